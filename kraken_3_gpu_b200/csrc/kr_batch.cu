@@ -23,6 +23,7 @@
 #include <string>
 #include <system_error>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "kr_batch_impl.h"
@@ -83,89 +84,65 @@ struct BatchArgs {
 // --- shared-memory layout, carved per template ------------------------------
 // Every region is a multiple of 4 words, so each region and each creature's
 // base stay 16-byte aligned (the f64 and float4 views included).
-constexpr int kLvlWords = (kr::kMaxTplLevels + 1 + 3) & ~3;                 // 68
-constexpr int kArmWords = (3 * KR_BATCH_MAX_ARMS + KR_BATCH_MAX_ARMS * KR_BATCH_MAX_SEGS + 3) & ~3;
+constexpr int kArmWords = (2 * KR_BATCH_MAX_ARMS + KR_BATCH_MAX_ARMS * KR_BATCH_MAX_SEGS + 3) & ~3;
 __host__ __device__ constexpr int r4(int n) { return (n + 3) & ~3; }
 
-// statics of the template, once per CTA
-__host__ __device__ inline int tpl_smem_words(int nb, int nc, int np) {
-  return 5 * r4(nb) + 11 * r4(nc) + 4 * r4(np) + kLvlWords + kArmWords;
+// statics of the template, once per CTA: unit records of the schedule for G
+// lanes, bodies, collision points, arm tables
+__host__ __device__ inline int tpl_smem_words(int npass, int G, int nb, int np) {
+  return npass * G * kr::kRecFloats + 4 * nb + 4 * np + kArmWords;
 }
-// one creature: the committed state (positions, angles, velocities: loaded
-// from the slot's HBM block when the creature starts, written back when its
-// run ends), predicted bodies and their sin/cos, grip and motor state,
-// lambda, collision scratch
-__host__ __device__ inline int creature_smem_words(int nb, int nc, int np, int arms, int segs) {
-  return 11 * r4(nb) + 2 * r4(nc) + r4(arms * segs) + r4(arms * segs + arms) + 4 * arms + 3 * r4(np) +
-         kr::kMaxCulled / 2;
+// one creature: the committed state and the predicted state (16-byte records;
+// the velocity lives in the predicted state's records between substeps), the
+// arms' anchors after the bodies, per motor {target, lambda}, per arm {lambda,
+// break force}, controls, collision scratch.  The proprioception's vector
+// shares the motors' words: it is read before the targets are written.
+__host__ __device__ inline int mot_words(int arms, int segs) {
+  const int m = 2 * arms * segs, o = 6 * arms + 6;
+  return r4(m > o ? m : o);
+}
+__host__ __device__ inline int creature_smem_words(int nb, int np, int arms, int segs) {
+  return 4 * nb + 4 * (nb + arms) + mot_words(arms, segs) + 4 * arms + r4(arms * segs + arms) + 2 * r4(nb) +
+         3 * r4(np) + kr::kMaxCulled / 2;
 }
 
 struct TplSmem {
-  float *im, *ii, *zero;
-  int *boff, *bcnt, *ab, *type, *motor, *garm;
-  float *lax, *lay, *lbx, *lby, *rest, *minA, *maxA;
-  int *lvl;
-  float *plx, *ply, *pr;
-  int *pbody;
-  int *arm_tip, *arm_grip, *arm_seg0, *arm_segs;
+  float4 *recs, *body, *pts;
+  int *arm_tip, *arm_seg0, *arm_segs;
 };
 
-__device__ inline void carve_tpl(TplSmem &P, float *p, const TplDev &td) {
-  const int mb = r4(td.nb), mc = r4(td.nc), mp = r4(td.np);
-  P.im = p; p += mb; P.ii = p; p += mb; P.zero = p; p += mb;
-  P.boff = reinterpret_cast<int *>(p); p += mb;
-  P.bcnt = reinterpret_cast<int *>(p); p += mb;
-  P.ab = reinterpret_cast<int *>(p); p += mc;
-  P.type = reinterpret_cast<int *>(p); p += mc;
-  P.motor = reinterpret_cast<int *>(p); p += mc;
-  P.garm = reinterpret_cast<int *>(p); p += mc;
-  P.lax = p; p += mc; P.lay = p; p += mc; P.lbx = p; p += mc; P.lby = p; p += mc;
-  P.rest = p; p += mc; P.minA = p; p += mc; P.maxA = p; p += mc;
-  P.lvl = reinterpret_cast<int *>(p); p += kLvlWords;
-  P.plx = p; p += mp; P.ply = p; p += mp; P.pr = p; p += mp;
-  P.pbody = reinterpret_cast<int *>(p); p += mp;
+__device__ inline void carve_tpl(TplSmem &P, float *p, const TplDev &td, int npass, int G) {
+  P.recs = reinterpret_cast<float4 *>(p); p += npass * G * kr::kRecFloats;
+  P.body = reinterpret_cast<float4 *>(p); p += 4 * td.nb;
+  P.pts = reinterpret_cast<float4 *>(p); p += 4 * td.np;
   P.arm_tip = reinterpret_cast<int *>(p); p += KR_BATCH_MAX_ARMS;
-  P.arm_grip = reinterpret_cast<int *>(p); p += KR_BATCH_MAX_ARMS;
   P.arm_seg0 = reinterpret_cast<int *>(p); p += KR_BATCH_MAX_ARMS;
   P.arm_segs = reinterpret_cast<int *>(p);
 }
 
 struct CreatureSmem {
   float *ctrl;     // arms * segs motor controls, then arms adhesion values
-  float *obs;      // proprioception (aliases the collision scratch pdy)
-  double *pair;    // atan2 terms of armCurl (aliases the collision scratch pdx)
+  float *obs;      // proprioception (aliases the motors' records)
 };
 
 __device__ inline void carve_creature(kr::Island &S, CreatureSmem &X, const TplSmem &P, float *p,
-                                      const TplDev &td) {
-  const int mb = r4(td.nb), mc = r4(td.nc), mp = r4(td.np), AS = td.arms * td.segs;
+                                      const TplDev &td, int npass) {
+  const int mb = r4(td.nb), mp = r4(td.np), AS = td.arms * td.segs;
   // committed state, resident for the creature's whole run
-  S.px = p; p += mb; S.py = p; p += mb; S.vx = p; p += mb; S.vy = p; p += mb;
-  S.ang = p; p += mb; S.av = p; p += mb;
-  S.ppx = p; p += mb; S.ppy = p; p += mb; S.angP = p; p += mb;
-  S.bs = p; p += mb; S.bc = p; p += mb;
-  S.lamX = p; p += mc; S.lamY = p; p += mc;
-  S.lam = S.lamX;  // pins use lamX/lamY, angles lam: never both on one slot
-  S.tgt_m = p; p += r4(AS);
+  S.P = reinterpret_cast<float4 *>(p); p += 4 * td.nb;
+  S.Q = reinterpret_cast<float4 *>(p); p += 4 * (td.nb + td.arms);
+  S.V = S.Q;
+  S.mot = reinterpret_cast<float2 *>(p);
+  X.obs = p; p += mot_words(td.arms, td.segs);
+  S.grip = reinterpret_cast<float4 *>(p); p += 4 * td.arms;
   X.ctrl = p; p += r4(AS + td.arms);
-  S.anc = p; p += 4 * td.arms;
+  S.bs = p; p += mb; S.bc = p; p += mb;
   S.pdx = p; p += mp; S.pdy = p; p += mp;
   S.pflag = reinterpret_cast<int *>(p); p += mp;
   S.cull = reinterpret_cast<short *>(p);
-  // proprioception scratch: live only before the XPBD step of an env step,
-  // when the collision scratch is dead (2 * arms * (segs - 1) <= np and
-  // 6 * arms + 6 <= np for every template shape)
-  X.pair = reinterpret_cast<double *>(S.pdx);
-  X.obs = S.pdy;
   // statics shared by the CTA
-  S.im = P.im; S.ii = P.ii; S.fx = P.zero; S.fy = P.zero; S.tq = P.zero;
-  S.ab = P.ab; S.type = P.type; S.garm = P.garm; S.motor = P.motor;
-  S.lax = P.lax; S.lay = P.lay; S.lbx = P.lbx; S.lby = P.lby;
-  S.rest = P.rest; S.minA = P.minA; S.maxA = P.maxA;
-  S.plx = P.plx; S.ply = P.ply; S.pr = P.pr; S.pbody = P.pbody; S.boff = P.boff; S.bcnt = P.bcnt;
-  S.lvl = P.lvl;
-  S.tb = nullptr; S.comp = nullptr; S.tgt = nullptr; S.brk = nullptr;
-  S.nb = td.nb; S.nc = td.nc; S.np = td.np;
+  S.recs = P.recs; S.body = P.body; S.pts = P.pts;
+  S.nb = td.nb; S.np = td.np; S.npass = npass; S.arms = td.arms;
 }
 
 // mulberry32 (src/world/map.js:11-20): the draw is a hash of the state, and
@@ -233,32 +210,30 @@ template <int G>
 __device__ unsigned proprio(const BatchArgs &A, const TplDev &td, const TplSmem &P, kr::Island &S,
                             CreatureSmem &X, SlotMeta &m, const double2 *cdp, const kr::Lanes<G> &L) {
   const int arms = td.arms, segs = td.segs, lane = L.lane;
-  const float4 *grip_st = reinterpret_cast<const float4 *>(S.anc);
-  const double cx = S.px[0], cy = S.py[0], cvx = S.vx[0], cvy = S.vy[0];
-  const double angle = S.ang[0], cav = S.av[0];
-  // armCurl terms: atan2(sin d, cos d) per adjacent segment pair, as wrap_pi
-  const int npair = arms * (segs - 1);
-  for (int q = lane; q < npair; q += G) {
-    const int a = q / (segs - 1), i = q % (segs - 1) + 1;
-    const double d = (double)S.ang[P.arm_segs[a * segs + i]] - (double)S.ang[P.arm_segs[a * segs + i - 1]];
-    X.pair[q] = wrap_pi(d);
-  }
-  L.sync();
+  const float4 p0 = S.P[0], v0 = S.V[0];
+  const double cx = p0.x, cy = p0.y, cvx = v0.x, cvy = v0.y;
+  const double angle = p0.z, cav = v0.z;
   double ext = 0.0, curl = 0.0, sh = 0.0, tx = 0.0, ty = 0.0;
   bool attached = false;
   if (lane < arms) {
     const int a = lane;
-    double s = 0.0;
-    for (int i = 0; i < segs - 1; i++) s += X.pair[a * (segs - 1) + i];
+    // armCurl: atan2(sin d, cos d) per adjacent segment pair, as wrap_pi
+    const int *sg = P.arm_segs + a * segs;
+    double s = 0.0, prev = S.P[sg[0]].z;
+    for (int i = 1; i < segs; i++) {
+      const double cur = S.P[sg[i]].z;
+      s += wrap_pi(cur - prev);
+      prev = cur;
+    }
     curl = segs > 1 ? s / (segs - 1) : 0.0;
-    const int s0 = P.arm_seg0[a], tip = P.arm_tip[a];
-    const double d = (double)S.ang[s0] - angle;
+    const float4 ps = S.P[P.arm_seg0[a]], pt = S.P[P.arm_tip[a]];
+    const double d = (double)ps.z - angle;
     sh = wrap_pi(d);
-    const double2 t = lib_sincos((double)S.ang[tip]);
-    tx = (double)S.px[tip] + kSegHalf * t.y;
-    ty = (double)S.py[tip] + kSegHalf * t.x;
-    ext = fmin(1.0, lib_hypot(tx - (double)S.px[s0], ty - (double)S.py[s0]) / fmax(1.0, td.reach));
-    attached = grip_st[a].w == 0.f;
+    const double2 t = lib_sincos((double)pt.z);
+    tx = (double)pt.x + kSegHalf * t.y;
+    ty = (double)pt.y + kSegHalf * t.x;
+    ext = fmin(1.0, lib_hypot(tx - (double)ps.x, ty - (double)ps.y) / fmax(1.0, td.reach));
+    attached = S.Q[S.nb + a].w == 0.f;
   }
   const unsigned att = L.ballot(attached) & ((1u << arms) - 1u);
   // sums in arm order, like the sequential loop
@@ -274,11 +249,11 @@ __device__ unsigned proprio(const BatchArgs &A, const TplDev &td, const TplSmem 
     const double dx = tx - cx, dy = ty - cy;
     X.obs[2 * arms + 2 * a] = (float)clamp_sym((dx * ca - dy * sa) / td.reach, 1.2);
     X.obs[2 * arms + 2 * a + 1] = (float)clamp_sym((dx * sa + dy * ca) / td.reach, 1.2);
-    const float4 g = grip_st[a];
+    const float4 g = S.grip[a];
     double force = 0.0;
-    if (g.w == 0.f) force = lib_hypot((double)S.lamX[P.arm_grip[a]], (double)S.lamY[P.arm_grip[a]]) * A.inv_h64;
-    X.obs[4 * arms + a] = g.w != 0.f ? 0.f : (float)fmin(1.0, force / fmax(1.0, cdp[a].y));
-    X.obs[5 * arms + a] = g.w != 0.f ? 0.f : 1.f;
+    if (attached) force = lib_hypot((double)g.x, (double)g.y) * A.inv_h64;
+    X.obs[4 * arms + a] = !attached ? 0.f : (float)fmin(1.0, force / fmax(1.0, cdp[a].y));
+    X.obs[5 * arms + a] = !attached ? 0.f : 1.f;
   }
   if (lane == 0) {
     const double ax = (cvx - m.prev_vx) / A.dt, ay = (cvy - m.prev_vy) / A.dt;
@@ -525,14 +500,14 @@ __device__ __noinline__ double2 net_sdf(const double *rects, int n, double px, d
 // step this is the end of (the slot's step counter, from 0 at its spawn):
 // below light_T the lights' positions come from the engine's table.
 template <int G>
-__device__ __noinline__ void net_senses(NetArgs N, int arms, const int *arm_tip, const float *px, const float *py,
-                                        const float *ang, int map, int slot, int t, kr::Lanes<G> L) {
+__device__ __noinline__ void net_senses(NetArgs N, int arms, const int *arm_tip, const float4 *pos, int map, int slot,
+                                        int t, kr::Lanes<G> L) {
   NetRec &R = N.net[slot];
   const int lane = L.lane;
   const int ro = N.map_off[map], nR = N.map_off[map + 1] - ro;
   const double *rects = N.rects64 + 4 * (size_t)ro;
-  const double x = px[0], y = py[0];
-  const double heading = (double)ang[0] - kPiD * 0.5;
+  const double x = pos[0].x, y = pos[0].y;
+  const double heading = (double)pos[0].z - kPiD * 0.5;
   const double dt = N.dt;
   const double time = R.time + dt;
   const int lo = N.light_off ? N.light_off[map] : 0, nl = N.light_off ? N.light_off[map + 1] - lo : 0;
@@ -621,9 +596,9 @@ __device__ __noinline__ void net_senses(NetArgs N, int arms, const int *arm_tip,
   }
   // tip contact: near = max(0, 1 - d / 9) of the map's SDF at the tip point
   for (int a = lane; a < arms; a += G) {
-    const int tip = arm_tip[a];
-    const double2 t = lib_sincos((double)ang[tip]);
-    const double tx = (double)px[tip] + kSegHalf * t.y, ty = (double)py[tip] + kSegHalf * t.x;
+    const float4 tip = pos[arm_tip[a]];
+    const double2 t = lib_sincos((double)tip.z);
+    const double tx = (double)tip.x + kSegHalf * t.y, ty = (double)tip.y + kSegHalf * t.x;
     // near is 0 unless a rect lies within 9 px: a rect whose box is 10 px
     // away or more cannot make it positive, so the SDF runs only when some
     // box is closer (the result is the same either way)
@@ -645,13 +620,12 @@ __device__ __noinline__ void net_senses(NetArgs N, int arms, const int *arm_tip,
 // NET: the kernel instance of engines in KR_CTRL_NET mode (the other modes'
 // kernels carry none of the net's code).
 template <int G, bool NET, int U>
-__device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, const TplSmem &P, float *base,
+__device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, const TplSmem &P, float *base,
                              int slot, const kr::Lanes<G> &L) {
   const int lane = L.lane;
   kr::Island S;
   CreatureSmem X;
-  carve_creature(S, X, P, base, td);
-  S.nlv = nlv;
+  carve_creature(S, X, P, base, td, npass);
   SlotMeta m = A.meta[slot];
   const int steps = min(A.max_steps, m.horizon - m.step);
   if (steps <= 0) return;
@@ -662,18 +636,16 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, cons
   // the committed state into shared memory (the slot's block is SoA, kBodyPad per field)
   float *hbm = A.state + (size_t)slot * kStateStride;
   for (int i = lane; i < td.nb; i += G) {
-    S.px[i] = hbm[i]; S.py[i] = hbm[kBodyPad + i]; S.vx[i] = hbm[2 * kBodyPad + i];
-    S.vy[i] = hbm[3 * kBodyPad + i]; S.ang[i] = hbm[4 * kBodyPad + i]; S.av[i] = hbm[5 * kBodyPad + i];
+    S.P[i] = make_float4(hbm[i], hbm[kBodyPad + i], hbm[4 * kBodyPad + i], 0.f);
+    S.V[i] = make_float4(hbm[2 * kBodyPad + i], hbm[3 * kBodyPad + i], hbm[5 * kBodyPad + i], 0.f);
   }
-  for (int k = lane; k < td.nc; k += G) { S.lamX[k] = 0.f; S.lamY[k] = 0.f; }
   S.comp_m = m.comp;
   double cd = 0.0;  // reflex cooldown of arm `lane` (its f64 break force stays in cdp)
-  L.sync();
   if (lane < arms) {
-    reinterpret_cast<float4 *>(S.anc)[lane] = gst[lane];
+    const float4 g = gst[lane];
     const float2 gl = glam[lane];
-    const int k = P.arm_grip[lane];
-    S.lamX[k] = gl.x; S.lamY[k] = gl.y;
+    S.Q[td.nb + lane] = make_float4(g.x, g.y, 0.f, g.w);  // the anchor's record: x, y, angle 0, broken
+    S.grip[lane] = make_float4(gl.x, gl.y, g.z, 0.f);
     cd = cdp[lane].x;
   }
   const float *cin = A.ctrl_cur + (size_t)slot * kCtrlStride;
@@ -721,26 +693,26 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, cons
     // 3. applyControl: targets (clamped) and the reflex, core.js:183-220
     for (int mo = lane; mo < AS; mo += G) {
       const double lim = (mo % td.segs) == 0 ? kPiD * 0.62 : kPiD * 0.42;
-      S.tgt_m[mo] = (float)fmax(-lim, fmin(lim, (double)X.ctrl[mo]));
+      S.mot[mo].x = (float)fmax(-lim, fmin(lim, (double)X.ctrl[mo]));
     }
     if (lane < arms) {
-      const int a = lane, k = P.arm_grip[a], tip = P.arm_tip[a];
-      float *an = S.anc + 4 * a;
+      const int a = lane, tip = P.arm_tip[a];
+      float4 &an = S.Q[td.nb + a], &gr = S.grip[a];
       const double adh = fmax(0.0, fmin(1.0, (double)X.ctrl[AS + a]));
       double c = cd;
       if (c > 0) c -= A.dt;
-      if (an[3] != 0.f) {
+      if (an.w != 0.f) {
         if (adh > 0.08 && c <= 0) {
-          const double slip = lib_hypot((double)S.vx[tip], (double)S.vy[tip]);
+          const float4 tv = S.V[tip];
+          const double slip = lib_hypot((double)tv.x, (double)tv.y);
           if (slip < A.slip_max) {
-            const double ta = (double)S.ang[tip];
-            an[0] = (float)((double)S.px[tip] + kSegHalf * lib_cos(ta));
-            an[1] = (float)((double)S.py[tip] + kSegHalf * lib_sin(ta));
+            const float4 tp = S.P[tip];
+            const double ta = (double)tp.z;
             const double brk = 40.0 + 860.0 * adh;
             cdp[a].y = brk;
-            an[2] = (float)brk;
-            an[3] = 0.f;
-            S.lamX[k] = 0.f; S.lamY[k] = 0.f;
+            an = make_float4((float)((double)tp.x + kSegHalf * lib_cos(ta)),
+                             (float)((double)tp.y + kSegHalf * lib_sin(ta)), 0.f, 0.f);
+            gr = make_float4(0.f, 0.f, (float)brk, 0.f);
           } else {
             c = A.cooldown;
           }
@@ -748,14 +720,14 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, cons
       } else {
         const double brk = 40.0 + 860.0 * adh;
         cdp[a].y = brk;
-        an[2] = (float)brk;
-        if (adh < 0.04) an[3] = 1.f;
+        gr.z = (float)brk;
+        if (adh < 0.04) an.w = 1.f;
       }
       cd = c;
     }
     L.sync();
     // 4. the XPBD step
-    kr::island_step<kr::CompactAccess, G, U>(A.K, S, rects, nR, cull_d, L, td.off_max + 1.f);
+    kr::island_step<false, G, U>(A.K, S, rects, nR, cull_d, L, td.off_max + 1.f);
     // 5. postStep, core.js:297-356 (f64 on the f32 state, as the
     //    reference's hybrid loop runs it on the mirrored state)
     //    The accumulators are read and written through the slot's HBM
@@ -764,14 +736,14 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, cons
     //    call on two lanes, beside lane 0's sincos of the heading.
     {
       const SlotMeta &gr = A.meta[slot];
-      const double x = S.px[0], y = S.py[0];
+      const double x = S.P[0].x, y = S.P[0].y;
       const double hx = lane == 1 ? x - gr.spawn_x : x - gr.last_x;
       const double hy = lane == 1 ? y - gr.spawn_y : y - gr.last_y;
       const double hv = lib_hypot(hx, hy);
       const double d_spawn_l = __shfl_sync(L.mask, hv, L.base + 1);
       if (lane == 0) {
         SlotMeta &g = A.meta[slot];
-        const double angle = S.ang[0], av = S.av[0];
+        const double angle = S.P[0].z, av = S.V[0].z;
         const double dx = hx, dy = hy;
         const double step_dist = hv;
         g.path_len += step_dist;
@@ -784,7 +756,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, cons
         int anchored = 0;
         unsigned now = 0;
         for (int a = 0; a < arms; a++)
-          if (S.anc[4 * a + 3] == 0.f) { anchored++; now |= 1u << a; }
+          if (S.Q[td.nb + a].w == 0.f) { anchored++; now |= 1u << a; }
         const double d_spawn = d_spawn_l;
         if (anchored > 0) {
           g.anchored_steps++;
@@ -803,20 +775,21 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int nlv, cons
       }
     }
     if constexpr (NET) {
-      if (m.ctrl == KR_CTRL_NET) net_senses<G>(net_args(A), arms, P.arm_tip, S.px, S.py, S.ang, m.map, slot, t, L);
+      if (m.ctrl == KR_CTRL_NET) net_senses<G>(net_args(A), arms, P.arm_tip, S.P, m.map, slot, t, L);
     }
     m.step = t + 1;
   }
   // write back: the committed state, grips, cooldowns, controls, the meta fields kept in registers
   L.sync();
   for (int i = lane; i < td.nb; i += G) {
-    hbm[i] = S.px[i]; hbm[kBodyPad + i] = S.py[i]; hbm[2 * kBodyPad + i] = S.vx[i];
-    hbm[3 * kBodyPad + i] = S.vy[i]; hbm[4 * kBodyPad + i] = S.ang[i]; hbm[5 * kBodyPad + i] = S.av[i];
+    const float4 p = S.P[i], v = S.V[i];
+    hbm[i] = p.x; hbm[kBodyPad + i] = p.y; hbm[2 * kBodyPad + i] = v.x;
+    hbm[3 * kBodyPad + i] = v.y; hbm[4 * kBodyPad + i] = p.z; hbm[5 * kBodyPad + i] = v.z;
   }
   if (lane < arms) {
-    const int k = P.arm_grip[lane];
-    gst[lane] = reinterpret_cast<const float4 *>(S.anc)[lane];
-    glam[lane] = make_float2(S.lamX[k], S.lamY[k]);
+    const float4 an = S.Q[td.nb + lane], g = S.grip[lane];
+    gst[lane] = make_float4(an.x, an.y, g.z, an.w);
+    glam[lane] = make_float2(g.x, g.y);
     cdp[lane].x = cd;
   }
   float *cout = A.ctrl_cur + (size_t)slot * kCtrlStride;
@@ -854,35 +827,25 @@ __global__ void __launch_bounds__(32 * kMaxW, 1) batch_kernel(BatchArgs A) {
     if (g >= A.n_groups) return;
     const int first = A.groups[g * A.cpc];
     const TplDev td = A.tpl[A.meta[first].tpl];
+    const int npass = td.npass[V];
     TplSmem P;
-    carve_tpl(P, smem, td);
+    carve_tpl(P, smem, td, npass, G);
     // stage the template statics (whole CTA)
-    for (int i = threadIdx.x; i < td.nb; i += blockDim.x) {
-      P.im[i] = A.T.im[td.o_b + i]; P.ii[i] = A.T.ii[td.o_b + i]; P.zero[i] = 0.f;
-      P.boff[i] = A.T.boff[td.o_b + i]; P.bcnt[i] = A.T.bcnt[td.o_b + i];
-    }
-    for (int k = threadIdx.x; k < td.nc; k += blockDim.x) {
-      const int o = td.o_c[V] + k;
-      P.ab[k] = A.T.ab[o]; P.type[k] = A.T.type[o]; P.motor[k] = A.T.motor[o]; P.garm[k] = A.T.garm[o];
-      P.lax[k] = A.T.lax[o]; P.lay[k] = A.T.lay[o]; P.lbx[k] = A.T.lbx[o]; P.lby[k] = A.T.lby[o];
-      P.rest[k] = A.T.rest[o]; P.minA[k] = A.T.minA[o]; P.maxA[k] = A.T.maxA[o];
-    }
-    for (int l = threadIdx.x; l <= td.nlv[V]; l += blockDim.x) P.lvl[l] = A.T.lvl[td.o_l[V] + l];
-    for (int p = threadIdx.x; p < td.np; p += blockDim.x) {
-      P.plx[p] = A.T.plx[td.o_p + p]; P.ply[p] = A.T.ply[td.o_p + p]; P.pr[p] = A.T.pr[td.o_p + p];
-      P.pbody[p] = A.T.pbody[td.o_p + p];
-    }
+    for (int i = threadIdx.x; i < npass * G * (kr::kRecFloats / 4); i += blockDim.x)
+      P.recs[i] = A.T.recs[td.o_r[V] + i];
+    for (int i = threadIdx.x; i < td.nb; i += blockDim.x) P.body[i] = A.T.body[td.o_b + i];
+    for (int p = threadIdx.x; p < td.np; p += blockDim.x) P.pts[p] = A.T.pts[td.o_p + p];
     for (int a = threadIdx.x; a < td.arms; a += blockDim.x) {
-      P.arm_tip[a] = A.T.arm_tip[td.o_a + a]; P.arm_grip[a] = A.T.arm_grip[td.o_g[V] + a];
+      P.arm_tip[a] = A.T.arm_tip[td.o_a + a];
       P.arm_seg0[a] = A.T.arm_seg0[td.o_a + a];
     }
     for (int q = threadIdx.x; q < td.arms * td.segs; q += blockDim.x) P.arm_segs[q] = A.T.arm_segs[td.o_s + q];
     __syncthreads();
     const int slot = c < A.cpc ? A.groups[g * A.cpc + c] : -1;
     if (slot >= 0) {
-      float *base = smem + tpl_smem_words(td.nb, td.nc, td.np) +
-                    c * creature_smem_words(td.nb, td.nc, td.np, td.arms, td.segs);
-      run_creature<G, NET, U>(A, td, td.nlv[V], P, base, slot, L);
+      float *base = smem + tpl_smem_words(npass, G, td.nb, td.np) +
+                    c * creature_smem_words(td.nb, td.np, td.arms, td.segs);
+      run_creature<G, NET, U>(A, td, npass, P, base, slot, L);
     }
   }
 }
@@ -1037,34 +1000,30 @@ int ensure_template(kr_batch *b, int arms, int segs) {
 }
 
 int upload_templates(kr_batch *b) {
-  std::vector<float> im, ii, lax, lay, lbx, lby, rest, minA, maxA, plx, ply, pr;
-  std::vector<int> boff, bcnt, ab, type, motor, garm, lvl, pbody, tip, grip, seg0, segs;
+  std::vector<float4> body, pts, recs;
+  std::vector<int> tip, seg0, segs;
+  auto word = [](int v) {
+    float f;
+    std::memcpy(&f, &v, sizeof(f));
+    return f;
+  };
   b->h_tpl.clear();
   for (const auto &t : b->tpls) {
     TplDev d{};
     d.nb = t.nb; d.nc = t.nc; d.np = t.np; d.arms = t.arms; d.segs = t.segs;
     d.r_max = t.r_max; d.off_max = t.off_max; d.reach = t.reach;
-    d.o_b = (int)im.size(); d.o_p = (int)plx.size(); d.o_a = (int)tip.size(); d.o_s = (int)segs.size();
-    im.insert(im.end(), t.im.begin(), t.im.end()); ii.insert(ii.end(), t.ii.begin(), t.ii.end());
-    boff.insert(boff.end(), t.boff.begin(), t.boff.end()); bcnt.insert(bcnt.end(), t.bcnt.begin(), t.bcnt.end());
+    d.o_b = (int)body.size(); d.o_p = (int)pts.size(); d.o_a = (int)tip.size(); d.o_s = (int)segs.size();
+    for (int i = 0; i < t.nb; i++)
+      body.push_back(make_float4(t.im[i], t.ii[i], t.breach[i], word(t.boff[i] | (t.bcnt[i] << 16))));
+    for (int p = 0; p < t.np; p++) pts.push_back(make_float4(t.plx[p], t.ply[p], t.pr[p], word(t.pbody[p])));
     for (int v = 0; v < kr::kSchedules; v++) {
       const kr::Schedule &S = t.sched[v];
-      d.nlv[v] = S.nlv;
-      d.o_c[v] = (int)ab.size(); d.o_l[v] = (int)lvl.size(); d.o_g[v] = (int)grip.size();
-      ab.insert(ab.end(), S.ab.begin(), S.ab.end()); type.insert(type.end(), S.type.begin(), S.type.end());
-      motor.insert(motor.end(), S.motor.begin(), S.motor.end());
-      std::vector<int> ga(t.nc, -1);
-      for (int a = 0; a < t.arms; a++) ga[S.arm_grip[a]] = a;
-      garm.insert(garm.end(), ga.begin(), ga.end());
-      lax.insert(lax.end(), S.lax.begin(), S.lax.end()); lay.insert(lay.end(), S.lay.begin(), S.lay.end());
-      lbx.insert(lbx.end(), S.lbx.begin(), S.lbx.end()); lby.insert(lby.end(), S.lby.begin(), S.lby.end());
-      rest.insert(rest.end(), S.rest.begin(), S.rest.end());
-      minA.insert(minA.end(), S.minA.begin(), S.minA.end()); maxA.insert(maxA.end(), S.maxA.begin(), S.maxA.end());
-      lvl.insert(lvl.end(), S.lvl.begin(), S.lvl.end());
-      grip.insert(grip.end(), S.arm_grip.begin(), S.arm_grip.end());
+      d.npass[v] = S.npass;
+      d.o_r[v] = (int)recs.size();
+      const size_t n4 = S.recs.size() / 4;
+      recs.resize(recs.size() + n4);
+      std::memcpy(recs.data() + d.o_r[v], S.recs.data(), n4 * sizeof(float4));
     }
-    plx.insert(plx.end(), t.plx.begin(), t.plx.end()); ply.insert(ply.end(), t.ply.begin(), t.ply.end());
-    pr.insert(pr.end(), t.pr.begin(), t.pr.end()); pbody.insert(pbody.end(), t.pbody.begin(), t.pbody.end());
     tip.insert(tip.end(), t.arm_tip.begin(), t.arm_tip.end());
     seg0.insert(seg0.end(), t.arm_seg0.begin(), t.arm_seg0.end());
     segs.insert(segs.end(), t.arm_segs.begin(), t.arm_segs.end());
@@ -1073,27 +1032,13 @@ int upload_templates(kr_batch *b) {
   // the device may still read the old tables in a queued launch
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return b->cuda_fail(e, "upload(templates) sync");
-  void **A = b->d_tpl_arrays;
-#define UP(i, vec) if (e == cudaSuccess) e = upload_vec(reinterpret_cast<decltype(vec.data()) *>(&A[i]), vec)
-  UP(0, im); UP(1, ii); UP(2, boff); UP(3, bcnt); UP(4, ab); UP(5, type); UP(6, motor); UP(7, lax);
-  UP(8, lay); UP(9, lbx); UP(10, lby); UP(11, rest); UP(12, minA); UP(13, maxA); UP(14, lvl);
-  UP(15, plx); UP(16, ply); UP(17, pr); UP(18, pbody); UP(19, tip); UP(20, grip); UP(21, seg0);
-  UP(22, garm);
-#undef UP
-  if (e != cudaSuccess) return b->cuda_fail(e, "upload(templates)");
-  int *d_segs = nullptr;
-  e = upload_vec(&d_segs, segs);
-  if (e != cudaSuccess) return b->cuda_fail(e, "upload(template segments)");
   TplArrays &T = b->T;
-  T.im = (const float *)A[0]; T.ii = (const float *)A[1]; T.boff = (const int *)A[2]; T.bcnt = (const int *)A[3];
-  T.ab = (const int *)A[4]; T.type = (const int *)A[5]; T.motor = (const int *)A[6];
-  T.lax = (const float *)A[7]; T.lay = (const float *)A[8]; T.lbx = (const float *)A[9]; T.lby = (const float *)A[10];
-  T.rest = (const float *)A[11]; T.minA = (const float *)A[12]; T.maxA = (const float *)A[13];
-  T.lvl = (const int *)A[14]; T.plx = (const float *)A[15]; T.ply = (const float *)A[16]; T.pr = (const float *)A[17];
-  T.pbody = (const int *)A[18]; T.arm_tip = (const int *)A[19]; T.arm_grip = (const int *)A[20];
-  T.arm_seg0 = (const int *)A[21]; T.garm = (const int *)A[22];
-  if (T.arm_segs) cudaFree(const_cast<int *>(T.arm_segs));
-  T.arm_segs = d_segs;
+  auto up = [&](auto *&dst, const auto &vec) {
+    if (e == cudaSuccess) e = upload_vec(const_cast<std::remove_const_t<std::remove_reference_t<decltype(*dst)>> **>(&dst), vec);
+  };
+  up(T.body, body); up(T.pts, pts); up(T.recs, recs);
+  up(T.arm_tip, tip); up(T.arm_seg0, seg0); up(T.arm_segs, segs);
+  if (e != cudaSuccess) return b->cuda_fail(e, "upload(templates)");
   if ((e = upload_vec(&b->d_tpl, b->h_tpl)) != cudaSuccess) return b->cuda_fail(e, "upload(template table)");
   b->shape_dirty = true;
   return KR_OK;
@@ -1113,8 +1058,8 @@ int plan_shape(kr_batch *b) {
   size_t need_max = 16;
   for (size_t t = 0; t < b->h_tpl.size(); t++) {
     const TplDev &d = b->h_tpl[t];
-    const long tw = tpl_smem_words(d.nb, d.nc, d.np);
-    const long cw = creature_smem_words(d.nb, d.nc, d.np, d.arms, d.segs);
+    const long tw = tpl_smem_words(d.npass[kr::schedule_index(b->G)], b->G, d.nb, d.np);
+    const long cw = creature_smem_words(d.nb, d.np, d.arms, d.segs);
     const long fit = (words - tw) / cw;
     if (fit < 1)
       return b->fail(KR_ERR_CAPACITY, "body " + std::to_string(d.arms) + "x" + std::to_string(d.segs) +
@@ -2266,10 +2211,9 @@ extern "C" int kr_batch_set_stream(kr_batch *b, void *stream) {
 extern "C" void kr_batch_destroy(kr_batch *b) {
   if (!b) return;
   cudaDeviceSynchronize();
-  for (void *p : b->d_tpl_arrays)
-    if (p) cudaFree(p);
-  free_part(b->main);
-  void *ptrs[] = {b->d_tpl, const_cast<int *>(b->T.arm_segs), b->d_rects, b->d_map_off, b->d_map_cull, b->d_rects64,
+  void *ptrs[] = {b->d_tpl, const_cast<float4 *>(b->T.body), const_cast<float4 *>(b->T.pts),
+                  const_cast<float4 *>(b->T.recs), const_cast<int *>(b->T.arm_tip), const_cast<int *>(b->T.arm_seg0),
+                  const_cast<int *>(b->T.arm_segs), b->d_rects, b->d_map_off, b->d_map_cull, b->d_rects64,
                   b->d_state, b->d_grip, b->d_glam, b->d_cd, b->d_ctrl, b->d_meta, b->d_obs,
                   b->d_pw, b->d_pw_idx, b->s_state, b->s_grip, b->s_glam, b->s_cd,
                   b->s_ctrl, b->s_meta, b->s_groups, b->d_net, b->s_net, b->d_lights, b->d_light_off,

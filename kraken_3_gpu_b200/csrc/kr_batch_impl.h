@@ -23,27 +23,23 @@ constexpr int kStateStride = 6 * kBodyPad;                     // px py vx vy an
 constexpr int kCtrlStride = KR_BATCH_MAX_ARMS * (KR_BATCH_MAX_SEGS + 1);  // 80
 
 // Template record on the device: sizes and offsets into the flat arrays.
-// Constraint slots, level offsets and arm grip slots exist once per solve
-// schedule (kr::schedule_index of the lanes per creature).
+// Unit records exist once per solve schedule (kr::schedule_index of the
+// lanes per creature).
 struct TplDev {
   int nb, nc, np, arms, segs;
-  int nlv[kr::kSchedules];
+  int npass[kr::kSchedules];
   float r_max;
   float off_max;   // largest distance of a collision point from its body's centre
   double reach;
-  int o_b, o_p, o_a, o_s;
-  int o_c[kr::kSchedules], o_l[kr::kSchedules], o_g[kr::kSchedules];
+  int o_b, o_p, o_a, o_s;     // bodies, collision points, arms, arm segments
+  int o_r[kr::kSchedules];    // unit records, in float4
 };
 
 struct TplArrays {
-  const float *im, *ii;
-  const int *boff, *bcnt;
-  const int *ab, *type, *motor, *garm;
-  const float *lax, *lay, *lbx, *lby, *rest, *minA, *maxA;
-  const int *lvl;
-  const float *plx, *ply, *pr;
-  const int *pbody;
-  const int *arm_tip, *arm_grip, *arm_seg0, *arm_segs;  // arm_grip: per schedule
+  const float4 *body;   // 1 / mass, 1 / inertia, reach, point offset | count << 16
+  const float4 *pts;    // x, y, radius, body
+  const float4 *recs;   // unit records (kr_template.h Schedule)
+  const int *arm_tip, *arm_seg0, *arm_segs;
 };
 
 // Per-slot record (device resident; the host keeps a mirror of the static
@@ -271,7 +267,6 @@ struct kr_batch {
   std::map<std::pair<int, int>, int> tpl_index;
   std::vector<krb::TplDev> h_tpl;
   krb::TplDev *d_tpl = nullptr;
-  void *d_tpl_arrays[23] = {nullptr};
   krb::TplArrays T{};
   // maps
   float4 *d_rects = nullptr;

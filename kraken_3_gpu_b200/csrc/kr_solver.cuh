@@ -1,10 +1,10 @@
 // kr_solver.cuh -- device side of the XPBD creature step (sm_100a).
 //
 // One connected component of the world (one creature, an "island") is
-// advanced by one warp.  Its bodies and constraints are staged in shared
-// memory for the whole launch; lanes split each constraint level and the
-// per-body collision work.  Nothing in here touches global memory except the
-// read-only rect list of the map.
+// advanced by a group of lanes of one warp.  Its bodies and constraints are
+// staged in shared memory for the whole launch; lanes split each pass of
+// solve units and the per-body collision work.  Nothing in here touches
+// global memory except the read-only rect list of the map.
 //
 // Arithmetic follows tools/f32solver.mjs operation by operation: every
 // intermediate is rounded to f32 with a non-contracting intrinsic
@@ -292,86 +292,78 @@ struct Lanes {
   }
 };
 
-// Shared-memory view of one island (one creature).  Constraint slots are in
-// schedule order: level by level, each level body-disjoint.  Two layouts:
-//  * per slot (gpuworld drop-in): every field an array over the slots;
-//  * compact (batched engine): the template's statics, plus per creature
-//    only lambda, the motor targets and the grip state (grips are the only
-//    constraints with a moving anchor, a break force and a broken flag;
-//    motors the only ones with a target and a nonzero compliance).
+// Shared-memory view of one island (one creature).
+//
+// The solve list is swept in units: a pin or grip constraint, an angle
+// constraint, or a pin and the angle constraint of the same two bodies when
+// no other constraint on either body lies between them in the list (every
+// joint of a creature).  A unit's two bodies are loaded once, solved in
+// registers -- pin, then angle, as the list orders them -- and stored once.
+// Units are grouped in passes of body-disjoint units, one unit per lane; a
+// pass order that keeps every pair of units sharing a body in list order
+// gives the sequential sweep's bits (the harness check color-order-free,
+// harness.js:1172-1193, pins this for the reference's colour classes).
+// The sweep is bound by its chain of dependent passes, each a round trip
+// through shared memory: per-constraint levels made a 6 x 7 body 12 of them,
+// as units it is 6 (12 creatures: 90 -> 64 us an env step; 16,384 mixed
+// creatures to their horizons: 391 -> 308 ms).
+//
+// Bodies are float4 records (one 16-byte load or store instead of three
+// 4-byte ones).
 struct Island {
-  // bodies (local index)
-  float *px, *py, *ppx, *ppy, *vx, *vy, *ang, *angP, *av, *im, *ii, *fx, *fy, *tq;
-  float *bs, *bc;  // sin / cos of angP during a collision pass
-  // constraint slots
-  const int *ab;   // a | (b << 16), b == 0xffff for a world anchor
-  int *tb;         // per slot: type | (broken << 8)
-  const float *lax, *lay, *rest, *minA, *maxA;
-  float *lbx, *lby;         // per slot (drop-in); template statics (batched)
-  float *comp, *tgt, *brk;  // per slot (drop-in)
-  float *lamX, *lamY, *lam;
-  // compact layout (batched engine)
-  const int *type;   // per slot static type
-  const int *garm;   // per slot: arm of a grip, else -1
-  const int *motor;  // per slot: motor index of an angle constraint, else -1
-  float *tgt_m;      // per motor target
-  float *anc;        // per arm: anchor x, y, break force, broken (1.f / 0.f)
-  float comp_m;      // motor compliance of the creature
-  // collision points, grouped per local body in groupCollPoints order
-  const float *plx, *ply, *pr;
-  const int *pbody;       // local body of each point
-  float *pdx, *pdy;       // speculative correction of each point
-  int *pflag;             // 1 if the speculative evaluation corrects
-  const int *boff, *bcnt;
-  short *cull;            // culled rect list (kMaxCulled)
-  int nb, nc, np, nlv;
-  const int *lvl;         // level offsets, nlv + 1
+  float4 *P;           // committed x, y, angle
+  float4 *Q;           // predicted x, y, angle
+  float4 *V;           // velocity vx, vy, av (batched engine: the same records as Q, see below)
+  const float4 *body;  // inverse mass, inverse inertia, reach, point offset | count << 16
+  const float4 *pts;   // collision points: x, y, radius, body; grouped per body in groupCollPoints order
+  float *bs, *bc;      // sin / cos of the predicted angle during a collision pass
+  float *pdx, *pdy;    // speculative correction of each point
+  int *pflag;          // 1 if the speculative evaluation corrects
+  short *cull;         // culled rect list (kMaxCulled)
+  int nb, np;
+  // drop-in world: one dynamic record of 4 float4 per unit, pass offsets
+  float4 *units;
+  int nu, npass;
+  const int *off;      // npass + 1 unit offsets
+  float4 *force;       // fx, fy, torque
+  // batched engine: the template's static records (3 float4 per lane and
+  // pass), per motor {target, lambda}, per arm {lambda x, y, break force}
+  const float4 *recs;
+  float2 *mot;
+  float4 *grip;
+  float comp_m;        // motor compliance of the creature
+  int arms;
 };
 
-// Field access of the two layouts (same values, different storage).
-struct SlotAccess {
-  __device__ static __forceinline__ int type(const Island &S, int k) { return S.tb[k] & 0xff; }
-  __device__ static __forceinline__ bool broken(const Island &S, int k) { return (S.tb[k] >> 8) != 0; }
-  __device__ static __forceinline__ void set_broken(Island &S, int k) { S.tb[k] |= 1 << 8; }
-  __device__ static __forceinline__ float lbx(const Island &S, int k) { return S.lbx[k]; }
-  __device__ static __forceinline__ float lby(const Island &S, int k) { return S.lby[k]; }
-  __device__ static __forceinline__ float comp(const Island &S, int k) { return S.comp[k]; }
-  __device__ static __forceinline__ float tgt(const Island &S, int k) { return S.tgt[k]; }
-  __device__ static __forceinline__ float brk(const Island &S, int k) { return S.brk[k]; }
-};
-struct CompactAccess {
-  __device__ static __forceinline__ int type(const Island &S, int k) { return S.type[k]; }
-  __device__ static __forceinline__ bool broken(const Island &S, int k) {
-    const int a = S.garm[k];
-    return a >= 0 && S.anc[4 * a + 3] != 0.f;
-  }
-  __device__ static __forceinline__ void set_broken(Island &S, int k) { S.anc[4 * S.garm[k] + 3] = 1.f; }
-  __device__ static __forceinline__ float lbx(const Island &S, int k) {
-    const int a = S.garm[k];
-    return a >= 0 ? S.anc[4 * a] : S.lbx[k];
-  }
-  __device__ static __forceinline__ float lby(const Island &S, int k) {
-    const int a = S.garm[k];
-    return a >= 0 ? S.anc[4 * a + 1] : S.lby[k];
-  }
-  __device__ static __forceinline__ float comp(const Island &S, int k) {
-    return S.type[k] == 1 ? S.comp_m : 0.f;
-  }
-  __device__ static __forceinline__ float tgt(const Island &S, int k) { return S.tgt_m[S.motor[k]]; }
-  __device__ static __forceinline__ float brk(const Island &S, int k) { return S.anc[4 * S.garm[k] + 2]; }
-};
+// ab word of a unit: body A, body B (or, in the batched engine, the record
+// of an arm's anchor; 0xff in the drop-in: the world), and flags.
+constexpr unsigned kUnitIdle = 0xffffffffu;
+// drop-in world flags
+constexpr unsigned kHasPin = 1u << 16, kPinBroken = 1u << 17, kHasAngle = 1u << 18, kAngleBroken = 1u << 19,
+                   kPinIsGrip = 1u << 20;
+// batched engine: bits 16..23 the motor of a joint, or 0xff for a grip
+constexpr unsigned kNoMotor = 0xffu;
 
-// integrateF, f32solver.mjs:177-200 (solver.wgsl:166-205)
+// integrateF, f32solver.mjs:177-200 (solver.wgsl:166-205).  World: the
+// drop-in's bodies (forces, immovable bodies, velocities in their own
+// records); otherwise the batched engine's, which have neither and whose
+// predicted state takes the place of the velocity: a substep reads the
+// velocity only here and writes it only in finalize_body.
+template <bool World>
 __device__ __forceinline__ void integrate_body(const SolverConsts &K, Island &S, int i) {
-  float im = S.im[i], ii = S.ii[i];
-  if (im == 0.f && ii == 0.f) {
-    S.ppx[i] = S.px[i]; S.ppy[i] = S.py[i]; S.angP[i] = S.ang[i];
-    S.vx[i] = 0.f; S.vy[i] = 0.f; S.av[i] = 0.f;
+  const float4 bd = S.body[i];
+  const float im = bd.x, ii = bd.y;
+  const float4 p = S.P[i];
+  if (World && im == 0.f && ii == 0.f) {
+    S.Q[i] = p;
+    S.V[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     return;
   }
-  float vx = fmul(fadd(S.vx[i], fmul(fmul(K.h, im), S.fx[i])), K.linDamp);
-  float vy = fmul(fadd(S.vy[i], fmul(fmul(K.h, im), S.fy[i])), K.linDamp);
-  float av = fmul(fadd(S.av[i], fmul(fmul(K.h, ii), S.tq[i])), K.angDamp);
+  float4 v = S.V[i];
+  const float4 f = World ? S.force[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float vx = fmul(fadd(v.x, fmul(fmul(K.h, im), f.x)), K.linDamp);
+  float vy = fmul(fadd(v.y, fmul(fmul(K.h, im), f.y)), K.linDamp);
+  float av = fmul(fadd(v.z, fmul(fmul(K.h, ii), f.z)), K.angDamp);
   float sp = length2(vx, vy);
   if (sp > K.maxSpeed) {
     float k = fdiv(K.maxSpeed, sp);
@@ -381,117 +373,183 @@ __device__ __forceinline__ void integrate_body(const SolverConsts &K, Island &S,
   else if (av < -K.maxAngSpeed) av = -K.maxAngSpeed;
   if (!(vx == vx) || !(vy == vy)) { vx = 0.f; vy = 0.f; }
   if (!(av == av)) av = 0.f;
-  S.vx[i] = vx; S.vy[i] = vy; S.av[i] = av;
-  S.ppx[i] = fadd(S.px[i], fmul(K.h, vx));
-  S.ppy[i] = fadd(S.py[i], fmul(K.h, vy));
-  S.angP[i] = fadd(S.ang[i], fmul(K.h, av));
-  S.fx[i] = 0.f; S.fy[i] = 0.f; S.tq[i] = 0.f;
+  if (World) S.V[i] = make_float4(vx, vy, av, v.w);
+  S.Q[i] = make_float4(fadd(p.x, fmul(K.h, vx)), fadd(p.y, fmul(K.h, vy)), fadd(p.z, fmul(K.h, av)), v.w);
+  if (World) S.force[i] = make_float4(0.f, 0.f, 0.f, f.w);
 }
 
-// solvePinF, f32solver.mjs:203-256 (solver.wgsl:225-290); grips are pins
-// against the world anchor (lbx, lby).
-template <class Acc>
-__device__ __forceinline__ void solve_pin(const SolverConsts &K, Island &S, int k) {
-  int ab = S.ab[k];
-  int A = ab & 0xffff, B = (ab >> 16) & 0xffff;
-  float sa, ca;
-  sincos_r(S.angP[A], &sa, &ca);
-  float lax = S.lax[k], lay = S.lay[k];
-  float rax = fsub(fmul(lax, ca), fmul(lay, sa));
-  float ray = fadd(fmul(lax, sa), fmul(lay, ca));
-  float gax = fadd(S.ppx[A], rax), gay = fadd(S.ppy[A], ray);
-  float gbx = Acc::lbx(S, k), gby = Acc::lby(S, k);
-  float rbx = 0.f, rby = 0.f, wB = 0.f, wIB = 0.f;
-  const bool hasB = B != 0xffff;
-  if (hasB) {
-    float sb, cb;
-    sincos_r(S.angP[B], &sb, &cb);
-    float lbx = gbx, lby = gby;
-    rbx = fsub(fmul(lbx, cb), fmul(lby, sb));
-    rby = fadd(fmul(lbx, sb), fmul(lby, cb));
-    gbx = fadd(S.ppx[B], rbx); gby = fadd(S.ppy[B], rby);
-    wB = S.im[B]; wIB = S.ii[B];
-  }
-  float Cx = fsub(gax, gbx), Cy = fsub(gay, gby);
+// solvePinF, f32solver.mjs:203-256 (solver.wgsl:225-290) on two body records
+// in registers; grips are pins against the world.  Without a body B: b holds
+// the anchor as its position with angle 0, lb and the masses of B are 0 (the
+// same values as the reference's branch).  lx, ly: the multiplier, updated.
+__device__ __forceinline__ void pin_math(float lax, float lay, float lbx, float lby, float wA, float wIA, float wB,
+                                         float wIB, float alphaTilde, bool hasB, float4 &a, float4 &b, float &lx,
+                                         float &ly) {
+  float sa, ca, sb, cb;
+  sincos_r(a.z, &sa, &ca);
+  sincos_r(b.z, &sb, &cb);
+  const float rax = fsub(fmul(lax, ca), fmul(lay, sa)), ray = fadd(fmul(lax, sa), fmul(lay, ca));
+  const float rbx = fsub(fmul(lbx, cb), fmul(lby, sb)), rby = fadd(fmul(lbx, sb), fmul(lby, cb));
+  const float Cx = fsub(fadd(a.x, rax), fadd(b.x, rbx)), Cy = fsub(fadd(a.y, ray), fadd(b.y, rby));
   if (!(Cx == Cx) || !(Cy == Cy)) return;
   if (fadd(fmul(Cx, Cx), fmul(Cy, Cy)) < fmul(kSlackPos, kSlackPos)) return;
-  float pax = -ray, pay = rax;
-  float pbx = -rby, pby = rbx;
-  float wA = S.im[A], wIA = S.ii[A];
-  float wSum = fadd(wA, wB);
-  float k00 = fadd(fadd(wSum, fmul(fmul(wIA, pax), pax)), fmul(fmul(wIB, pbx), pbx));
-  float k01 = fadd(fmul(fmul(wIA, pax), pay), fmul(fmul(wIB, pbx), pby));
-  float k11 = fadd(fadd(wSum, fmul(fmul(wIA, pay), pay)), fmul(fmul(wIB, pby), pby));
-  float det = fsub(fmul(k00, k11), fmul(k01, k01));
+  const float pax = -ray, pay = rax, pbx = -rby, pby = rbx;
+  const float wSum = fadd(wA, wB);
+  const float k00 = fadd(fadd(wSum, fmul(fmul(wIA, pax), pax)), fmul(fmul(wIB, pbx), pbx));
+  const float k01 = fadd(fmul(fmul(wIA, pax), pay), fmul(fmul(wIB, pbx), pby));
+  const float k11 = fadd(fadd(wSum, fmul(fmul(wIA, pay), pay)), fmul(fmul(wIB, pby), pby));
+  const float det = fsub(fmul(k00, k11), fmul(k01, k01));
   if (fabsf(det) < kEpsDet) return;
-  float alphaTilde = fmul(Acc::comp(S, k), K.invH2);
-  float lx0 = S.lamX[k], ly0 = S.lamY[k];
-  float bx = fadd(Cx, fmul(alphaTilde, lx0));
-  float by = fadd(Cy, fmul(alphaTilde, ly0));
-  float i00 = fdiv(k11, det), i11 = fdiv(k00, det), i01 = -fdiv(k01, det);
-  float dlx = -fadd(fmul(i00, bx), fmul(i01, by));
-  float dly = -fadd(fmul(i01, bx), fmul(i11, by));
+  const float bx = fadd(Cx, fmul(alphaTilde, lx)), by = fadd(Cy, fmul(alphaTilde, ly));
+  const float i00 = fdiv(k11, det), i11 = fdiv(k00, det), i01 = -fdiv(k01, det);
+  const float dlx = -fadd(fmul(i00, bx), fmul(i01, by)), dly = -fadd(fmul(i01, bx), fmul(i11, by));
   if (!(dlx == dlx) || !(dly == dly)) return;
-  S.lamX[k] = fadd(lx0, dlx);
-  S.lamY[k] = fadd(ly0, dly);
-  S.ppx[A] = fadd(S.ppx[A], fmul(wA, dlx));
-  S.ppy[A] = fadd(S.ppy[A], fmul(wA, dly));
-  S.angP[A] = fadd(S.angP[A], fmul(wIA, fadd(fmul(pax, dlx), fmul(pay, dly))));
+  lx = fadd(lx, dlx);
+  ly = fadd(ly, dly);
+  a.x = fadd(a.x, fmul(wA, dlx));
+  a.y = fadd(a.y, fmul(wA, dly));
+  a.z = fadd(a.z, fmul(wIA, fadd(fmul(pax, dlx), fmul(pay, dly))));
   if (hasB) {
-    S.ppx[B] = fsub(S.ppx[B], fmul(wB, dlx));
-    S.ppy[B] = fsub(S.ppy[B], fmul(wB, dly));
-    S.angP[B] = fsub(S.angP[B], fmul(wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
+    b.x = fsub(b.x, fmul(wB, dlx));
+    b.y = fsub(b.y, fmul(wB, dly));
+    b.z = fsub(b.z, fmul(wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
   }
 }
 
 // solveAngleF, f32solver.mjs:258-301 (solver.wgsl:292-350): muscle
-// (compliant) part, then the one-sided joint limit.
-template <class Acc>
-__device__ __forceinline__ void solve_angle(const SolverConsts &K, Island &S, int k) {
-  int ab = S.ab[k];
-  int A = ab & 0xffff, B = (ab >> 16) & 0xffff;
-  const bool hasB = B != 0xffff;
-  float wA = S.ii[A];
-  float wB = 0.f;
-  float rel = S.angP[A];
-  if (hasB) {
-    wB = S.ii[B];
-    rel = angle_delta(S.angP[B], S.angP[A]);
-  }
-  float wSum = fadd(wA, wB);
+// (compliant) part, then the one-sided joint limit.  az, bz: the angles; l:
+// the multiplier, updated.
+__device__ __forceinline__ void angle_math(float rest, float mn, float mx, float tgt, float alphaTilde, float wA,
+                                           float wB, bool hasB, float &az, float &bz, float &l) {
+  const float rel = hasB ? angle_delta(bz, az) : az;
+  const float wSum = fadd(wA, wB);
   if (wSum <= 0.f) return;
-  float rest = S.rest[k];
-  float dev = angle_delta(rel, rest);
-  float C = angle_delta(dev, Acc::tgt(S, k));
+  const float dev = angle_delta(rel, rest);
+  const float C = angle_delta(dev, tgt);
   if (!(C == C)) return;
   if (fabsf(C) >= kSlackAng) {
-    float alphaTilde = fmul(Acc::comp(S, k), K.invH2);
-    float l0 = S.lam[k];
-    float dl = -fdiv(fadd(C, fmul(alphaTilde, l0)), fadd(wSum, alphaTilde));
+    const float dl = -fdiv(fadd(C, fmul(alphaTilde, l)), fadd(wSum, alphaTilde));
     if (!(dl == dl)) return;
-    S.lam[k] = fadd(l0, dl);
+    l = fadd(l, dl);
     if (hasB) {
-      S.angP[B] = fadd(S.angP[B], fmul(wB, dl));
-      S.angP[A] = fsub(S.angP[A], fmul(wA, dl));
+      bz = fadd(bz, fmul(wB, dl));
+      az = fsub(az, fmul(wA, dl));
     } else {
-      S.angP[A] = fadd(S.angP[A], fmul(wA, dl));
+      az = fadd(az, fmul(wA, dl));
     }
   }
-  float rel2 = S.angP[A];
-  if (hasB) rel2 = angle_delta(S.angP[B], S.angP[A]);
-  float dev2 = angle_delta(rel2, rest);
+  const float dev2 = angle_delta(hasB ? angle_delta(bz, az) : az, rest);
   float over = 0.f;
-  float mx = S.maxA[k], mn = S.minA[k];
   if (dev2 > mx) over = fsub(dev2, mx);
   else if (dev2 < mn) over = fsub(dev2, mn);
   if (fabsf(over) >= kSlackAng) {
-    float dl2 = -fdiv(over, wSum);
+    const float dl2 = -fdiv(over, wSum);
     if (hasB) {
-      S.angP[B] = fadd(S.angP[B], fmul(wB, dl2));
-      S.angP[A] = fsub(S.angP[A], fmul(wA, dl2));
+      bz = fadd(bz, fmul(wB, dl2));
+      az = fsub(az, fmul(wA, dl2));
     } else {
-      S.angP[A] = fadd(S.angP[A], fmul(wA, dl2));
+      az = fadd(az, fmul(wA, dl2));
     }
+  }
+}
+
+// One sweep of the solve list, batched engine.  first: the first sweep of a
+// substep, where every multiplier starts from 0.  A pin's multiplier only
+// enters its own equation times its compliance, which is 0 for the
+// template's pins and grips, so only the grips' (the break test) and the
+// motors' are kept.
+template <int G>
+__device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
+  const float alpha_m = fmul(S.comp_m, K.invH2);
+  const float4 *rec = S.recs + 3 * L.lane;
+  for (int p = 0; p < S.npass; p++, rec += 3 * G) {
+    const float4 r0 = rec[0];
+    const unsigned ab = __float_as_uint(r0.x);
+    if (ab != kUnitIdle) {
+      const int A = ab & 0xff, B = (ab >> 8) & 0xff, m = (ab >> 16) & 0xff;
+      float4 a = S.Q[A], b = S.Q[B];
+      const float4 r1 = rec[1], r2 = rec[2];
+      if (m != (int)kNoMotor) {
+        float lx = 0.f, ly = 0.f;
+        pin_math(r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, 0.f, true, a, b, lx, ly);
+        const float2 mo = S.mot[m];
+        float l = first ? 0.f : mo.y;
+        angle_math(r2.y, r2.z, r2.w, mo.x, alpha_m, r1.z, r2.x, true, a.z, b.z, l);
+        S.mot[m].y = l;
+        S.Q[A] = a;
+        S.Q[B] = b;
+      } else {
+        float4 g = S.grip[B - S.nb];
+        if (first) g.x = g.y = 0.f;
+        if (b.w == 0.f) {  // holding
+          pin_math(r0.y, r0.z, 0.f, 0.f, r1.y, r1.z, 0.f, 0.f, 0.f, false, a, b, g.x, g.y);
+          S.Q[A] = a;
+        }
+        S.grip[B - S.nb] = g;
+      }
+    }
+    L.sync();
+  }
+}
+
+// A drop-in unit whose two bodies are one: every update sees the one before
+// it (a and b are the same record).  Out of line: no creature has one.
+static __device__ __noinline__ void solve_self(const SolverConsts &K, unsigned ab, float4 wa, float4 &a, float4 *rec) {
+  const float4 r0 = rec[0], r2 = rec[2];
+  float4 r1 = rec[1], r3 = rec[3];
+  if ((ab & (kHasPin | kPinBroken)) == kHasPin)
+    pin_math(r0.y, r0.z, r0.w, r1.x, wa.x, wa.y, wa.x, wa.y, fmul(r1.y, K.invH2), true, a, a, r1.z, r1.w);
+  if ((ab & (kHasAngle | kAngleBroken)) == kHasAngle)
+    angle_math(r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wa.y, true, a.z, a.z, r3.y);
+  rec[1] = r1;
+  rec[3] = r3;
+}
+
+// One sweep of the solve list, drop-in world: unit records
+// {ab, lax, lay, lbx} {lby, pin compliance, lambda x, y}
+// {rest, min, max, target} {angle compliance, lambda, break force, -}.
+template <int G>
+__device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
+  for (int p = 0; p < S.npass; p++) {
+    for (int u = S.off[p] + L.lane; u < S.off[p + 1]; u += G) {  // at most one: passes hold up to 32 units
+      float4 *rec = S.units + 4 * u;
+      const float4 r0 = rec[0];
+      const unsigned ab = __float_as_uint(r0.x);
+      const int A = ab & 0xff, B = (ab >> 8) & 0xff;
+      const bool hasB = B != 0xff;
+      float4 a = S.Q[A], b = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 wa = S.body[A];
+      if (A == B) {
+        if (first) { rec[1].z = rec[1].w = 0.f; rec[3].y = 0.f; }
+        solve_self(K, ab, wa, a, rec);
+        S.Q[A] = a;
+        continue;
+      }
+      float4 wb = b;
+      if (hasB) { b = S.Q[B]; wb = S.body[B]; }
+      if (ab & kHasPin) {
+        float4 r1 = rec[1];
+        if (first) r1.z = r1.w = 0.f;
+        if (!(ab & kPinBroken)) {
+          float4 anchor = make_float4(r0.w, r1.x, 0.f, 0.f);
+          pin_math(r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y, fmul(r1.y, K.invH2),
+                   hasB, a, hasB ? b : anchor, r1.z, r1.w);
+        }
+        rec[1] = r1;
+      }
+      if (ab & kHasAngle) {
+        float4 r3 = rec[3];
+        if (first) r3.y = 0.f;
+        if (!(ab & kAngleBroken)) {
+          const float4 r2 = rec[2];
+          angle_math(r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wb.y, hasB, a.z, b.z, r3.y);
+        }
+        rec[3] = r3;
+      }
+      S.Q[A] = a;
+      if (hasB) S.Q[B] = b;
+    }
+    L.sync();
   }
 }
 
@@ -523,8 +581,8 @@ __device__ __forceinline__ bool collide_bodies(Island &S, const float4 *__restri
                                                const Lanes<G> &L, float reach) {
   float lx = __int_as_float(0x7f800000), ly = lx, hx = -lx, hy = -lx;
   for (int j = L.lane; j < S.nb; j += G) {
-    lx = fminf(lx, S.ppx[j]); hx = fmaxf(hx, S.ppx[j]);
-    ly = fminf(ly, S.ppy[j]); hy = fmaxf(hy, S.ppy[j]);
+    lx = fminf(lx, S.Q[j].x); hx = fmaxf(hx, S.Q[j].x);
+    ly = fminf(ly, S.Q[j].y); hy = fmaxf(hy, S.Q[j].y);
   }
   lx = L.min(lx); ly = L.min(ly);
   hx = L.max(hx); hy = L.max(hy);
@@ -552,7 +610,7 @@ __device__ __forceinline__ bool collide_bodies(Island &S, const float4 *__restri
   if (ncull == 0) return true;
   L.sync();
   for (int j = L.lane; j < S.nb; j += G) {
-    const float cx = S.ppx[j], cy = S.ppy[j];
+    const float cx = S.Q[j].x, cy = S.Q[j].y;
     bool near = false;
     for (int q = 0; q < ncull && !near; q++) {
       const float4 r = __ldg(rects + S.cull[q]);
@@ -560,7 +618,7 @@ __device__ __forceinline__ bool collide_bodies(Island &S, const float4 *__restri
     }
     if (near) {
       float sn, cs;
-      sincos_r(S.angP[j], &sn, &cs);
+      sincos_r(S.Q[j].z, &sn, &cs);
       S.bs[j] = sn;
       S.bc[j] = cs;
     } else {
@@ -569,17 +627,18 @@ __device__ __forceinline__ bool collide_bodies(Island &S, const float4 *__restri
   }
   L.sync();
   for (int p = L.lane; p < S.np; p += G) {
-    const int j = S.pbody[p];
+    const float4 pt = S.pts[p];
+    const int j = __float_as_int(pt.w);
     const float ca = S.bc[j];
     int flag = 0;
     float cx = 0.f, cy = 0.f;
-    if (ca != 2.f && S.im[j] != 0.f) {
-      const float sa = S.bs[j], ox = S.plx[p], oy = S.ply[p];
-      const float wx = fadd(S.ppx[j], fsub(fmul(ox, ca), fmul(oy, sa)));
-      const float wy = fadd(S.ppy[j], fadd(fmul(ox, sa), fmul(oy, ca)));
+    if (ca != 2.f && S.body[j].x != 0.f) {
+      const float sa = S.bs[j], ox = pt.x, oy = pt.y;
+      const float wx = fadd(S.Q[j].x, fsub(fmul(ox, ca), fmul(oy, sa)));
+      const float wy = fadd(S.Q[j].y, fadd(fmul(ox, sa), fmul(oy, ca)));
       float d, nx, ny;
       if (sdf(rects, S.cull, ncull, wx, wy, &d, &nx, &ny)) {
-        const float pen = fsub(S.pr[p], d);
+        const float pen = fsub(pt.z, d);
         if (pen > kSlackPos) {
           flag = 1;
           cx = fmul(nx, pen);
@@ -595,9 +654,9 @@ __device__ __forceinline__ bool collide_bodies(Island &S, const float4 *__restri
   const float sx0 = lx - reach - kCullSlack, sx1 = hx + reach + kCullSlack;
   const float sy0 = ly - reach - kCullSlack, sy1 = hy + reach + kCullSlack;
   for (int j = L.lane; j < S.nb; j += G) {
-    if (S.im[j] == 0.f || S.bc[j] == 2.f) continue;
-    const int o = S.boff[j], cnt = S.bcnt[j];
-    float px = S.ppx[j], py = S.ppy[j];
+    if (S.body[j].x == 0.f || S.bc[j] == 2.f) continue;
+    const int pr = __float_as_int(S.body[j].w), o = pr & 0xffff, cnt = pr >> 16;
+    float px = S.Q[j].x, py = S.Q[j].y;
     const float ca = S.bc[j], sa = S.bs[j];
     bool moved = false;
     for (int q = 0; q < cnt; q++) {
@@ -610,19 +669,20 @@ __device__ __forceinline__ bool collide_bodies(Island &S, const float4 *__restri
         }
         continue;
       }
-      const float ox = S.plx[p], oy = S.ply[p];
+      const float4 pt = S.pts[p];
+      const float ox = pt.x, oy = pt.y;
       const float wx = fadd(px, fsub(fmul(ox, ca), fmul(oy, sa)));
       const float wy = fadd(py, fadd(fmul(ox, sa), fmul(oy, ca)));
       const bool in_box = wx >= sx0 && wx <= sx1 && wy >= sy0 && wy <= sy1;
       float d, nx, ny;
       if (!sdf(rects, in_box ? S.cull : nullptr, in_box ? ncull : nR, wx, wy, &d, &nx, &ny)) continue;
-      const float pen = fsub(S.pr[p], d);
+      const float pen = fsub(pt.z, d);
       if (pen <= kSlackPos) continue;
       px = fadd(px, fmul(nx, pen));
       py = fadd(py, fmul(ny, pen));
     }
-    S.ppx[j] = px;
-    S.ppy[j] = py;
+    S.Q[j].x = px;
+    S.Q[j].y = py;
   }
   L.sync();
   return true;
@@ -638,17 +698,18 @@ __device__ __forceinline__ void collide_island(Island &S, const float4 *__restri
   if (reach >= 0.f && collide_bodies<G>(S, rects, nR, cull_d, L, reach)) return;
   for (int j = L.lane; j < S.nb; j += G) {
     float s, c;
-    sincos_r(S.angP[j], &s, &c);
+    sincos_r(S.Q[j].z, &s, &c);
     S.bs[j] = s;
     S.bc[j] = c;
   }
   L.sync();
   float mnx = __int_as_float(0x7f800000), mny = mnx, mxx = -mnx, mxy = -mnx;
   for (int p = L.lane; p < S.np; p += G) {
-    const int j = S.pbody[p];
-    const float ca = S.bc[j], sa = S.bs[j], lx = S.plx[p], ly = S.ply[p];
-    const float wx = fadd(S.ppx[j], fsub(fmul(lx, ca), fmul(ly, sa)));
-    const float wy = fadd(S.ppy[j], fadd(fmul(lx, sa), fmul(ly, ca)));
+    const float4 pt = S.pts[p];
+    const int j = __float_as_int(pt.w);
+    const float ca = S.bc[j], sa = S.bs[j], lx = pt.x, ly = pt.y;
+    const float wx = fadd(S.Q[j].x, fsub(fmul(lx, ca), fmul(ly, sa)));
+    const float wy = fadd(S.Q[j].y, fadd(fmul(lx, sa), fmul(ly, ca)));
     S.pdx[p] = wx;  // position for now, correction below
     S.pdy[p] = wy;
     mnx = fminf(mnx, wx); mxx = fmaxf(mxx, wx);
@@ -679,13 +740,14 @@ __device__ __forceinline__ void collide_island(Island &S, const float4 *__restri
   const float sx0 = mnx - kCullSlack, sx1 = mxx + kCullSlack;
   const float sy0 = mny - kCullSlack, sy1 = mxy + kCullSlack;
   for (int p = L.lane; p < S.np; p += G) {
-    const int j = S.pbody[p];
+    const float4 pt = S.pts[p];
+    const int j = __float_as_int(pt.w);
     int flag = 0;
     float cx = 0.f, cy = 0.f;
-    if (S.im[j] != 0.f) {
+    if (S.body[j].x != 0.f) {
       float d, nx, ny;
       if (sdf(rects, list, nlist, S.pdx[p], S.pdy[p], &d, &nx, &ny)) {
-        const float pen = fsub(S.pr[p], d);
+        const float pen = fsub(pt.z, d);
         if (pen > kSlackPos) {
           flag = 1;
           cx = fmul(nx, pen);
@@ -699,9 +761,9 @@ __device__ __forceinline__ void collide_island(Island &S, const float4 *__restri
   }
   L.sync();
   for (int j = L.lane; j < S.nb; j += G) {
-    if (S.im[j] == 0.f) continue;
-    const int o = S.boff[j], cnt = S.bcnt[j];
-    float px = S.ppx[j], py = S.ppy[j];
+    if (S.body[j].x == 0.f) continue;
+    const int pr = __float_as_int(S.body[j].w), o = pr & 0xffff, cnt = pr >> 16;
+    float px = S.Q[j].x, py = S.Q[j].y;
     const float ca = S.bc[j], sa = S.bs[j];
     bool moved = false;
     for (int q = 0; q < cnt; q++) {
@@ -714,32 +776,39 @@ __device__ __forceinline__ void collide_island(Island &S, const float4 *__restri
         }
         continue;
       }
-      const float lx = S.plx[p], ly = S.ply[p];
+      const float4 pt = S.pts[p];
+      const float lx = pt.x, ly = pt.y;
       const float wx = fadd(px, fsub(fmul(lx, ca), fmul(ly, sa)));
       const float wy = fadd(py, fadd(fmul(lx, sa), fmul(ly, ca)));
       const bool in_box = wx >= sx0 && wx <= sx1 && wy >= sy0 && wy <= sy1;
       float d, nx, ny;
       if (!sdf(rects, in_box ? list : nullptr, in_box ? nlist : nR, wx, wy, &d, &nx, &ny)) continue;
-      const float pen = fsub(S.pr[p], d);
+      const float pen = fsub(pt.z, d);
       if (pen <= kSlackPos) continue;
       px = fadd(px, fmul(nx, pen));
       py = fadd(py, fmul(ny, pen));
     }
-    S.ppx[j] = px;
-    S.ppy[j] = py;
+    S.Q[j].x = px;
+    S.Q[j].y = py;
   }
   L.sync();
 }
 
 // finalizeF, f32solver.mjs:376-399 (solver.wgsl:405-430)
+template <bool World>
 __device__ __forceinline__ void finalize_body(const SolverConsts &K, Island &S, int i) {
-  if (S.im[i] == 0.f && S.ii[i] == 0.f) {
-    S.vx[i] = 0.f; S.vy[i] = 0.f; S.av[i] = 0.f;
-    return;
+  if (World) {
+    const float4 bd = S.body[i];
+    if (bd.x == 0.f && bd.y == 0.f) {
+      S.V[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      return;
+    }
   }
-  float vx = fmul(fsub(S.ppx[i], S.px[i]), K.invH);
-  float vy = fmul(fsub(S.ppy[i], S.py[i]), K.invH);
-  float av = fmul(angle_delta(S.angP[i], S.ang[i]), K.invH);
+  float4 q = S.Q[i];
+  const float4 p = S.P[i];
+  float vx = fmul(fsub(q.x, p.x), K.invH);
+  float vy = fmul(fsub(q.y, p.y), K.invH);
+  float av = fmul(angle_delta(q.z, p.z), K.invH);
   float sp = length2(vx, vy);
   if (sp > K.maxSpeed) {
     float k = fdiv(K.maxSpeed, sp);
@@ -747,59 +816,61 @@ __device__ __forceinline__ void finalize_body(const SolverConsts &K, Island &S, 
   }
   if (av > K.maxAngSpeed) av = K.maxAngSpeed;
   else if (av < -K.maxAngSpeed) av = -K.maxAngSpeed;
-  S.vx[i] = vx; S.vy[i] = vy; S.av[i] = av;
-  S.px[i] = S.ppx[i]; S.py[i] = S.ppy[i];
-  float a = S.angP[i];
-  if (a > 50.f || a < -50.f) {
-    a = wrap_angle(a);
-    S.angP[i] = a;
+  if (q.z > 50.f || q.z < -50.f) {
+    q.z = wrap_angle(q.z);
+    if (World) S.Q[i].z = q.z;
   }
-  S.ang[i] = a;
+  S.P[i] = make_float4(q.x, q.y, q.z, p.w);
+  S.V[i] = make_float4(vx, vy, av, World ? 0.f : q.w);
 }
 
-// gripBreakF, f32solver.mjs:402-416 (solver.wgsl:433-442)
-template <class Acc>
-__device__ __forceinline__ void grip_break(const SolverConsts &K, Island &S, int k) {
-  if (Acc::type(S, k) != 2 || Acc::broken(S, k)) return;
-  float f = fmul(length2(S.lamX[k], S.lamY[k]), K.invH);
-  if (f > Acc::brk(S, k)) {
-    Acc::set_broken(S, k);
-    S.lamX[k] = 0.f;
-    S.lamY[k] = 0.f;
-  }
+// gripBreakF, f32solver.mjs:402-416 (solver.wgsl:433-442): true if the
+// constraint with this multiplier and break force breaks
+__device__ __forceinline__ bool grip_breaks(const SolverConsts &K, float lx, float ly, float brk) {
+  return fmul(length2(lx, ly), K.invH) > brk;
 }
 
 // One env step of one island by a group of G lanes (xpbd.js:487-490 with the
 // substep of f32solver.mjs:419-428): substeps x (reset lambda, integrate,
-// iterations x (constraint levels, collisions), finalize), then grip break.
+// iterations x (solve passes, collisions), finalize), then grip break.
 // U: unroll factor of the substep loop (1: a loop; 2: its body twice per
 // trip, remainder handled) -- the same operations in the same order, so the
 // results do not depend on it; the batched engine's autotuner picks it.
-template <class Acc, int G, int U = 1>
+template <bool World, int G, int U = 1>
 __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
                                             const float4 *__restrict__ rects, int nR, float cull_d,
                                             const Lanes<G> &L, float reach) {
 #pragma unroll U
   for (int s = 0; s < K.substeps; s++) {
-    for (int k = L.lane; k < S.nc; k += G) { S.lamX[k] = 0.f; S.lamY[k] = 0.f; S.lam[k] = 0.f; }
-    for (int i = L.lane; i < S.nb; i += G) integrate_body(K, S, i);
+    for (int i = L.lane; i < S.nb; i += G) integrate_body<World>(K, S, i);
     L.sync();
     for (int it = 0; it < K.iterations; it++) {
-      for (int l = 0; l < S.nlv; l++) {
-        const int beg = S.lvl[l], end = S.lvl[l + 1];
-        for (int k = beg + L.lane; k < end; k += G) {
-          if (Acc::broken(S, k)) continue;
-          if (Acc::type(S, k) == 1) solve_angle<Acc>(K, S, k);
-          else solve_pin<Acc>(K, S, k);
-        }
-        L.sync();
-      }
+      if constexpr (World) solve_world<G>(K, S, it == 0, L);
+      else solve_engine<G>(K, S, it == 0, L);
       collide_island<G>(S, rects, nR, cull_d, L, reach);
     }
-    for (int i = L.lane; i < S.nb; i += G) finalize_body(K, S, i);
+    for (int i = L.lane; i < S.nb; i += G) finalize_body<World>(K, S, i);
     L.sync();
   }
-  for (int k = L.lane; k < S.nc; k += G) grip_break<Acc>(K, S, k);
+  if constexpr (World) {
+    for (int u = L.lane; u < S.nu; u += G) {
+      float4 *rec = S.units + 4 * u;
+      const unsigned ab = __float_as_uint(rec[0].x);
+      if ((ab & (kHasPin | kPinIsGrip | kPinBroken)) != (kHasPin | kPinIsGrip)) continue;
+      const float4 r1 = rec[1];
+      if (grip_breaks(K, r1.z, r1.w, rec[3].z)) {
+        rec[0].x = __uint_as_float(ab | kPinBroken);
+        rec[1] = make_float4(r1.x, r1.y, 0.f, 0.f);
+      }
+    }
+  } else if (L.lane < S.arms) {
+    const float4 g = S.grip[L.lane];
+    float4 &an = S.Q[S.nb + L.lane];
+    if (an.w == 0.f && grip_breaks(K, g.x, g.y, g.z)) {
+      an.w = 1.f;
+      S.grip[L.lane] = make_float4(0.f, 0.f, g.z, g.w);
+    }
+  }
   L.sync();
 }
 

@@ -3,6 +3,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+
+#include "kr_units.h"
 
 namespace kr {
 
@@ -29,71 +32,10 @@ struct RawCon {
 
 double rect_inertia(double m, double w, double h) { return m * (w * w + h * h) / 12; }
 
-// Levels balanced for G lanes.  Input: the solve list (type and bodies of
-// each entry, in list order) and its as-early-as-possible levels.  Any level
-// assignment in which every pair of entries sharing a body keeps its list
-// order gives bit-identical results (a level holds body-disjoint entries, so
-// their order inside it is free).  This one keeps the number of levels and
-// each level's constraint type (so a level's lanes never diverge between
-// the pin and the angle solve) and fills levels from the first: each level
-// takes the entries that cannot go later, then fills its last pass of G
-// lanes with the most urgent of the others whose predecessors are placed.
-// Returns false (leaving `out` unset) if the list's levels mix types.
-bool balance_levels(const std::vector<int> &ty, const std::vector<int> &ea, const std::vector<int> &eb,
-                    const std::vector<int> &asap0, int L, int G, std::vector<int> *out) {
-  const int n = (int)ty.size();
-  std::vector<int> ltype(L, -1);
-  for (int i = 0; i < n; i++) {
-    if (ltype[asap0[i]] >= 0 && ltype[asap0[i]] != ty[i]) return false;
-    ltype[asap0[i]] = ty[i];
-  }
-  std::vector<std::vector<int>> pred(n), succ(n);
-  std::vector<int> last_of;
-  for (int i = 0; i < n; i++) {
-    for (int b : {ea[i], eb[i]}) {
-      if (b < 0) continue;
-      if ((int)last_of.size() <= b) last_of.resize(b + 1, -1);
-      if (last_of[b] >= 0) { pred[i].push_back(last_of[b]); succ[last_of[b]].push_back(i); }
-      last_of[b] = i;
-    }
-  }
-  std::vector<int> asap(n), alap(n);
-  for (int i = 0; i < n; i++) {
-    int lo = 0;
-    for (int p : pred[i]) lo = std::max(lo, asap[p] + 1);
-    while (lo < L && ltype[lo] != ty[i]) lo++;
-    if (lo >= L) return false;
-    asap[i] = lo;
-  }
-  for (int i = n - 1; i >= 0; i--) {
-    int hi = L - 1;
-    for (int j : succ[i]) hi = std::min(hi, alap[j] - 1);
-    while (hi >= 0 && ltype[hi] != ty[i]) hi--;
-    if (hi < asap[i]) return false;
-    alap[i] = hi;
-  }
-  std::vector<int> lvl(n, -1);
-  for (int l = 0; l < L; l++) {
-    std::vector<int> mand, rest;
-    for (int i = 0; i < n; i++) {
-      if (lvl[i] >= 0 || ty[i] != ltype[l] || asap[i] > l) continue;
-      bool ready = true;
-      for (int p : pred[i]) ready = ready && lvl[p] >= 0 && lvl[p] < l;
-      if (!ready) continue;
-      (alap[i] == l ? mand : rest).push_back(i);
-    }
-    std::stable_sort(rest.begin(), rest.end(), [&](int x, int y) { return alap[x] < alap[y]; });
-    const int cap = std::max(1, (int)(mand.size() + G - 1) / G) * G;
-    for (int i : mand) lvl[i] = l;
-    for (size_t k = 0; k < rest.size() && (int)(mand.size() + k) < cap; k++) lvl[rest[k]] = l;
-  }
-  for (int i = 0; i < n; i++) {
-    if (lvl[i] < 0) return false;
-    for (int j : succ[i])
-      if (lvl[i] >= lvl[j]) return false;
-  }
-  *out = lvl;
-  return true;
+float word(unsigned u) {
+  float f;
+  std::memcpy(&f, &u, sizeof(f));
+  return f;
 }
 
 }  // namespace
@@ -137,7 +79,6 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
   t->arm_tip.resize(arms);
   t->arm_seg0.resize(arms);
   t->arm_segs.resize((size_t)arms * segs);
-  std::vector<int> grip_raw(arms);
   for (int a = 0; a < arms; a++) {
     const double relAng = ((double)a / arms) * kPi * 2;
     std::vector<int> sg(segs);
@@ -169,7 +110,6 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
     }
     int g = add_con(2, sg[segs - 1], -1, kSegLen * 0.5, 0, 0, 0);
     cons[g].arm = a;
-    grip_raw[a] = g;
     t->arm_tip[a] = sg[segs - 1];
     t->arm_seg0[a] = sg[0];
   }
@@ -188,71 +128,63 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
   for (int i = 0; i < nc; i++) list[i] = i;
   std::stable_sort(list.begin(), list.end(),
                    [&](int x, int y) { return cons[x].color < cons[y].color; });
-  // levels from the list order
-  std::vector<int> last(nb, -1), level(nc);
-  int nlv = 0;
-  for (int q = 0; q < nc; q++) {
-    const RawCon &c = cons[list[q]];
-    int L = last[c.a] + 1;
-    if (c.b >= 0) L = std::max(L, last[c.b] + 1);
-    level[q] = L;
-    last[c.a] = L;
-    if (c.b >= 0) last[c.b] = L;
-    nlv = std::max(nlv, L + 1);
-  }
-  if (nlv > kMaxTplLevels) {
-    *err = "body shape needs " + std::to_string(nlv) + " levels";
-    return false;
-  }
   t->nb = nb; t->nc = nc; t->np = np;
   t->im.resize(nb); t->ii.resize(nb);
   for (int i = 0; i < nb; i++) { t->im[i] = (float)im[i]; t->ii[i] = (float)ii[i]; }
-  // the list's types and bodies, for the balanced schedules
-  std::vector<int> lty(nc), la(nc), lb(nc);
+  // units of the solve list and, per lane-group size, their passes
+  std::vector<SolveEntry> entries(nc);
   for (int q = 0; q < nc; q++) {
     const RawCon &c = cons[list[q]];
-    lty[q] = c.type == 1 ? 1 : 0;
-    la[q] = c.a;
-    lb[q] = c.b;
+    entries[q] = SolveEntry{c.type == 1 ? 1 : 0, c.a, c.b};
+  }
+  std::vector<SolveUnit> units;
+  std::vector<int> last;
+  build_units(entries, nb, &units, last);
+  for (const SolveUnit &u : units) {
+    // the engine's records hold a joint (pin and angle constraint) or a grip
+    const bool joint = u.pin >= 0 && u.ang >= 0 && u.b >= 0;
+    const bool grip = u.pin >= 0 && u.ang < 0 && u.b < 0 && cons[list[u.pin]].type == 2;
+    if (!joint && !grip) {
+      *err = "body shape " + std::to_string(arms) + "x" + std::to_string(segs) + ": a constraint outside the joints";
+      return false;
+    }
   }
   for (int v = 0; v < kSchedules; v++) {
     const int G = v == 0 ? 32 : v == 1 ? 16 : 8;
-    std::vector<int> lv = level, bal;
-    if (balance_levels(lty, la, lb, level, nlv, G, &bal)) lv = bal;
+    std::vector<int> order, off;
+    schedule_units(units, nb, G, &order, &off);
     Schedule &S = t->sched[v];
-    S.nlv = nlv;
-    std::vector<int> cnt(nlv + 1, 0);
-    for (int q = 0; q < nc; q++) cnt[lv[q] + 1]++;
-    for (int L = 0; L < nlv; L++) cnt[L + 1] += cnt[L];
-    std::vector<int> order(nc), cur(cnt.begin(), cnt.end() - 1);
-    for (int q = 0; q < nc; q++) order[cur[lv[q]]++] = list[q];
-    S.lvl = cnt;
-    std::vector<int> slot_of(nc);
-    for (int s = 0; s < nc; s++) {
-      const RawCon &c = cons[order[s]];
-      slot_of[order[s]] = s;
-      const uint32_t b = c.b >= 0 ? (uint32_t)c.b : 0xffffu;
-      S.ab.push_back((int)((uint32_t)c.a | (b << 16)));
-      S.type.push_back(c.type);
-      S.lax.push_back((float)c.lax); S.lay.push_back((float)c.lay);
-      S.lbx.push_back((float)c.lbx); S.lby.push_back((float)c.lby);
-      S.rest.push_back((float)c.rest);
-      S.minA.push_back((float)c.minA); S.maxA.push_back((float)c.maxA);
-      S.motor.push_back(c.motor);
+    S.npass = (int)off.size() - 1;
+    S.recs.assign((size_t)S.npass * G * kRecFloats, 0.f);
+    for (int p = 0; p < S.npass; p++) {
+      for (int l = 0; l < G; l++) {
+        float *r = &S.recs[((size_t)p * G + l) * kRecFloats];
+        if (off[p] + l >= off[p + 1]) {
+          r[0] = word(0xffffffffu);
+          continue;
+        }
+        const SolveUnit &u = units[order[off[p] + l]];
+        const RawCon &c = cons[list[u.pin]];
+        const unsigned B = u.b >= 0 ? (unsigned)u.b : (unsigned)(nb + c.arm);
+        const unsigned m = u.ang >= 0 ? (unsigned)cons[list[u.ang]].motor : 0xffu;
+        r[0] = word((unsigned)u.a | (B << 8) | (m << 16));
+        r[1] = (float)c.lax; r[2] = (float)c.lay;
+        r[5] = t->im[u.a]; r[6] = t->ii[u.a];
+        if (u.b >= 0) {
+          r[3] = (float)c.lbx; r[4] = (float)c.lby;
+          r[7] = t->im[u.b]; r[8] = t->ii[u.b];
+        }
+        if (u.ang >= 0) {
+          const RawCon &g = cons[list[u.ang]];
+          r[9] = (float)g.rest; r[10] = (float)g.minA; r[11] = (float)g.maxA;
+        }
+      }
     }
-    S.arm_grip.resize(arms);
-    for (int a = 0; a < arms; a++) S.arm_grip[a] = slot_of[grip_raw[a]];
   }
-  const Schedule &S0 = t->sched[0];
-  t->nlv = nlv;
-  t->lvl = S0.lvl;
-  t->ab = S0.ab; t->type = S0.type; t->motor = S0.motor;
-  t->lax = S0.lax; t->lay = S0.lay; t->lbx = S0.lbx; t->lby = S0.lby;
-  t->rest = S0.rest; t->minA = S0.minA; t->maxA = S0.maxA;
-  t->arm_grip = S0.arm_grip;
   // points grouped per body, creation order within a body (groupCollPoints)
   t->boff.assign(nb, 0);
   t->bcnt.assign(nb, 0);
+  t->breach.assign(nb, 0.f);
   for (int p = 0; p < np; p++) t->bcnt[pbody[p]]++;
   int acc = 0;
   for (int b = 0; b < nb; b++) { t->boff[b] = acc; acc += t->bcnt[b]; }
@@ -265,6 +197,7 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
     t->r_max = std::max(t->r_max, (float)pr[p]);
     const double off = std::sqrt((double)t->plx[q] * t->plx[q] + (double)t->ply[q] * t->ply[q]);
     t->off_max = std::max(t->off_max, (float)off);
+    t->breach[pbody[p]] = std::max(t->breach[pbody[p]], (float)off + 1.f);
   }
   return true;
 }

@@ -10,12 +10,11 @@
 // (gpuworld.js:353-366); a colour class is body-disjoint, so the classes in
 // order are one valid sequential order of the solve list.  Here every
 // connected component of the constraint graph (a creature) gets its own
-// schedule: each constraint is placed on the first level after every earlier
-// constraint (in solve-list order) that shares one of its bodies.  Levels are
-// body-disjoint, and any order that keeps every pair of constraints sharing a
-// body in list order gives bit-identical results (the harness check
-// color-order-free, harness.js:1172-1193, pins this property for the
-// reference), so the warp's level sweep reproduces the list order exactly.
+// schedule of solve units in passes (kr_units.h, kr::Island): any order that
+// keeps every pair of constraints sharing a body in list order gives
+// bit-identical results (the harness check color-order-free,
+// harness.js:1172-1193, pins this property for the reference), so the warp's
+// pass sweep reproduces the list order exactly.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +28,7 @@
 
 #include "../../include/kraken_b200.h"
 #include "kr_solver.cuh"
+#include "kr_units.h"
 
 namespace {
 
@@ -37,16 +37,16 @@ thread_local std::string g_last_error;
 constexpr int kWarpsPerBlock = 4;
 
 // Per-island record, one int array of kIslandInts per island.
-enum { I_BODY_OFF = 0, I_NB, I_CON_OFF, I_NC, I_PT_OFF, I_NP, I_LVL_OFF, I_NLV, kIslandInts };
+enum { I_BODY_OFF = 0, I_NB, I_UNIT_OFF, I_NU, I_PT_OFF, I_NP, I_PASS_OFF, I_NPASS, kIslandInts };
 
 struct DeviceTables {
   const int *isl;          // nI x kIslandInts
   const int *bodies;       // global body id per island body
-  const int *cons;         // global constraint index per schedule slot
-  const int *ab;           // local a | local b << 16 per schedule slot
+  const int4 *units;       // per unit, pass by pass: local a | b << 8 (0xff: the world), global constraint
+                           // index of its pin and of its angle constraint (-1: none)
   const int *pts;          // global collision point index, local-body grouped
   const int2 *bpt;         // per island body: (offset within island points, count)
-  const int *lvl;          // level offsets per island (nlv + 1 each)
+  const int *pass;         // pass offsets per island (npass + 1 each)
 };
 
 struct StepArgs {
@@ -60,121 +60,129 @@ struct StepArgs {
   float cull_d;            // rect culling distance of a collision pass
   float reach;             // bound on a collision point's distance from its body (+1 px), < 0: none
   int nI;
-  int maxB, maxC, maxP;    // smem carve sizes (per warp)
+  int maxB, maxU, maxP;    // smem carve sizes (per warp)
   DeviceTables T;
 };
 
-__host__ __device__ inline int warp_smem_words(int mb, int mc, int mp) {
-  return 18 * mb + 15 * mc + 7 * mp + kr::kMaxCulled / 2;
+__host__ __device__ inline int warp_smem_words(int mb, int mu, int mp) {
+  return 22 * mb + 16 * mu + 7 * mp + kr::kMaxCulled / 2;
 }
 
-// Writable views of the per-slot statics while they are staged; the solver
-// reads them through the const pointers of kr::Island.
+// Writable views of the statics while they are staged; the solver reads them
+// through the const pointers of kr::Island.
 struct StageView {
-  int *ab, *boff, *bcnt, *pbody;
-  float *lax, *lay, *rest, *minA, *maxA, *plx, *ply, *pr;
+  float4 *body, *pts;
 };
 
-__device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, int mc, int mp) {
-  float *p = base;
-  S.px = p; p += mb; S.py = p; p += mb; S.ppx = p; p += mb; S.ppy = p; p += mb;
-  S.vx = p; p += mb; S.vy = p; p += mb; S.ang = p; p += mb; S.angP = p; p += mb;
-  S.av = p; p += mb; S.im = p; p += mb; S.ii = p; p += mb;
-  S.fx = p; p += mb; S.fy = p; p += mb; S.tq = p; p += mb;
+__device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, int mu, int mp) {
+  float4 *q = reinterpret_cast<float4 *>(base);
+  S.P = q; q += mb; S.Q = q; q += mb; S.V = q; q += mb; S.force = q; q += mb;
+  V.body = q; q += mb;
+  S.units = q; q += 4 * mu;
+  V.pts = q; q += mp;
+  float *p = reinterpret_cast<float *>(q);
   S.bs = p; p += mb; S.bc = p; p += mb;
-  V.boff = reinterpret_cast<int *>(p); p += mb;
-  V.bcnt = reinterpret_cast<int *>(p); p += mb;
-  V.ab = reinterpret_cast<int *>(p); p += mc;
-  S.tb = reinterpret_cast<int *>(p); p += mc;
-  V.lax = p; p += mc; V.lay = p; p += mc; S.lbx = p; p += mc; S.lby = p; p += mc;
-  S.comp = p; p += mc; V.rest = p; p += mc; S.tgt = p; p += mc; V.minA = p; p += mc;
-  V.maxA = p; p += mc; S.lamX = p; p += mc; S.lamY = p; p += mc; S.lam = p; p += mc;
-  S.brk = p; p += mc;
-  V.plx = p; p += mp; V.ply = p; p += mp; V.pr = p; p += mp;
   S.pdx = p; p += mp; S.pdy = p; p += mp;
-  V.pbody = reinterpret_cast<int *>(p); p += mp;
   S.pflag = reinterpret_cast<int *>(p); p += mp;
   S.cull = reinterpret_cast<short *>(p);
-  S.ab = V.ab; S.boff = V.boff; S.bcnt = V.bcnt; S.pbody = V.pbody;
-  S.lax = V.lax; S.lay = V.lay; S.rest = V.rest; S.minA = V.minA; S.maxA = V.maxA;
-  S.plx = V.plx; S.ply = V.ply; S.pr = V.pr;
+  S.body = V.body; S.pts = V.pts;
 }
 
 // One launch of the plain step for the island of this warp (shared by the
 // plain kernel and its allocation-free variant).
 __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int island = blockIdx.x * kWarpsPerBlock + warp;
   if (island >= A.nI) return;
   kr::Island S;
   StageView V;
-  carve(S, V, smem + warp * warp_smem_words(A.maxB, A.maxC, A.maxP), A.maxB, A.maxC, A.maxP);
+  carve(S, V, smem + warp * warp_smem_words(A.maxB, A.maxU, A.maxP), A.maxB, A.maxU, A.maxP);
   const int *rec = A.T.isl + island * kIslandInts;
-  const int bo = rec[I_BODY_OFF], co = rec[I_CON_OFF], po = rec[I_PT_OFF];
-  S.nb = rec[I_NB]; S.nc = rec[I_NC]; S.np = rec[I_NP];
-  S.nlv = rec[I_NLV];
-  S.lvl = A.T.lvl + rec[I_LVL_OFF];
+  const int bo = rec[I_BODY_OFF], uo = rec[I_UNIT_OFF], po = rec[I_PT_OFF];
+  S.nb = rec[I_NB]; S.nu = rec[I_NU]; S.np = rec[I_NP];
+  S.npass = rec[I_NPASS];
+  S.off = A.T.pass + rec[I_PASS_OFF];
 
-  // stage bodies (48 B AoS -> SoA) and forces
+  // stage bodies (48 B AoS), forces and the bodies' collision points
   for (int i = lane; i < S.nb; i += 32) {
     const int g = A.T.bodies[bo + i];
     const float4 *b4 = reinterpret_cast<const float4 *>(A.bodies + 12 * (size_t)g);
     const float4 q0 = b4[0], q1 = b4[1], q2 = b4[2];
-    S.px[i] = q0.x; S.py[i] = q0.y; S.ppx[i] = q0.z; S.ppy[i] = q0.w;
-    S.vx[i] = q1.x; S.vy[i] = q1.y; S.ang[i] = q1.z; S.angP[i] = q1.w;
-    S.av[i] = q2.x; S.im[i] = q2.y; S.ii[i] = q2.z;
-    const float4 f = reinterpret_cast<const float4 *>(A.forces)[g];
-    S.fx[i] = f.x; S.fy[i] = f.y; S.tq[i] = f.z;
+    S.P[i] = make_float4(q0.x, q0.y, q1.z, 0.f);
+    S.Q[i] = make_float4(q0.z, q0.w, q1.w, 0.f);
+    S.V[i] = make_float4(q1.x, q1.y, q2.x, 0.f);
+    S.force[i] = reinterpret_cast<const float4 *>(A.forces)[g];
     const int2 bp = A.T.bpt[bo + i];
-    V.boff[i] = bp.x; V.bcnt[i] = bp.y;
-    for (int q = 0; q < bp.y; q++) V.pbody[bp.x + q] = i;
+    V.body[i] = make_float4(q2.y, q2.z, 0.f, __int_as_float(bp.x | (bp.y << 16)));
+    for (int q = 0; q < bp.y; q++) {
+      const uint4 cp = A.coll[A.T.pts[po + bp.x + q]];
+      V.pts[bp.x + q] = make_float4(__uint_as_float(cp.y), __uint_as_float(cp.z), __uint_as_float(cp.w),
+                                    __int_as_float(i));
+    }
   }
-  // stage constraints (80 B AoS -> SoA, schedule order)
-  for (int k = lane; k < S.nc; k += 32) {
-    const int g = A.T.cons[co + k];
-    const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)g);
-    const uint4 w0 = c4[0], w1 = c4[1], w2 = c4[2], w3 = c4[3], w4 = c4[4];
-    V.ab[k] = A.T.ab[co + k];
-    S.tb[k] = static_cast<int>(w0.z & 0xffu) | ((w4.y != 0u ? 1 : 0) << 8);
-    V.lax[k] = __uint_as_float(w1.x); V.lay[k] = __uint_as_float(w1.y);
-    S.lbx[k] = __uint_as_float(w1.z); S.lby[k] = __uint_as_float(w1.w);
-    S.comp[k] = __uint_as_float(w2.x); V.rest[k] = __uint_as_float(w2.y);
-    S.tgt[k] = __uint_as_float(w2.z); V.minA[k] = __uint_as_float(w2.w);
-    V.maxA[k] = __uint_as_float(w3.x); S.lamX[k] = __uint_as_float(w3.y);
-    S.lamY[k] = __uint_as_float(w3.z); S.lam[k] = __uint_as_float(w3.w);
-    S.brk[k] = __uint_as_float(w4.x);
-  }
-  // stage collision points
-  for (int p = lane; p < S.np; p += 32) {
-    const uint4 cp = A.coll[A.T.pts[po + p]];
-    V.plx[p] = __uint_as_float(cp.y); V.ply[p] = __uint_as_float(cp.z);
-    V.pr[p] = __uint_as_float(cp.w);
+  // stage the units' constraints (80 B AoS -> unit records)
+  for (int u = lane; u < S.nu; u += 32) {
+    const int4 t = A.T.units[uo + u];
+    unsigned ab = (unsigned)t.x;
+    float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0, r3 = r0;
+    if (t.y >= 0) {
+      const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)t.y);
+      const uint4 w0 = c4[0], w1 = c4[1], w2 = c4[2], w4 = c4[4];
+      ab |= kr::kHasPin | (w4.y != 0u ? kr::kPinBroken : 0u) | ((w0.z & 0xffu) == 2u ? kr::kPinIsGrip : 0u);
+      r0.y = __uint_as_float(w1.x); r0.z = __uint_as_float(w1.y);
+      r0.w = __uint_as_float(w1.z); r1.x = __uint_as_float(w1.w);
+      r1.y = __uint_as_float(w2.x);
+      r3.z = __uint_as_float(w4.x);
+    }
+    if (t.z >= 0) {
+      const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)t.z);
+      const uint4 w2 = c4[2], w3 = c4[3], w4 = c4[4];
+      ab |= kr::kHasAngle | (w4.y != 0u ? kr::kAngleBroken : 0u);
+      r2 = make_float4(__uint_as_float(w2.y), __uint_as_float(w2.w), __uint_as_float(w3.x), __uint_as_float(w2.z));
+      r3.x = __uint_as_float(w2.x);
+    }
+    r0.x = __uint_as_float(ab);
+    S.units[4 * u] = r0; S.units[4 * u + 1] = r1; S.units[4 * u + 2] = r2; S.units[4 * u + 3] = r3;
   }
   __syncwarp();
 
-  kr::island_step<kr::SlotAccess, 32>(A.K, S, A.rects, A.nR, A.cull_d, kr::Lanes<32>(lane), A.reach);
+  kr::island_step<true, 32>(A.K, S, A.rects, A.nR, A.cull_d, kr::Lanes<32>(lane), A.reach);
 
   // write back bodies, consumed forces and constraint multipliers / flags
   for (int i = lane; i < S.nb; i += 32) {
     const int g = A.T.bodies[bo + i];
     float4 *b4 = reinterpret_cast<float4 *>(A.bodies + 12 * (size_t)g);
     const float pad = A.bodies[12 * (size_t)g + 11];
-    b4[0] = make_float4(S.px[i], S.py[i], S.ppx[i], S.ppy[i]);
-    b4[1] = make_float4(S.vx[i], S.vy[i], S.ang[i], S.angP[i]);
-    b4[2] = make_float4(S.av[i], S.im[i], S.ii[i], pad);
-    if (!(S.im[i] == 0.f && S.ii[i] == 0.f)) {
+    const float4 p = S.P[i], q = S.Q[i], v = S.V[i], bd = S.body[i];
+    b4[0] = make_float4(p.x, p.y, q.x, q.y);
+    b4[1] = make_float4(v.x, v.y, p.z, q.z);
+    b4[2] = make_float4(v.z, bd.x, bd.y, pad);
+    if (!(bd.x == 0.f && bd.y == 0.f)) {
       float *f = A.forces + 4 * (size_t)g;
       f[0] = 0.f; f[1] = 0.f; f[2] = 0.f;  // consumed, adhesion kept (solver.wgsl:204)
     }
   }
-  for (int k = lane; k < S.nc; k += 32) {
-    const int g = A.T.cons[co + k];
-    uint32_t *c = A.cons + 20 * (size_t)g;
-    c[13] = __float_as_uint(S.lamX[k]);
-    c[14] = __float_as_uint(S.lamY[k]);
-    c[15] = __float_as_uint(S.lam[k]);
-    c[17] = (S.tb[k] >> 8) != 0 ? 1u : 0u;
+  // every multiplier starts each substep at 0, so a pin's angle multiplier
+  // and an angle constraint's pin multiplier end at 0
+  for (int u = lane; u < S.nu; u += 32) {
+    const int4 t = A.T.units[uo + u];
+    const unsigned ab = __float_as_uint(S.units[4 * u].x);
+    if (t.y >= 0) {
+      const float4 r1 = S.units[4 * u + 1];
+      uint32_t *c = A.cons + 20 * (size_t)t.y;
+      c[13] = __float_as_uint(r1.z);
+      c[14] = __float_as_uint(r1.w);
+      c[15] = 0u;
+      c[17] = (ab & kr::kPinBroken) ? 1u : 0u;
+    }
+    if (t.z >= 0) {
+      uint32_t *c = A.cons + 20 * (size_t)t.z;
+      c[13] = 0u;
+      c[14] = 0u;
+      c[15] = __float_as_uint(S.units[4 * u + 3].y);
+      c[17] = (ab & kr::kAngleBroken) ? 1u : 0u;
+    }
   }
 }
 
@@ -211,14 +219,14 @@ struct kr_world {
   uint4 *d_coll = nullptr;
   std::vector<uint32_t> h_coll_range;   // 2 x nB
   // island tables
-  int *d_isl = nullptr, *d_ibodies = nullptr, *d_icons = nullptr, *d_iab = nullptr,
-      *d_ipts = nullptr, *d_lvl = nullptr;
+  int *d_isl = nullptr, *d_ibodies = nullptr, *d_ipts = nullptr, *d_pass = nullptr;
+  int4 *d_units = nullptr;
   int2 *d_bpt = nullptr;
-  size_t c_isl = 0, c_ibodies = 0, c_icons = 0, c_iab = 0, c_ipts = 0, c_lvl = 0, c_bpt = 0;
+  size_t c_isl = 0, c_ibodies = 0, c_units = 0, c_ipts = 0, c_pass = 0, c_bpt = 0;
   float max_half_thick = 0.f;  // largest min(w, h) / 2 of the map's rects
   float cull_d = 0.f;
   float reach = -1.f;          // largest collision-point offset + 1 px (kr_solver.cuh collide_bodies)
-  int nI = 0, maxB = 1, maxC = 1, maxP = 1, maxLv = 0;
+  int nI = 0, maxB = 1, maxU = 1, maxP = 1, maxLv = 0;
   bool uploaded = false;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -399,7 +407,7 @@ extern "C" int kr_create(const kr_solver_params *params, uint32_t n_bodies, uint
 
 namespace {
 
-// Connected components, per-component levels and lane tables (see the file
+// Connected components, per-component unit passes and lane tables (see the file
 // comment).  Returns KR_OK or an error code with w->err set.
 int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
   const uint32_t nB = w->nB, nC = w->nC;
@@ -439,11 +447,14 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
   std::vector<std::vector<int>> ic(nI);  // constraints per island, list order
   for (uint32_t k = 0; k < nC; k++) ic[island_of[cons[20 * k]]].push_back((int)k);
 
-  std::vector<int> isl(nI * (size_t)kIslandInts), h_bodies, h_cons, h_ab, h_pts, h_lvl;
+  std::vector<int> isl(nI * (size_t)kIslandInts), h_bodies, h_pts, h_pass;
+  std::vector<int4> h_units;
   std::vector<int2> h_bpt;
-  h_bodies.reserve(nB); h_cons.reserve(nC); h_ab.reserve(nC);
-  int maxB = 1, maxC = 1, maxP = 1, maxLv = 0;
-  std::vector<int> last_level, level, order, cnt_per_level;
+  h_bodies.reserve(nB); h_units.reserve(nC);
+  int maxB = 1, maxU = 1, maxP = 1, maxLv = 0;
+  std::vector<int> last_level, order, off;
+  std::vector<kr::SolveEntry> list;
+  std::vector<kr::SolveUnit> units;
   for (int I = 0; I < nI; I++) {
     const auto &bl = ib[I];
     const auto &cl = ic[I];
@@ -458,9 +469,10 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
     rec[I_BODY_OFF] = (int)h_bodies.size();
     rec[I_NB] = nb;
     for (int g : bl) h_bodies.push_back(g);
-    // levels: first level after every earlier constraint sharing a body
+    // the list, and its constraint levels (each on the first level after
+    // every earlier constraint sharing a body)
     last_level.assign(nb, -1);
-    level.resize(nc);
+    list.resize(nc);
     int nlv = 0;
     for (int q = 0; q < nc; q++) {
       const uint32_t *c = cons + 20 * (size_t)cl[q];
@@ -468,35 +480,26 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
       const int b = c[1] == 0xffffffffu ? -1 : local[c[1]];
       int L = last_level[a] + 1;
       if (b >= 0) L = std::max(L, last_level[b] + 1);
-      level[q] = L;
       last_level[a] = L;
       if (b >= 0) last_level[b] = L;
       nlv = std::max(nlv, L + 1);
+      list[q] = kr::SolveEntry{(c[2] & 0xffu) == 1u ? 1 : 0, a, b};
     }
     if (nlv > KR_MAX_LEVELS)
       return w->fail(KR_ERR_CAPACITY, "connected component " + std::to_string(I) + " needs " +
                                           std::to_string(nlv) + " constraint levels; the kernel holds " +
                                           std::to_string(KR_MAX_LEVELS));
-    cnt_per_level.assign(nlv + 1, 0);
-    for (int q = 0; q < nc; q++) cnt_per_level[level[q] + 1]++;
-    for (int L = 0; L < nlv; L++) cnt_per_level[L + 1] += cnt_per_level[L];
-    rec[I_LVL_OFF] = (int)h_lvl.size();
-    rec[I_NLV] = nlv;
-    for (int L = 0; L <= nlv; L++) h_lvl.push_back(cnt_per_level[L]);
-    order.assign(nc, 0);
-    {
-      std::vector<int> cur(cnt_per_level.begin(), cnt_per_level.end() - 1);
-      for (int q = 0; q < nc; q++) order[cur[level[q]]++] = q;  // stable within a level
-    }
-    rec[I_CON_OFF] = (int)h_cons.size();
-    rec[I_NC] = nc;
-    for (int s = 0; s < nc; s++) {
-      const int k = cl[order[s]];
-      const uint32_t *c = cons + 20 * (size_t)k;
-      const uint32_t a = (uint32_t)local[c[0]];
-      const uint32_t b = c[1] == 0xffffffffu ? 0xffffu : (uint32_t)local[c[1]];
-      h_cons.push_back(k);
-      h_ab.push_back((int)(a | (b << 16)));
+    kr::build_units(list, nb, &units, last_level);
+    kr::schedule_units(units, nb, 32, &order, &off);
+    rec[I_PASS_OFF] = (int)h_pass.size();
+    rec[I_NPASS] = (int)off.size() - 1;
+    h_pass.insert(h_pass.end(), off.begin(), off.end());
+    rec[I_UNIT_OFF] = (int)h_units.size();
+    rec[I_NU] = (int)units.size();
+    for (int u : order) {
+      const kr::SolveUnit &x = units[u];
+      h_units.push_back(make_int4(x.a | ((x.b >= 0 ? x.b : 0xff) << 8), x.pin >= 0 ? cl[x.pin] : -1,
+                                  x.ang >= 0 ? cl[x.ang] : -1, 0));
     }
     // collision points in local body order
     rec[I_PT_OFF] = (int)h_pts.size();
@@ -514,26 +517,25 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
                                           std::to_string(KR_MAX_ISLAND_COLLPTS));
     rec[I_NP] = np;
     maxB = std::max(maxB, nb);
-    maxC = std::max(maxC, nc);
+    maxU = std::max(maxU, (int)units.size());
     maxP = std::max(maxP, np);
     maxLv = std::max(maxLv, nlv);
   }
   cudaError_t e;
   if ((e = dev_upload(&w->d_isl, &w->c_isl, isl)) != cudaSuccess) return w->cuda_fail(e, "upload(islands)");
   if ((e = dev_upload(&w->d_ibodies, &w->c_ibodies, h_bodies)) != cudaSuccess) return w->cuda_fail(e, "upload(island bodies)");
-  if ((e = dev_upload(&w->d_icons, &w->c_icons, h_cons)) != cudaSuccess) return w->cuda_fail(e, "upload(island constraints)");
-  if ((e = dev_upload(&w->d_iab, &w->c_iab, h_ab)) != cudaSuccess) return w->cuda_fail(e, "upload(island ab)");
+  if ((e = dev_upload(&w->d_units, &w->c_units, h_units)) != cudaSuccess) return w->cuda_fail(e, "upload(island units)");
   if ((e = dev_upload(&w->d_ipts, &w->c_ipts, h_pts)) != cudaSuccess) return w->cuda_fail(e, "upload(island points)");
   if ((e = dev_upload(&w->d_bpt, &w->c_bpt, h_bpt)) != cudaSuccess) return w->cuda_fail(e, "upload(body point ranges)");
-  if ((e = dev_upload(&w->d_lvl, &w->c_lvl, h_lvl)) != cudaSuccess) return w->cuda_fail(e, "upload(levels)");
+  if ((e = dev_upload(&w->d_pass, &w->c_pass, h_pass)) != cudaSuccess) return w->cuda_fail(e, "upload(passes)");
   w->nI = nI;
   // round up so every per-warp region keeps 16-byte alignment of its arrays
   w->maxB = (maxB + 3) & ~3;
-  w->maxC = (maxC + 3) & ~3;
+  w->maxU = maxU;
   w->maxP = (maxP + 3) & ~3;
   w->maxLv = maxLv;
   w->smem_bytes =
-      sizeof(float) * kWarpsPerBlock * (size_t)warp_smem_words(w->maxB, w->maxC, w->maxP);
+      sizeof(float) * kWarpsPerBlock * (size_t)warp_smem_words(w->maxB, w->maxU, w->maxP);
   if ((e = cudaFuncSetAttribute(plain_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)w->smem_bytes)) != cudaSuccess)
     return w->cuda_fail(e, "cudaFuncSetAttribute(plain_step_kernel)");
@@ -620,8 +622,8 @@ extern "C" int kr_step(kr_world *w, int32_t n_steps) {
   A.rects = w->d_rects;
   A.nR = (int)w->nR;
   A.nI = w->nI;
-  A.maxB = w->maxB; A.maxC = w->maxC; A.maxP = w->maxP;
-  A.T = DeviceTables{w->d_isl, w->d_ibodies, w->d_icons, w->d_iab, w->d_ipts, w->d_bpt, w->d_lvl};
+  A.maxB = w->maxB; A.maxU = w->maxU; A.maxP = w->maxP;
+  A.T = DeviceTables{w->d_isl, w->d_ibodies, w->d_units, w->d_ipts, w->d_bpt, w->d_pass};
   A.cull_d = w->cull_d;
   A.reach = w->reach;
   const size_t smem = w->smem_bytes;
@@ -683,7 +685,7 @@ extern "C" void kr_destroy(kr_world *w) {
   if (!w) return;
   if (w->stream) cudaStreamSynchronize(w->stream);
   void *ptrs[] = {w->d_bodies, w->d_cons, w->d_stage, w->d_forces, w->d_rects, w->d_coll, w->d_isl,
-                  w->d_ibodies, w->d_icons, w->d_iab, w->d_ipts, w->d_lvl, w->d_bpt};
+                  w->d_ibodies, w->d_units, w->d_ipts, w->d_pass, w->d_bpt};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (w->own_stream && w->stream) cudaStreamDestroy(w->stream);
@@ -701,9 +703,9 @@ extern "C" void kr_destroy(kr_world *w) {
 // lives in one file-scope device array of fixed size, so the call allocates
 // nothing on the device or the host.
 //
-// Scratch layout (words): island records, island bodies, schedule slots,
-// slot body pairs, island points, body point ranges, level offsets, rects,
-// and the builder's temporaries.  The array is shared by every call on a
+// Scratch layout (words): island records, island bodies, units, island
+// points, body point ranges, pass offsets, rects, and the builder's
+// temporaries.  The array is shared by every call on a
 // device and keeps the last call's contents; the builder initializes every
 // word it reads before reading it.
 // ---------------------------------------------------------------------------
@@ -717,20 +719,22 @@ constexpr int kNaR = KR_NOALLOC_MAX_RECTS;
 constexpr int kOffHdr = 0;                                  // n_islands, cull_d, status, pad
 constexpr int kOffIsl = 4;
 constexpr int kOffBodies = kOffIsl + kNaB * kIslandInts;
-constexpr int kOffCons = kOffBodies + kNaB;
-constexpr int kOffAb = kOffCons + kNaC;
-constexpr int kOffPts = kOffAb + kNaC;
+constexpr int kOffUnits = (kOffBodies + kNaB + 3) & ~3;    // int4, 16-byte aligned
+constexpr int kOffPts = kOffUnits + 4 * kNaC;
 constexpr int kOffBpt = ((kOffPts + kNaP) + 1) & ~1;       // int2, 8-byte aligned
-constexpr int kOffLvl = kOffBpt + 2 * kNaB;
-constexpr int kOffRects = ((kOffLvl + kNaC + kNaB) + 3) & ~3;  // float4, 16-byte aligned
+constexpr int kOffPass = kOffBpt + 2 * kNaB;
+constexpr int kOffRects = ((kOffPass + kNaC + kNaB) + 3) & ~3;  // float4, 16-byte aligned
 constexpr int kOffParent = kOffRects + 4 * kNaR;
 constexpr int kOffIslandOf = kOffParent + kNaB;
 constexpr int kOffLocal = kOffIslandOf + kNaB;
 constexpr int kOffRootIsl = kOffLocal + kNaB;
 constexpr int kOffCnt = kOffRootIsl + kNaB;                 // kNaB + 1
 constexpr int kOffLast = kOffCnt + kNaB + 1;
-constexpr int kOffLevel = kOffLast + kNaB;
-constexpr int kOffCur = kOffLevel + kNaC;                   // kNaC + 1
+constexpr int kOffLastUnit = kOffLast + kNaB;
+constexpr int kOffList = kOffLastUnit + kNaB;               // constraints per island, list order
+constexpr int kOffLevel = kOffList + kNaC;                  // level of each unit
+constexpr int kOffTmp = (kOffLevel + kNaC + 3) & ~3;        // units in list order, int4
+constexpr int kOffCur = kOffTmp + 4 * kNaC;                 // kNaC + 1
 constexpr int kScratchWords = kOffCur + kNaC + 1;
 
 static __device__ __align__(256) int g_noalloc_scratch[kScratchWords];
@@ -741,13 +745,14 @@ __global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint3
                                         const float *rects, const uint32_t *coll_pts,
                                         const uint32_t *coll_range, int nB, int nC, int nP, int nR) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int *isl = W + kOffIsl, *ib = W + kOffBodies, *icons = W + kOffCons, *iab = W + kOffAb;
-  int *ipts = W + kOffPts, *lvl = W + kOffLvl;
+  int *isl = W + kOffIsl, *ib = W + kOffBodies, *icons = W + kOffList;
+  int4 *units = reinterpret_cast<int4 *>(W + kOffUnits), *tmp = reinterpret_cast<int4 *>(W + kOffTmp);
+  int *ipts = W + kOffPts, *pass = W + kOffPass;
   int2 *bpt = reinterpret_cast<int2 *>(W + kOffBpt);
   float4 *r4 = reinterpret_cast<float4 *>(W + kOffRects);
   int *parent = W + kOffParent, *island_of = W + kOffIslandOf, *local = W + kOffLocal;
   int *root_isl = W + kOffRootIsl, *cnt = W + kOffCnt, *last = W + kOffLast;
-  int *level = W + kOffLevel, *cur = W + kOffCur;
+  int *last_unit = W + kOffLastUnit, *level = W + kOffLevel, *cur = W + kOffCur;
   W[kOffHdr + 0] = 0;
   W[kOffHdr + 2] = KR_OK;
   // collRange must tile the points in body order (gpuworld.js:193-199).  The
@@ -800,52 +805,58 @@ __global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint3
   for (int I = 0; I < nI; I++) cnt[I + 1] += cnt[I];
   for (int I = 0; I < nI; I++) cur[I] = cnt[I];
   for (int k = 0; k < nC; k++) icons[cur[island_of[cons[20 * (size_t)k]]]++] = k;
-  // levels per island, then a stable counting sort of its slots by level
-  int lvl_off = 0, pt_off = 0;
+  // units per island and their levels (each on the first level after every
+  // earlier unit sharing a body), then a stable counting sort by level; a
+  // level of more than 32 units takes several passes
+  int pass_off = 0, pt_off = 0, unit_off = 0;
   for (int I = 0; I < nI; I++) {
     int *rec = isl + I * kIslandInts;
     const int co = cnt[I], nc = cnt[I + 1] - cnt[I], bo = rec[I_BODY_OFF], nb = rec[I_NB];
     if (nc > KR_MAX_ISLAND_CONSTRAINTS) { W[kOffHdr + 2] = KR_ERR_CAPACITY; return; }
-    for (int j = 0; j < nb; j++) last[j] = -1;
-    int nlv = 0;
+    for (int j = 0; j < nb; j++) { last[j] = -1; last_unit[j] = -1; }
+    int nlv = 0, nu = 0, nul = 0;
     for (int q = 0; q < nc; q++) {
-      const uint32_t *c = cons + 20 * (size_t)icons[co + q];
+      const int k = icons[co + q];
+      const uint32_t *c = cons + 20 * (size_t)k;
       const int a = local[c[0]];
       const int b = c[1] == 0xffffffffu ? -1 : local[c[1]];
+      const bool angle = (c[2] & 0xffu) == 1u;
       int L = last[a] + 1;
       if (b >= 0) L = max(L, last[b] + 1);
-      level[q] = L;
       last[a] = L;
       if (b >= 0) last[b] = L;
       nlv = max(nlv, L + 1);
+      const int ab = a | ((b >= 0 ? b : 0xff) << 8), u = last_unit[a];
+      if (angle && u >= 0 && (b < 0 || last_unit[b] == u) && tmp[u].y >= 0 && tmp[u].z < 0 && tmp[u].x == ab) {
+        tmp[u].z = k;
+        continue;
+      }
+      int ul = u >= 0 ? level[u] + 1 : 0;
+      if (b >= 0 && last_unit[b] >= 0) ul = max(ul, level[last_unit[b]] + 1);
+      tmp[nu] = make_int4(ab, angle ? -1 : k, angle ? k : -1, 0);
+      level[nu] = ul;
+      nul = max(nul, ul + 1);
+      last_unit[a] = nu;
+      if (b >= 0) last_unit[b] = nu;
+      nu++;
     }
     if (nlv > KR_MAX_LEVELS) { W[kOffHdr + 2] = KR_ERR_CAPACITY; return; }
-    int *lv = lvl + lvl_off;
-    for (int L = 0; L <= nlv; L++) lv[L] = 0;
-    for (int q = 0; q < nc; q++) lv[level[q] + 1]++;
-    for (int L = 0; L < nlv; L++) lv[L + 1] += lv[L];
-    // stable sort of the island's slots by level; `last` is reused as the
-    // per-level cursor (nlv <= KR_MAX_LEVELS < bodies region) and `level`
-    // then holds each list position's destination slot
-    for (int L = 0; L < nlv; L++) last[L] = lv[L];
-    for (int q = 0; q < nc; q++) {
-      const int k = icons[co + q];
-      const int s = last[level[q]]++;
-      // iab holds the final slot's body pair; icons is rewritten after
-      const uint32_t *c = cons + 20 * (size_t)k;
-      const uint32_t a = (uint32_t)local[c[0]];
-      const uint32_t b = c[1] == 0xffffffffu ? 0xffffu : (uint32_t)local[c[1]];
-      iab[co + s] = (int)(a | (b << 16));
-      level[q] = s;  // destination slot of list position q
+    for (int L = 0; L <= nul; L++) cur[L] = 0;
+    for (int u = 0; u < nu; u++) cur[level[u] + 1]++;
+    int *po = pass + pass_off;
+    int np_ = 0;
+    po[0] = 0;
+    for (int L = 0; L < nul; L++) {
+      cur[L + 1] += cur[L];
+      for (int s = cur[L]; s < cur[L + 1]; s += 32) po[++np_] = min(s + 32, cur[L + 1]);
     }
-    // permute constraint ids into slot order via the `cur` tail as temp
-    for (int q = 0; q < nc; q++) cur[q] = icons[co + q];
-    for (int q = 0; q < nc; q++) icons[co + level[q]] = cur[q];
-    rec[I_CON_OFF] = co;
-    rec[I_NC] = nc;
-    rec[I_LVL_OFF] = lvl_off;
-    rec[I_NLV] = nlv;
-    lvl_off += nlv + 1;
+    for (int u = 0; u < nu; u++) units[unit_off + cur[level[u]]++] = tmp[u];
+    rec[I_UNIT_OFF] = unit_off;
+    rec[I_NU] = nu;
+    rec[I_PASS_OFF] = pass_off;
+    rec[I_NPASS] = np_;
+    unit_off += nu;
+    pass_off += np_ + 1;
     // collision points in local body order; the island's count is checked
     // against the kernel's capacity before any of its points is written
     rec[I_PT_OFF] = pt_off;
@@ -961,11 +972,11 @@ extern "C" int kr_step_noalloc(const kr_solver_params *params, uint32_t n_bodies
   A.nI = 0;
   // shared memory for the largest island the world can hold
   A.maxB = ((int)std::min<uint32_t>(n_bodies, KR_MAX_ISLAND_BODIES) + 3) & ~3;
-  A.maxC = ((int)std::min<uint32_t>(std::max<uint32_t>(n_constraints, 1), KR_MAX_ISLAND_CONSTRAINTS) + 3) & ~3;
+  A.maxU = (int)std::min<uint32_t>(std::max<uint32_t>(n_constraints, 1), KR_MAX_ISLAND_CONSTRAINTS);
   A.maxP = ((int)std::min<uint32_t>(std::max<uint32_t>(n_coll_pts, 1), KR_MAX_ISLAND_COLLPTS) + 3) & ~3;
-  A.T = DeviceTables{W + kOffIsl, W + kOffBodies, W + kOffCons, W + kOffAb, W + kOffPts,
-                     reinterpret_cast<const int2 *>(W + kOffBpt), W + kOffLvl};
-  const size_t smem = sizeof(float) * kWarpsPerBlock * (size_t)warp_smem_words(A.maxB, A.maxC, A.maxP);
+  A.T = DeviceTables{W + kOffIsl, W + kOffBodies, reinterpret_cast<const int4 *>(W + kOffUnits), W + kOffPts,
+                     reinterpret_cast<const int2 *>(W + kOffBpt), W + kOffPass};
+  const size_t smem = sizeof(float) * kWarpsPerBlock * (size_t)warp_smem_words(A.maxB, A.maxU, A.maxP);
   if (cudaFuncSetAttribute(noalloc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return KR_ERR_CUDA;

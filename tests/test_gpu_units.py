@@ -1,0 +1,114 @@
+"""The drop-in's solve units against the f32 oracle's sequential sweep, on
+worlds no creature looks like: random constraint lists with repeated and
+reversed pairs, both bodies the same, angle constraints against the world,
+pins with compliance, grips between bodies, broken flags on every type,
+immovable bodies, forces, and passes of more than 32 units.  The oracle solves
+the list constraint by constraint; the kernel solves units in passes, the same
+operations per body in the same order, so every value must be equal -- up to
+the step in which a world that tears itself apart throws a body beyond 1e6 px
+(angles then jump by more than the f32 quotient of the angle wrap covers)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from kraken_3_gpu_b200 import _native
+from oracle import binding as ob
+
+pytestmark = pytest.mark.gpu
+
+_F32P, _U32P = C.POINTER(C.c_float), C.POINTER(C.c_uint32)
+RECTS = np.array([[0, 0, 400, 14], [0, 286, 400, 14], [0, 0, 14, 300], [386, 0, 14, 300], [150, 120, 90, 18]], float)
+
+
+def _random_world(seed, nb, nc, spread):
+    r = np.random.default_rng(seed)
+    o = ob.World()
+    o.set_rects(RECTS)
+    for i in range(nb):
+        fixed = r.random() < 0.1
+        o.add_body(r.uniform(30, 30 + spread), r.uniform(30, 30 + 0.6 * spread), r.uniform(-7, 7),
+                   0 if fixed else r.uniform(1, 20), 0 if fixed and r.random() < 0.5 else r.uniform(20, 900))
+        for _ in range(int(r.integers(0, 4))):
+            o.add_collision_point(i, r.uniform(-8, 8), r.uniform(-8, 8), r.uniform(2, 7))
+    pair = (0, -1)
+    for k in range(nc):
+        if r.random() < 0.6 or k == 0:
+            a = int(r.integers(nb))
+            b = -1 if r.random() < 0.2 else int(r.integers(nb))
+            if b == a and r.random() < 0.5:
+                b = -1
+            pair = (a, b)
+        elif pair[1] >= 0 and r.random() < 0.2:
+            pair = pair[::-1]
+        a, b = pair
+        t = int(r.integers(3))
+        c = o.add_constraint(t, a, b, r.uniform(-7, 7), r.uniform(-7, 7),
+                             r.uniform(40, 200) if b < 0 else r.uniform(-7, 7),
+                             r.uniform(40, 150) if b < 0 else r.uniform(-7, 7),
+                             r.choice([0.0, 1e-6, 1e-5]))
+        c.rest, c.target = r.uniform(-3, 3), r.uniform(-1, 1)
+        c.minAngle, c.maxAngle = -r.uniform(0.1, 2), r.uniform(0.1, 2)
+        c.broken = r.random() < 0.15
+        c.breakForce = r.uniform(5, 400)
+    o.set_list(np.arange(nc))
+    o.f32ify()
+    o.round_state()
+    return o, r.uniform(-400, 400, (nb, 3)).astype(np.float32)
+
+
+def _blocks(o, force):
+    bodies = np.zeros((o.n, 12), np.float32)
+    for c, f in enumerate(("px", "py", "ppx", "ppy", "vx", "vy", "ang", "angP", "av", "im", "ii")):
+        bodies[:, c] = o.arr(f)
+    cons = np.zeros((o.nC, 20), np.float32)
+    cu = cons.view(np.uint32)
+    for k, c in enumerate(o.constraints):
+        cu[k, 0], cu[k, 1], cu[k, 2] = c.a, c.b & 0xFFFFFFFF, c.type
+        cons[k, 4:13] = (c.lax, c.lay, c.lbx, c.lby, c.compliance, c.rest, c.target, c.minAngle, c.maxAngle)
+        cons[k, 16] = c.breakForce
+        cu[k, 17] = c.broken
+    pts = np.array(o.coll_pts(), np.float32).reshape(-1, 4)
+    body = pts[:, 0].astype(np.int64)
+    order = np.argsort(body, kind="stable")
+    pts, body = np.ascontiguousarray(pts[order]), body[order]
+    pts.view(np.uint32)[:, 0] = body
+    cnt = np.bincount(body, minlength=o.n).astype(np.uint32)
+    rng = np.concatenate([np.cumsum(cnt) - cnt, cnt]).astype(np.uint32)
+    forces = np.zeros((o.n, 4), np.float32)
+    forces[:, :3] = force
+    return bodies, cons, pts, rng, forces
+
+
+@pytest.mark.parametrize("seed,nb,nc,spread", [(s, 12, 40, 160) for s in range(8)] + [(8, 2, 6, 20), (9, 1, 3, 30),
+                                                                                    (10, 90, 110, 300), (11, 5, 0, 60)])
+def test_random_lists_equal_the_sequential_oracle(seed, nb, nc, spread):
+    o, force = _random_world(seed, nb, nc, spread)
+    bodies, cons, pts, rng, forces = _blocks(o, force)
+    L = _native.lib()
+    h = C.c_void_p()
+    p = _native.SolverParams(1 / 120, 2, 4, 3.0, 3.0, 360.0, 18.0)
+    rects = RECTS.astype(np.float32)
+    _native.check(L.kr_create(C.byref(p), nb, nc, rects.ctypes.data_as(_F32P), len(rects), pts.ctypes.data_as(_U32P),
+                              len(pts), rng.ctypes.data_as(_U32P), C.byref(h)))
+    try:
+        cp = cons.ctypes.data_as(_U32P) if nc else None
+        _native.check(L.kr_upload(h, bodies.ctypes.data_as(_F32P), cp, forces.ctypes.data_as(_F32P), None), h)
+        for f, k in (("fx", 0), ("fy", 1), ("tq", 2)):
+            o.arr(f)[:] = force[:, k]
+        for s in range(12):
+            _native.check(L.kr_step(h, 1), h)
+            _native.check(L.kr_download(h, bodies.ctypes.data_as(_F32P), cp), h)
+            o.step32()
+            if np.abs(o.arr("px")).max() > 1e6 or np.abs(o.arr("py")).max() > 1e6:
+                assert s >= 2
+                break
+            for c, f in ((0, "px"), (1, "py"), (4, "vx"), (5, "vy"), (6, "ang"), (8, "av")):
+                assert np.array_equal(bodies[:, c], o.arr(f).astype(np.float32)), (s, f)
+            for k, c in enumerate(o.constraints):
+                lam = (cons[k, 15],) if c.type == 1 else (cons[k, 13], cons[k, 14])
+                ref = (getattr(c, "lambda"),) if c.type == 1 else (c.lambdaX, c.lambdaY)
+                assert tuple(np.float32(v) for v in ref) == tuple(lam), (s, k)
+                assert bool(cons.view(np.uint32)[k, 17]) == c.broken, (s, k)
+    finally:
+        L.kr_destroy(h)
