@@ -95,15 +95,15 @@ __host__ __device__ inline int tpl_smem_words(int npass, int G, int nb, int np) 
 // one creature: the committed state and the predicted state (16-byte records;
 // the velocity lives in the predicted state's records between substeps), the
 // arms' anchors after the bodies, per motor {target, lambda}, per arm {lambda,
-// break force}, controls, collision scratch.  The proprioception's vector
+// break force}, controls, the near lists of the collision pass.  The proprioception's vector
 // shares the motors' words: it is read before the targets are written.
 __host__ __device__ inline int mot_words(int arms, int segs) {
   const int m = 2 * arms * segs, o = 6 * arms + 6;
   return r4(m > o ? m : o);
 }
-__host__ __device__ inline int creature_smem_words(int nb, int np, int arms, int segs) {
-  return 4 * nb + 4 * (nb + arms) + mot_words(arms, segs) + 4 * arms + r4(arms * segs + arms) + 2 * r4(nb) +
-         3 * r4(np) + kr::kMaxCulled / 2;
+__host__ __device__ inline int creature_smem_words(int nb, int arms, int segs) {
+  return 4 * nb + 4 * (nb + arms) + mot_words(arms, segs) + 4 * arms + r4(arms * segs + arms) +
+         kr::kMaxCulled / 2 + r4((nb + 3) / 4);
 }
 
 struct TplSmem {
@@ -127,7 +127,7 @@ struct CreatureSmem {
 
 __device__ inline void carve_creature(kr::Island &S, CreatureSmem &X, const TplSmem &P, float *p,
                                       const TplDev &td, int npass) {
-  const int mb = r4(td.nb), mp = r4(td.np), AS = td.arms * td.segs;
+  const int AS = td.arms * td.segs;
   // committed state, resident for the creature's whole run
   S.P = reinterpret_cast<float4 *>(p); p += 4 * td.nb;
   S.Q = reinterpret_cast<float4 *>(p); p += 4 * (td.nb + td.arms);
@@ -136,13 +136,11 @@ __device__ inline void carve_creature(kr::Island &S, CreatureSmem &X, const TplS
   X.obs = p; p += mot_words(td.arms, td.segs);
   S.grip = reinterpret_cast<float4 *>(p); p += 4 * td.arms;
   X.ctrl = p; p += r4(AS + td.arms);
-  S.bs = p; p += mb; S.bc = p; p += mb;
-  S.pdx = p; p += mp; S.pdy = p; p += mp;
-  S.pflag = reinterpret_cast<int *>(p); p += mp;
-  S.cull = reinterpret_cast<short *>(p);
+  S.cull = reinterpret_cast<unsigned short *>(p); p += kr::kMaxCulled / 2;
+  S.list = reinterpret_cast<unsigned char *>(p);
   // statics shared by the CTA
   S.recs = P.recs; S.body = P.body; S.pts = P.pts;
-  S.nb = td.nb; S.np = td.np; S.npass = npass; S.arms = td.arms;
+  S.nb = td.nb; S.npass = npass; S.arms = td.arms;
 }
 
 // mulberry32 (src/world/map.js:11-20): the draw is a hash of the state, and
@@ -653,7 +651,8 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
   L.sync();
   const float4 *rects = A.rects + A.map_off[m.map];
   const int nR = A.map_off[m.map + 1] - A.map_off[m.map];
-  const float cull_d = fmaxf(A.map_cull[m.map], td.r_max + 2.f + kr::kCullSlack + 1.f);
+  const float near_d = fmaxf(A.map_cull[m.map], td.r_max + 2.f + kr::kCullPad);
+  kr::Near near;
   int halt_next = 0;  // the stop word as loaded during the previous step
   for (int s = 0; s < steps; s++) {
     if (A.stop) {
@@ -727,7 +726,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
     }
     L.sync();
     // 4. the XPBD step
-    kr::island_step<false, G, U>(A.K, S, rects, nR, cull_d, L, td.off_max + 1.f);
+    kr::island_step<false, G, U>(A.K, S, rects, nR, near_d, L, near);
     // 5. postStep, core.js:297-356 (f64 on the f32 state, as the
     //    reference's hybrid loop runs it on the mirrored state)
     //    The accumulators are read and written through the slot's HBM
@@ -844,7 +843,7 @@ __global__ void __launch_bounds__(32 * kMaxW, 1) batch_kernel(BatchArgs A) {
     const int slot = c < A.cpc ? A.groups[g * A.cpc + c] : -1;
     if (slot >= 0) {
       float *base = smem + tpl_smem_words(npass, G, td.nb, td.np) +
-                    c * creature_smem_words(td.nb, td.np, td.arms, td.segs);
+                    c * creature_smem_words(td.nb, td.arms, td.segs);
       run_creature<G, NET, U>(A, td, npass, P, base, slot, L);
     }
   }
@@ -1011,7 +1010,7 @@ int upload_templates(kr_batch *b) {
   for (const auto &t : b->tpls) {
     TplDev d{};
     d.nb = t.nb; d.nc = t.nc; d.np = t.np; d.arms = t.arms; d.segs = t.segs;
-    d.r_max = t.r_max; d.off_max = t.off_max; d.reach = t.reach;
+    d.r_max = t.r_max; d.reach = t.reach;
     d.o_b = (int)body.size(); d.o_p = (int)pts.size(); d.o_a = (int)tip.size(); d.o_s = (int)segs.size();
     for (int i = 0; i < t.nb; i++)
       body.push_back(make_float4(t.im[i], t.ii[i], t.breach[i], word(t.boff[i] | (t.bcnt[i] << 16))));
@@ -1059,7 +1058,7 @@ int plan_shape(kr_batch *b) {
   for (size_t t = 0; t < b->h_tpl.size(); t++) {
     const TplDev &d = b->h_tpl[t];
     const long tw = tpl_smem_words(d.npass[kr::schedule_index(b->G)], b->G, d.nb, d.np);
-    const long cw = creature_smem_words(d.nb, d.np, d.arms, d.segs);
+    const long cw = creature_smem_words(d.nb, d.arms, d.segs);
     const long fit = (words - tw) / cw;
     if (fit < 1)
       return b->fail(KR_ERR_CAPACITY, "body " + std::to_string(d.arms) + "x" + std::to_string(d.segs) +
@@ -1613,7 +1612,7 @@ extern "C" int kr_batch_create(const kr_batch_desc *desc, kr_batch **out) {
       const double t = 0.5 * std::min(std::fabs((double)w), std::fabs((double)h));
       ht = std::isfinite(t) ? std::max(ht, t) : HUGE_VAL;
     }
-    const double c = ht + 2.0 + kr::kCullSlack + 1.0;
+    const double c = ht + 2.0 + kr::kCullPad;
     b->h_map_cull[m] = std::isfinite(c) && c < 1e30 ? (float)c : 1e30f;
   }
   b->h_rects.assign(d.rects, d.rects + 4 * (size_t)n_rects);

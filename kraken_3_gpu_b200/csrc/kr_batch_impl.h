@@ -29,7 +29,6 @@ struct TplDev {
   int nb, nc, np, arms, segs;
   int npass[kr::kSchedules];
   float r_max;
-  float off_max;   // largest distance of a collision point from its body's centre
   double reach;
   int o_b, o_p, o_a, o_s;     // bodies, collision points, arms, arm segments
   int o_r[kr::kSchedules];    // unit records, in float4

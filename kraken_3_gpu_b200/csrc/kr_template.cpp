@@ -196,7 +196,6 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
     t->pbody[q] = pbody[p];
     t->r_max = std::max(t->r_max, (float)pr[p]);
     const double off = std::sqrt((double)t->plx[q] * t->plx[q] + (double)t->ply[q] * t->ply[q]);
-    t->off_max = std::max(t->off_max, (float)off);
     t->breach[pbody[p]] = std::max(t->breach[pbody[p]], (float)off + 1.f);
   }
   return true;

@@ -37,7 +37,7 @@ thread_local std::string g_last_error;
 constexpr int kWarpsPerBlock = 4;
 
 // Per-island record, one int array of kIslandInts per island.
-enum { I_BODY_OFF = 0, I_NB, I_UNIT_OFF, I_NU, I_PT_OFF, I_NP, I_PASS_OFF, I_NPASS, kIslandInts };
+enum { I_BODY_OFF = 0, I_NB, I_UNIT_OFF, I_NU, I_PT_OFF, I_PASS_OFF, I_NPASS, kIslandInts };
 
 struct DeviceTables {
   const int *isl;          // nI x kIslandInts
@@ -57,15 +57,14 @@ struct StepArgs {
   const uint4 *coll;       // nP x 4 words
   const float4 *rects;     // nR x (x, y, x+w, y+h)
   int nR;
-  float cull_d;            // rect culling distance of a collision pass
-  float reach;             // bound on a collision point's distance from its body (+1 px), < 0: none
+  float near_d;            // rect culling distance of a collision pass (kr_solver.cuh)
   int nI;
   int maxB, maxU, maxP;    // smem carve sizes (per warp)
   DeviceTables T;
 };
 
 __host__ __device__ inline int warp_smem_words(int mb, int mu, int mp) {
-  return 22 * mb + 16 * mu + 7 * mp + kr::kMaxCulled / 2;
+  return 20 * mb + 16 * mu + 4 * mp + kr::kMaxCulled / 2 + mb;
 }
 
 // Writable views of the statics while they are staged; the solver reads them
@@ -80,11 +79,8 @@ __device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, i
   V.body = q; q += mb;
   S.units = q; q += 4 * mu;
   V.pts = q; q += mp;
-  float *p = reinterpret_cast<float *>(q);
-  S.bs = p; p += mb; S.bc = p; p += mb;
-  S.pdx = p; p += mp; S.pdy = p; p += mp;
-  S.pflag = reinterpret_cast<int *>(p); p += mp;
-  S.cull = reinterpret_cast<short *>(p);
+  S.cull = reinterpret_cast<unsigned short *>(q); q += kr::kMaxCulled / 8;
+  S.list = reinterpret_cast<unsigned char *>(q);
   S.body = V.body; S.pts = V.pts;
 }
 
@@ -100,7 +96,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   carve(S, V, smem + warp * warp_smem_words(A.maxB, A.maxU, A.maxP), A.maxB, A.maxU, A.maxP);
   const int *rec = A.T.isl + island * kIslandInts;
   const int bo = rec[I_BODY_OFF], uo = rec[I_UNIT_OFF], po = rec[I_PT_OFF];
-  S.nb = rec[I_NB]; S.nu = rec[I_NU]; S.np = rec[I_NP];
+  S.nb = rec[I_NB]; S.nu = rec[I_NU];
   S.npass = rec[I_NPASS];
   S.off = A.T.pass + rec[I_PASS_OFF];
 
@@ -114,12 +110,15 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
     S.V[i] = make_float4(q1.x, q1.y, q2.x, 0.f);
     S.force[i] = reinterpret_cast<const float4 *>(A.forces)[g];
     const int2 bp = A.T.bpt[bo + i];
-    V.body[i] = make_float4(q2.y, q2.z, 0.f, __int_as_float(bp.x | (bp.y << 16)));
+    float reach = 0.f;  // every point lies within it of the centre (+1 px for rounding)
     for (int q = 0; q < bp.y; q++) {
       const uint4 cp = A.coll[A.T.pts[po + bp.x + q]];
-      V.pts[bp.x + q] = make_float4(__uint_as_float(cp.y), __uint_as_float(cp.z), __uint_as_float(cp.w),
-                                    __int_as_float(i));
+      const float lx = __uint_as_float(cp.y), ly = __uint_as_float(cp.z);
+      V.pts[bp.x + q] = make_float4(lx, ly, __uint_as_float(cp.w), __int_as_float(i));
+      const float d = kr::length2(lx, ly) + 1.f;
+      if (!(d <= reach)) reach = d;  // NaN stays: such a body is tested against every rect
     }
+    V.body[i] = make_float4(q2.y, q2.z, reach, __int_as_float(bp.x | (bp.y << 16)));
   }
   // stage the units' constraints (80 B AoS -> unit records)
   for (int u = lane; u < S.nu; u += 32) {
@@ -147,7 +146,8 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   }
   __syncwarp();
 
-  kr::island_step<true, 32>(A.K, S, A.rects, A.nR, A.cull_d, kr::Lanes<32>(lane), A.reach);
+  kr::Near near;
+  kr::island_step<true, 32>(A.K, S, A.rects, A.nR, A.near_d, kr::Lanes<32>(lane), near);
 
   // write back bodies, consumed forces and constraint multipliers / flags
   for (int i = lane; i < S.nb; i += 32) {
@@ -223,9 +223,7 @@ struct kr_world {
   int4 *d_units = nullptr;
   int2 *d_bpt = nullptr;
   size_t c_isl = 0, c_ibodies = 0, c_units = 0, c_ipts = 0, c_pass = 0, c_bpt = 0;
-  float max_half_thick = 0.f;  // largest min(w, h) / 2 of the map's rects
-  float cull_d = 0.f;
-  float reach = -1.f;          // largest collision-point offset + 1 px (kr_solver.cuh collide_bodies)
+  float near_d = 0.f;
   int nI = 0, maxB = 1, maxU = 1, maxP = 1, maxLv = 0;
   bool uploaded = false;
   cudaStream_t stream = nullptr;
@@ -369,25 +367,16 @@ extern "C" int kr_create(const kr_solver_params *params, uint32_t n_bodies, uint
     if (std::isfinite(ht)) half_thick = std::max(half_thick, ht);
     else half_thick = HUGE_VAL;
   }
-  double off_max = 0.0;
   for (uint32_t i = 0; i < n_coll_pts; i++) {
-    float r, lx, ly;
-    std::memcpy(&lx, &coll_pts[4 * i + 1], sizeof(float));
-    std::memcpy(&ly, &coll_pts[4 * i + 2], sizeof(float));
+    float r;
     std::memcpy(&r, &coll_pts[4 * i + 3], sizeof(float));
     if (std::isfinite(r)) r_max = std::max(r_max, std::fabs((double)r));
     else r_max = HUGE_VAL;
-    const double off = std::sqrt((double)lx * lx + (double)ly * ly);
-    off_max = std::isfinite(off) ? std::max(off_max, off) : HUGE_VAL;
   }
-  // every collision point lies within off_max of its body's centre: the
-  // collision pass may skip bodies with no rect nearby (collide_bodies)
-  w->reach = off_max < 1e5 ? (float)off_max + 1.f : -1.f;
-  // D = max(radius, half thickness) + 2, plus the slack of the culling box;
-  // the f32 rounding of the box test is covered by the +1
-  const double cull = std::max(r_max, half_thick) + 2.0 + kr::kCullSlack + 1.0;
-  w->cull_d = std::isfinite(cull) && cull < 1e30 ? (float)cull : 1e30f;
-  w->max_half_thick = (float)std::min(half_thick, 1e30);
+  // D = max(radius, half thickness) + 2; the f32 rounding of the box tests is
+  // covered by the pad
+  const double cull = std::max(r_max, half_thick) + 2.0 + kr::kCullPad;
+  w->near_d = std::isfinite(cull) && cull < 1e30 ? (float)cull : 1e30f;
   if ((e = cudaMalloc(&w->d_rects, sizeof(float4) * n_rects)) != cudaSuccess)
     return cleanup_fail(e, "cudaMalloc(rects)");
   if ((e = cudaMemcpy(w->d_rects, r4.data(), sizeof(float4) * n_rects, cudaMemcpyHostToDevice)) !=
@@ -515,7 +504,6 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
       return w->fail(KR_ERR_CAPACITY, "connected component " + std::to_string(I) + " has " +
                                           std::to_string(np) + " collision points; the kernel holds " +
                                           std::to_string(KR_MAX_ISLAND_COLLPTS));
-    rec[I_NP] = np;
     maxB = std::max(maxB, nb);
     maxU = std::max(maxU, (int)units.size());
     maxP = std::max(maxP, np);
@@ -624,8 +612,7 @@ extern "C" int kr_step(kr_world *w, int32_t n_steps) {
   A.nI = w->nI;
   A.maxB = w->maxB; A.maxU = w->maxU; A.maxP = w->maxP;
   A.T = DeviceTables{w->d_isl, w->d_ibodies, w->d_units, w->d_ipts, w->d_bpt, w->d_pass};
-  A.cull_d = w->cull_d;
-  A.reach = w->reach;
+  A.near_d = w->near_d;
   const size_t smem = w->smem_bytes;
   cudaError_t e;
   const int grid = (w->nI + kWarpsPerBlock - 1) / kWarpsPerBlock;
@@ -716,7 +703,7 @@ constexpr int kNaC = KR_NOALLOC_MAX_CONSTRAINTS;
 constexpr int kNaP = KR_NOALLOC_MAX_COLLPTS;
 constexpr int kNaR = KR_NOALLOC_MAX_RECTS;
 // region offsets in words
-constexpr int kOffHdr = 0;                                  // n_islands, cull_d, status, pad
+constexpr int kOffHdr = 0;                                  // n_islands, near_d, status, pad
 constexpr int kOffIsl = 4;
 constexpr int kOffBodies = kOffIsl + kNaB * kIslandInts;
 constexpr int kOffUnits = (kOffBodies + kNaB + 3) & ~3;    // int4, 16-byte aligned
@@ -871,7 +858,6 @@ __global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint3
       for (uint32_t q = 0; q < cn; q++) ipts[pt_off + np + (int)q] = (int)(off + q);
       np += (int)cn;
     }
-    rec[I_NP] = np;
     pt_off += np;
   }
   // rects and the culling distance, as kr_create derives them
@@ -886,7 +872,7 @@ __global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint3
     const float r = __uint_as_float(coll_pts[4 * i + 3]);
     r_max = isfinite(r) ? fmax(r_max, fabs((double)r)) : HUGE_VAL;
   }
-  const double cull = fmax(r_max, half_thick) + 2.0 + kr::kCullSlack + 1.0;
+  const double cull = fmax(r_max, half_thick) + 2.0 + kr::kCullPad;
   reinterpret_cast<float *>(W)[kOffHdr + 1] = (isfinite(cull) && cull < 1e30) ? (float)cull : 1e30f;
   W[kOffHdr + 0] = nI;
 }
@@ -894,7 +880,7 @@ __global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint3
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) noalloc_step_kernel(StepArgs A, const int *W) {
   StepArgs B = A;
   B.nI = W[kOffHdr + 0];
-  B.cull_d = reinterpret_cast<const float *>(W)[kOffHdr + 1];
+  B.near_d = reinterpret_cast<const float *>(W)[kOffHdr + 1];
   if (W[kOffHdr + 2] != KR_OK) return;
   plain_step_body(B);
 }
@@ -967,8 +953,7 @@ extern "C" int kr_step_noalloc(const kr_solver_params *params, uint32_t n_bodies
   A.coll = reinterpret_cast<const uint4 *>(coll_pts);
   A.rects = reinterpret_cast<const float4 *>(W + kOffRects);
   A.nR = (int)n_rects;
-  A.cull_d = 0.f;
-  A.reach = -1.f;
+  A.near_d = 0.f;
   A.nI = 0;
   // shared memory for the largest island the world can hold
   A.maxB = ((int)std::min<uint32_t>(n_bodies, KR_MAX_ISLAND_BODIES) + 3) & ~3;

@@ -21,13 +21,13 @@ _F32P, _U32P = C.POINTER(C.c_float), C.POINTER(C.c_uint32)
 RECTS = np.array([[0, 0, 400, 14], [0, 286, 400, 14], [0, 0, 14, 300], [386, 0, 14, 300], [150, 120, 90, 18]], float)
 
 
-def _random_world(seed, nb, nc, spread):
+def _random_world(seed, nb, nc, spread, rects=RECTS, offset=0.0):
     r = np.random.default_rng(seed)
     o = ob.World()
-    o.set_rects(RECTS)
+    o.set_rects(rects)
     for i in range(nb):
         fixed = r.random() < 0.1
-        o.add_body(r.uniform(30, 30 + spread), r.uniform(30, 30 + 0.6 * spread), r.uniform(-7, 7),
+        o.add_body(offset + r.uniform(30, 30 + spread), offset + r.uniform(30, 30 + 0.6 * spread), r.uniform(-7, 7),
                    0 if fixed else r.uniform(1, 20), 0 if fixed and r.random() < 0.5 else r.uniform(20, 900))
         for _ in range(int(r.integers(0, 4))):
             o.add_collision_point(i, r.uniform(-8, 8), r.uniform(-8, 8), r.uniform(2, 7))
@@ -44,8 +44,8 @@ def _random_world(seed, nb, nc, spread):
         a, b = pair
         t = int(r.integers(3))
         c = o.add_constraint(t, a, b, r.uniform(-7, 7), r.uniform(-7, 7),
-                             r.uniform(40, 200) if b < 0 else r.uniform(-7, 7),
-                             r.uniform(40, 150) if b < 0 else r.uniform(-7, 7),
+                             offset + r.uniform(40, 200) if b < 0 else r.uniform(-7, 7),
+                             offset + r.uniform(40, 150) if b < 0 else r.uniform(-7, 7),
                              r.choice([0.0, 1e-6, 1e-5]))
         c.rest, c.target = r.uniform(-3, 3), r.uniform(-1, 1)
         c.minAngle, c.maxAngle = -r.uniform(0.1, 2), r.uniform(0.1, 2)
@@ -80,17 +80,16 @@ def _blocks(o, force):
     return bodies, cons, pts, rng, forces
 
 
-@pytest.mark.parametrize("seed,nb,nc,spread", [(s, 12, 40, 160) for s in range(8)] + [(8, 2, 6, 20), (9, 1, 3, 30),
-                                                                                    (10, 90, 110, 300), (11, 5, 0, 60)])
-def test_random_lists_equal_the_sequential_oracle(seed, nb, nc, spread):
-    o, force = _random_world(seed, nb, nc, spread)
+def _run(seed, nb, nc, spread, rects=RECTS, offset=0.0):
+    o, force = _random_world(seed, nb, nc, spread, rects, offset)
     bodies, cons, pts, rng, forces = _blocks(o, force)
     L = _native.lib()
     h = C.c_void_p()
     p = _native.SolverParams(1 / 120, 2, 4, 3.0, 3.0, 360.0, 18.0)
-    rects = RECTS.astype(np.float32)
-    _native.check(L.kr_create(C.byref(p), nb, nc, rects.ctypes.data_as(_F32P), len(rects), pts.ctypes.data_as(_U32P),
+    r32 = rects.astype(np.float32)
+    _native.check(L.kr_create(C.byref(p), nb, nc, r32.ctypes.data_as(_F32P), len(r32), pts.ctypes.data_as(_U32P),
                               len(pts), rng.ctypes.data_as(_U32P), C.byref(h)))
+    hits = 0
     try:
         cp = cons.ctypes.data_as(_U32P) if nc else None
         _native.check(L.kr_upload(h, bodies.ctypes.data_as(_F32P), cp, forces.ctypes.data_as(_F32P), None), h)
@@ -100,6 +99,7 @@ def test_random_lists_equal_the_sequential_oracle(seed, nb, nc, spread):
             _native.check(L.kr_step(h, 1), h)
             _native.check(L.kr_download(h, bodies.ctypes.data_as(_F32P), cp), h)
             o.step32()
+            hits += o.stats["collisions"]
             if np.abs(o.arr("px")).max() > 1e6 or np.abs(o.arr("py")).max() > 1e6:
                 assert s >= 2
                 break
@@ -112,3 +112,33 @@ def test_random_lists_equal_the_sequential_oracle(seed, nb, nc, spread):
                 assert bool(cons.view(np.uint32)[k, 17]) == c.broken, (s, k)
     finally:
         L.kr_destroy(h)
+    return hits
+
+
+@pytest.mark.parametrize("seed,nb,nc,spread", [(s, 12, 40, 160) for s in range(8)] + [(8, 2, 6, 20), (9, 1, 3, 30),
+                                                                                    (10, 90, 110, 300), (11, 5, 0, 60)])
+def test_random_lists_equal_the_sequential_oracle(seed, nb, nc, spread):
+    _run(seed, nb, nc, spread)
+
+
+def _clutter(n, seed):
+    """The walls and n small rects among the bodies."""
+    r = np.random.default_rng(seed)
+    return np.concatenate([RECTS, np.stack([r.uniform(20, 260, n), r.uniform(20, 200, n), r.uniform(4, 30, n),
+                                            r.uniform(4, 30, n)], 1)])
+
+
+@pytest.mark.parametrize("n,offset", [(0, 0.0), (12, 0.0), (40, 0.0), (58, 0.0), (59, 0.0), (60, 0.0), (200, 0.0),
+                                      (70000, 0.0), (12, 31900.0), (12, 40000.0)])
+def test_near_rects_equal_the_full_list(n, offset):
+    """Collision passes over the near sets (one rect or two per mask bit), and
+    over every rect where a creature has more than 64 near it, coordinates
+    outside the references' range or the map more than 65,535 rects: the
+    oracle folds over every rect each time."""
+    rects = _clutter(min(n, 200), n)
+    if n > 200:  # the rest far away, the near ones last
+        far = np.tile([1e5, 1e5, 20.0, 20.0], (n - 200, 1))
+        rects = np.concatenate([far, rects])
+    rects = rects + np.array([offset, offset, 0, 0])
+    for seed in range(2 if n > 200 else 4):
+        _run(100 + seed, 14, 10, 200, rects, offset)
