@@ -142,3 +142,44 @@ def test_near_rects_equal_the_full_list(n, offset):
     rects = rects + np.array([offset, offset, 0, 0])
     for seed in range(2 if n > 200 else 4):
         _run(100 + seed, 14, 10, 200, rects, offset)
+
+
+def test_angle_wrap_edges():
+    """Pairs of bodies whose angle differences lie at the edges of the wrap:
+    multiples of pi / 2 up to 8 pi, and where the near form ends, within a few
+    ulp and on both sides."""
+    o = ob.World()
+    o.set_rects(RECTS)
+    r = np.random.default_rng(3)
+    edges = [k * np.pi / 2 for k in range(-16, 17)] + [9.42, -9.42, 4.0, -4.0, 49.9, -49.9]
+    k = 0
+    for e in edges:
+        for d in (0.0, 3e-7, -3e-7, 2e-4, -2e-4, r.uniform(-0.3, 0.3)):
+            for base in (0.0, r.uniform(-6, 6)):
+                x, y = 20.0 + 5 * (k % 70), 20.0 + 5 * (k // 70)
+                a = o.add_body(x, y, base, 2.0, 60.0)
+                b = o.add_body(x, y, base + e + d, 3.0, 90.0)
+                c = o.add_constraint(1, a, b, 0, 0, 0, 0, 1e-6 if k % 3 else 0.0)
+                c.rest, c.target = (0.0, 0.0) if k % 2 else (r.uniform(0, 6.3), r.uniform(-1.9, 1.9))
+                c.minAngle, c.maxAngle = -1.3, 1.3
+                k += 1
+    o.set_list(np.arange(o.nC))
+    o.f32ify()
+    o.round_state()
+    bodies, cons, pts, rng, forces = _blocks(o, np.zeros((o.n, 3), np.float32))
+    L = _native.lib()
+    h = C.c_void_p()
+    p = _native.SolverParams(1 / 120, 2, 4, 3.0, 3.0, 360.0, 18.0)
+    r32 = RECTS.astype(np.float32)
+    _native.check(L.kr_create(C.byref(p), o.n, o.nC, r32.ctypes.data_as(_F32P), len(r32), None, 0, None, C.byref(h)))
+    try:
+        cp = cons.ctypes.data_as(_U32P)
+        _native.check(L.kr_upload(h, bodies.ctypes.data_as(_F32P), cp, None, None), h)
+        for s in range(4):
+            _native.check(L.kr_step(h, 1), h)
+            _native.check(L.kr_download(h, bodies.ctypes.data_as(_F32P), cp), h)
+            o.step32()
+            assert np.array_equal(bodies[:, 6], o.arr("ang").astype(np.float32)), s
+            assert np.array_equal(bodies[:, 8], o.arr("av").astype(np.float32)), s
+    finally:
+        L.kr_destroy(h)
