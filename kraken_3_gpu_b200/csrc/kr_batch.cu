@@ -642,7 +642,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
   if (lane < arms) {
     const float4 g = gst[lane];
     const float2 gl = glam[lane];
-    S.Q[td.nb + lane] = make_float4(g.x, g.y, 0.f, g.w);  // the anchor's record: x, y, angle 0, broken
+    S.Q[td.nb + lane] = make_float4(g.x, g.y, 1.f, g.w);  // the anchor's record: x, y, angle, broken
     S.grip[lane] = make_float4(gl.x, gl.y, g.z, 0.f);
     cd = cdp[lane].x;
   }
@@ -710,7 +710,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
             const double brk = 40.0 + 860.0 * adh;
             cdp[a].y = brk;
             an = make_float4((float)((double)tp.x + kSegHalf * lib_cos(ta)),
-                             (float)((double)tp.y + kSegHalf * lib_sin(ta)), 0.f, 0.f);
+                             (float)((double)tp.y + kSegHalf * lib_sin(ta)), 1.f, 0.f);
             gr = make_float4(0.f, 0.f, (float)brk, 0.f);
           } else {
             c = A.cooldown;

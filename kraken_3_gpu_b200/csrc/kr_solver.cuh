@@ -14,6 +14,8 @@
 #pragma once
 #include <cstdint>
 
+#include "kr_sincos_tab.h"
+
 namespace kr {
 
 // solver.wgsl:81, 93-94 and f32solver.mjs:26-33, as f32
@@ -126,14 +128,9 @@ static __device__ __noinline__ float2 sincos_far(double x) {
   return make_float2(static_cast<float>(sd), static_cast<float>(cd));
 }
 
-__device__ __forceinline__ void sincos_r(float a, float *s, float *c) {
+static __device__ __noinline__ float2 sincos_f64(float a) {
   const double x = static_cast<double>(a);
-  if (!(fabs(x) <= 1048576.0)) {
-    const float2 f = sincos_far(x);
-    *s = f.x;
-    *c = f.y;
-    return;
-  }
+  if (!(fabs(x) <= 1048576.0)) return sincos_far(x);
   // x = k pi/32 + r, |r| <= pi/64: pi/32 in three parts (29, 29 and 53
   // bits), so k p1 and k p2 are exact for |k| < 2^24
   const double k = rint(x * 10.185916357881302);  // 32/pi
@@ -155,8 +152,66 @@ __device__ __forceinline__ void sincos_r(float a, float *s, float *c) {
   // sin(t + r) = S + (S (cos r - 1) + C sin r), cos(t + r) = C + (C (cos r - 1) - S sin r):
   // the table value plus a small correction
   const double2 t = __ldg(&kSinCosTab[static_cast<int>(static_cast<long long>(k) & 63)]);
-  *s = static_cast<float>(t.x + fma(t.x, cm1, t.y * sr));
-  *c = static_cast<float>(t.y + fma(t.y, cm1, -(t.x * sr)));
+  return make_float2(static_cast<float>(t.x + fma(t.x, cm1, t.y * sr)),
+                     static_cast<float>(t.y + fma(t.y, cm1, -(t.x * sr))));
+}
+
+// The same values in f32 arithmetic (Ziv's rounding test): sin and cos as an
+// unevaluated sum h + l of two f32 whose error bound err is known; where
+// h + (l - err) and h + (l + err) round to one f32, that is the rounding of
+// the exact value and of the f64 value above, whose own error err includes.
+// Returns false where they do not (about one value in 3,000) or |a| > 64:
+// sincos_f64 decides.  The f64 chain cost 241 cycles, mostly conversions
+// (18 cycles each) and the serial reduction and series.
+//
+// a = k pi/256 + r1 + rl: p1 = pi/256 to 24 bits, so r1 = a - k p1 is exact
+// (a multiple of 2^-31 below 2^-7.3, or a itself for k = 0), and rl = -k p2
+// with |rl| < 2^-18.6.  With the table's S + Sl, C + Cl, r = r1 + rl, m =
+// cos r - 1 and n = rl - r^3 / 6:
+//   sin = S + C r1 + (Sl + Cl r1 + C n + S m),
+//   cos = C - S r1 + (Cl - Sl r1 - S n + C m),
+// S + C r1 and its two rounding errors exact (the product by fma, the sum
+// because |S| is 0 or above |C r1|).  Error: r^2 (|m| <= r^2 / 2) times
+// below 12 units of 2^-24 for the roundings of r, r^2, m and the two sums
+// it enters, Sl m among them; below 2^-40 for the roundings of rl, n, its
+// sum and p2 (2^-42.6 each), r^5 / 120 (2^-43.7), Cl n (2^-43.6) and the f64
+// value (2^-51).
+__device__ __forceinline__ bool sincos_near(float a, float *s, float *c) {
+  const float t = fmaf(a, 0x1.45f306p6f, 12582912.f);  // 256/pi; the sum's low bits hold k
+  const float4 T = __ldg(&kSinCosNear[__float_as_int(t) & 511]);
+  const float k = fsub(t, 12582912.f);
+  const float r1 = fmaf(-k, 0x1.921fb6p-7f, a), rl = fmul(-k, -0x1.777a5cp-32f);
+  const float r = fadd(r1, rl), rr = fmul(r, r);
+  const float n = fmaf(fmul(r, rr), -1.f / 6, rl);
+  const float m = fmul(rr, fmaf(rr, 1.f / 24, -0.5f));
+  const float err = fmaf(rr, 0x1.8p-22f, 0x1p-40f);
+  const float qs = fmul(T.z, r1), hs = fadd(T.x, qs);
+  const float ls = fadd(fmaf(T.x, m, fmaf(T.z, n, fmaf(T.w, r1, T.y))),
+                        fadd(fmaf(T.z, r1, -qs), fsub(qs, fsub(hs, T.x))));
+  const float qc = fmul(-T.x, r1), hc = fadd(T.z, qc);
+  const float lc = fadd(fmaf(T.z, m, fmaf(-T.x, n, fmaf(-T.y, r1, T.w))),
+                        fadd(fmaf(-T.x, r1, -qc), fsub(qc, fsub(hc, T.z))));
+  *s = fadd(hs, fadd(ls, err));
+  *c = fadd(hc, fadd(lc, err));
+  return fabsf(a) <= 64.f && *s == fadd(hs, fsub(ls, err)) && *c == fadd(hc, fsub(lc, err));
+}
+
+__device__ __forceinline__ void sincos_r(float a, float *s, float *c) {
+  if (!sincos_near(a, s, c)) {
+    const float2 f = sincos_f64(a);
+    *s = f.x;
+    *c = f.y;
+  }
+}
+
+// sincos_r of two angles: their chains run side by side
+__device__ __forceinline__ void sincos2_r(float a, float b, float *sa, float *ca, float *sb, float *cb) {
+  const bool oa = sincos_near(a, sa, ca), ob = sincos_near(b, sb, cb);
+  if (!(oa && ob)) {
+    const float2 f = sincos_f64(a), g = sincos_f64(b);
+    *sa = f.x; *ca = f.y;
+    *sb = g.x; *cb = g.y;
+  }
 }
 
 // trunc(x / TAU) exactly, as the f64 quotient of f32solver.mjs:38 gives it.
@@ -399,14 +454,14 @@ __device__ __forceinline__ void integrate_body(const SolverConsts &K, Island &S,
 
 // solvePinF, f32solver.mjs:203-256 (solver.wgsl:225-290) on two body records
 // in registers; grips are pins against the world.  Without a body B: b holds
-// the anchor as its position with angle 0, lb and the masses of B are 0 (the
-// same values as the reference's branch).  lx, ly: the multiplier, updated.
+// the anchor as its position with angle 1 (any angle with positive sine and
+// cosine), lb and the masses of B are 0 (the same values as the reference's
+// branch).  lx, ly: the multiplier, updated.
 __device__ __forceinline__ void pin_math(float lax, float lay, float lbx, float lby, float wA, float wIA, float wB,
                                          float wIB, float alphaTilde, bool hasB, float4 &a, float4 &b, float &lx,
                                          float &ly) {
   float sa, ca, sb, cb;
-  sincos_r(a.z, &sa, &ca);
-  sincos_r(b.z, &sb, &cb);
+  sincos2_r(a.z, b.z, &sa, &ca, &sb, &cb);
   const float rax = fsub(fmul(lax, ca), fmul(lay, sa)), ray = fadd(fmul(lax, sa), fmul(lay, ca));
   const float rbx = fsub(fmul(lbx, cb), fmul(lby, sb)), rby = fadd(fmul(lbx, sb), fmul(lby, cb));
   const float Cx = fsub(fadd(a.x, rax), fadd(b.x, rbx)), Cy = fsub(fadd(a.y, ray), fadd(b.y, rby));
@@ -564,7 +619,7 @@ __device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bo
         float4 r1 = rec[1];
         if (first) r1.z = r1.w = 0.f;
         if (!(ab & kPinBroken)) {
-          float4 anchor = make_float4(r0.w, r1.x, 0.f, 0.f);
+          float4 anchor = make_float4(r0.w, r1.x, 1.f, 0.f);
           pin_math(r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y, fmul(r1.y, K.invH2),
                    hasB, a, hasB ? b : anchor, r1.z, r1.w);
         }
