@@ -114,6 +114,7 @@ def _lib():
         "kr_probe_fp32_rate": (C.c_int, [_F64P]),
         "kr_probe_sincos": (C.c_int, [_F32P, i32, _F32P, _F32P]),
         "kr_probe_wrap": (C.c_int, [_F64P, i32, _F64P]),
+        "kr_probe_quot": (C.c_int, [_F32P, _F32P, i32, _F32P]),
     }
     for name, (res, args) in sigs.items():
         fn = getattr(L, name)
@@ -373,6 +374,16 @@ def probe_wrap(d):
     out = np.zeros_like(d)
     _check(_lib().kr_probe_wrap(d.ctypes.data_as(_F64P), len(d), out.ctypes.data_as(_F64P)), None)
     return out
+
+
+def probe_quot(a, b):
+    """The solver's quotients a / b of f32 arrays (kr_probe_quot's ranges)."""
+    a = np.ascontiguousarray(a, dtype=np.float32)
+    b = np.ascontiguousarray(b, dtype=np.float32)
+    q = np.zeros_like(a)
+    _check(_lib().kr_probe_quot(a.ctypes.data_as(_F32P), b.ctypes.data_as(_F32P), len(a),
+                                q.ctypes.data_as(_F32P)), None)
+    return q
 
 
 def probe_sincos(x):

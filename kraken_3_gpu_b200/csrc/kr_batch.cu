@@ -2315,6 +2315,11 @@ __global__ void sincos_probe_kernel(const float *x, int n, float *s, float *c) {
   if (i < n) kr::sincos_r(x[i], s + i, c + i);
 }
 
+__global__ void quot_probe_kernel(const float *a, const float *b, int n, float *q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) q[i] = kr::quot(a[i], b[i], kr::recip(b[i]));
+}
+
 __global__ void wrap_probe_kernel(const double *d, int n, double *out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = wrap_pi(d[i]);
@@ -2333,6 +2338,23 @@ extern "C" int kr_probe_sincos(const float *x, int32_t n, float *s, float *c) {
   }
   if (e == cudaSuccess) e = cudaMemcpy(s, d + n, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(c, d + 2 * (size_t)n, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) { g_batch_error = cudaGetErrorString(e); return KR_ERR_CUDA; }
+  return KR_OK;
+}
+
+extern "C" int kr_probe_quot(const float *a, const float *b, int32_t n, float *q) {
+  if (!a || !b || !q || n < 0) { g_batch_error = "kr_probe_quot: bad arguments"; return KR_ERR_INVALID; }
+  if (n == 0) return KR_OK;
+  float *d = nullptr;
+  cudaError_t e = cudaMalloc(&d, (size_t)n * 3 * sizeof(float));
+  if (e == cudaSuccess) e = cudaMemcpy(d, a, (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + n, b, (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    quot_probe_kernel<<<(n + 255) / 256, 256>>>(d, d + n, n, d + 2 * (size_t)n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(q, d + 2 * (size_t)n, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost);
   cudaFree(d);
   if (e != cudaSuccess) { g_batch_error = cudaGetErrorString(e); return KR_ERR_CUDA; }
   return KR_OK;

@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "kr_sincos_tab.h"
+#include "kr_units.h"
 
 namespace kr {
 
@@ -160,7 +161,8 @@ static __device__ __noinline__ float2 sincos_f64(float a) {
 // unevaluated sum h + l of two f32 whose error bound err is known; where
 // h + (l - err) and h + (l + err) round to one f32, that is the rounding of
 // the exact value and of the f64 value above, whose own error err includes.
-// Returns false where they do not (about one value in 3,000) or |a| > 64:
+// Returns the distance of the two roundings, 0 where the values stand; where
+// it is not (about one value in 3,000) and for |a| > kSinCosNearMax
 // sincos_f64 decides.  The f64 chain cost 241 cycles, mostly conversions
 // (18 cycles each) and the serial reduction and series.
 //
@@ -173,10 +175,12 @@ static __device__ __noinline__ float2 sincos_f64(float a) {
 // S + C r1 and its two rounding errors exact (the product by fma, the sum
 // because |S| is 0 or above |C r1|).  Error: r^2 (|m| <= r^2 / 2) times
 // below 12 units of 2^-24 for the roundings of r, r^2, m and the two sums
-// it enters, Sl m among them; below 2^-40 for the roundings of rl, n, its
-// sum and p2 (2^-42.6 each), r^5 / 120 (2^-43.7), Cl n (2^-43.6) and the f64
-// value (2^-51).
-__device__ __forceinline__ bool sincos_near(float a, float *s, float *c) {
+// it enters, Sl m among them, times |S| (cos: |C|); |k| 2^-53 for the
+// roundings of rl, n, its sum and p2 (2^-55.4 |k| each); below 2^-43 for
+// r^5 / 120 (2^-43.7), the other roundings and the f64 value (2^-51).  All
+// 1.8e8 arguments of each sign from 2^-20 to 64: no value accepted that
+// differs from sincos_f64's.
+__device__ __forceinline__ float sincos_near(float a, float *s, float *c) {
   const float t = fmaf(a, 0x1.45f306p6f, 12582912.f);  // 256/pi; the sum's low bits hold k
   const float4 T = __ldg(&kSinCosNear[__float_as_int(t) & 511]);
   const float k = fsub(t, 12582912.f);
@@ -184,34 +188,53 @@ __device__ __forceinline__ bool sincos_near(float a, float *s, float *c) {
   const float r = fadd(r1, rl), rr = fmul(r, r);
   const float n = fmaf(fmul(r, rr), -1.f / 6, rl);
   const float m = fmul(rr, fmaf(rr, 1.f / 24, -0.5f));
-  const float err = fmaf(rr, 0x1.8p-22f, 0x1p-40f);
+  const float w = fmul(rr, 0x1.8p-22f), e0 = fmaf(fabsf(k), 0x1p-53f, 0x1p-43f);
+  const float es = fmaf(fabsf(T.x), w, e0), ec = fmaf(fabsf(T.z), w, e0);
   const float qs = fmul(T.z, r1), hs = fadd(T.x, qs);
   const float ls = fadd(fmaf(T.x, m, fmaf(T.z, n, fmaf(T.w, r1, T.y))),
                         fadd(fmaf(T.z, r1, -qs), fsub(qs, fsub(hs, T.x))));
   const float qc = fmul(-T.x, r1), hc = fadd(T.z, qc);
   const float lc = fadd(fmaf(T.z, m, fmaf(-T.x, n, fmaf(-T.y, r1, T.w))),
                         fadd(fmaf(-T.x, r1, -qc), fsub(qc, fsub(hc, T.z))));
-  *s = fadd(hs, fadd(ls, err));
-  *c = fadd(hc, fadd(lc, err));
-  return fabsf(a) <= 64.f && *s == fadd(hs, fsub(ls, err)) && *c == fadd(hc, fsub(lc, err));
+  *s = fadd(hs, fadd(ls, es));
+  *c = fadd(hc, fadd(lc, ec));
+  return fadd(fabsf(fsub(*s, fadd(hs, fsub(ls, es)))), fabsf(fsub(*c, fadd(hc, fsub(lc, ec)))));
 }
+constexpr float kSinCosNearMax = 64.f;
 
 __device__ __forceinline__ void sincos_r(float a, float *s, float *c) {
-  if (!sincos_near(a, s, c)) {
+  if (!(sincos_near(a, s, c) == 0.f && fabsf(a) <= kSinCosNearMax)) {
     const float2 f = sincos_f64(a);
     *s = f.x;
     *c = f.y;
   }
 }
 
-// sincos_r of two angles: their chains run side by side
-__device__ __forceinline__ void sincos2_r(float a, float b, float *sa, float *ca, float *sb, float *cb) {
-  const bool oa = sincos_near(a, sa, ca), ob = sincos_near(b, sb, cb);
-  if (!(oa && ob)) {
-    const float2 f = sincos_f64(a), g = sincos_f64(b);
-    *sa = f.x; *ca = f.y;
-    *sb = g.x; *cb = g.y;
-  }
+// Several quotients by one divisor: RN(1 / b) once, then each RN(a / b) by
+// Markstein's theorem (P. Markstein, IBM J. Res. Dev. 34(1), 1990): with y =
+// RN(1 / b) and q within one ulp of a / b, q + y (a - b q) rounds to RN(a / b),
+// the residual exact in one fma.  The first correction brings q within one
+// ulp, the second rounds.  y itself comes from the hardware estimate (one
+// ulp) by the same step twice; the theorem gives RN(1 / b) except for the
+// divisor with all mantissa bits set.  Five instructions in sequence per
+// quotient and no branch, against about 45 cycles and a branch per __fdiv_rn;
+// the GPU tests compare every mantissa of b and random quotients with it.
+// Valid for |b| in 2^-60 .. 2^60 and |a| in 2^-100 .. 2^60 or a = 0: no
+// exponent comes near its limits, a residual is a multiple of 2^-149.
+__device__ __forceinline__ float recip(float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  y = fmaf(fmaf(-b, y, 1.f), y, y);
+  return fmaf(fmaf(-b, y, 1.f), y, y);
+}
+__device__ __forceinline__ bool mantissa_ok(float b) { return (__float_as_uint(b) & 0x7fffffu) != 0x7fffffu; }
+__device__ __forceinline__ bool recip_ok(float b) {
+  return fabsf(b) > 0x1p-60f && fabsf(b) < 0x1p60f && mantissa_ok(b);
+}
+__device__ __forceinline__ float quot(float a, float b, float y) {
+  float q = fmul(a, y);
+  q = fmaf(fmaf(-b, q, a), y, q);
+  return fmaf(fmaf(-b, q, a), y, q);
 }
 
 // trunc(x / TAU) exactly, as the f64 quotient of f32solver.mjs:38 gives it.
@@ -413,7 +436,7 @@ struct Island {
 constexpr unsigned kUnitIdle = 0xffffffffu;
 // drop-in world flags
 constexpr unsigned kHasPin = 1u << 16, kPinBroken = 1u << 17, kHasAngle = 1u << 18, kAngleBroken = 1u << 19,
-                   kPinIsGrip = 1u << 20;
+                   kPinIsGrip = 1u << 20, kPinTame = 1u << 21;
 // batched engine: bits 16..23 the motor of a joint, or 0xff for a grip
 constexpr unsigned kNoMotor = 0xffu;
 
@@ -457,88 +480,169 @@ __device__ __forceinline__ void integrate_body(const SolverConsts &K, Island &S,
 // the anchor as its position with angle 1 (any angle with positive sine and
 // cosine), lb and the masses of B are 0 (the same values as the reference's
 // branch).  lx, ly: the multiplier, updated.
-__device__ __forceinline__ void pin_math(float lax, float lay, float lbx, float lby, float wA, float wIA, float wB,
-                                         float wIB, float alphaTilde, bool hasB, float4 &a, float4 &b, float &lx,
-                                         float &ly) {
-  float sa, ca, sb, cb;
-  sincos2_r(a.z, b.z, &sa, &ca, &sb, &cb);
-  const float rax = fsub(fmul(lax, ca), fmul(lay, sa)), ray = fadd(fmul(lax, sa), fmul(lay, ca));
-  const float rbx = fsub(fmul(lbx, cb), fmul(lby, sb)), rby = fadd(fmul(lbx, sb), fmul(lby, cb));
+struct PinArgs {
+  float lax, lay, lbx, lby, wA, wIA, wB, wIB, alphaTilde;
+  bool hasB;
+};
+
+// The reference form: every branch as the reference takes it.  Out of line:
+// for the arguments pin_math cannot take, and for units whose two bodies are
+// one (self: a and b the same record, the result in b).
+// Values in, values out: records passed by address would live in local memory
+// on the near path as well.
+struct PinOut {
+  float4 a, b;
+  float lx, ly;
+};
+static __device__ __noinline__ PinOut pin_any(PinArgs U, float4 a, float4 b, float lx, float ly, bool self) {
+  const PinOut in{a, b, lx, ly};
+  const float2 ta = sincos_f64(a.z), tb = sincos_f64(b.z);
+  const float sa = ta.x, ca = ta.y, sb = tb.x, cb = tb.y;
+  const float rax = fsub(fmul(U.lax, ca), fmul(U.lay, sa)), ray = fadd(fmul(U.lax, sa), fmul(U.lay, ca));
+  const float rbx = fsub(fmul(U.lbx, cb), fmul(U.lby, sb)), rby = fadd(fmul(U.lbx, sb), fmul(U.lby, cb));
   const float Cx = fsub(fadd(a.x, rax), fadd(b.x, rbx)), Cy = fsub(fadd(a.y, ray), fadd(b.y, rby));
-  if (!(Cx == Cx) || !(Cy == Cy)) return;
-  if (fadd(fmul(Cx, Cx), fmul(Cy, Cy)) < fmul(kSlackPos, kSlackPos)) return;
+  if (!(Cx == Cx) || !(Cy == Cy)) return in;
+  if (fadd(fmul(Cx, Cx), fmul(Cy, Cy)) < fmul(kSlackPos, kSlackPos)) return in;
   const float pax = -ray, pay = rax, pbx = -rby, pby = rbx;
-  const float wSum = fadd(wA, wB);
-  const float k00 = fadd(fadd(wSum, fmul(fmul(wIA, pax), pax)), fmul(fmul(wIB, pbx), pbx));
-  const float k01 = fadd(fmul(fmul(wIA, pax), pay), fmul(fmul(wIB, pbx), pby));
-  const float k11 = fadd(fadd(wSum, fmul(fmul(wIA, pay), pay)), fmul(fmul(wIB, pby), pby));
+  const float wSum = fadd(U.wA, U.wB);
+  const float k00 = fadd(fadd(wSum, fmul(fmul(U.wIA, pax), pax)), fmul(fmul(U.wIB, pbx), pbx));
+  const float k01 = fadd(fmul(fmul(U.wIA, pax), pay), fmul(fmul(U.wIB, pbx), pby));
+  const float k11 = fadd(fadd(wSum, fmul(fmul(U.wIA, pay), pay)), fmul(fmul(U.wIB, pby), pby));
   const float det = fsub(fmul(k00, k11), fmul(k01, k01));
-  if (fabsf(det) < kEpsDet) return;
-  const float bx = fadd(Cx, fmul(alphaTilde, lx)), by = fadd(Cy, fmul(alphaTilde, ly));
+  if (fabsf(det) < kEpsDet) return in;
+  const float bx = fadd(Cx, fmul(U.alphaTilde, lx)), by = fadd(Cy, fmul(U.alphaTilde, ly));
   const float i00 = fdiv(k11, det), i11 = fdiv(k00, det), i01 = -fdiv(k01, det);
   const float dlx = -fadd(fmul(i00, bx), fmul(i01, by)), dly = -fadd(fmul(i01, bx), fmul(i11, by));
-  if (!(dlx == dlx) || !(dly == dly)) return;
+  if (!(dlx == dlx) || !(dly == dly)) return in;
   lx = fadd(lx, dlx);
   ly = fadd(ly, dly);
-  a.x = fadd(a.x, fmul(wA, dlx));
-  a.y = fadd(a.y, fmul(wA, dly));
-  a.z = fadd(a.z, fmul(wIA, fadd(fmul(pax, dlx), fmul(pay, dly))));
-  if (hasB) {
-    b.x = fsub(b.x, fmul(wB, dlx));
-    b.y = fsub(b.y, fmul(wB, dly));
-    b.z = fsub(b.z, fmul(wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
+  a.x = fadd(a.x, fmul(U.wA, dlx));
+  a.y = fadd(a.y, fmul(U.wA, dly));
+  a.z = fadd(a.z, fmul(U.wIA, fadd(fmul(pax, dlx), fmul(pay, dly))));
+  if (self) b = a;
+  if (U.hasB) {
+    b.x = fsub(b.x, fmul(U.wB, dlx));
+    b.y = fsub(b.y, fmul(U.wB, dly));
+    b.z = fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
   }
+  return PinOut{a, b, lx, ly};
 }
 
-// The deviation of the joint angle from rest, and that deviation from the
-// target (x, y): up to three wrapped differences in a row, one test for all
-// of them instead of a branch each.
-static __device__ __noinline__ float2 deviation_far(float az, float bz, float rest, float tgt, bool hasB) {
-  const float dev = angle_delta(hasB ? angle_delta(bz, az) : az, rest);
-  return make_float2(dev, angle_delta(dev, tgt));
-}
-__device__ __forceinline__ float2 deviation(float az, float bz, float rest, float tgt, bool hasB) {
-  const float x1 = hasB ? fsub(bz, az) : 0.f;
-  const float x2 = fsub(hasB ? wrap_near(x1) : az, rest), dev = wrap_near(x2);
-  const float x3 = fsub(dev, tgt);
-  if (fmaxf(fmaxf(fabsf(x1), fabsf(x2)), fabsf(x3)) > kWrapNear) return deviation_far(az, bz, rest, tgt, hasB);
-  return make_float2(dev, wrap_near(x3));
+// The same operations for a tame pin (kr_units.h pin_tame), without the
+// branches: the reference's
+// early returns become one condition on the update, and what needs another
+// path (an angle the rounding test does not decide, a divisor that recip
+// does not cover, an error of 1e15 or more or NaN) is evaluated again by
+// pin_any.  A predicate costs about 13 cycles and a branch on it 25 more in a
+// chain that nothing else hides, so the tests are folded into sums.
+__device__ __forceinline__ void pin_math(const PinArgs &U, float4 &a, float4 &b, float &lx, float &ly) {
+  float sa, ca, sb, cb;
+  const float spread = fadd(sincos_near(a.z, &sa, &ca), sincos_near(b.z, &sb, &cb));
+  const float rax = fsub(fmul(U.lax, ca), fmul(U.lay, sa)), ray = fadd(fmul(U.lax, sa), fmul(U.lay, ca));
+  const float rbx = fsub(fmul(U.lbx, cb), fmul(U.lby, sb)), rby = fadd(fmul(U.lbx, sb), fmul(U.lby, cb));
+  const float Cx = fsub(fadd(a.x, rax), fadd(b.x, rbx)), Cy = fsub(fadd(a.y, ray), fadd(b.y, rby));
+  const float pax = -ray, pay = rax, pbx = -rby, pby = rbx;
+  const float wSum = fadd(U.wA, U.wB);
+  const float k00 = fadd(fadd(wSum, fmul(fmul(U.wIA, pax), pax)), fmul(fmul(U.wIB, pbx), pbx));
+  const float k01 = fadd(fmul(fmul(U.wIA, pax), pay), fmul(fmul(U.wIB, pbx), pby));
+  const float k11 = fadd(fadd(wSum, fmul(fmul(U.wIA, pay), pay)), fmul(fmul(U.wIB, pby), pby));
+  const float det = fsub(fmul(k00, k11), fmul(k01, k01));
+  const float bx = fadd(Cx, fmul(U.alphaTilde, lx)), by = fadd(Cy, fmul(U.alphaTilde, ly));
+  const float y = recip(det);
+  const float i00 = quot(k11, det, y), i11 = quot(k00, det, y), i01 = -quot(k01, det, y);
+  const float dlx = -fadd(fmul(i00, bx), fmul(i01, by)), dly = -fadd(fmul(i01, bx), fmul(i11, by));
+  if (!(fmaxf(fabsf(a.z), fabsf(b.z)) <= kSinCosNearMax && fadd(fabsf(bx), fabsf(by)) < 1e15f && mantissa_ok(det) &&
+        spread == 0.f)) {
+    const PinOut o = pin_any(U, a, b, lx, ly, false);
+    a = o.a; b = o.b; lx = o.lx; ly = o.ly;
+    return;
+  }
+  const bool upd = fadd(fmul(Cx, Cx), fmul(Cy, Cy)) >= fmul(kSlackPos, kSlackPos), updb = upd && U.hasB;
+  lx = upd ? fadd(lx, dlx) : lx;
+  ly = upd ? fadd(ly, dly) : ly;
+  a.x = upd ? fadd(a.x, fmul(U.wA, dlx)) : a.x;
+  a.y = upd ? fadd(a.y, fmul(U.wA, dly)) : a.y;
+  a.z = upd ? fadd(a.z, fmul(U.wIA, fadd(fmul(pax, dlx), fmul(pay, dly)))) : a.z;
+  b.x = updb ? fsub(b.x, fmul(U.wB, dlx)) : b.x;
+  b.y = updb ? fsub(b.y, fmul(U.wB, dly)) : b.y;
+  b.z = updb ? fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly)))) : b.z;
 }
 
 // solveAngleF, f32solver.mjs:258-301 (solver.wgsl:292-350): muscle
 // (compliant) part, then the one-sided joint limit.  az, bz: the angles; l:
 // the multiplier, updated.
-__device__ __forceinline__ void angle_math(float rest, float mn, float mx, float tgt, float alphaTilde, float wA,
-                                           float wB, bool hasB, float &az, float &bz, float &l) {
-  const float wSum = fadd(wA, wB);
-  if (wSum <= 0.f) return;
-  const float2 dc = deviation(az, bz, rest, tgt, hasB);
-  const float C = dc.y;
-  if (!(C == C)) return;
+struct AngleArgs {
+  float rest, mn, mx, tgt, alphaTilde, wA, wB;
+  bool hasB;
+};
+
+// The reference form (as pin_any)
+static __device__ __noinline__ float3 angle_any(AngleArgs U, float az, float bz, float l, bool self) {
+  const float wSum = fadd(U.wA, U.wB);
+  if (wSum <= 0.f) return make_float3(az, bz, l);
+  const float dev = angle_delta(U.hasB ? angle_delta(bz, az) : az, U.rest);
+  const float C = angle_delta(dev, U.tgt);
+  if (!(C == C)) return make_float3(az, bz, l);
   if (fabsf(C) >= kSlackAng) {
-    const float dl = -fdiv(fadd(C, fmul(alphaTilde, l)), fadd(wSum, alphaTilde));
-    if (!(dl == dl)) return;
+    const float dl = -fdiv(fadd(C, fmul(U.alphaTilde, l)), fadd(wSum, U.alphaTilde));
+    if (!(dl == dl)) return make_float3(az, bz, l);
     l = fadd(l, dl);
-    if (hasB) {
-      bz = fadd(bz, fmul(wB, dl));
-      az = fsub(az, fmul(wA, dl));
+    if (U.hasB) {
+      bz = fadd(bz, fmul(U.wB, dl));
+      az = fsub(self ? bz : az, fmul(U.wA, dl));
+      if (self) bz = az;
     } else {
-      az = fadd(az, fmul(wA, dl));
+      az = fadd(az, fmul(U.wA, dl));
     }
   }
-  const float dev2 = deviation(az, bz, rest, 0.f, hasB).x;
+  const float dev2 = angle_delta(U.hasB ? angle_delta(bz, az) : az, U.rest);
   float over = 0.f;
-  if (dev2 > mx) over = fsub(dev2, mx);
-  else if (dev2 < mn) over = fsub(dev2, mn);
+  if (dev2 > U.mx) over = fsub(dev2, U.mx);
+  else if (dev2 < U.mn) over = fsub(dev2, U.mn);
   if (fabsf(over) >= kSlackAng) {
     const float dl2 = -fdiv(over, wSum);
-    if (hasB) {
-      bz = fadd(bz, fmul(wB, dl2));
-      az = fsub(az, fmul(wA, dl2));
+    if (U.hasB) {
+      bz = fadd(bz, fmul(U.wB, dl2));
+      az = fsub(self ? bz : az, fmul(U.wA, dl2));
+      if (self) bz = az;
     } else {
-      az = fadd(az, fmul(wA, dl2));
+      az = fadd(az, fmul(U.wA, dl2));
     }
   }
+  return make_float3(az, bz, l);
+}
+
+// The same operations in near form (see pin_math).  Where a term is used,
+// |C| and |over| are at least kSlackAng, so the quotients' numerators are 0
+// or above 2^-40.
+__device__ __forceinline__ void angle_math(const AngleArgs &U, float &az, float &bz, float &l) {
+  const float wSum = fadd(U.wA, U.wB), den = fadd(wSum, U.alphaTilde);
+  const float y = recip(den), yw = recip(wSum);
+  const bool tame = recip_ok(den) && recip_ok(wSum) && wSum > 0.f;
+  const float x1 = U.hasB ? fsub(bz, az) : 0.f;
+  const float x2 = fsub(U.hasB ? wrap_near(x1) : az, U.rest);
+  const float x3 = fsub(wrap_near(x2), U.tgt);
+  const float C = wrap_near(x3);
+  const float num = fadd(C, fmul(U.alphaTilde, l));
+  const float dl = -quot(num, den, y);
+  const bool act = fabsf(C) >= kSlackAng;
+  const float na = act ? (U.hasB ? fsub(az, fmul(U.wA, dl)) : fadd(az, fmul(U.wA, dl))) : az;
+  const float nb = act && U.hasB ? fadd(bz, fmul(U.wB, dl)) : bz;
+  const float x4 = U.hasB ? fsub(nb, na) : 0.f;
+  const float x5 = fsub(U.hasB ? wrap_near(x4) : na, U.rest);
+  const float dev2 = wrap_near(x5);
+  const float o1 = fsub(dev2, U.mx), o2 = fsub(dev2, U.mn);
+  const bool hi = o1 >= kSlackAng, lim = hi || o2 <= -kSlackAng;
+  const float over = hi ? o1 : o2, dl2 = -quot(over, wSum, yw);
+  const float far = fmaxf(fmaxf(fmaxf(fabsf(x1), fabsf(x2)), fmaxf(fabsf(x3), fabsf(x4))), fabsf(x5));
+  if (!(tame && fabsf(num) < 0x1p60f && far <= kWrapNear)) {  // NaN fails by num
+    const float3 o = angle_any(U, az, bz, l, false);
+    az = o.x; bz = o.y; l = o.z;
+    return;
+  }
+  l = act ? fadd(l, dl) : l;
+  az = lim ? (U.hasB ? fsub(na, fmul(U.wA, dl2)) : fadd(na, fmul(U.wA, dl2))) : na;
+  bz = lim && U.hasB ? fadd(nb, fmul(U.wB, dl2)) : nb;
 }
 
 // One sweep of the solve list, batched engine.  first: the first sweep of a
@@ -550,47 +654,60 @@ template <int G>
 __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
   const float alpha_m = fmul(S.comp_m, K.invH2);
   const float4 *rec = S.recs + 3 * L.lane;
-  for (int p = 0; p < S.npass; p++, rec += 3 * G) {
-    const float4 r0 = rec[0];
+  float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
+  for (int p = 0; p < S.npass; p++) {
     const unsigned ab = __float_as_uint(r0.x);
+    const PinArgs U{r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, 0.f, (ab >> 16) != kNoMotor};
+    AngleArgs V{r2.y, r2.z, r2.w, 0.f, alpha_m, r1.z, r2.x, true};
+    // the next pass's records: the loads wait on nothing the sweep computes
+    rec += 3 * G;
+    if (p + 1 < S.npass) { r0 = rec[0]; r1 = rec[1]; r2 = rec[2]; }
     if (ab != kUnitIdle) {
-      const int A = ab & 0xff, B = (ab >> 8) & 0xff, m = (ab >> 16) & 0xff;
+      const int A = ab & 0xff, B = (ab >> 8) & 0xff, m = ab >> 16;
       float4 a = S.Q[A], b = S.Q[B];
-      const float4 r1 = rec[1], r2 = rec[2];
-      if (m != (int)kNoMotor) {
-        float lx = 0.f, ly = 0.f;
-        pin_math(r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, 0.f, true, a, b, lx, ly);
+      const bool joint = U.hasB;
+      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+      float l = 0.f;
+      if (joint) {
         const float2 mo = S.mot[m];
-        float l = first ? 0.f : mo.y;
-        angle_math(r2.y, r2.z, r2.w, mo.x, alpha_m, r1.z, r2.x, true, a.z, b.z, l);
+        V.tgt = mo.x;
+        l = first ? 0.f : mo.y;
+      } else {
+        g = S.grip[B - S.nb];
+        if (first) g.x = g.y = 0.f;
+      }
+      // joints and grips that hold (b.w: the anchor's broken flag)
+      if (joint || b.w == 0.f) pin_math(U, a, b, g.x, g.y);
+      if (joint) {
+        angle_math(V, a.z, b.z, l);
         S.mot[m].y = l;
-        S.Q[A] = a;
         S.Q[B] = b;
       } else {
-        float4 g = S.grip[B - S.nb];
-        if (first) g.x = g.y = 0.f;
-        if (b.w == 0.f) {  // holding
-          pin_math(r0.y, r0.z, 0.f, 0.f, r1.y, r1.z, 0.f, 0.f, 0.f, false, a, b, g.x, g.y);
-          S.Q[A] = a;
-        }
         S.grip[B - S.nb] = g;
       }
+      S.Q[A] = a;
     }
     L.sync();
   }
 }
 
 // A drop-in unit whose two bodies are one: every update sees the one before
-// it (a and b are the same record).  Out of line: no creature has one.
-static __device__ __noinline__ void solve_self(const SolverConsts &K, unsigned ab, float4 wa, float4 &a, float4 *rec) {
-  const float4 r0 = rec[0], r2 = rec[2];
-  float4 r1 = rec[1], r3 = rec[3];
-  if ((ab & (kHasPin | kPinBroken)) == kHasPin)
-    pin_math(r0.y, r0.z, r0.w, r1.x, wa.x, wa.y, wa.x, wa.y, fmul(r1.y, K.invH2), true, a, a, r1.z, r1.w);
-  if ((ab & (kHasAngle | kAngleBroken)) == kHasAngle)
-    angle_math(r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wa.y, true, a.z, a.z, r3.y);
-  rec[1] = r1;
-  rec[3] = r3;
+// it.  Out of line: no creature has one.
+static __device__ __noinline__ float4 solve_self(const SolverConsts &K, unsigned ab, float4 wa, float4 a, float4 *rec) {
+  const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3];
+  if ((ab & (kHasPin | kPinBroken)) == kHasPin) {
+    const PinOut o = pin_any(PinArgs{r0.y, r0.z, r0.w, r1.x, wa.x, wa.y, wa.x, wa.y, fmul(r1.y, K.invH2), true}, a, a,
+                             r1.z, r1.w, true);
+    a = o.b;
+    rec[1] = make_float4(r1.x, r1.y, o.lx, o.ly);
+  }
+  if ((ab & (kHasAngle | kAngleBroken)) == kHasAngle) {
+    const float3 o = angle_any(AngleArgs{r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wa.y, true}, a.z, a.z,
+                               r3.y, true);
+    a.z = o.y;
+    rec[3].y = o.z;
+  }
+  return a;
 }
 
 // One sweep of the solve list, drop-in world: unit records
@@ -609,8 +726,7 @@ __device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bo
       const float4 wa = S.body[A];
       if (A == B) {
         if (first) { rec[1].z = rec[1].w = 0.f; rec[3].y = 0.f; }
-        solve_self(K, ab, wa, a, rec);
-        S.Q[A] = a;
+        S.Q[A] = solve_self(K, ab, wa, a, rec);
         continue;
       }
       float4 wb = b;
@@ -619,9 +735,15 @@ __device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bo
         float4 r1 = rec[1];
         if (first) r1.z = r1.w = 0.f;
         if (!(ab & kPinBroken)) {
-          float4 anchor = make_float4(r0.w, r1.x, 1.f, 0.f);
-          pin_math(r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y, fmul(r1.y, K.invH2),
-                   hasB, a, hasB ? b : anchor, r1.z, r1.w);
+          if (!hasB) b = make_float4(r0.w, r1.x, 1.f, 0.f);  // the anchor
+          const PinArgs U{r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y,
+                          fmul(r1.y, K.invH2), hasB};
+          if (ab & kPinTame) {
+            pin_math(U, a, b, r1.z, r1.w);
+          } else {
+            const PinOut o = pin_any(U, a, b, r1.z, r1.w, false);
+            a = o.a; b = o.b; r1.z = o.lx; r1.w = o.ly;
+          }
         }
         rec[1] = r1;
       }
@@ -630,7 +752,7 @@ __device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bo
         if (first) r3.y = 0.f;
         if (!(ab & kAngleBroken)) {
           const float4 r2 = rec[2];
-          angle_math(r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wb.y, hasB, a.z, b.z, r3.y);
+          angle_math(AngleArgs{r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wb.y, hasB}, a.z, b.z, r3.y);
         }
         rec[3] = r3;
       }

@@ -144,7 +144,14 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
     // the engine's records hold a joint (pin and angle constraint) or a grip
     const bool joint = u.pin >= 0 && u.ang >= 0 && u.b >= 0;
     const bool grip = u.pin >= 0 && u.ang < 0 && u.b < 0 && cons[list[u.pin]].type == 2;
-    if (!joint && !grip) {
+    bool tame = joint || grip;
+    if (tame) {
+      const RawCon &c = cons[list[u.pin]];
+      tame = joint ? pin_tame((float)c.lax, (float)c.lay, (float)c.lbx, (float)c.lby, t->im[u.a], t->ii[u.a],
+                              t->im[u.b], t->ii[u.b])
+                   : pin_tame((float)c.lax, (float)c.lay, 0.f, 0.f, t->im[u.a], t->ii[u.a], 0.f, 0.f);
+    }
+    if (!tame) {
       *err = "body shape " + std::to_string(arms) + "x" + std::to_string(segs) + ": a constraint outside the joints";
       return false;
     }

@@ -1,11 +1,37 @@
 // kr_units.h -- host side of the solve schedule: a solve list (constraints in
 // order, each with its one or two bodies) as units and passes of units (see
-// kr::Island in kr_solver.cuh).
+// kr::Island in kr_solver.cuh), and which pins take the short form.
 #pragma once
 #include <algorithm>
 #include <vector>
 
+#ifdef __CUDACC__
+#define KR_HD __host__ __device__
+#else
+#define KR_HD
+#endif
+
 namespace kr {
+
+// Levers and masses for which the quotients of kr_solver.cuh pin_math stay in
+// range whatever the angles (every pin of a creature): with wI |l|^2 <= 16 wS
+// the matrix entries lie in wS .. 33 wS and det in wS^2 .. 2^11 wS^2, wS in
+// 2^-10 .. 2^10 (so |det| >= kEpsDet); k01 is 0 or above 2^-100, since |sin|
+// and |cos| are above 2^-21 where sincos_near stands and a lever's components
+// are not small unless the other is large.
+KR_HD inline bool lever_tame(float x, float y, float wI, float wS) {
+  const float ax = x < 0.f ? -x : x, ay = y < 0.f ? -y : y;
+  if (!(wI >= 0.f && wI <= 0x1p10f && ax <= 0x1p20f && ay <= 0x1p20f)) return false;
+  if (wI == 0.f || (ax == 0.f && ay == 0.f)) return true;
+  if (wI < 0x1p-16f || !(ax >= 0x1p-4f || ay >= 0x1p-4f)) return false;
+  if ((ax > 0x1p-30f && ax < 0x1p-4f) || (ay > 0x1p-30f && ay < 0x1p-4f)) return false;
+  return wI * (ax * ax + ay * ay) <= 16.f * wS;
+}
+KR_HD inline bool pin_tame(float lax, float lay, float lbx, float lby, float wA, float wIA, float wB, float wIB) {
+  const float wS = wA + wB;
+  return wA >= 0.f && wB >= 0.f && wS >= 0x1p-10f && wS <= 0x1p10f && lever_tame(lax, lay, wIA, wS) &&
+         lever_tame(lbx, lby, wIB, wS);
+}
 
 struct SolveEntry {
   int angle;  // 1: angle constraint, 0: pin or grip

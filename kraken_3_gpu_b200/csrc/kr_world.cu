@@ -120,6 +120,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
     }
     V.body[i] = make_float4(q2.y, q2.z, reach, __int_as_float(bp.x | (bp.y << 16)));
   }
+  __syncwarp();  // the units read the bodies' masses
   // stage the units' constraints (80 B AoS -> unit records)
   for (int u = lane; u < S.nu; u += 32) {
     const int4 t = A.T.units[uo + u];
@@ -133,6 +134,10 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
       r0.w = __uint_as_float(w1.z); r1.x = __uint_as_float(w1.w);
       r1.y = __uint_as_float(w2.x);
       r3.z = __uint_as_float(w4.x);
+      const bool has_b = ((ab >> 8) & 0xffu) != 0xffu;
+      const float4 wa = S.body[ab & 0xffu];
+      const float4 wb = has_b ? S.body[(ab >> 8) & 0xffu] : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (kr::pin_tame(r0.y, r0.z, has_b ? r0.w : 0.f, has_b ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y)) ab |= kr::kPinTame;
     }
     if (t.z >= 0) {
       const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)t.z);

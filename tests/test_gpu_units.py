@@ -12,7 +12,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from kraken_3_gpu_b200 import _native
+from kraken_3_gpu_b200 import _native, batch
 from oracle import binding as ob
 
 pytestmark = pytest.mark.gpu
@@ -183,3 +183,24 @@ def test_angle_wrap_edges():
             assert np.array_equal(bodies[:, 8], o.arr("av").astype(np.float32)), s
     finally:
         L.kr_destroy(h)
+
+
+def test_quotients_equal_ieee_division():
+    """The shared-reciprocal quotients: 1 / b for every mantissa of b but the
+    one with all bits set, and quotients of random and extreme mantissas over
+    the stated exponents, against IEEE f32 division."""
+    m = np.arange((1 << 23) - 1, dtype=np.uint32)
+    b = (m | np.uint32(127 << 23)).view(np.float32)
+    one = np.ones_like(b)
+    assert np.array_equal(batch.probe_quot(one, b), one / b)
+    r = np.random.default_rng(5)
+    n = 1 << 21
+    for ea, eb in ((0, 0), (59, -59), (-99, 59), (-60, -59), (20, -20), (-7, 3)):
+        ma, mb = r.integers(0, 1 << 23, n), r.integers(0, (1 << 23) - 1, n)
+        ma[: n // 4] = np.where(r.random(n // 4) < 0.5, r.integers(0, 8, n // 4), (1 << 23) - 1 - r.integers(0, 8, n // 4))
+        mb[n // 8: n // 2] = np.where(r.random(n // 2 - n // 8) < 0.5, r.integers(0, 8, n // 2 - n // 8),
+                                      (1 << 23) - 2 - r.integers(0, 8, n // 2 - n // 8))
+        a = np.ldexp(1 + ma / 2.0 ** 23, ea).astype(np.float32) * r.choice([-1, 1], n).astype(np.float32)
+        b = np.ldexp(1 + mb / 2.0 ** 23, eb).astype(np.float32)
+        a[-1000:] = 0
+        assert np.array_equal(batch.probe_quot(a, b), a / b), (ea, eb)
