@@ -87,6 +87,9 @@ struct BatchArgs {
 constexpr int kArmWords = (2 * KR_BATCH_MAX_ARMS + KR_BATCH_MAX_ARMS * KR_BATCH_MAX_SEGS + 3) & ~3;
 __host__ __device__ constexpr int r4(int n) { return (n + 3) & ~3; }
 
+// static shared memory of the kernel: the sine table and the group word
+constexpr long kStaticSmem = 512 * sizeof(float2) + 64;
+
 // statics of the template, once per CTA: unit records of the schedule for G
 // lanes, bodies, collision points, arm tables
 __host__ __device__ inline int tpl_smem_words(int npass, int G, int nb, int np) {
@@ -94,16 +97,14 @@ __host__ __device__ inline int tpl_smem_words(int npass, int G, int nb, int np) 
 }
 // one creature: the committed state and the predicted state (16-byte records;
 // the velocity lives in the predicted state's records between substeps), the
-// arms' anchors after the bodies, per motor {target, lambda}, per arm {lambda,
-// break force}, controls, the near lists of the collision pass.  The proprioception's vector
-// shares the motors' words: it is read before the targets are written.
-__host__ __device__ inline int mot_words(int arms, int segs) {
-  const int m = 2 * arms * segs, o = 6 * arms + 6;
-  return r4(m > o ? m : o);
-}
+// arms' anchors and a spare record after the bodies, the motors' and grips'
+// pairs, break forces, controls, the near lists of the collision pass.  The
+// proprioception's vector shares the motors' words: it is read before the
+// targets are written.
+__host__ __device__ inline int mot_words(int arms, int segs) { return r4(2 * (kr::grip_pair0(arms, segs) + arms + 1)); }
 __host__ __device__ inline int creature_smem_words(int nb, int arms, int segs) {
-  return 4 * nb + 4 * (nb + arms) + mot_words(arms, segs) + 4 * arms + r4(arms * segs + arms) +
-         kr::kMaxCulled / 2 + r4((nb + 3) / 4);
+  return 4 * nb + 4 * (nb + arms + 1) + mot_words(arms, segs) + r4(arms) + r4(arms * segs + arms) +
+         r4((kr::kMaxCulled + 1) / 2) + r4((nb + 3) / 4);
 }
 
 struct TplSmem {
@@ -130,13 +131,14 @@ __device__ inline void carve_creature(kr::Island &S, CreatureSmem &X, const TplS
   const int AS = td.arms * td.segs;
   // committed state, resident for the creature's whole run
   S.P = reinterpret_cast<float4 *>(p); p += 4 * td.nb;
-  S.Q = reinterpret_cast<float4 *>(p); p += 4 * (td.nb + td.arms);
+  S.Q = reinterpret_cast<float4 *>(p); p += 4 * (td.nb + td.arms + 1);
   S.V = S.Q;
   S.mot = reinterpret_cast<float2 *>(p);
   X.obs = p; p += mot_words(td.arms, td.segs);
-  S.grip = reinterpret_cast<float4 *>(p); p += 4 * td.arms;
+  S.brk = p; p += r4(td.arms);
+  S.grip0 = kr::grip_pair0(td.arms, td.segs);
   X.ctrl = p; p += r4(AS + td.arms);
-  S.cull = reinterpret_cast<unsigned short *>(p); p += kr::kMaxCulled / 2;
+  S.cull = reinterpret_cast<unsigned short *>(p); p += r4((kr::kMaxCulled + 1) / 2);
   S.list = reinterpret_cast<unsigned char *>(p);
   // statics shared by the CTA
   S.recs = P.recs; S.body = P.body; S.pts = P.pts;
@@ -247,7 +249,7 @@ __device__ unsigned proprio(const BatchArgs &A, const TplDev &td, const TplSmem 
     const double dx = tx - cx, dy = ty - cy;
     X.obs[2 * arms + 2 * a] = (float)clamp_sym((dx * ca - dy * sa) / td.reach, 1.2);
     X.obs[2 * arms + 2 * a + 1] = (float)clamp_sym((dx * sa + dy * ca) / td.reach, 1.2);
-    const float4 g = S.grip[a];
+    const float2 g = S.mot[S.grip0 + a];
     double force = 0.0;
     if (attached) force = lib_hypot((double)g.x, (double)g.y) * A.inv_h64;
     X.obs[4 * arms + a] = !attached ? 0.f : (float)fmin(1.0, force / fmax(1.0, cdp[a].y));
@@ -619,11 +621,12 @@ __device__ __noinline__ void net_senses(NetArgs N, int arms, const int *arm_tip,
 // kernels carry none of the net's code).
 template <int G, bool NET, int U>
 __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, const TplSmem &P, float *base,
-                             int slot, const kr::Lanes<G> &L) {
+                             const float2 *tab, int slot, const kr::Lanes<G> &L) {
   const int lane = L.lane;
   kr::Island S;
   CreatureSmem X;
   carve_creature(S, X, P, base, td, npass);
+  S.tab = tab;
   SlotMeta m = A.meta[slot];
   const int steps = min(A.max_steps, m.horizon - m.step);
   if (steps <= 0) return;
@@ -643,8 +646,13 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
     const float4 g = gst[lane];
     const float2 gl = glam[lane];
     S.Q[td.nb + lane] = make_float4(g.x, g.y, 1.f, g.w);  // the anchor's record: x, y, angle, broken
-    S.grip[lane] = make_float4(gl.x, gl.y, g.z, 0.f);
+    S.mot[S.grip0 + lane] = gl;
+    S.brk[lane] = g.z;
     cd = cdp[lane].x;
+  }
+  if (lane == 0) {  // idle lanes' spare records
+    S.Q[td.nb + arms] = make_float4(0.f, 0.f, 1.f, 1.f);
+    S.mot[S.grip0 + arms] = make_float2(0.f, 0.f);
   }
   const float *cin = A.ctrl_cur + (size_t)slot * kCtrlStride;
   for (int q = lane; q < AS + arms; q += G) X.ctrl[q] = cin[q];
@@ -696,7 +704,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
     }
     if (lane < arms) {
       const int a = lane, tip = P.arm_tip[a];
-      float4 &an = S.Q[td.nb + a], &gr = S.grip[a];
+      float4 &an = S.Q[td.nb + a];
       const double adh = fmax(0.0, fmin(1.0, (double)X.ctrl[AS + a]));
       double c = cd;
       if (c > 0) c -= A.dt;
@@ -711,7 +719,8 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
             cdp[a].y = brk;
             an = make_float4((float)((double)tp.x + kSegHalf * lib_cos(ta)),
                              (float)((double)tp.y + kSegHalf * lib_sin(ta)), 1.f, 0.f);
-            gr = make_float4(0.f, 0.f, (float)brk, 0.f);
+            S.brk[a] = (float)brk;
+            S.mot[S.grip0 + a] = make_float2(0.f, 0.f);
           } else {
             c = A.cooldown;
           }
@@ -719,7 +728,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
       } else {
         const double brk = 40.0 + 860.0 * adh;
         cdp[a].y = brk;
-        gr.z = (float)brk;
+        S.brk[a] = (float)brk;
         if (adh < 0.04) an.w = 1.f;
       }
       cd = c;
@@ -786,9 +795,9 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
     hbm[3 * kBodyPad + i] = v.y; hbm[4 * kBodyPad + i] = p.z; hbm[5 * kBodyPad + i] = v.z;
   }
   if (lane < arms) {
-    const float4 an = S.Q[td.nb + lane], g = S.grip[lane];
-    gst[lane] = make_float4(an.x, an.y, g.z, an.w);
-    glam[lane] = make_float2(g.x, g.y);
+    const float4 an = S.Q[td.nb + lane];
+    gst[lane] = make_float4(an.x, an.y, S.brk[lane], an.w);
+    glam[lane] = S.mot[S.grip0 + lane];
     cdp[lane].x = cd;
   }
   float *cout = A.ctrl_cur + (size_t)slot * kCtrlStride;
@@ -814,6 +823,8 @@ __global__ void __launch_bounds__(32 * kMaxW, 1) batch_kernel(BatchArgs A) {
   constexpr int V = G == 32 ? 0 : G == 16 ? 1 : 2;  // kr::schedule_index(G): the schedule for G lanes
   extern __shared__ __align__(16) float smem[];
   __shared__ int s_group;
+  __shared__ float2 s_sin[512];
+  kr::stage_sin(s_sin);  // the group loop's first barrier precedes its use
   const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31;
   const kr::Lanes<G> L(wl);
   const int c = warp * CPW + wl / G;  // creature entry of this lane group
@@ -844,7 +855,7 @@ __global__ void __launch_bounds__(32 * kMaxW, 1) batch_kernel(BatchArgs A) {
     if (slot >= 0) {
       float *base = smem + tpl_smem_words(npass, G, td.nb, td.np) +
                     c * creature_smem_words(td.nb, td.arms, td.segs);
-      run_creature<G, NET, U>(A, td, npass, P, base, slot, L);
+      run_creature<G, NET, U>(A, td, npass, P, base, s_sin, slot, L);
     }
   }
 }
@@ -1050,7 +1061,7 @@ int upload_templates(kr_batch *b) {
 int plan_shape(kr_batch *b) {
   b->cpc = b->W * (32 / b->G);
   const int ctas = b->ctas_per_sm > 0 ? b->ctas_per_sm : std::max(1, 16 / b->W);
-  long budget = std::min<long>(b->smem_optin, (long)b->smem_per_sm / ctas - b->smem_reserved) - 64;
+  long budget = std::min<long>(b->smem_optin, (long)b->smem_per_sm / ctas - b->smem_reserved) - kStaticSmem;
   budget = (budget / 16) * 16;
   const long words = budget / 4;
   b->tpl_cpg.assign(b->h_tpl.size(), 0);
@@ -2311,8 +2322,11 @@ __global__ void fma_probe_kernel(float *out, int iters) {
 
 namespace {
 __global__ void sincos_probe_kernel(const float *x, int n, float *s, float *c) {
+  __shared__ float2 tab[512];
+  kr::stage_sin(tab);
+  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) kr::sincos_r(x[i], s + i, c + i);
+  if (i < n) kr::sincos_r(tab, x[i], s + i, c + i);
 }
 
 __global__ void quot_probe_kernel(const float *a, const float *b, int n, float *q) {

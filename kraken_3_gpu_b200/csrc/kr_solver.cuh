@@ -180,9 +180,14 @@ static __device__ __noinline__ float2 sincos_f64(float a) {
 // r^5 / 120 (2^-43.7), the other roundings and the f64 value (2^-51).  All
 // 1.8e8 arguments of each sign from 2^-20 to 64: no value accepted that
 // differs from sincos_f64's.
-__device__ __forceinline__ float sincos_near(float a, float *s, float *c) {
+//
+// tab: kSinNear in shared memory.  As 16-byte __ldg gathers its look-ups were
+// the longest part of a pin (32 lanes, 32 lines: two of them 360 of 550
+// cycles); two 8-byte shared loads take a few bank conflicts each.
+__device__ __forceinline__ float sincos_near(const float2 *tab, float a, float *s, float *c) {
   const float t = fmaf(a, 0x1.45f306p6f, 12582912.f);  // 256/pi; the sum's low bits hold k
-  const float4 T = __ldg(&kSinCosNear[__float_as_int(t) & 511]);
+  const float2 ts = tab[__float_as_int(t) & 511], tc = tab[(__float_as_int(t) + 128) & 511];
+  const float4 T = make_float4(ts.x, ts.y, tc.x, tc.y);
   const float k = fsub(t, 12582912.f);
   const float r1 = fmaf(-k, 0x1.921fb6p-7f, a), rl = fmul(-k, -0x1.777a5cp-32f);
   const float r = fadd(r1, rl), rr = fmul(r, r);
@@ -202,8 +207,14 @@ __device__ __forceinline__ float sincos_near(float a, float *s, float *c) {
 }
 constexpr float kSinCosNearMax = 64.f;
 
-__device__ __forceinline__ void sincos_r(float a, float *s, float *c) {
-  if (!(sincos_near(a, s, c) == 0.f && fabsf(a) <= kSinCosNearMax)) {
+// The table into shared memory, by every thread of the block; __syncthreads
+// before its first use.
+__device__ __forceinline__ void stage_sin(float2 *tab) {
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = kSinNear[i];
+}
+
+__device__ __forceinline__ void sincos_r(const float2 *tab, float a, float *s, float *c) {
+  if (!(sincos_near(tab, a, s, c) == 0.f && fabsf(a) <= kSinCosNearMax)) {
     const float2 f = sincos_f64(a);
     *s = f.x;
     *c = f.y;
@@ -351,8 +362,9 @@ struct SdfFold {
 //    without the dropped rects hold equal states or two far states.
 //
 // Each body keeps the set of rects that can lie within D of one of its points
-// while its centre stays within kNearMove of a reference position: a bit mask
-// over the creature's near list (the rects near any of its bodies, ascending).
+// while its centre stays within kNearMove of a reference position (kFarMove
+// if no rect is that near): a bit mask over the creature's near list (the
+// rects near any of its bodies, ascending).
 // Bodies move a few px per env step, so the sets are rebuilt every few steps
 // instead of once per collision pass, and a body whose set is empty needs
 // nothing but the test that it still is near its reference.  A pass used to
@@ -360,8 +372,9 @@ struct SdfFold {
 // rects against it each time, the largest part of a pass in which no body
 // touched a wall: 16,384 mixed creatures 308 -> 289 ms, 1,024 creatures x 400
 // steps 31.8 -> 29.0 ms.
-constexpr int kMaxCulled = 64;      // near list entries; bit b of a mask covers entries b << shift ...
-constexpr float kNearMove = 8.f;
+constexpr int kMaxCulled = 62;      // near list entries; bit b of a mask covers entries b << shift ...
+constexpr unsigned kNearBit = 1u << 31;  // of a mask: the body holds within kNearMove only
+constexpr float kNearMove = 8.f, kFarMove = 32.f;
 constexpr float kCullPad = 1.f;     // rounding of the box tests
 
 // A group of G lanes of one warp advancing one creature (G = 32, 16, 8):
@@ -412,6 +425,7 @@ struct Island {
   float4 *P;           // committed x, y, angle; w: the collision reference position (near_pack)
   float4 *Q;           // predicted x, y, angle; w: the mask of near rects
   float4 *V;           // velocity vx, vy, av (batched engine: the same records as Q, see below)
+  const float2 *tab;   // kSinNear in shared memory
   const float4 *body;  // inverse mass, inverse inertia, reach, point offset | count << 16
   const float4 *pts;   // collision points: x, y, radius, body; grouped per body in groupCollPoints order
   unsigned short *cull;       // near list (kMaxCulled rect indices)
@@ -423,22 +437,34 @@ struct Island {
   const int *off;      // npass + 1 unit offsets
   float4 *force;       // fx, fy, torque
   // batched engine: the template's static records (3 float4 per lane and
-  // pass), per motor {target, lambda}, per arm {lambda x, y, break force}
+  // pass), per motor {target, lambda}, from grip0 on per arm the grip's lambda
+  // and one pair for idle lanes, break force per arm
   const float4 *recs;
   float2 *mot;
-  float4 *grip;
+  float *brk;
+  int grip0;
   float comp_m;        // motor compliance of the creature
   int arms;
 };
 
-// ab word of a unit: body A, body B (or, in the batched engine, the record
-// of an arm's anchor; 0xff in the drop-in: the world), and flags.
-constexpr unsigned kUnitIdle = 0xffffffffu;
-// drop-in world flags
+// ab word of a unit: body A, body B << 8, and flags.  Drop-in world: B is 0xff
+// for the world.
 constexpr unsigned kHasPin = 1u << 16, kPinBroken = 1u << 17, kHasAngle = 1u << 18, kAngleBroken = 1u << 19,
                    kPinIsGrip = 1u << 20, kPinTame = 1u << 21;
-// batched engine: bits 16..23 the motor of a joint, or 0xff for a grip
-constexpr unsigned kNoMotor = 0xffu;
+
+// The speed clamp of integrateF and finalizeF.  A squared speed of at most
+// 0.999 maxSpeed^2 has a length of at most maxSpeed however it rounds, so the
+// square root is taken only near the limit.
+__device__ __forceinline__ void clamp_speed(const SolverConsts &K, float &vx, float &vy) {
+  const float s2 = fadd(fmul(vx, vx), fmul(vy, vy));
+  if (s2 > (K.maxSpeed > 0.f ? 0.999f * K.maxSpeed * K.maxSpeed : -1.f)) {
+    const float sp = fsqrt(s2);
+    if (sp > K.maxSpeed) {
+      const float k = fdiv(K.maxSpeed, sp);
+      vx = fmul(vx, k); vy = fmul(vy, k);
+    }
+  }
+}
 
 // integrateF, f32solver.mjs:177-200 (solver.wgsl:166-205).  World: the
 // drop-in's bodies (forces, immovable bodies, velocities in their own
@@ -461,11 +487,7 @@ __device__ __forceinline__ void integrate_body(const SolverConsts &K, Island &S,
   float vx = fmul(fadd(v.x, fmul(fmul(K.h, im), f.x)), K.linDamp);
   float vy = fmul(fadd(v.y, fmul(fmul(K.h, im), f.y)), K.linDamp);
   float av = fmul(fadd(v.z, fmul(fmul(K.h, ii), f.z)), K.angDamp);
-  float sp = length2(vx, vy);
-  if (sp > K.maxSpeed) {
-    float k = fdiv(K.maxSpeed, sp);
-    vx = fmul(vx, k); vy = fmul(vy, k);
-  }
+  clamp_speed(K, vx, vy);
   if (av > K.maxAngSpeed) av = K.maxAngSpeed;
   else if (av < -K.maxAngSpeed) av = -K.maxAngSpeed;
   if (!(vx == vx) || !(vy == vy)) { vx = 0.f; vy = 0.f; }
@@ -485,16 +507,14 @@ struct PinArgs {
   bool hasB;
 };
 
-// The reference form: every branch as the reference takes it.  Out of line:
-// for the arguments pin_math cannot take, and for units whose two bodies are
-// one (self: a and b the same record, the result in b).
-// Values in, values out: records passed by address would live in local memory
-// on the near path as well.
+// The reference form: every branch as the reference takes it, for the
+// arguments pin_near cannot take, and for units whose two bodies are one
+// (self: a and b the same record, the result in b).
 struct PinOut {
   float4 a, b;
   float lx, ly;
 };
-static __device__ __noinline__ PinOut pin_any(PinArgs U, float4 a, float4 b, float lx, float ly, bool self) {
+__device__ inline PinOut pin_any(PinArgs U, float4 a, float4 b, float lx, float ly, bool self) {
   const PinOut in{a, b, lx, ly};
   const float2 ta = sincos_f64(a.z), tb = sincos_f64(b.z);
   const float sa = ta.x, ca = ta.y, sb = tb.x, cb = tb.y;
@@ -528,44 +548,47 @@ static __device__ __noinline__ PinOut pin_any(PinArgs U, float4 a, float4 b, flo
   return PinOut{a, b, lx, ly};
 }
 
-// The same operations for a tame pin (kr_units.h pin_tame), without the
-// branches: the reference's
-// early returns become one condition on the update, and what needs another
-// path (an angle the rounding test does not decide, a divisor that recip
-// does not cover, an error of 1e15 or more or NaN) is evaluated again by
-// pin_any.  A predicate costs about 13 cycles and a branch on it 25 more in a
-// chain that nothing else hides, so the tests are folded into sums.
-__device__ __forceinline__ void pin_math(const PinArgs &U, float4 &a, float4 &b, float &lx, float &ly) {
+// The same operations for a tame pin (kr_units.h pin_tame), without a branch:
+// the reference's early returns become one condition on the update (on: the
+// pin is there and not broken), which otherwise adds 0.  Returns false, with
+// a, b, lx, ly of no use, where another path is needed: an angle the rounding
+// test does not decide, a divisor that recip does not cover, an error beyond
+// 1e15 or NaN.  A predicate costs about 13 cycles and a branch on it 25 more
+// in a chain that nothing else hides, so the tests are folded into sums.
+// World: lby and the compliance may be other than 0 (the engine's pins have
+// neither, so their terms are left out: the same values).
+template <bool World>
+__device__ __forceinline__ bool pin_near(const float2 *tab, const PinArgs &U, bool on, float4 &a, float4 &b, float &lx,
+                                         float &ly) {
   float sa, ca, sb, cb;
-  const float spread = fadd(sincos_near(a.z, &sa, &ca), sincos_near(b.z, &sb, &cb));
+  const float spread = fadd(sincos_near(tab, a.z, &sa, &ca), sincos_near(tab, b.z, &sb, &cb));
+  const float amax = fmaxf(fabsf(a.z), fabsf(b.z));
   const float rax = fsub(fmul(U.lax, ca), fmul(U.lay, sa)), ray = fadd(fmul(U.lax, sa), fmul(U.lay, ca));
-  const float rbx = fsub(fmul(U.lbx, cb), fmul(U.lby, sb)), rby = fadd(fmul(U.lbx, sb), fmul(U.lby, cb));
+  const float rbx = World ? fsub(fmul(U.lbx, cb), fmul(U.lby, sb)) : fmul(U.lbx, cb);
+  const float rby = World ? fadd(fmul(U.lbx, sb), fmul(U.lby, cb)) : fmul(U.lbx, sb);
   const float Cx = fsub(fadd(a.x, rax), fadd(b.x, rbx)), Cy = fsub(fadd(a.y, ray), fadd(b.y, rby));
   const float pax = -ray, pay = rax, pbx = -rby, pby = rbx;
-  const float wSum = fadd(U.wA, U.wB);
+  const float wSum = fadd(U.wA, U.wB), csq = fadd(fmul(Cx, Cx), fmul(Cy, Cy));
   const float k00 = fadd(fadd(wSum, fmul(fmul(U.wIA, pax), pax)), fmul(fmul(U.wIB, pbx), pbx));
   const float k01 = fadd(fmul(fmul(U.wIA, pax), pay), fmul(fmul(U.wIB, pbx), pby));
   const float k11 = fadd(fadd(wSum, fmul(fmul(U.wIA, pay), pay)), fmul(fmul(U.wIB, pby), pby));
   const float det = fsub(fmul(k00, k11), fmul(k01, k01));
-  const float bx = fadd(Cx, fmul(U.alphaTilde, lx)), by = fadd(Cy, fmul(U.alphaTilde, ly));
+  const float bx = World ? fadd(Cx, fmul(U.alphaTilde, lx)) : Cx, by = World ? fadd(Cy, fmul(U.alphaTilde, ly)) : Cy;
   const float y = recip(det);
   const float i00 = quot(k11, det, y), i11 = quot(k00, det, y), i01 = -quot(k01, det, y);
-  const float dlx = -fadd(fmul(i00, bx), fmul(i01, by)), dly = -fadd(fmul(i01, bx), fmul(i11, by));
-  if (!(fmaxf(fabsf(a.z), fabsf(b.z)) <= kSinCosNearMax && fadd(fabsf(bx), fabsf(by)) < 1e15f && mantissa_ok(det) &&
-        spread == 0.f)) {
-    const PinOut o = pin_any(U, a, b, lx, ly, false);
-    a = o.a; b = o.b; lx = o.lx; ly = o.ly;
-    return;
-  }
-  const bool upd = fadd(fmul(Cx, Cx), fmul(Cy, Cy)) >= fmul(kSlackPos, kSlackPos), updb = upd && U.hasB;
-  lx = upd ? fadd(lx, dlx) : lx;
-  ly = upd ? fadd(ly, dly) : ly;
-  a.x = upd ? fadd(a.x, fmul(U.wA, dlx)) : a.x;
-  a.y = upd ? fadd(a.y, fmul(U.wA, dly)) : a.y;
-  a.z = upd ? fadd(a.z, fmul(U.wIA, fadd(fmul(pax, dlx), fmul(pay, dly)))) : a.z;
-  b.x = updb ? fsub(b.x, fmul(U.wB, dlx)) : b.x;
-  b.y = updb ? fsub(b.y, fmul(U.wB, dly)) : b.y;
-  b.z = updb ? fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly)))) : b.z;
+  const bool upd = on && csq >= fmul(kSlackPos, kSlackPos);
+  const float dlx = upd ? -fadd(fmul(i00, bx), fmul(i01, by)) : 0.f;
+  const float dly = upd ? -fadd(fmul(i01, bx), fmul(i11, by)) : 0.f;
+  lx = fadd(lx, dlx);
+  ly = fadd(ly, dly);
+  a.x = fadd(a.x, fmul(U.wA, dlx));
+  a.y = fadd(a.y, fmul(U.wA, dly));
+  a.z = fadd(a.z, fmul(U.wIA, fadd(fmul(pax, dlx), fmul(pay, dly))));
+  b.x = fsub(b.x, fmul(U.wB, dlx));
+  b.y = fsub(b.y, fmul(U.wB, dly));
+  b.z = fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
+  const bool small = World ? fadd(fabsf(bx), fabsf(by)) < 1e15f : csq < 1e30f;
+  return !on || (amax <= kSinCosNearMax && small && mantissa_ok(det) && spread == 0.f);
 }
 
 // solveAngleF, f32solver.mjs:258-301 (solver.wgsl:292-350): muscle
@@ -577,7 +600,7 @@ struct AngleArgs {
 };
 
 // The reference form (as pin_any)
-static __device__ __noinline__ float3 angle_any(AngleArgs U, float az, float bz, float l, bool self) {
+__device__ inline float3 angle_any(AngleArgs U, float az, float bz, float l, bool self) {
   const float wSum = fadd(U.wA, U.wB);
   if (wSum <= 0.f) return make_float3(az, bz, l);
   const float dev = angle_delta(U.hasB ? angle_delta(bz, az) : az, U.rest);
@@ -612,44 +635,69 @@ static __device__ __noinline__ float3 angle_any(AngleArgs U, float az, float bz,
   return make_float3(az, bz, l);
 }
 
-// The same operations in near form (see pin_math).  Where a term is used,
-// |C| and |over| are at least kSlackAng, so the quotients' numerators are 0
-// or above 2^-40.
-__device__ __forceinline__ void angle_math(const AngleArgs &U, float &az, float &bz, float &l) {
+// The same operations in near form (as pin_near).  Where a term is used, |C|
+// and |over| are at least kSlackAng, so the quotients' numerators are 0 or
+// above 2^-40.  yw: recip(wA + wB).  World: any rest, target, masses and a
+// missing body B; the engine's joints have 0 <= rest <= 6.27 and |target| <
+// 1.95, so only the differences of the two angles can exceed kWrapNear.
+template <bool World>
+__device__ __forceinline__ bool angle_near(const AngleArgs &U, float yw, bool on, float &az, float &bz, float &l) {
+  const bool hasB = !World || U.hasB;
   const float wSum = fadd(U.wA, U.wB), den = fadd(wSum, U.alphaTilde);
-  const float y = recip(den), yw = recip(wSum);
-  const bool tame = recip_ok(den) && recip_ok(wSum) && wSum > 0.f;
-  const float x1 = U.hasB ? fsub(bz, az) : 0.f;
-  const float x2 = fsub(U.hasB ? wrap_near(x1) : az, U.rest);
+  const float y = recip(den);
+  const float x1 = hasB ? fsub(bz, az) : 0.f;
+  const float x2 = fsub(hasB ? wrap_near(x1) : az, U.rest);
   const float x3 = fsub(wrap_near(x2), U.tgt);
   const float C = wrap_near(x3);
   const float num = fadd(C, fmul(U.alphaTilde, l));
-  const float dl = -quot(num, den, y);
-  const bool act = fabsf(C) >= kSlackAng;
-  const float na = act ? (U.hasB ? fsub(az, fmul(U.wA, dl)) : fadd(az, fmul(U.wA, dl))) : az;
-  const float nb = act && U.hasB ? fadd(bz, fmul(U.wB, dl)) : bz;
-  const float x4 = U.hasB ? fsub(nb, na) : 0.f;
-  const float x5 = fsub(U.hasB ? wrap_near(x4) : na, U.rest);
+  const float dl = on && fabsf(C) >= kSlackAng ? -quot(num, den, y) : 0.f;
+  l = fadd(l, dl);
+  az = hasB ? fsub(az, fmul(U.wA, dl)) : fadd(az, fmul(U.wA, dl));
+  bz = hasB ? fadd(bz, fmul(U.wB, dl)) : bz;
+  const float x4 = hasB ? fsub(bz, az) : 0.f;
+  const float x5 = fsub(hasB ? wrap_near(x4) : az, U.rest);
   const float dev2 = wrap_near(x5);
   const float o1 = fsub(dev2, U.mx), o2 = fsub(dev2, U.mn);
-  const bool hi = o1 >= kSlackAng, lim = hi || o2 <= -kSlackAng;
-  const float over = hi ? o1 : o2, dl2 = -quot(over, wSum, yw);
-  const float far = fmaxf(fmaxf(fmaxf(fabsf(x1), fabsf(x2)), fmaxf(fabsf(x3), fabsf(x4))), fabsf(x5));
-  if (!(tame && fabsf(num) < 0x1p60f && far <= kWrapNear)) {  // NaN fails by num
-    const float3 o = angle_any(U, az, bz, l, false);
-    az = o.x; bz = o.y; l = o.z;
-    return;
+  // (limits the wrong way round: above the maximum the minimum does not act)
+  const bool hi = o1 >= kSlackAng, lim = hi || (o2 <= -kSlackAng && !(World && dev2 > U.mx));
+  const float dl2 = on && lim ? -quot(hi ? o1 : o2, wSum, yw) : 0.f;
+  az = hasB ? fsub(az, fmul(U.wA, dl2)) : fadd(az, fmul(U.wA, dl2));
+  bz = hasB ? fadd(bz, fmul(U.wB, dl2)) : bz;
+  float far = fmaxf(fabsf(x1), fabsf(x4));
+  if (World) far = fmaxf(fmaxf(far, fabsf(x2)), fmaxf(fabsf(x3), fabsf(x5)));
+  const bool tame = World ? recip_ok(den) && recip_ok(wSum) && wSum > 0.f : mantissa_ok(den);
+  return !on || (tame && fabsf(num) < 0x1p60f && far <= kWrapNear);  // NaN fails by num
+}
+
+// A unit in the reference form.  Out of line, values in and values out:
+// records passed by address would live in local memory on the near path too.
+struct UnitOut {
+  float4 a, b;
+  float lx, ly, l;
+};
+static __device__ __noinline__ UnitOut unit_any(PinArgs U, AngleArgs V, bool pin, bool angle, bool self, float4 a,
+                                                float4 b, float lx, float ly, float l) {
+  if (pin) {
+    const PinOut o = pin_any(U, a, b, lx, ly, self);
+    a = self ? o.b : o.a; b = o.b; lx = o.lx; ly = o.ly;
   }
-  l = act ? fadd(l, dl) : l;
-  az = lim ? (U.hasB ? fsub(na, fmul(U.wA, dl2)) : fadd(na, fmul(U.wA, dl2))) : na;
-  bz = lim && U.hasB ? fadd(nb, fmul(U.wB, dl2)) : nb;
+  if (angle) {
+    const float3 o = angle_any(V, a.z, b.z, l, self);
+    a.z = o.x; b.z = o.y; l = o.z;
+  }
+  return UnitOut{a, b, lx, ly, l};
 }
 
 // One sweep of the solve list, batched engine.  first: the first sweep of a
 // substep, where every multiplier starts from 0.  A pin's multiplier only
 // enters its own equation times its compliance, which is 0 for the
 // template's pins and grips, so only the grips' (the break test) and the
-// motors' are kept.
+// motors' are kept.  Joints, grips (held or not) and idle lanes run one
+// instruction stream; a pass ends in its only branch, for units that need
+// the reference form (their bodies are still in shared memory as they were).
+// The pass's 230 + 340 cycles of dependent arithmetic are what a creature's
+// step consists of; 12 creatures' solve took 104,000 cycles a step as
+// separate pin and angle levels with the reference's branches.
 template <int G>
 __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
   const float alpha_m = fmul(S.comp_m, K.invH2);
@@ -657,57 +705,31 @@ __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, b
   float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
   for (int p = 0; p < S.npass; p++) {
     const unsigned ab = __float_as_uint(r0.x);
-    const PinArgs U{r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, 0.f, (ab >> 16) != kNoMotor};
-    AngleArgs V{r2.y, r2.z, r2.w, 0.f, alpha_m, r1.z, r2.x, true};
+    const int A = ab & 0xff, B = (ab >> 8) & 0xff, m = (ab >> 16) & 0xff;
+    const bool joint = (ab & kRecJoint) != 0;
+    float4 a = S.Q[A], b = S.Q[B];
+    const float2 mo = S.mot[m];
+    const PinArgs U{r0.y, r0.z, r0.w, 0.f, r1.x, r1.y, r1.z, r1.w, 0.f, joint};
+    const AngleArgs V{r2.x, r2.y, r2.z, mo.x, alpha_m, r1.y, r1.w, true};
+    const float yw = r2.w;
     // the next pass's records: the loads wait on nothing the sweep computes
     rec += 3 * G;
     if (p + 1 < S.npass) { r0 = rec[0]; r1 = rec[1]; r2 = rec[2]; }
-    if (ab != kUnitIdle) {
-      const int A = ab & 0xff, B = (ab >> 8) & 0xff, m = ab >> 16;
-      float4 a = S.Q[A], b = S.Q[B];
-      const bool joint = U.hasB;
-      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-      float l = 0.f;
-      if (joint) {
-        const float2 mo = S.mot[m];
-        V.tgt = mo.x;
-        l = first ? 0.f : mo.y;
-      } else {
-        g = S.grip[B - S.nb];
-        if (first) g.x = g.y = 0.f;
-      }
-      // joints and grips that hold (b.w: the anchor's broken flag)
-      if (joint || b.w == 0.f) pin_math(U, a, b, g.x, g.y);
-      if (joint) {
-        angle_math(V, a.z, b.z, l);
-        S.mot[m].y = l;
-        S.Q[B] = b;
-      } else {
-        S.grip[B - S.nb] = g;
-      }
-      S.Q[A] = a;
+    const bool held = joint || ((ab & kRecIdle) == 0 && b.w == 0.f);  // b.w: an anchor's broken flag
+    const float l0 = first || !joint ? 0.f : mo.y;
+    const float lx0 = first || joint ? 0.f : mo.x, ly0 = first || joint ? 0.f : mo.y;
+    float lx = lx0, ly = ly0, l = l0;
+    const bool op = pin_near<false>(S.tab, U, held, a, b, lx, ly);
+    const bool oa = angle_near<false>(V, yw, joint, a.z, b.z, l);
+    if (!(op && oa && alpha_m < 0x1p59f)) {
+      const UnitOut o = unit_any(U, V, held, joint, false, S.Q[A], S.Q[B], lx0, ly0, l0);
+      a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;
     }
+    S.Q[A] = a;
+    if (joint) S.Q[B] = b;
+    S.mot[m] = joint ? make_float2(mo.x, l) : make_float2(lx, ly);
     L.sync();
   }
-}
-
-// A drop-in unit whose two bodies are one: every update sees the one before
-// it.  Out of line: no creature has one.
-static __device__ __noinline__ float4 solve_self(const SolverConsts &K, unsigned ab, float4 wa, float4 a, float4 *rec) {
-  const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3];
-  if ((ab & (kHasPin | kPinBroken)) == kHasPin) {
-    const PinOut o = pin_any(PinArgs{r0.y, r0.z, r0.w, r1.x, wa.x, wa.y, wa.x, wa.y, fmul(r1.y, K.invH2), true}, a, a,
-                             r1.z, r1.w, true);
-    a = o.b;
-    rec[1] = make_float4(r1.x, r1.y, o.lx, o.ly);
-  }
-  if ((ab & (kHasAngle | kAngleBroken)) == kHasAngle) {
-    const float3 o = angle_any(AngleArgs{r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wa.y, true}, a.z, a.z,
-                               r3.y, true);
-    a.z = o.y;
-    rec[3].y = o.z;
-  }
-  return a;
 }
 
 // One sweep of the solve list, drop-in world: unit records
@@ -716,48 +738,35 @@ static __device__ __noinline__ float4 solve_self(const SolverConsts &K, unsigned
 template <int G>
 __device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
   for (int p = 0; p < S.npass; p++) {
-    for (int u = S.off[p] + L.lane; u < S.off[p + 1]; u += G) {  // at most one: passes hold up to 32 units
+    const int u = S.off[p] + L.lane;  // passes hold at most 32 units
+    if (u < S.off[p + 1]) {
       float4 *rec = S.units + 4 * u;
-      const float4 r0 = rec[0];
+      const float4 r0 = rec[0], r2 = rec[2];
+      float4 r1 = rec[1], r3 = rec[3];
       const unsigned ab = __float_as_uint(r0.x);
       const int A = ab & 0xff, B = (ab >> 8) & 0xff;
       const bool hasB = B != 0xff;
-      float4 a = S.Q[A], b = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 wa = S.body[A];
-      if (A == B) {
-        if (first) { rec[1].z = rec[1].w = 0.f; rec[3].y = 0.f; }
-        S.Q[A] = solve_self(K, ab, wa, a, rec);
-        continue;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), anchor = make_float4(r0.w, r1.x, 1.f, 0.f);
+      const float4 wa = S.body[A], wb = hasB ? S.body[B] : zero;
+      float4 a = S.Q[A], b = hasB ? S.Q[B] : anchor;
+      const bool pin = (ab & (kHasPin | kPinBroken)) == kHasPin, angle = (ab & (kHasAngle | kAngleBroken)) == kHasAngle;
+      const PinArgs U{r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y, fmul(r1.y, K.invH2),
+                      hasB};
+      const AngleArgs V{r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wb.y, hasB};
+      if (first) r1.z = r1.w = r3.y = 0.f;
+      float lx = r1.z, ly = r1.w, l = r3.y;
+      const bool op = pin_near<true>(S.tab, U, pin, a, b, lx, ly) && (!pin || (ab & kPinTame) != 0);
+      const bool oa = angle_near<true>(V, recip(fadd(V.wA, V.wB)), angle, a.z, b.z, l);
+      // an inverse mass without bound times an update of 0 is not 0
+      const bool bounded = fadd(fadd(wa.x, wa.y), fadd(wb.x, wb.y)) < 1e30f;
+      if (!(op && oa && bounded) || A == B) {
+        const UnitOut o = unit_any(U, V, pin, angle, A == B, S.Q[A], hasB ? S.Q[B] : anchor, r1.z, r1.w, r3.y);
+        a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;
       }
-      float4 wb = b;
-      if (hasB) { b = S.Q[B]; wb = S.body[B]; }
-      if (ab & kHasPin) {
-        float4 r1 = rec[1];
-        if (first) r1.z = r1.w = 0.f;
-        if (!(ab & kPinBroken)) {
-          if (!hasB) b = make_float4(r0.w, r1.x, 1.f, 0.f);  // the anchor
-          const PinArgs U{r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y,
-                          fmul(r1.y, K.invH2), hasB};
-          if (ab & kPinTame) {
-            pin_math(U, a, b, r1.z, r1.w);
-          } else {
-            const PinOut o = pin_any(U, a, b, r1.z, r1.w, false);
-            a = o.a; b = o.b; r1.z = o.lx; r1.w = o.ly;
-          }
-        }
-        rec[1] = r1;
-      }
-      if (ab & kHasAngle) {
-        float4 r3 = rec[3];
-        if (first) r3.y = 0.f;
-        if (!(ab & kAngleBroken)) {
-          const float4 r2 = rec[2];
-          angle_math(AngleArgs{r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wb.y, hasB}, a.z, b.z, r3.y);
-        }
-        rec[3] = r3;
-      }
+      rec[1].z = lx; rec[1].w = ly;
+      rec[3].y = l;
       S.Q[A] = a;
-      if (hasB) S.Q[B] = b;
+      if (hasB && A != B) S.Q[B] = b;
     }
     L.sync();
   }
@@ -767,12 +776,19 @@ __device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bo
 // (solver.wgsl:373-402) -- per body, its points in order, each correction
 // cumulative.
 //
-// State of the near sets, the same in every lane of the group.
+// State of the near sets, the same in every lane of the group, in one word
+// (a struct returned by the out-of-line rebuild would live in local memory):
+// listed bodies with at most kFewPoints points, listed bodies with more, near
+// list entries, entries per mask bit (log2), valid (every body has a
+// reference), full (no usable list: every body against every rect).
 struct Near {
-  int few = 0, many = 0;   // listed bodies with at most kFewPoints points / with more
-  int n = 0, shift = 0;    // near list entries, entries per mask bit (log2)
-  bool valid = false;      // every body has a reference
-  bool full = false;       // no usable list: every body against every rect
+  unsigned w = 0;
+  __device__ __forceinline__ int few() const { return w & 0xff; }
+  __device__ __forceinline__ int many() const { return (w >> 8) & 0xff; }
+  __device__ __forceinline__ int n() const { return (w >> 16) & 0x7f; }
+  __device__ __forceinline__ int shift() const { return (w >> 23) & 1; }
+  __device__ __forceinline__ bool valid() const { return (w >> 24) & 1; }
+  __device__ __forceinline__ bool full() const { return (w >> 25) & 1; }
 };
 constexpr int kFewPoints = 2;
 
@@ -784,8 +800,8 @@ __device__ __forceinline__ float2 near_unpack(unsigned w) {
   return make_float2(__uint_as_float(0x4b000000u | (w & 0xffffu)) - 8421376.f,
                      __uint_as_float(0x4b000000u | (w >> 16)) - 8421376.f);
 }
-__device__ __forceinline__ bool near_holds(const float2 ref, float x, float y) {
-  return fabsf(x - ref.x) <= kNearMove && fabsf(y - ref.y) <= kNearMove;
+__device__ __forceinline__ bool near_holds(const float2 ref, float x, float y, unsigned mask) {
+  return fmaxf(fabsf(x - ref.x), fabsf(y - ref.y)) <= ((mask & kNearBit) ? kNearMove : kFarMove) && x == x && y == y;
 }
 // false only if the rect lies outside the box x0..x1 x y0..y1 (extents of
 // either sign; NaN counts as inside)
@@ -797,35 +813,43 @@ __device__ __forceinline__ bool in_box(const float4 r, float x0, float x1, float
 // positions.  near_d = D + kCullPad.  Out of line: it runs once per several
 // dozen passes.
 template <int G>
-__device__ __noinline__ Near near_rebuild(float4 *P, float4 *Q, const float4 *body, unsigned short *cull,
+__device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4 *body, unsigned short *cull,
                                           unsigned char *list, int nb, const float4 *__restrict__ rects, int nR,
                                           float near_d, Lanes<G> L) {
-  Near N;
+  int few_n = 0, many_n = 0, n = 0;
   float lx = kInf, ly = kInf, hx = -kInf, hy = -kInf;
   bool bad = nR > 65535;
   for (int j = L.lane; j < nb; j += G) {
     const float4 bd = body[j];
     if (bd.x == 0.f || (__float_as_int(bd.w) >> 16) == 0) continue;
     const float4 q = Q[j];
-    const float e = bd.z + near_d + kNearMove + kCullPad;
+    const float e = bd.z + near_d + kFarMove + kCullPad;
     if (!(fabsf(q.x) < 32000.f && fabsf(q.y) < 32000.f && e < 1e6f)) { bad = true; continue; }
     lx = fminf(lx, q.x - e); hx = fmaxf(hx, q.x + e);
     ly = fminf(ly, q.y - e); hy = fmaxf(hy, q.y + e);
   }
   lx = L.min(lx); ly = L.min(ly);
   hx = L.max(hx); hy = L.max(hy);
-  N.full = L.ballot(bad) != 0;
-  for (int base = 0; base < nR && !N.full; base += G) {
+  bool full = L.ballot(bad) != 0;
+  // the near list, with the wide move if it fits
+  float move = kFarMove;
+  for (int base = 0; base < nR && !full; base += G) {
     const int i = base + L.lane;
-    const bool keep = i < nR && in_box(__ldg(rects + i), lx, hx, ly, hy);
+    const float d = kFarMove - move;
+    const bool keep = i < nR && in_box(__ldg(rects + i), lx + d, hx - d, ly + d, hy - d);
     const unsigned m = L.ballot(keep);
-    const int at = N.n + __popc(m & ((1u << L.lane) - 1u));
+    const int at = n + __popc(m & ((1u << L.lane) - 1u));
     if (keep && at < kMaxCulled) cull[at] = (unsigned short)i;
-    N.n += __popc(m);
-    N.full = N.n > kMaxCulled;
+    n += __popc(m);
+    if (n > kMaxCulled) {
+      full = move == kNearMove;
+      move = kNearMove;
+      n = 0;
+      base = -G;
+      L.sync();
+    }
   }
-  N.shift = N.n > 32 ? 1 : 0;
-  N.valid = !N.full;
+  const int shift = n > 31 ? 1 : 0;
   L.sync();
   for (int base = 0; base < nb; base += G) {
     const int j = base + L.lane;
@@ -836,32 +860,39 @@ __device__ __noinline__ Near near_rebuild(float4 *P, float4 *Q, const float4 *bo
       unsigned mask = 0u;
       if (bd.x != 0.f && cnt != 0) {
         const float4 q = Q[j];
-        if (N.full) {
+        if (full) {
           mask = 1u;
         } else {
           const unsigned w = near_pack(q.x, q.y);
           const float2 ref = near_unpack(w);
-          const float e = bd.z + near_d + kNearMove;
-          for (int i = 0; i < N.n; i++)
-            if (in_box(__ldg(rects + cull[i]), ref.x - e, ref.x + e, ref.y - e, ref.y + e)) mask |= 1u << (i >> N.shift);
+          const float e = bd.z + near_d, en = e + kNearMove, ef = e + kFarMove;
+          bool wide = move == kNearMove;
+#pragma unroll 4
+          for (int i = 0; i < n; i++) {
+            const float4 r = __ldg(rects + cull[i]);
+            wide |= in_box(r, ref.x - ef, ref.x + ef, ref.y - ef, ref.y + ef);
+            if (in_box(r, ref.x - en, ref.x + en, ref.y - en, ref.y + en)) mask |= 1u << (i >> shift);
+          }
+          if (wide) mask |= kNearBit;
           P[j].w = __uint_as_float(w);
         }
         Q[j].w = __uint_as_float(mask);
-      } else if (!N.full) {
-        // a body without points is never tested: the reference only has to hold
+      } else if (!full) {
+        // a body without points meets no rect: the reference only has to hold
         P[j].w = __uint_as_float(near_pack(fminf(fmaxf(Q[j].x, -32000.f), 32000.f), fminf(fmaxf(Q[j].y, -32000.f), 32000.f)));
       }
-      few = mask != 0u && cnt <= kFewPoints;
-      many = mask != 0u && cnt > kFewPoints;
+      few = (mask & ~kNearBit) != 0u && cnt <= kFewPoints;
+      many = (mask & ~kNearBit) != 0u && cnt > kFewPoints;
     }
     const unsigned mf = L.ballot(few), mm = L.ballot(many), below = (1u << L.lane) - 1u;
-    if (few) list[N.few + __popc(mf & below)] = (unsigned char)j;
-    if (many) list[nb - 1 - (N.many + __popc(mm & below))] = (unsigned char)j;
-    N.few += __popc(mf);
-    N.many += __popc(mm);
+    if (few) list[few_n + __popc(mf & below)] = (unsigned char)j;
+    if (many) list[nb - 1 - (many_n + __popc(mm & below))] = (unsigned char)j;
+    few_n += __popc(mf);
+    many_n += __popc(mm);
   }
   L.sync();
-  return N;
+  return full ? (unsigned)few_n | ((unsigned)many_n << 8) | (1u << 25)
+              : (unsigned)few_n | ((unsigned)many_n << 8) | ((unsigned)n << 16) | ((unsigned)shift << 23) | (1u << 24);
 }
 
 // The fold at (x, y) over a body's near rects (or every rect)
@@ -871,8 +902,8 @@ __device__ __forceinline__ SdfFold near_fold(const Island &S, const Near &N, con
   if (all) {
     for (int i = 0; i < nR; i++) f.add(__ldg(rects + i), x, y);
   } else {
-    for (unsigned m = mask; m; m &= m - 1u) {
-      const int b = (__ffs(m) - 1) << N.shift, e = min(b + 1 + N.shift, N.n);
+    for (unsigned m = mask & ~kNearBit; m; m &= m - 1u) {
+      const int b = (__ffs(m) - 1) << N.shift(), e = min(b + 1 + N.shift(), N.n());
       for (int i = b; i < e; i++) f.add(__ldg(rects + S.cull[i]), x, y);
     }
   }
@@ -884,7 +915,7 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
                                                int j, float4 q, float sa, float ca, int from) {
   const int pr = __float_as_int(S.body[j].w), off = pr & 0xffff, cnt = pr >> 16;
   const unsigned mask = __float_as_uint(q.w);
-  bool all = N.full, moved = false;
+  bool all = N.full(), moved = false;
   for (int k = from; k < cnt; k++) {
     const float4 pt = S.pts[off + k];
     const float wx = fadd(q.x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
@@ -895,7 +926,7 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
       q.y = fadd(q.y, dy);
       moved = true;
       // pushed away from its reference: its near set may miss a rect
-      all = N.full || !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y);
+      all = N.full() || !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, mask);
     }
   }
   if (moved) S.Q[j] = q;
@@ -908,29 +939,30 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
 template <int G>
 __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 *__restrict__ rects, int nR,
                                                float near_d, const Lanes<G> &L) {
-  bool stale = !N.valid;
+  bool stale = !N.valid();
   if (!stale) {
     bool moved = false;
+#pragma unroll 2
     for (int j = L.lane; j < S.nb; j += G) {
       const float4 q = S.Q[j];
-      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y);
+      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, __float_as_uint(q.w));
     }
     stale = L.ballot(moved) != 0;
   }
-  if (stale) N = near_rebuild<G>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
-  for (int t = L.lane; t < N.few; t += G) {
+  if (stale) N.w = near_rebuild<G>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
+  for (int t = L.lane; t < N.few(); t += G) {
     const int j = S.list[t];
     const float4 q = S.Q[j];
     float sa, ca;
-    sincos_r(q.z, &sa, &ca);
+    sincos_r(S.tab, q.z, &sa, &ca);
     collide_points(S, N, rects, nR, j, q, sa, ca, 0);
   }
-  for (int t = 0; t < N.many; t++) {
+  for (int t = 0; t < N.many(); t++) {
     const int j = S.list[S.nb - 1 - t];
     const float4 q = S.Q[j];
     const int pr = __float_as_int(S.body[j].w), off = pr & 0xffff, cnt = pr >> 16;
     float sa, ca;
-    sincos_r(q.z, &sa, &ca);
+    sincos_r(S.tab, q.z, &sa, &ca);
     int first = -1;
     for (int base = 0; base < cnt && first < 0; base += G) {
       bool hit = false;
@@ -939,7 +971,7 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
         const float wx = fadd(q.x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
         const float wy = fadd(q.y, fadd(fmul(pt.x, sa), fmul(pt.y, ca)));
         float dx, dy;
-        hit = near_fold(S, N, rects, nR, N.full, __float_as_uint(q.w), wx, wy).push(pt.z, &dx, &dy);
+        hit = near_fold(S, N, rects, nR, N.full(), __float_as_uint(q.w), wx, wy).push(pt.z, &dx, &dy);
       }
       const unsigned m = L.ballot(hit);
       if (m) first = base + __ffs(m) - 1;
@@ -964,11 +996,7 @@ __device__ __forceinline__ void finalize_body(const SolverConsts &K, Island &S, 
   float vx = fmul(fsub(q.x, p.x), K.invH);
   float vy = fmul(fsub(q.y, p.y), K.invH);
   float av = fmul(angle_delta(q.z, p.z), K.invH);
-  float sp = length2(vx, vy);
-  if (sp > K.maxSpeed) {
-    float k = fdiv(K.maxSpeed, sp);
-    vx = fmul(vx, k); vy = fmul(vy, k);
-  }
+  clamp_speed(K, vx, vy);
   if (av > K.maxAngSpeed) av = K.maxAngSpeed;
   else if (av < -K.maxAngSpeed) av = -K.maxAngSpeed;
   if (q.z > 50.f || q.z < -50.f) {
@@ -997,6 +1025,7 @@ __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
                                             const Lanes<G> &L, Near &N) {
 #pragma unroll U
   for (int s = 0; s < K.substeps; s++) {
+#pragma unroll 2
     for (int i = L.lane; i < S.nb; i += G) integrate_body<World>(K, S, i);
     L.sync();
     for (int it = 0; it < K.iterations; it++) {
@@ -1004,6 +1033,7 @@ __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
       else solve_engine<G>(K, S, it == 0, L);
       collide_island<G>(S, N, rects, nR, near_d, L);
     }
+#pragma unroll 2
     for (int i = L.lane; i < S.nb; i += G) finalize_body<World>(K, S, i);
     L.sync();
   }
@@ -1019,11 +1049,11 @@ __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
       }
     }
   } else if (L.lane < S.arms) {
-    const float4 g = S.grip[L.lane];
+    const float2 g = S.mot[S.grip0 + L.lane];
     float4 &an = S.Q[S.nb + L.lane];
-    if (an.w == 0.f && grip_breaks(K, g.x, g.y, g.z)) {
+    if (an.w == 0.f && grip_breaks(K, g.x, g.y, S.brk[L.lane])) {
       an.w = 1.f;
-      S.grip[L.lane] = make_float4(0.f, 0.f, g.z, g.w);
+      S.mot[S.grip0 + L.lane] = make_float2(0.f, 0.f);
     }
   }
   L.sync();

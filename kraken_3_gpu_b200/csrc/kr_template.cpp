@@ -150,6 +150,15 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
       tame = joint ? pin_tame((float)c.lax, (float)c.lay, (float)c.lbx, (float)c.lby, t->im[u.a], t->ii[u.a],
                               t->im[u.b], t->ii[u.b])
                    : pin_tame((float)c.lax, (float)c.lay, 0.f, 0.f, t->im[u.a], t->ii[u.a], 0.f, 0.f);
+      tame = tame && c.lby == 0;
+    }
+    if (tame && joint) {
+      // what the engine's angle constraint relies on (kr_solver.cuh angle_near)
+      const RawCon &g = cons[list[u.ang]];
+      const float w = t->ii[u.a] + t->ii[u.b];
+      unsigned m;
+      std::memcpy(&m, &w, sizeof(m));
+      tame = g.rest >= 0 && g.rest <= 6.27 && w > 0x1p-60f && w < 0x1p60f && (m & 0x7fffffu) != 0x7fffffu;
     }
     if (!tame) {
       *err = "body shape " + std::to_string(arms) + "x" + std::to_string(segs) + ": a constraint outside the joints";
@@ -167,23 +176,28 @@ bool build_template(int arms, int segs, Template *t, std::string *err) {
       for (int l = 0; l < G; l++) {
         float *r = &S.recs[((size_t)p * G + l) * kRecFloats];
         if (off[p] + l >= off[p + 1]) {
-          r[0] = word(0xffffffffu);
+          const unsigned spare = (unsigned)(nb + arms);
+          r[0] = word(spare | (spare << 8) | ((unsigned)(grip_pair0(arms, segs) + arms) << 16) | kRecIdle);
+          r[4] = 1.f;
           continue;
         }
         const SolveUnit &u = units[order[off[p] + l]];
         const RawCon &c = cons[list[u.pin]];
         const unsigned B = u.b >= 0 ? (unsigned)u.b : (unsigned)(nb + c.arm);
-        const unsigned m = u.ang >= 0 ? (unsigned)cons[list[u.ang]].motor : 0xffu;
+        const unsigned m = u.ang >= 0 ? (unsigned)cons[list[u.ang]].motor | (kRecJoint >> 16)
+                                      : (unsigned)(grip_pair0(arms, segs) + c.arm);
         r[0] = word((unsigned)u.a | (B << 8) | (m << 16));
         r[1] = (float)c.lax; r[2] = (float)c.lay;
-        r[5] = t->im[u.a]; r[6] = t->ii[u.a];
+        r[4] = t->im[u.a]; r[5] = t->ii[u.a];
         if (u.b >= 0) {
-          r[3] = (float)c.lbx; r[4] = (float)c.lby;
-          r[7] = t->im[u.b]; r[8] = t->ii[u.b];
+          r[3] = (float)c.lbx;
+          r[6] = t->im[u.b]; r[7] = t->ii[u.b];
         }
         if (u.ang >= 0) {
           const RawCon &g = cons[list[u.ang]];
-          r[9] = (float)g.rest; r[10] = (float)g.minA; r[11] = (float)g.maxA;
+          r[8] = (float)g.rest; r[9] = (float)g.minA; r[10] = (float)g.maxA;
+          // rounded once: no f32 reciprocal lies within a f64 rounding of a midpoint
+          r[11] = (float)(1.0 / (double)(t->ii[u.a] + t->ii[u.b]));
         }
       }
     }

@@ -27,10 +27,10 @@ constexpr int schedule_index(int lanes) { return lanes == 32 ? 0 : lanes == 16 ?
 
 // One solve schedule of the constraint list: unit records pass by pass, one
 // per lane (idle lanes included), 3 float4 each:
-//   {A | B << 8 | motor << 16, lax, lay, lbx} {lby, 1 / mass A, 1 / inertia A,
-//   1 / mass B} {1 / inertia B, rest, min, max}
-// B of a grip is nb + arm, the record that holds its anchor, and its motor
-// 0xff; an idle lane's first word is 0xffffffff.
+//   {A | B << 8 | pair << 16 | flags, lax, lay, lbx} {1 / mass A, 1 / inertia
+//   A, 1 / mass B, 1 / inertia B} {rest, min, max, 1 / (sum of 1 / inertia)}
+// (kr_units.h kRecJoint, grip_pair0; lby is 0).  B of a grip is nb + arm, the record
+// that holds its anchor; an idle lane's bodies are nb + arms, a spare record.
 struct Schedule {
   int npass = 0;
   std::vector<float> recs;              // npass x lanes x kRecFloats

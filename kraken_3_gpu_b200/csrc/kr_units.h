@@ -33,6 +33,16 @@ KR_HD inline bool pin_tame(float lax, float lay, float lbx, float lby, float wA,
          lever_tame(lbx, lby, wIB, wS);
 }
 
+// The batched engine's unit records: flags of the ab word above body A, body B
+// << 8 and the index of its pair in the motors' records << 16; motors come
+// first, then (their words also hold the proprioception's 6 arms + 6) one
+// pair per grip and one for idle lanes.
+constexpr unsigned kRecJoint = 1u << 24, kRecIdle = 1u << 25;
+KR_HD inline int grip_pair0(int arms, int segs) {
+  const int m = 2 * arms * segs, o = 6 * arms + 6;
+  return (m > o ? m : o) / 2;
+}
+
 struct SolveEntry {
   int angle;  // 1: angle constraint, 0: pin or grip
   int a, b;   // bodies, b < 0: the world

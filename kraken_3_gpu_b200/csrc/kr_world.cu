@@ -64,7 +64,7 @@ struct StepArgs {
 };
 
 __host__ __device__ inline int warp_smem_words(int mb, int mu, int mp) {
-  return 20 * mb + 16 * mu + 4 * mp + kr::kMaxCulled / 2 + mb;
+  return 20 * mb + 16 * mu + 4 * mp + 4 * ((kr::kMaxCulled + 7) / 8) + mb;
 }
 
 // Writable views of the statics while they are staged; the solver reads them
@@ -79,7 +79,7 @@ __device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, i
   V.body = q; q += mb;
   S.units = q; q += 4 * mu;
   V.pts = q; q += mp;
-  S.cull = reinterpret_cast<unsigned short *>(q); q += kr::kMaxCulled / 8;
+  S.cull = reinterpret_cast<unsigned short *>(q); q += (kr::kMaxCulled + 7) / 8;
   S.list = reinterpret_cast<unsigned char *>(q);
   S.body = V.body; S.pts = V.pts;
 }
@@ -88,6 +88,9 @@ __device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, i
 // plain kernel and its allocation-free variant).
 __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   extern __shared__ __align__(16) float smem[];
+  __shared__ float2 s_sin[512];
+  kr::stage_sin(s_sin);
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int island = blockIdx.x * kWarpsPerBlock + warp;
   if (island >= A.nI) return;
@@ -99,6 +102,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   S.nb = rec[I_NB]; S.nu = rec[I_NU];
   S.npass = rec[I_NPASS];
   S.off = A.T.pass + rec[I_PASS_OFF];
+  S.tab = s_sin;
 
   // stage bodies (48 B AoS), forces and the bodies' collision points
   for (int i = lane; i < S.nb; i += 32) {
@@ -191,7 +195,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   }
 }
 
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) plain_step_kernel(StepArgs A) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) plain_step_kernel(StepArgs A) {
   plain_step_body(A);
 }
 
@@ -882,7 +886,7 @@ __global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint3
   W[kOffHdr + 0] = nI;
 }
 
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) noalloc_step_kernel(StepArgs A, const int *W) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) noalloc_step_kernel(StepArgs A, const int *W) {
   StepArgs B = A;
   B.nI = W[kOffHdr + 0];
   B.near_d = reinterpret_cast<const float *>(W)[kOffHdr + 1];

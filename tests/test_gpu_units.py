@@ -128,11 +128,12 @@ def _clutter(n, seed):
                                             r.uniform(4, 30, n)], 1)])
 
 
-@pytest.mark.parametrize("n,offset", [(0, 0.0), (12, 0.0), (40, 0.0), (58, 0.0), (59, 0.0), (60, 0.0), (200, 0.0),
+@pytest.mark.parametrize("n,offset", [(0, 0.0), (12, 0.0), (25, 0.0), (26, 0.0), (27, 0.0), (40, 0.0), (56, 0.0),
+                                      (57, 0.0), (58, 0.0), (200, 0.0),
                                       (70000, 0.0), (12, 31900.0), (12, 40000.0)])
 def test_near_rects_equal_the_full_list(n, offset):
     """Collision passes over the near sets (one rect or two per mask bit), and
-    over every rect where a creature has more than 64 near it, coordinates
+    over every rect where a creature has more than 62 near it, coordinates
     outside the references' range or the map more than 65,535 rects: the
     oracle folds over every rect each time."""
     rects = _clutter(min(n, 200), n)

@@ -94,11 +94,14 @@ int main() {
           for (int l = 0; l < G; l++) {
             unsigned ab;
             std::memcpy(&ab, &s.recs[((size_t)p * G + l) * kr::kRecFloats], 4);
-            if (ab == 0xffffffffu) continue;
-            const int a = ab & 0xff, b = (ab >> 8) & 0xff, m = ab >> 16;
+            const int a = ab & 0xff, b = (ab >> 8) & 0xff, m = (ab >> 16) & 0xff, g0 = kr::grip_pair0(A, S);
+            if (ab & kr::kRecIdle) {
+              if (a != T.nb + A || b != a || m != g0 + A || (ab & kr::kRecJoint)) return fail("idle", A * 10 + S);
+              continue;
+            }
             if (a >= T.nb || b >= T.nb + A || used[a]++ || used[b]++) return fail("record bodies", A * 10 + S);
-            if (m == 0xff) { if (b < T.nb || grip[b - T.nb]++ || a != T.arm_tip[b - T.nb]) return fail("grip", m); }
-            else if (m >= A * S || joint[m]++ || b != T.arm_segs[m]) return fail("joint", m);
+            if (ab & kr::kRecJoint) { if (m >= A * S || joint[m]++ || b != T.arm_segs[m]) return fail("joint", m); }
+            else if (b < T.nb || grip[b - T.nb]++ || a != T.arm_tip[b - T.nb] || m != g0 + b - T.nb) return fail("grip", m);
           }
         }
         for (int j : joint) if (j != 1) return fail("joints", A * 10 + S);
