@@ -374,8 +374,9 @@ int prepare_spawn(kr_batch *b, int n, const int32_t *arms, const int32_t *segs, 
                   const uint32_t *control_seed, const float *tone, int ctrl_mode, SpawnInit *out,
                   int *first_bad);
 // writes prepared creatures into the given slots (device copies of the
-// pose / meta / slot arrays), asynchronous on `stream`
-cudaError_t launch_spawn(kr_batch *b, const int *d_slots, const float *d_pose, const SlotMeta *d_meta,
+// pose / meta / slot arrays; without a slot array first, first + 1, ...),
+// asynchronous on `stream`
+cudaError_t launch_spawn(kr_batch *b, const int *d_slots, int first, const float *d_pose, const SlotMeta *d_meta,
                          int n, cudaStream_t stream);
 cudaStream_t part_stream(const kr_batch *b, const Part &p);
 // the metrics record of a slot (kraken_batch.h, KR_METRIC_WORDS), score included

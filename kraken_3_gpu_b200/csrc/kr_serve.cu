@@ -457,7 +457,7 @@ int admit(kr_server *S, int p) {
                                   cudaMemcpyHostToDevice, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(st.d_meta, st.h_meta, (size_t)n_new * sizeof(SlotMeta), cudaMemcpyHostToDevice, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(st.d_slots, st.h_slots, (size_t)n_new * sizeof(int), cudaMemcpyHostToDevice, stream);
-  if (e == cudaSuccess) e = launch_spawn(S->b, st.d_slots, st.d_pose, st.d_meta, n_new, stream);
+  if (e == cudaSuccess) e = launch_spawn(S->b, st.d_slots, 0, st.d_pose, st.d_meta, n_new, stream);
   if (e == cudaSuccess && S->d_done) {
     clear_done_kernel<<<(n_new + 255) / 256, 256, 0, stream>>>(st.d_meta, st.d_slots, n_new, S->d_done);
     e = cudaGetLastError();

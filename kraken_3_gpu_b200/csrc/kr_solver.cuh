@@ -431,7 +431,7 @@ struct Island {
   unsigned short *cull;       // near list (kMaxCulled rect indices)
   unsigned char *list;        // bodies with near rects: one or two points from the front, more from the back
   int nb;
-  // drop-in world: one dynamic record of 4 float4 per unit, pass offsets
+  // drop-in world: one dynamic record of 5 float4 per unit, pass offsets
   float4 *units;
   int nu, npass;
   const int *off;      // npass + 1 unit offsets
@@ -450,7 +450,9 @@ struct Island {
 // ab word of a unit: body A, body B << 8, and flags.  Drop-in world: B is 0xff
 // for the world.
 constexpr unsigned kHasPin = 1u << 16, kPinBroken = 1u << 17, kHasAngle = 1u << 18, kAngleBroken = 1u << 19,
-                   kPinIsGrip = 1u << 20, kPinTame = 1u << 21;
+                   kPinIsGrip = 1u << 20, kPinTame = 1u << 21,
+                   // two bodies whose inverse masses are finite (an update of 0 times them is 0)
+                   kBounded = 1u << 22;
 
 // The speed clamp of integrateF and finalizeF.  A squared speed of at most
 // 0.999 maxSpeed^2 has a length of at most maxSpeed however it rounds, so the
@@ -733,41 +735,52 @@ __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, b
 }
 
 // One sweep of the solve list, drop-in world: unit records
-// {ab, lax, lay, lbx} {lby, pin compliance, lambda x, y}
-// {rest, min, max, target} {angle compliance, lambda, break force, -}.
+// {ab, lax, lay, lbx} {lby, 1 / mass A, 1 / inertia A, 1 / mass B}
+// {1 / inertia B, rest, min, max} {target, pin compliance / h^2, angle
+// compliance / h^2, recip of the inertias' sum} {lambda x, y, lambda, break
+// force}; lb is 0 without a body B.  As solve_engine, the next pass's static
+// part loads while the current one computes.
+constexpr int kWorldRec = 5;
 template <int G>
-__device__ __forceinline__ void solve_world(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
+__device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G> &L) {
+  int beg = 0, end = S.npass > 0 ? S.off[1] : 0;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 r0 = zero, r1 = zero, r2 = zero, r3 = zero;
+  auto load = [&](int u) {
+    const float4 *rec = S.units + kWorldRec * u;
+    r0 = rec[0]; r1 = rec[1]; r2 = rec[2]; r3 = rec[3];
+  };
+  if (L.lane < end) load(L.lane);
   for (int p = 0; p < S.npass; p++) {
-    const int u = S.off[p] + L.lane;  // passes hold at most 32 units
-    if (u < S.off[p + 1]) {
-      float4 *rec = S.units + 4 * u;
-      const float4 r0 = rec[0], r2 = rec[2];
-      float4 r1 = rec[1], r3 = rec[3];
-      const unsigned ab = __float_as_uint(r0.x);
-      const int A = ab & 0xff, B = (ab >> 8) & 0xff;
-      const bool hasB = B != 0xff;
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), anchor = make_float4(r0.w, r1.x, 1.f, 0.f);
-      const float4 wa = S.body[A], wb = hasB ? S.body[B] : zero;
+    const int u = beg + L.lane;  // passes hold at most 32 units
+    const bool mine = u < end;
+    const int next = p + 1 < S.npass ? S.off[p + 2] : end;
+    const unsigned ab = __float_as_uint(r0.x);
+    const int A = ab & 0xff, B = (ab >> 8) & 0xff;
+    const bool hasB = B != 0xff;
+    const float4 anchor = make_float4(r0.w, r1.x, 1.f, 0.f);
+    const PinArgs U{r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, r1.y, r1.z, r1.w, r2.x, r3.y, hasB};
+    const AngleArgs V{r2.y, r2.z, r2.w, r3.x, r3.z, r1.z, r2.x, hasB};
+    const float yw = r3.w;
+    if (end + L.lane < next) load(end + L.lane);
+    if (mine) {
       float4 a = S.Q[A], b = hasB ? S.Q[B] : anchor;
+      float4 d = S.units[kWorldRec * u + 4];
+      if (first) d.x = d.y = d.z = 0.f;
       const bool pin = (ab & (kHasPin | kPinBroken)) == kHasPin, angle = (ab & (kHasAngle | kAngleBroken)) == kHasAngle;
-      const PinArgs U{r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y, fmul(r1.y, K.invH2),
-                      hasB};
-      const AngleArgs V{r2.x, r2.y, r2.z, r2.w, fmul(r3.x, K.invH2), wa.y, wb.y, hasB};
-      if (first) r1.z = r1.w = r3.y = 0.f;
-      float lx = r1.z, ly = r1.w, l = r3.y;
+      float lx = d.x, ly = d.y, l = d.z;
       const bool op = pin_near<true>(S.tab, U, pin, a, b, lx, ly) && (!pin || (ab & kPinTame) != 0);
-      const bool oa = angle_near<true>(V, recip(fadd(V.wA, V.wB)), angle, a.z, b.z, l);
-      // an inverse mass without bound times an update of 0 is not 0
-      const bool bounded = fadd(fadd(wa.x, wa.y), fadd(wb.x, wb.y)) < 1e30f;
-      if (!(op && oa && bounded) || A == B) {
-        const UnitOut o = unit_any(U, V, pin, angle, A == B, S.Q[A], hasB ? S.Q[B] : anchor, r1.z, r1.w, r3.y);
+      const bool oa = angle_near<true>(V, yw, angle, a.z, b.z, l);
+      if (!(op && oa && (ab & kBounded))) {
+        const UnitOut o = unit_any(U, V, pin, angle, A == B, S.Q[A], hasB ? S.Q[B] : anchor, d.x, d.y, d.z);
         a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;
       }
-      rec[1].z = lx; rec[1].w = ly;
-      rec[3].y = l;
+      S.units[kWorldRec * u + 4] = make_float4(lx, ly, l, d.w);
       S.Q[A] = a;
       if (hasB && A != B) S.Q[B] = b;
     }
+    beg = end;
+    end = next;
     L.sync();
   }
 }
@@ -1029,7 +1042,7 @@ __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
     for (int i = L.lane; i < S.nb; i += G) integrate_body<World>(K, S, i);
     L.sync();
     for (int it = 0; it < K.iterations; it++) {
-      if constexpr (World) solve_world<G>(K, S, it == 0, L);
+      if constexpr (World) solve_world<G>(S, it == 0, L);
       else solve_engine<G>(K, S, it == 0, L);
       collide_island<G>(S, N, rects, nR, near_d, L);
     }
@@ -1039,13 +1052,13 @@ __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
   }
   if constexpr (World) {
     for (int u = L.lane; u < S.nu; u += G) {
-      float4 *rec = S.units + 4 * u;
+      float4 *rec = S.units + kWorldRec * u;
       const unsigned ab = __float_as_uint(rec[0].x);
       if ((ab & (kHasPin | kPinIsGrip | kPinBroken)) != (kHasPin | kPinIsGrip)) continue;
-      const float4 r1 = rec[1];
-      if (grip_breaks(K, r1.z, r1.w, rec[3].z)) {
+      const float4 d = rec[4];
+      if (grip_breaks(K, d.x, d.y, d.w)) {
         rec[0].x = __uint_as_float(ab | kPinBroken);
-        rec[1] = make_float4(r1.x, r1.y, 0.f, 0.f);
+        rec[4] = make_float4(0.f, 0.f, d.z, d.w);
       }
     }
   } else if (L.lane < S.arms) {

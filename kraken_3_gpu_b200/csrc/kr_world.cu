@@ -1,5 +1,5 @@
 // kr_world.cu -- the gpuworld.js drop-in: handle, schedule and the plain
-// per-step kernel (one launch per env step, one warp per creature).
+// step kernel (one launch per kr_step call, one warp per creature).
 //
 // Device buffers hold the reference's own AoS blocks (48 B bodies, 80 B
 // constraints, 16 B forces / collision points), so upload and download are
@@ -35,6 +35,9 @@ namespace {
 thread_local std::string g_last_error;
 
 constexpr int kWarpsPerBlock = 4;
+// Env steps of one launch at most (a few ms): a launch stages the whole world
+// from and to global memory, which took a fifth of a one-step launch.
+constexpr int kStepsPerLaunch = 128;
 
 // Per-island record, one int array of kIslandInts per island.
 enum { I_BODY_OFF = 0, I_NB, I_UNIT_OFF, I_NU, I_PT_OFF, I_PASS_OFF, I_NPASS, kIslandInts };
@@ -59,12 +62,13 @@ struct StepArgs {
   int nR;
   float near_d;            // rect culling distance of a collision pass (kr_solver.cuh)
   int nI;
+  int n_steps;             // env steps of the launch
   int maxB, maxU, maxP;    // smem carve sizes (per warp)
   DeviceTables T;
 };
 
 __host__ __device__ inline int warp_smem_words(int mb, int mu, int mp) {
-  return 20 * mb + 16 * mu + 4 * mp + 4 * ((kr::kMaxCulled + 7) / 8) + mb;
+  return 20 * mb + 4 * kr::kWorldRec * mu + 4 * mp + 4 * ((kr::kMaxCulled + 7) / 8) + mb;
 }
 
 // Writable views of the statics while they are staged; the solver reads them
@@ -77,7 +81,7 @@ __device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, i
   float4 *q = reinterpret_cast<float4 *>(base);
   S.P = q; q += mb; S.Q = q; q += mb; S.V = q; q += mb; S.force = q; q += mb;
   V.body = q; q += mb;
-  S.units = q; q += 4 * mu;
+  S.units = q; q += kr::kWorldRec * mu;
   V.pts = q; q += mp;
   S.cull = reinterpret_cast<unsigned short *>(q); q += (kr::kMaxCulled + 7) / 8;
   S.list = reinterpret_cast<unsigned char *>(q);
@@ -129,34 +133,43 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   for (int u = lane; u < S.nu; u += 32) {
     const int4 t = A.T.units[uo + u];
     unsigned ab = (unsigned)t.x;
-    float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0, r3 = r0;
+    const int bA = ab & 0xffu, bB = (ab >> 8) & 0xffu;
+    const bool has_b = bB != 0xff;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 wa = S.body[bA], wb = has_b ? S.body[bB] : zero;
+    float4 r0 = zero, r1 = make_float4(0.f, wa.x, wa.y, wb.x), r2 = make_float4(wb.y, 0.f, 0.f, 0.f), r3 = zero;
+    float brk = 0.f;
     if (t.y >= 0) {
       const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)t.y);
       const uint4 w0 = c4[0], w1 = c4[1], w2 = c4[2], w4 = c4[4];
       ab |= kr::kHasPin | (w4.y != 0u ? kr::kPinBroken : 0u) | ((w0.z & 0xffu) == 2u ? kr::kPinIsGrip : 0u);
       r0.y = __uint_as_float(w1.x); r0.z = __uint_as_float(w1.y);
       r0.w = __uint_as_float(w1.z); r1.x = __uint_as_float(w1.w);
-      r1.y = __uint_as_float(w2.x);
-      r3.z = __uint_as_float(w4.x);
-      const bool has_b = ((ab >> 8) & 0xffu) != 0xffu;
-      const float4 wa = S.body[ab & 0xffu];
-      const float4 wb = has_b ? S.body[(ab >> 8) & 0xffu] : make_float4(0.f, 0.f, 0.f, 0.f);
+      r3.y = kr::fmul(__uint_as_float(w2.x), A.K.invH2);
+      brk = __uint_as_float(w4.x);
       if (kr::pin_tame(r0.y, r0.z, has_b ? r0.w : 0.f, has_b ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y)) ab |= kr::kPinTame;
     }
     if (t.z >= 0) {
       const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)t.z);
       const uint4 w2 = c4[2], w3 = c4[3], w4 = c4[4];
       ab |= kr::kHasAngle | (w4.y != 0u ? kr::kAngleBroken : 0u);
-      r2 = make_float4(__uint_as_float(w2.y), __uint_as_float(w2.w), __uint_as_float(w3.x), __uint_as_float(w2.z));
-      r3.x = __uint_as_float(w2.x);
+      r2 = make_float4(wb.y, __uint_as_float(w2.y), __uint_as_float(w2.w), __uint_as_float(w3.x));
+      r3.x = __uint_as_float(w2.z);
+      r3.z = kr::fmul(__uint_as_float(w2.x), A.K.invH2);
+      r3.w = kr::recip(kr::fadd(wa.y, wb.y));
     }
+    if (bA != bB && wa.x + wa.y + wb.x + wb.y < 1e30f) ab |= kr::kBounded;
     r0.x = __uint_as_float(ab);
-    S.units[4 * u] = r0; S.units[4 * u + 1] = r1; S.units[4 * u + 2] = r2; S.units[4 * u + 3] = r3;
+    float4 *rec = S.units + kr::kWorldRec * u;
+    rec[0] = r0; rec[1] = r1; rec[2] = r2; rec[3] = r3; rec[4] = make_float4(0.f, 0.f, 0.f, brk);
   }
   __syncwarp();
 
+  // env steps back to back: what a launch per step would write back and stage
+  // again is what shared memory holds
   kr::Near near;
-  kr::island_step<true, 32>(A.K, S, A.rects, A.nR, A.near_d, kr::Lanes<32>(lane), near);
+  for (int s = 0; s < A.n_steps; s++)
+    kr::island_step<true, 32>(A.K, S, A.rects, A.nR, A.near_d, kr::Lanes<32>(lane), near);
 
   // write back bodies, consumed forces and constraint multipliers / flags
   for (int i = lane; i < S.nb; i += 32) {
@@ -176,12 +189,12 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   // and an angle constraint's pin multiplier end at 0
   for (int u = lane; u < S.nu; u += 32) {
     const int4 t = A.T.units[uo + u];
-    const unsigned ab = __float_as_uint(S.units[4 * u].x);
+    const unsigned ab = __float_as_uint(S.units[kr::kWorldRec * u].x);
+    const float4 d = S.units[kr::kWorldRec * u + 4];
     if (t.y >= 0) {
-      const float4 r1 = S.units[4 * u + 1];
       uint32_t *c = A.cons + 20 * (size_t)t.y;
-      c[13] = __float_as_uint(r1.z);
-      c[14] = __float_as_uint(r1.w);
+      c[13] = __float_as_uint(d.x);
+      c[14] = __float_as_uint(d.y);
       c[15] = 0u;
       c[17] = (ab & kr::kPinBroken) ? 1u : 0u;
     }
@@ -189,7 +202,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
       uint32_t *c = A.cons + 20 * (size_t)t.z;
       c[13] = 0u;
       c[14] = 0u;
-      c[15] = __float_as_uint(S.units[4 * u + 3].y);
+      c[15] = __float_as_uint(d.z);
       c[17] = (ab & kr::kAngleBroken) ? 1u : 0u;
     }
   }
@@ -625,7 +638,8 @@ extern "C" int kr_step(kr_world *w, int32_t n_steps) {
   const size_t smem = w->smem_bytes;
   cudaError_t e;
   const int grid = (w->nI + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  for (int s = 0; s < n_steps; s++) {
+  for (int s = 0; s < n_steps; s += kStepsPerLaunch) {
+    A.n_steps = std::min(kStepsPerLaunch, n_steps - s);
     plain_step_kernel<<<grid, 32 * kWarpsPerBlock, smem, w->stream>>>(A);
     e = cudaGetLastError();
     if (e != cudaSuccess) return w->cuda_fail(e, "plain_step_kernel launch");
@@ -975,7 +989,8 @@ extern "C" int kr_step_noalloc(const kr_solver_params *params, uint32_t n_bodies
                            (int)smem) != cudaSuccess)
     return KR_ERR_CUDA;
   const int grid = ((int)n_bodies + kWarpsPerBlock - 1) / kWarpsPerBlock;  // islands <= bodies
-  for (int s = 0; s < n_steps; s++) {
+  for (int s = 0; s < n_steps; s += kStepsPerLaunch) {
+    A.n_steps = std::min(kStepsPerLaunch, n_steps - s);
     noalloc_step_kernel<<<grid, 32 * kWarpsPerBlock, smem, st>>>(A, W);
     if (cudaGetLastError() != cudaSuccess) return KR_ERR_CUDA;
   }
