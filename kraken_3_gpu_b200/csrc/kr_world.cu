@@ -714,8 +714,8 @@ extern "C" void kr_destroy(kr_world *w) {
 // nothing on the device or the host.
 //
 // Scratch layout (words): island records, island bodies, units, island
-// points, body point ranges, pass offsets, rects, and the builder's
-// temporaries.  The array is shared by every call on a
+// points, body point ranges, pass offsets, rects.  The builder's temporaries
+// are in its block's shared memory.  The array is shared by every call on a
 // device and keeps the last call's contents; the builder initializes every
 // word it reads before reading it.
 // ---------------------------------------------------------------------------
@@ -734,170 +734,290 @@ constexpr int kOffPts = kOffUnits + 4 * kNaC;
 constexpr int kOffBpt = ((kOffPts + kNaP) + 1) & ~1;       // int2, 8-byte aligned
 constexpr int kOffPass = kOffBpt + 2 * kNaB;
 constexpr int kOffRects = ((kOffPass + kNaC + kNaB) + 3) & ~3;  // float4, 16-byte aligned
-constexpr int kOffParent = kOffRects + 4 * kNaR;
-constexpr int kOffIslandOf = kOffParent + kNaB;
-constexpr int kOffLocal = kOffIslandOf + kNaB;
-constexpr int kOffRootIsl = kOffLocal + kNaB;
-constexpr int kOffCnt = kOffRootIsl + kNaB;                 // kNaB + 1
-constexpr int kOffLast = kOffCnt + kNaB + 1;
-constexpr int kOffLastUnit = kOffLast + kNaB;
-constexpr int kOffList = kOffLastUnit + kNaB;               // constraints per island, list order
-constexpr int kOffLevel = kOffList + kNaC;                  // level of each unit
-constexpr int kOffTmp = (kOffLevel + kNaC + 3) & ~3;        // units in list order, int4
-constexpr int kOffCur = kOffTmp + 4 * kNaC;                 // kNaC + 1
-constexpr int kScratchWords = kOffCur + kNaC + 1;
+constexpr int kScratchWords = kOffRects + 4 * kNaR;
 
 static __device__ __align__(256) int g_noalloc_scratch[kScratchWords];
 
-// Single-thread schedule builder: the same islands, bodies, levels, slot
-// order and point ranges as build_schedule(), written into the scratch.
-__global__ void noalloc_schedule_kernel(int *W, const float *bodies, const uint32_t *cons,
-                                        const float *rects, const uint32_t *coll_pts,
-                                        const uint32_t *coll_range, int nB, int nC, int nP, int nR) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int *isl = W + kOffIsl, *ib = W + kOffBodies, *icons = W + kOffList;
-  int4 *units = reinterpret_cast<int4 *>(W + kOffUnits), *tmp = reinterpret_cast<int4 *>(W + kOffTmp);
-  int *ipts = W + kOffPts, *pass = W + kOffPass;
+// Schedule builder, one block: the islands, bodies and point ranges of
+// build_schedule() and the same units, in passes by level.  A single thread
+// over global memory took 5.3 ms for 40 creatures, all of it load latency;
+// here (a 40-creature call of 4 steps: 5.6 -> 0.27 ms) the temporaries are in
+// shared memory and only what is sequential by
+// nature runs in order -- the ranks within an island by one warp, 32 entries
+// at a time, and an island's units by one thread per island.
+constexpr int kBuildThreads = 1024;
+
+// Exclusive scan of v[0..n) in place, n <= 2 * kBuildThreads; returns the
+// total.  sums: 32 ints.  Every thread of the block calls it.
+__device__ __forceinline__ int block_scan(int *v, int n, int *sums) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int x0 = 2 * t < n ? v[2 * t] : 0, x1 = 2 * t + 1 < n ? v[2 * t + 1] : 0;
+  int x = x0 + x1;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sums[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int s = sums[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += y;
+    }
+    sums[lane] = s;
+  }
+  __syncthreads();
+  const int before = x - x0 - x1 + (warp ? sums[warp - 1] : 0), total = sums[31];
+  if (2 * t < n) v[2 * t] = before;
+  if (2 * t + 1 < n) v[2 * t + 1] = before + x0;
+  __syncthreads();
+  return total;
+}
+
+// The builder's shared memory
+struct BuildSmem {
+  int par[kNaB];             // union-find parent
+  int isl[kNaB];             // island of a body
+  int loc[kNaB];             // its index in the island
+  int bo[kNaB + 1];          // islands' body offsets
+  int co[kNaB + 1];          // islands' constraint offsets
+  int po[kNaB + 1];          // islands' point offsets
+  int cnt[kNaB + 1];
+  int last[kNaB], last_unit[kNaB];  // level and unit last on a body (by its place in island order)
+  int con[kNaC];             // island order: local a | b << 8 | angle << 16
+  int cur[kNaC + kNaB];      // level counts, nc + 1 words per island
+  unsigned short list[kNaC]; // island order: constraint index
+  short pin[kNaC], ang[kNaC];  // units in list order: place of their constraints
+  short level[kNaC];
+  int sums[32];
+  int bad;
+  double half_thick, r_max;
+};
+
+// Ranks by key in index order, by one warp: rank(i) = how many of 0..i-1 have
+// key(i); count[key] ends up as the number of entries.
+template <class Key, class Out>
+__device__ __forceinline__ void ordered_ranks(int n, int *count, Key key, Out out) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < n; base += 32) {
+    const int i = base + lane;
+    const int k = i < n ? key(i) : -1;
+    const unsigned m = __match_any_sync(0xffffffffu, k);
+    const int before = k >= 0 ? count[k] : 0;
+    __syncwarp();
+    const int r = __popc(m & ((1u << lane) - 1u));
+    if (k >= 0) {
+      out(i, before + r);
+      if (r == 0) count[k] = before + __popc(m);
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(kBuildThreads) noalloc_schedule_kernel(
+    int *W, const float *bodies, const uint32_t *cons, const float *rects, const uint32_t *coll_pts,
+    const uint32_t *coll_range, int nB, int nC, int nP, int nR) {
+  extern __shared__ __align__(16) unsigned char build_smem[];
+  BuildSmem &M = *reinterpret_cast<BuildSmem *>(build_smem);
+  const int t = threadIdx.x;
+  int *isl = W + kOffIsl, *ib = W + kOffBodies, *ipts = W + kOffPts, *pass = W + kOffPass;
+  int4 *units = reinterpret_cast<int4 *>(W + kOffUnits);
   int2 *bpt = reinterpret_cast<int2 *>(W + kOffBpt);
   float4 *r4 = reinterpret_cast<float4 *>(W + kOffRects);
-  int *parent = W + kOffParent, *island_of = W + kOffIslandOf, *local = W + kOffLocal;
-  int *root_isl = W + kOffRootIsl, *cnt = W + kOffCnt, *last = W + kOffLast;
-  int *last_unit = W + kOffLastUnit, *level = W + kOffLevel, *cur = W + kOffCur;
-  W[kOffHdr + 0] = 0;
-  W[kOffHdr + 2] = KR_OK;
-  // collRange must tile the points in body order (gpuworld.js:193-199).  The
-  // running sum is 64-bit and may never pass nP, so no count can wrap it and
-  // every range lies inside [0, nP): the point loops below stay in bounds.
-  uint64_t acc = 0;
-  for (int g = 0; g < nB; g++) {
-    if ((uint64_t)coll_range[g] != acc) { W[kOffHdr + 2] = KR_ERR_INVALID; return; }
-    acc += coll_range[nB + g];
-    if (acc > (uint64_t)nP) { W[kOffHdr + 2] = KR_ERR_INVALID; return; }
-  }
-  if (acc != (uint64_t)nP) { W[kOffHdr + 2] = KR_ERR_INVALID; return; }
-  for (int g = 0; g < nB; g++) { parent[g] = g; root_isl[g] = -1; }
-  for (int k = 0; k < nC; k++) {
-    const uint32_t a = cons[20 * (size_t)k], b = cons[20 * (size_t)k + 1];
-    if (a >= (uint32_t)nB || (b != 0xffffffffu && b >= (uint32_t)nB)) { W[kOffHdr + 2] = KR_ERR_INDEX; return; }
-    if (b != 0xffffffffu) {
-      int ra = (int)a, rb = (int)b;
-      while (parent[ra] != ra) { parent[ra] = parent[parent[ra]]; ra = parent[ra]; }
-      while (parent[rb] != rb) { parent[rb] = parent[parent[rb]]; rb = parent[rb]; }
-      if (ra != rb) parent[max(ra, rb)] = min(ra, rb);
+  auto fail = [&](int code) {
+    if (t == 0) {
+      W[kOffHdr + 0] = 0;
+      W[kOffHdr + 2] = code;
     }
+  };
+  // collRange must tile the points in body order (gpuworld.js:193-199).  A
+  // count above nP is refused by itself, so the 32-bit prefix sums of the
+  // others stay below 2^24 and every range lies inside [0, nP).
+  bool bad = false;
+  for (int g = t; g < nB; g += kBuildThreads) {
+    const uint32_t c = coll_range[nB + g];
+    bad |= c > (uint32_t)nP;
+    M.cnt[g] = c > (uint32_t)nP ? 0 : (int)c;
   }
-  int nI = 0;
-  for (int g = 0; g < nB; g++) {
-    int r = g;
-    while (parent[r] != r) r = parent[r];
-    if (root_isl[r] < 0) root_isl[r] = nI++;
-    island_of[g] = root_isl[r];
+  if (__syncthreads_or(bad)) { fail(KR_ERR_INVALID); return; }
+  const int total = block_scan(M.cnt, nB, M.sums);
+  for (int g = t; g < nB; g += kBuildThreads) bad |= coll_range[g] != (uint32_t)M.cnt[g];
+  if (__syncthreads_or(bad || total != nP)) { fail(KR_ERR_INVALID); return; }
+  // connected components: hook the larger root below the smaller until no
+  // constraint joins two; a component's root is its smallest body
+  for (int k = t; k < nC; k += kBuildThreads) {
+    const uint32_t a = cons[20 * (size_t)k], b = cons[20 * (size_t)k + 1];
+    bad |= a >= (uint32_t)nB || (b != 0xffffffffu && b >= (uint32_t)nB);
   }
-  // bodies per island, ascending
-  for (int I = 0; I <= nI; I++) cnt[I] = 0;
-  for (int g = 0; g < nB; g++) cnt[island_of[g] + 1]++;
-  for (int I = 0; I < nI; I++) cnt[I + 1] += cnt[I];
-  for (int I = 0; I < nI; I++) {
-    int *rec = isl + I * kIslandInts;
-    rec[I_BODY_OFF] = cnt[I];
-    rec[I_NB] = cnt[I + 1] - cnt[I];
-    if (rec[I_NB] > KR_MAX_ISLAND_BODIES) { W[kOffHdr + 2] = KR_ERR_CAPACITY; return; }
+  if (__syncthreads_or(bad)) { fail(KR_ERR_INDEX); return; }
+  for (int g = t; g < nB; g += kBuildThreads) M.par[g] = g;
+  __syncthreads();
+  auto root = [&](int x) {
+    for (;;) {
+      const int p = *(volatile int *)&M.par[x];
+      if (p == x) return x;
+      x = p;
+    }
+  };
+  for (int round = 0; round < nB; round++) {  // ends after a few rounds: every round joins what it finds apart
+    bool joined = false;
+    for (int k = t; k < nC; k += kBuildThreads) {
+      const uint32_t b = cons[20 * (size_t)k + 1];
+      if (b == 0xffffffffu) continue;
+      const int ra = root((int)cons[20 * (size_t)k]), rb = root((int)b);
+      if (ra != rb) {
+        atomicMin(&M.par[max(ra, rb)], min(ra, rb));
+        joined = true;
+      }
+    }
+    if (!__syncthreads_or(joined)) break;
+    for (int g = t; g < nB; g += kBuildThreads) M.par[g] = root(g);
+    __syncthreads();
   }
-  for (int I = 0; I < nI; I++) cur[I] = cnt[I];
-  for (int g = 0; g < nB; g++) {
-    const int I = island_of[g];
-    local[g] = cur[I] - cnt[I];
-    ib[cur[I]++] = g;
+  // islands in order of their smallest body
+  for (int g = t; g < nB; g += kBuildThreads) M.last[g] = M.par[g] == g ? 1 : 0;
+  __syncthreads();
+  const int nI = block_scan(M.last, nB, M.sums);
+  for (int g = t; g < nB; g += kBuildThreads) {
+    M.isl[g] = M.last[M.par[g]];
+    M.cnt[g] = 0;
   }
-  // constraints per island, list order
-  for (int I = 0; I <= nI; I++) cnt[I] = 0;
-  for (int k = 0; k < nC; k++) cnt[island_of[cons[20 * (size_t)k]] + 1]++;
-  for (int I = 0; I < nI; I++) cnt[I + 1] += cnt[I];
-  for (int I = 0; I < nI; I++) cur[I] = cnt[I];
-  for (int k = 0; k < nC; k++) icons[cur[island_of[cons[20 * (size_t)k]]]++] = k;
-  // units per island and their levels (each on the first level after every
-  // earlier unit sharing a body), then a stable counting sort by level; a
-  // level of more than 32 units takes several passes
-  int pass_off = 0, pt_off = 0, unit_off = 0;
-  for (int I = 0; I < nI; I++) {
-    int *rec = isl + I * kIslandInts;
-    const int co = cnt[I], nc = cnt[I + 1] - cnt[I], bo = rec[I_BODY_OFF], nb = rec[I_NB];
-    if (nc > KR_MAX_ISLAND_CONSTRAINTS) { W[kOffHdr + 2] = KR_ERR_CAPACITY; return; }
-    for (int j = 0; j < nb; j++) { last[j] = -1; last_unit[j] = -1; }
+  __syncthreads();
+  // bodies per island, ascending; constraints per island, list order
+  if (t < 32) ordered_ranks(nB, M.cnt, [&](int g) { return M.isl[g]; }, [&](int g, int r) { M.loc[g] = r; });
+  __syncthreads();
+  for (int I = t; I < nI; I += kBuildThreads) {
+    bad |= M.cnt[I] > KR_MAX_ISLAND_BODIES;
+    M.bo[I] = M.cnt[I];
+    M.co[I] = 0;
+    M.cnt[I] = 0;
+  }
+  if (__syncthreads_or(bad)) { fail(KR_ERR_CAPACITY); return; }
+  const int nb_all = block_scan(M.bo, nI, M.sums);
+  for (int k = t; k < nC; k += kBuildThreads) {
+    const int I = M.isl[cons[20 * (size_t)k]];
+    M.con[k] = I;  // for now: the constraint's island
+    atomicAdd(&M.co[I], 1);
+  }
+  if (t == 0) M.bo[nI] = nb_all;
+  __syncthreads();
+  for (int I = t; I < nI; I += kBuildThreads) bad |= M.co[I] > KR_MAX_ISLAND_CONSTRAINTS;
+  if (__syncthreads_or(bad)) { fail(KR_ERR_CAPACITY); return; }
+  const int nc_all = block_scan(M.co, nI, M.sums);
+  if (t == 0) M.co[nI] = nc_all;
+  __syncthreads();
+  if (t < 32)
+    ordered_ranks(nC, M.cnt, [&](int k) { return M.con[k]; },
+                  [&](int k, int r) { M.list[M.co[M.con[k]] + r] = (unsigned short)k; });
+  for (int g = t; g < nB; g += kBuildThreads) {
+    const int at = M.bo[M.isl[g]] + M.loc[g];
+    ib[at] = g;
+    M.last[at] = -1;
+    M.last_unit[at] = -1;
+  }
+  __syncthreads();
+  for (int q = t; q < nC; q += kBuildThreads) {
+    const uint32_t *c = cons + 20 * (size_t)M.list[q];
+    const int b = c[1] == 0xffffffffu ? 0xff : M.loc[c[1]];
+    M.con[q] = M.loc[c[0]] | (b << 8) | ((c[2] & 0xffu) == 1u ? 1 << 16 : 0);
+  }
+  __syncthreads();
+  // per island: units and their levels (each on the first level after every
+  // earlier unit sharing a body), a stable counting sort by level (a level of
+  // more than 32 units takes several passes), point ranges of its bodies
+  for (int I = t; I < nI; I += kBuildThreads) {
+    const int co = M.co[I], nc = M.co[I + 1] - co, bo = M.bo[I], nb = M.bo[I + 1] - bo;
+    int *last = M.last + bo, *last_unit = M.last_unit + bo;
     int nlv = 0, nu = 0, nul = 0;
-    for (int q = 0; q < nc; q++) {
-      const int k = icons[co + q];
-      const uint32_t *c = cons + 20 * (size_t)k;
-      const int a = local[c[0]];
-      const int b = c[1] == 0xffffffffu ? -1 : local[c[1]];
-      const bool angle = (c[2] & 0xffu) == 1u;
+    for (int q = co; q < co + nc; q++) {
+      const int c = M.con[q], a = c & 0xff, b = (c >> 8) & 0xff, angle = c >> 16;
       int L = last[a] + 1;
-      if (b >= 0) L = max(L, last[b] + 1);
+      if (b != 0xff) L = max(L, last[b] + 1);
       last[a] = L;
-      if (b >= 0) last[b] = L;
+      if (b != 0xff) last[b] = L;
       nlv = max(nlv, L + 1);
-      const int ab = a | ((b >= 0 ? b : 0xff) << 8), u = last_unit[a];
-      if (angle && u >= 0 && (b < 0 || last_unit[b] == u) && tmp[u].y >= 0 && tmp[u].z < 0 && tmp[u].x == ab) {
-        tmp[u].z = k;
+      const int u = last_unit[a], ub = b != 0xff ? last_unit[b] : u;
+      if (angle && u >= 0 && ub == u && M.pin[co + u] >= 0 && M.ang[co + u] < 0 &&
+          (M.con[M.pin[co + u]] & 0xffff) == (c & 0xffff)) {
+        M.ang[co + u] = (short)q;
         continue;
       }
-      int ul = u >= 0 ? level[u] + 1 : 0;
-      if (b >= 0 && last_unit[b] >= 0) ul = max(ul, level[last_unit[b]] + 1);
-      tmp[nu] = make_int4(ab, angle ? -1 : k, angle ? k : -1, 0);
-      level[nu] = ul;
+      int ul = u >= 0 ? M.level[co + u] + 1 : 0;
+      if (ub >= 0) ul = max(ul, M.level[co + ub] + 1);
+      M.pin[co + nu] = angle ? -1 : (short)q;
+      M.ang[co + nu] = angle ? (short)q : -1;
+      M.level[co + nu] = (short)ul;
       nul = max(nul, ul + 1);
       last_unit[a] = nu;
-      if (b >= 0) last_unit[b] = nu;
+      if (b != 0xff) last_unit[b] = nu;
       nu++;
     }
-    if (nlv > KR_MAX_LEVELS) { W[kOffHdr + 2] = KR_ERR_CAPACITY; return; }
+    bad |= nlv > KR_MAX_LEVELS;
+    // cur has nc + 1 words per island
+    int *cur = M.cur + co + I, *po = pass + co + I;
     for (int L = 0; L <= nul; L++) cur[L] = 0;
-    for (int u = 0; u < nu; u++) cur[level[u] + 1]++;
-    int *po = pass + pass_off;
-    int np_ = 0;
+    for (int u = 0; u < nu; u++) cur[M.level[co + u] + 1]++;
+    int np = 0;
     po[0] = 0;
     for (int L = 0; L < nul; L++) {
       cur[L + 1] += cur[L];
-      for (int s = cur[L]; s < cur[L + 1]; s += 32) po[++np_] = min(s + 32, cur[L + 1]);
+      for (int s = cur[L]; s < cur[L + 1]; s += 32) po[++np] = min(s + 32, cur[L + 1]);
     }
-    for (int u = 0; u < nu; u++) units[unit_off + cur[level[u]]++] = tmp[u];
-    rec[I_UNIT_OFF] = unit_off;
-    rec[I_NU] = nu;
-    rec[I_PASS_OFF] = pass_off;
-    rec[I_NPASS] = np_;
-    unit_off += nu;
-    pass_off += np_ + 1;
-    // collision points in local body order; the island's count is checked
-    // against the kernel's capacity before any of its points is written
-    rec[I_PT_OFF] = pt_off;
-    uint64_t np_isl = 0;
-    for (int j = 0; j < nb; j++) np_isl += coll_range[nB + ib[bo + j]];
-    if (np_isl > (uint64_t)KR_MAX_ISLAND_COLLPTS) { W[kOffHdr + 2] = KR_ERR_CAPACITY; return; }
-    int np = 0;
+    for (int u = 0; u < nu; u++) {
+      const int p = M.pin[co + u], q = M.ang[co + u];
+      units[co + cur[M.level[co + u]]++] =
+          make_int4(M.con[p >= 0 ? p : q] & 0xffff, p >= 0 ? (int)M.list[p] : -1, q >= 0 ? (int)M.list[q] : -1, 0);
+    }
+    int pts = 0;
     for (int j = 0; j < nb; j++) {
-      const int g = ib[bo + j];
-      const uint32_t off = coll_range[g], cn = coll_range[nB + g];
-      bpt[bo + j] = make_int2(np, (int)cn);
-      for (uint32_t q = 0; q < cn; q++) ipts[pt_off + np + (int)q] = (int)(off + q);
-      np += (int)cn;
+      const int cn = (int)coll_range[nB + ib[bo + j]];
+      bpt[bo + j] = make_int2(pts, cn);
+      pts += cn;
     }
-    pt_off += np;
+    bad |= pts > KR_MAX_ISLAND_COLLPTS;
+    M.po[I] = pts;
+    int *rec = isl + I * kIslandInts;
+    rec[I_BODY_OFF] = bo;
+    rec[I_NB] = nb;
+    rec[I_UNIT_OFF] = co;
+    rec[I_NU] = nu;
+    rec[I_PASS_OFF] = co + I;
+    rec[I_NPASS] = np;
   }
-  // rects and the culling distance, as kr_create derives them
-  double half_thick = 0.0, r_max = 0.0;
-  for (int i = 0; i < nR; i++) {
+  if (__syncthreads_or(bad)) { fail(KR_ERR_CAPACITY); return; }
+  block_scan(M.po, nI, M.sums);
+  for (int I = t; I < nI; I += kBuildThreads) isl[I * kIslandInts + I_PT_OFF] = M.po[I];
+  for (int g = t; g < nB; g += kBuildThreads) {
+    const int I = M.isl[g], at = M.bo[I] + M.loc[g];
+    const int2 r = bpt[at];
+    for (int q = 0; q < r.y; q++) ipts[M.po[I] + r.x + q] = (int)coll_range[g] + q;
+  }
+  // rects and the culling distance, as kr_create derives them: the largest
+  // half thickness and radius (an infinite or undefined one counts as no
+  // bound), as the bit patterns of non-negative doubles
+  if (t == 0) M.half_thick = M.r_max = 0.0;
+  __syncthreads();
+  auto raise = [](double *m, double v) {
+    atomicMax(reinterpret_cast<unsigned long long *>(m), (unsigned long long)__double_as_longlong(v));
+  };
+  for (int i = t; i < nR; i += kBuildThreads) {
     const float x = rects[4 * i], y = rects[4 * i + 1], rw = rects[4 * i + 2], rh = rects[4 * i + 3];
     r4[i] = make_float4(x, y, x + rw, y + rh);
     const double ht = 0.5 * fmin(fabs((double)rw), fabs((double)rh));
-    half_thick = isfinite(ht) ? fmax(half_thick, ht) : HUGE_VAL;
+    raise(&M.half_thick, isfinite(ht) ? ht : HUGE_VAL);
   }
-  for (int i = 0; i < nP; i++) {
+  for (int i = t; i < nP; i += kBuildThreads) {
     const float r = __uint_as_float(coll_pts[4 * i + 3]);
-    r_max = isfinite(r) ? fmax(r_max, fabs((double)r)) : HUGE_VAL;
+    raise(&M.r_max, isfinite(r) ? fabs((double)r) : HUGE_VAL);
   }
-  const double cull = fmax(r_max, half_thick) + 2.0 + kr::kCullPad;
-  reinterpret_cast<float *>(W)[kOffHdr + 1] = (isfinite(cull) && cull < 1e30) ? (float)cull : 1e30f;
-  W[kOffHdr + 0] = nI;
+  __syncthreads();
+  if (t == 0) {
+    const double cull = fmax(M.r_max, M.half_thick) + 2.0 + kr::kCullPad;
+    reinterpret_cast<float *>(W)[kOffHdr + 1] = (isfinite(cull) && cull < 1e30) ? (float)cull : 1e30f;
+    W[kOffHdr + 0] = nI;
+    W[kOffHdr + 2] = KR_OK;
+  }
 }
 
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) noalloc_step_kernel(StepArgs A, const int *W) {
@@ -948,7 +1068,10 @@ extern "C" int kr_step_noalloc(const kr_solver_params *params, uint32_t n_bodies
   int *W = static_cast<int *>(g_noalloc_ptr[dev]);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (n_steps == 0) return KR_OK;
-  noalloc_schedule_kernel<<<1, 32, 0, st>>>(W, bodies, cons, rects, coll_pts, coll_range,
+  if (cudaFuncSetAttribute(noalloc_schedule_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(BuildSmem)) != cudaSuccess)
+    return KR_ERR_CUDA;
+  noalloc_schedule_kernel<<<1, kBuildThreads, sizeof(BuildSmem), st>>>(W, bodies, cons, rects, coll_pts, coll_range,
                                            (int)n_bodies, (int)n_constraints, (int)n_coll_pts,
                                            (int)n_rects);
   if (cudaGetLastError() != cudaSuccess) return KR_ERR_CUDA;

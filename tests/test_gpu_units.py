@@ -205,3 +205,84 @@ def test_quotients_equal_ieee_division():
         b = np.ldexp(1 + mb / 2.0 ** 23, eb).astype(np.float32)
         a[-1000:] = 0
         assert np.array_equal(batch.probe_quot(a, b), a / b), (ea, eb)
+
+
+def _noalloc(L):
+    L.kr_step_noalloc.restype = C.c_int
+    L.kr_step_noalloc.argtypes = [C.POINTER(_native.SolverParams), C.c_uint32, C.c_uint32, C.c_void_p, C.c_void_p,
+                                  C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p, C.c_int32,
+                                  C.c_void_p]
+    return L
+
+
+@pytest.mark.parametrize("islands,nb,nc,steps", [(1, 1, 1, 1), (1, 160, 384, 2), (33, 5, 9, 3), (300, 2, 3, 1),
+                                                 (1024, 2, 4, 130), (2048, 1, 2, 1), (12, 160, 330, 2)])
+def test_noalloc_schedule_equals_the_handles_step(islands, nb, nc, steps):
+    """The allocation-free entry builds its schedule on the device: random
+    islands whose bodies and constraints are shuffled among one another, from
+    one body to the entry's limits, must step to the bytes that the handle's
+    host-built schedule gives."""
+    import torch
+
+    r = np.random.default_rng(islands * 1000 + nb)
+    n = islands * nb
+    place = r.permutation(n)  # body (island, j) -> index
+    bodies = np.zeros((n, 12), np.float32)
+    bodies[:, 0], bodies[:, 1] = r.uniform(30, 350, n), r.uniform(30, 250, n)
+    bodies[:, 2:4] = bodies[:, :2]
+    bodies[:, 6] = bodies[:, 7] = r.uniform(-3, 3, n)
+    bodies[:, 9], bodies[:, 10] = 1 / r.uniform(1, 20, n), 1 / r.uniform(20, 900, n)
+    rows = []
+    for i in range(islands):
+        own = place[i * nb:(i + 1) * nb]
+        level = np.zeros(nb, int)
+        for k in range(nc):
+            a = k % (nb - 1) if nb > 1 and k < nb - 1 else int(np.argmin(level))
+            b = a + 1 if nb > 1 and k < nb - 1 else (-1 if nb == 1 or r.random() < 0.3 else int((a + 1 + r.integers(nb - 1)) % nb))
+            t = int(r.integers(3))
+            if b >= 0 and max(level[a], level[b]) > 80:
+                b = -1
+            level[a] = max(level[a], level[b] if b >= 0 else 0) + 1
+            if b >= 0:
+                level[b] = level[a]
+            rows.append((i * nc + k, own[a], own[b] if b >= 0 else -1, t))
+    order = np.argsort(r.random(len(rows)) * islands + np.array([q[0] % nc for q in rows]), kind="stable")
+    cons = np.zeros((len(rows), 20), np.float32)
+    cu = cons.view(np.uint32)
+    for at, k in enumerate(order):
+        _, a, b, t = rows[k]
+        cu[at, 0], cu[at, 1], cu[at, 2] = a, b & 0xFFFFFFFF, t
+        cons[at, 4:8] = r.uniform(-7, 7, 4)
+        if b < 0:
+            cons[at, 6:8] = r.uniform(40, 250, 2)
+        cons[at, 8], cons[at, 9], cons[at, 10] = 1e-5, r.uniform(-1, 1), r.uniform(-1, 1)
+        cons[at, 11], cons[at, 12], cons[at, 16] = -1, 1, r.uniform(50, 500)
+    cnt = np.minimum(r.integers(0, 4, n), 4096 // n + 1).astype(np.uint32)
+    while cnt.sum() > 4096:
+        cnt[int(np.argmax(cnt))] -= 1
+    rng = np.concatenate([np.cumsum(cnt) - cnt, cnt]).astype(np.uint32)
+    pts = np.zeros((int(cnt.sum()), 4), np.float32)
+    pts.view(np.uint32)[:, 0] = np.repeat(np.arange(n), cnt)
+    pts[:, 1:3], pts[:, 3] = r.uniform(-6, 6, (len(pts), 2)), r.uniform(2, 7, len(pts))
+    rects = RECTS.astype(np.float32)
+    L = _noalloc(_native.lib())
+    p = _native.SolverParams(1 / 120, 2, 4, 3.0, 3.0, 360.0, 18.0)
+    dev = [torch.from_numpy(np.ascontiguousarray(v).view(np.int32)).cuda() for v in (bodies, cons, rects, pts, rng)]
+    forces = torch.zeros((n, 4), device="cuda")
+    args = (C.byref(p), n, len(cons), dev[0].data_ptr(), dev[1].data_ptr(), forces.data_ptr(), dev[2].data_ptr(),
+            len(rects), dev[3].data_ptr(), len(pts), dev[4].data_ptr())
+    rc = L.kr_step_noalloc(*args, steps, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    h = C.c_void_p()
+    _native.check(L.kr_create(C.byref(p), n, len(cons), rects.ctypes.data_as(_F32P), len(rects),
+                              pts.ctypes.data_as(_U32P), len(pts), rng.ctypes.data_as(_U32P), C.byref(h)))
+    try:
+        up = L.kr_upload(h, bodies.ctypes.data_as(_F32P), cu.ctypes.data_as(_U32P), None, None)
+        assert rc == up
+        if rc == 0:
+            _native.check(L.kr_step(h, steps), h)
+            _native.check(L.kr_download(h, bodies.ctypes.data_as(_F32P), cu.ctypes.data_as(_U32P)), h)
+        assert np.array_equal(dev[0].cpu().numpy(), bodies.view(np.int32))
+        assert np.array_equal(dev[1].cpu().numpy(), cons.view(np.int32))
+    finally:
+        L.kr_destroy(h)
