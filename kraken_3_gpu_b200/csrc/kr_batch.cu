@@ -1095,8 +1095,6 @@ void gather_live(kr_batch *b, Part &p) {
   p.g_tpl.clear();
   p.g_rem.clear();
   p.g_ctrl.clear();
-  p.g_per_arm = 0;
-  p.g_net = 0;
   auto take = [&](int s) {
     const int r = b->h_remaining[s];
     if (r <= 0) return;
@@ -1106,8 +1104,6 @@ void gather_live(kr_batch *b, Part &p) {
     p.g_tpl.push_back(m.tpl);
     p.g_rem.push_back(r);
     p.g_ctrl.push_back(m.ctrl);
-    p.g_per_arm += m.ctrl == KR_CTRL_POLICY || m.ctrl == KR_CTRL_NET;
-    p.g_net += m.ctrl == KR_CTRL_NET;
   };
   if (p.all) {
     for (int s = 0; s < b->capacity; s++) take(s);
@@ -1257,15 +1253,20 @@ cudaError_t launch_g(const BatchArgs &A, kr_batch *b, cudaStream_t st, int n_gro
 
 namespace krb {
 
-// Few creatures (under 16 per SM): one per warp, the shortest step latency;
+// Few creatures (under 8 per SM): one per warp, the shortest step latency;
 // up to 96 per SM two per warp; beyond, four per warp, the most
-// creature-steps per issue slot (measured on the 16k workload).
-// Proprioception and the fused policy run per arm, so creatures that need
-// them pack four per warp from 16 per SM on.
-int auto_lanes(const kr_batch *b, long live, long per_arm) {
-  const bool arm_heavy = b->d.obs_ring > 0 || 2 * per_arm > live;
-  return live < 16L * b->n_sm ? 32 : (arm_heavy || live >= 96L * b->n_sm) ? 8 : 16;
+// creature-steps per issue slot.  Measured at the edges, always with CTAs of
+// 4 warps: 2,000 default creatures x 200 steps (13.5 per SM) 9.1 ms at 16
+// lanes against 11.2 at 32, 1,024 x 400 (7 per SM) 16.1 at either; 16,384
+// mixed creatures 154 ms with 8 lanes above 96 per SM, 166 above 64.
+// Creatures under the policy or the net and ring-keeping ones used to take 8
+// lanes from 16 per SM on; since a pass runs one unit per lane at any width
+// they do better with 16: 8,000 under the policy 32 against 39 ms, under the
+// net 37 against 41, 6,000 with rings 24 against 27.
+int auto_lanes(const kr_batch *b, long live) {
+  return live < 8L * b->n_sm ? 32 : live >= 96L * b->n_sm ? 8 : 16;
 }
+constexpr int kAutoWarps = 4;
 
 int launch_part(kr_batch *b, Part &p, int max_steps, bool timed) {
   if (b->tpls.empty()) return KR_OK;
@@ -1273,14 +1274,7 @@ int launch_part(kr_batch *b, Part &p, int max_steps, bool timed) {
     return b->fail(KR_ERR_STATE, "policy control without kr_batch_set_policy");
   if (b->auto_shape && p.dirty) {
     gather_live(b, p);  // build_groups below takes the same gather
-    const int g = auto_lanes(b, (long)p.g_live.size(), p.g_per_arm);
-    // at 8 lanes, creatures under the reference net or keeping an
-    // observation ring run faster as one CTA of 16 warps per SM than as two
-    // of 8 (served net ES stream 2.60e7 -> 2.90e7 creature-steps/s; 65k
-    // creatures with 128-step rings 4.32e7 -> 4.54e7); under the fused
-    // policy the two are within noise, and stream controls keep 8
-    const bool wide = b->d.obs_ring > 0 || 2 * p.g_net > (long)p.g_live.size();
-    const int w = g == 32 ? 4 : (g == 8 && wide) ? 16 : 8;
+    const int g = auto_lanes(b, (long)p.g_live.size()), w = kAutoWarps;
     if (g != b->G || w != b->W) {
       b->G = g;
       b->W = w;
@@ -2012,7 +2006,7 @@ extern "C" int kr_batch_autotune(kr_batch *b, int32_t steps, int32_t *lanes_out,
   if (!b) return KR_ERR_INVALID;
   if (steps < 1) return b->fail(KR_ERR_INVALID, "autotune steps < 1");
   // (lanes per creature, warps per CTA, CTAs per SM, substep unroll)
-  static const int kCand[][4] = {{8, 8, 0, 1},  {8, 16, 1, 1},  {8, 4, 4, 1},  {16, 8, 0, 1}, {16, 16, 1, 1},
+  static const int kCand[][4] = {{8, 8, 0, 1},  {8, 16, 1, 1},  {8, 4, 4, 1},  {16, 8, 0, 1}, {16, 4, 0, 1},
                                  {32, 4, 0, 1}, {32, 8, 0, 1},  {8, 8, 0, 2},  {8, 16, 1, 2}, {16, 8, 0, 2},
                                  {32, 4, 0, 2}};
   const size_t C = (size_t)b->capacity;

@@ -242,7 +242,6 @@ struct Part {
   // the next build_groups; then the launch order's scratch
   std::vector<int> g_live, g_tpl, g_rem, g_ctrl, s_live, perm, perm2;
   std::vector<uint64_t> keys, keys2;
-  long g_per_arm = 0, g_net = 0;   // live slots under the policy or the net / under the net
   bool gathered = false;
 };
 
@@ -348,10 +347,8 @@ int ensure_template(kr_batch *b, int arms, int segs);
 int upload_templates(kr_batch *b);
 // creatures per group of every template and the CTA's shared memory
 int plan_shape(kr_batch *b);
-// lanes per creature the automatic launch shape gives `live` creatures, of
-// which `per_arm` run the policy or net controller (their proprioception
-// and controller run per arm)
-int auto_lanes(const kr_batch *b, long live, long per_arm);
+// lanes per creature the automatic launch shape gives `live` creatures
+int auto_lanes(const kr_batch *b, long live);
 // the part's live slots (remaining steps > 0) with their template, remaining
 // steps and control mode, in slot-list order, into p.g_*
 void gather_live(kr_batch *b, Part &p);

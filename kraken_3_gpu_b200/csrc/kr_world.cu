@@ -742,9 +742,9 @@ static __device__ __align__(256) int g_noalloc_scratch[kScratchWords];
 // build_schedule() and the same units, in passes by level.  A single thread
 // over global memory took 5.3 ms for 40 creatures, all of it load latency;
 // here (a 40-creature call of 4 steps: 5.6 -> 0.27 ms) the temporaries are in
-// shared memory and only what is sequential by
-// nature runs in order -- the ranks within an island by one warp, 32 entries
-// at a time, and an island's units by one thread per island.
+// shared memory and only what is sequential by nature runs in order -- the
+// ranks within an island by one warp, 32 entries at a time, and an island's
+// units by one thread per island.
 constexpr int kBuildThreads = 1024;
 
 // Exclusive scan of v[0..n) in place, n <= 2 * kBuildThreads; returns the
