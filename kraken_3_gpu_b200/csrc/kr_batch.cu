@@ -913,6 +913,16 @@ __global__ void spawn_kernel(float *state, float4 *grip, float2 *glam, double2 *
   }
 }
 
+// slots' bodies from the field arrays of their state blocks into records of
+// px py vx vy ang av (kr_batch_read_state's layout)
+__global__ void bodies_kernel(const float *state, float *out, int n) {
+  constexpr int per = 6 * kr::kMaxTplBodies;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n * per) return;
+  const int i = q / per, w = q - i * per;
+  out[q] = state[(size_t)i * kStateStride + (w % 6) * kBodyPad + w / 6];
+}
+
 // every slot's step counter into one contiguous array (read back after a
 // time slice: a preempted slice leaves each creature at its own step)
 __global__ void step_counts_kernel(const SlotMeta *meta, int n, int *out) {
@@ -2097,32 +2107,72 @@ extern "C" int kr_batch_live(kr_batch *b, int32_t *live) {
   return KR_OK;
 }
 
+// Device buffers of bodies in the public layout, one per readback lane, for a
+// read of n slots (one lane if one buffer holds them); kept with the engine,
+// at most 4 x 4 MB.  Returns 0 where there is no memory for them.
+static int bodies_buffers(kr_batch *b, int n) {
+  constexpr size_t kSlot = 6 * kr::kMaxTplBodies * sizeof(float);
+  const size_t slots = std::min<size_t>(n, kr::Readback::kChunk / kSlot);
+  if (b->bodies_slots < slots) {
+    for (float *&p : b->d_bodies) {
+      if (p) cudaFree(p);
+      p = nullptr;
+    }
+    b->bodies_slots = slots;
+  }
+  const int lanes = (size_t)n > b->bodies_slots ? kr::Readback::kLanes : 1;
+  for (int i = 0; i < lanes; i++)
+    if (!b->d_bodies[i] && cudaMalloc(&b->d_bodies[i], b->bodies_slots * kSlot) != cudaSuccess) {
+      cudaGetLastError();
+      b->d_bodies[i] = nullptr;
+      return 0;
+    }
+  return lanes;
+}
+
 extern "C" int kr_batch_read_state(kr_batch *b, int32_t first, int32_t n, float *bodies, float *grips,
                                    int32_t *steps) {
   if (!b) return KR_ERR_INVALID;
   if (first < 0 || n < 0 || first + n > b->capacity) return b->fail(KR_ERR_INVALID, "read range outside the slots");
   if (n == 0) return KR_OK;
-  std::vector<float> st((size_t)n * kStateStride);
-  std::vector<float4> gr((size_t)n * KR_BATCH_MAX_ARMS);
-  std::vector<SlotMeta> m(n);
-  cudaError_t e = cudaMemcpyAsync(st.data(), b->d_state + (size_t)first * kStateStride, st.size() * sizeof(float), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(gr.data(), b->d_grip + (size_t)first * KR_BATCH_MAX_ARMS, gr.size() * sizeof(float4), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(m.data(), b->d_meta + first, m.size() * sizeof(SlotMeta), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  if (e != cudaSuccess) return b->cuda_fail(e, "kr_batch_read_state");
-  constexpr int NB = kr::kMaxTplBodies;
-  for (int i = 0; i < n; i++) {
-    if (bodies)
-      for (int j = 0; j < NB; j++)
-        for (int f = 0; f < 6; f++) bodies[((size_t)i * NB + j) * 6 + f] = st[(size_t)i * kStateStride + f * kBodyPad + j];
-    if (grips)
-      for (int a = 0; a < KR_BATCH_MAX_ARMS; a++) {
-        const float4 g = gr[(size_t)i * KR_BATCH_MAX_ARMS + a];
-        float *o = grips + ((size_t)i * KR_BATCH_MAX_ARMS + a) * 4;
-        o[0] = g.x; o[1] = g.y; o[2] = g.z; o[3] = g.w;
+  // A kernel puts the bodies in the public layout (on the host that was 438
+  // strided element copies a slot), chunk by chunk into a lane's buffer; grips
+  // are laid out as they are read.
+  constexpr size_t kPer = 6 * kr::kMaxTplBodies;
+  cudaError_t e = cudaSuccess;
+  if (bodies) {
+    const int lanes = bodies_buffers(b, n);
+    const float *state = b->d_state + (size_t)first * kStateStride;
+    if (lanes > 0) {
+      e = b->rb.read(reinterpret_cast<char *>(bodies), (size_t)n * kPer * sizeof(float), b->stream,
+                     b->bodies_slots * kPer * sizeof(float), [&](int lane, size_t off, size_t bytes, cudaStream_t st) {
+                       const int i0 = (int)(off / (kPer * sizeof(float))), k = (int)(bytes / (kPer * sizeof(float)));
+                       bodies_kernel<<<(unsigned)((k * kPer + 255) / 256), 256, 0, st>>>(
+                           state + (size_t)i0 * kStateStride, b->d_bodies[lane], k);
+                       return reinterpret_cast<const char *>(b->d_bodies[lane]);
+                     });
+    } else {  // no device memory for the buffers
+      std::vector<float> blk((size_t)std::min(n, 1024) * kStateStride);
+      for (int i0 = 0; i0 < n && e == cudaSuccess; i0 += 1024) {
+        const int k = std::min(1024, n - i0);
+        e = cudaMemcpyAsync(blk.data(), state + (size_t)i0 * kStateStride, (size_t)k * kStateStride * sizeof(float),
+                            cudaMemcpyDeviceToHost, b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+        for (size_t q = 0; q < (size_t)k * kPer && e == cudaSuccess; q++)
+          bodies[(size_t)i0 * kPer + q] = blk[q / kPer * kStateStride + (q % 6) * kBodyPad + q % kPer / 6];
       }
-    if (steps) steps[i] = m[i].step;
+    }
   }
+  if (e == cudaSuccess && grips)
+    e = b->rb.read(grips, b->d_grip + (size_t)first * KR_BATCH_MAX_ARMS, (size_t)n * KR_BATCH_MAX_ARMS * sizeof(float4),
+                   b->stream);
+  if (e == cudaSuccess && steps) {
+    std::vector<SlotMeta> m(n);
+    e = cudaMemcpyAsync(m.data(), b->d_meta + first, m.size() * sizeof(SlotMeta), cudaMemcpyDeviceToHost, b->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+    for (int i = 0; i < n && e == cudaSuccess; i++) steps[i] = m[i].step;
+  }
+  if (e != cudaSuccess) return b->cuda_fail(e, "kr_batch_read_state");
   return KR_OK;
 }
 
@@ -2131,9 +2181,7 @@ extern "C" int kr_batch_read_obs(kr_batch *b, int32_t first, int32_t n, float *o
   if (b->d.obs_ring <= 0) return b->fail(KR_ERR_STATE, "no observation ring (obs_ring == 0)");
   if (first < 0 || n < 0 || first + n > b->capacity) return b->fail(KR_ERR_INVALID, "read range outside the slots");
   const size_t per = (size_t)b->d.obs_ring * KR_OBS_STRIDE;
-  cudaError_t e = cudaMemcpyAsync(obs, b->d_obs + (size_t)first * per, (size_t)n * per * sizeof(float),
-                                  cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  cudaError_t e = b->rb.read(obs, b->d_obs + (size_t)first * per, (size_t)n * per * sizeof(float), b->stream);
   if (e != cudaSuccess) return b->cuda_fail(e, "kr_batch_read_obs");
   return KR_OK;
 }
@@ -2208,6 +2256,8 @@ extern "C" int kr_batch_set_stream(kr_batch *b, void *stream) {
 extern "C" void kr_batch_destroy(kr_batch *b) {
   if (!b) return;
   cudaDeviceSynchronize();
+  for (float *p : b->d_bodies)
+    if (p) cudaFree(p);
   void *ptrs[] = {b->d_tpl, const_cast<float4 *>(b->T.body), const_cast<float4 *>(b->T.pts),
                   const_cast<float4 *>(b->T.recs), const_cast<int *>(b->T.arm_tip), const_cast<int *>(b->T.arm_seg0),
                   const_cast<int *>(b->T.arm_segs), b->d_rects, b->d_map_off, b->d_map_cull, b->d_rects64,

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/kraken_b200.h"
+#include "kr_readback.h"
 #include "kr_solver.cuh"
 #include "kr_units.h"
 
@@ -250,6 +251,7 @@ struct kr_world {
   bool uploaded = false;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  kr::Readback rb;
   std::string err;
 
   int fail(int code, const std::string &msg) {
@@ -464,7 +466,8 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
   h_bodies.reserve(nB); h_units.reserve(nC);
   int maxB = 1, maxU = 1, maxP = 1, maxLv = 0;
   std::vector<int> last_level, order, off;
-  std::vector<kr::SolveEntry> list;
+  std::vector<kr::SolveEntry> list, list_of;
+  int list_nb = 0;
   std::vector<kr::SolveUnit> units;
   for (int I = 0; I < nI; I++) {
     const auto &bl = ib[I];
@@ -500,8 +503,18 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
       return w->fail(KR_ERR_CAPACITY, "connected component " + std::to_string(I) + " needs " +
                                           std::to_string(nlv) + " constraint levels; the kernel holds " +
                                           std::to_string(KR_MAX_LEVELS));
-    kr::build_units(list, nb, &units, last_level);
-    kr::schedule_units(units, nb, 32, &order, &off);
+    // islands of one structure (a population of one body shape) follow one
+    // another: the last one's units serve again
+    const bool again = I > 0 && nb == list_nb && list.size() == list_of.size() &&
+                       std::equal(list.begin(), list.end(), list_of.begin(), [](const auto &x, const auto &y) {
+                         return x.angle == y.angle && x.a == y.a && x.b == y.b;
+                       });
+    if (!again) {
+      kr::build_units(list, nb, &units, last_level);
+      kr::schedule_units(units, nb, 32, &order, &off);
+      list_of = list;
+      list_nb = nb;
+    }
     rec[I_PASS_OFF] = (int)h_pass.size();
     rec[I_NPASS] = (int)off.size() - 1;
     h_pass.insert(h_pass.end(), off.begin(), off.end());
@@ -651,11 +664,17 @@ extern "C" int kr_download(kr_world *w, float *bodies, uint32_t *cons) {
   if (!w) return KR_ERR_INVALID;
   if (!w->uploaded) return w->fail(KR_ERR_STATE, "download before upload");
   cudaError_t e;
-  if (bodies && (e = cudaMemcpyAsync(bodies, w->d_bodies, sizeof(float) * 12 * w->nB,
-                                     cudaMemcpyDeviceToHost, w->stream)) != cudaSuccess)
+  const size_t nb = sizeof(float) * 12 * (size_t)w->nB, nc = cons ? sizeof(uint32_t) * 20 * (size_t)w->nC : 0;
+  if (nc > kr::Readback::kChunk) {
+    // a large world: in chunks by several threads
+    if (bodies && (e = w->rb.read(bodies, w->d_bodies, nb, w->stream)) != cudaSuccess)
+      return w->cuda_fail(e, "download(bodies)");
+    if ((e = w->rb.read(cons, w->d_cons, nc, w->stream)) != cudaSuccess) return w->cuda_fail(e, "download(cons)");
+    return KR_OK;
+  }
+  if (bodies && (e = cudaMemcpyAsync(bodies, w->d_bodies, nb, cudaMemcpyDeviceToHost, w->stream)) != cudaSuccess)
     return w->cuda_fail(e, "download(bodies)");
-  if (cons && w->nC && (e = cudaMemcpyAsync(cons, w->d_cons, sizeof(uint32_t) * 20 * w->nC,
-                                            cudaMemcpyDeviceToHost, w->stream)) != cudaSuccess)
+  if (nc && (e = cudaMemcpyAsync(cons, w->d_cons, nc, cudaMemcpyDeviceToHost, w->stream)) != cudaSuccess)
     return w->cuda_fail(e, "download(cons)");
   if ((e = cudaStreamSynchronize(w->stream)) != cudaSuccess) return w->cuda_fail(e, "download(sync)");
   return KR_OK;
