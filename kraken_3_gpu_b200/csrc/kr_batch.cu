@@ -88,7 +88,7 @@ constexpr int kArmWords = (2 * KR_BATCH_MAX_ARMS + KR_BATCH_MAX_ARMS * KR_BATCH_
 __host__ __device__ constexpr int r4(int n) { return (n + 3) & ~3; }
 
 // static shared memory of the kernel: the sine table and the group word
-constexpr long kStaticSmem = 512 * sizeof(float2) + 64;
+constexpr long kStaticSmem = kr::kSinEntries * sizeof(float2) + 64;
 
 // statics of the template, once per CTA: unit records of the schedule for G
 // lanes, bodies, collision points, arm tables
@@ -735,7 +735,7 @@ __device__ void run_creature(const BatchArgs &A, const TplDev &td, int npass, co
     }
     L.sync();
     // 4. the XPBD step
-    kr::island_step<false, G, U>(A.K, S, rects, nR, near_d, L, near);
+    kr::island_step<false, G, U, NET>(A.K, S, rects, nR, near_d, L, near);
     // 5. postStep, core.js:297-356 (f64 on the f32 state, as the
     //    reference's hybrid loop runs it on the mirrored state)
     //    The accumulators are read and written through the slot's HBM
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(32 * kMaxW, 1) batch_kernel(BatchArgs A) {
   constexpr int V = G == 32 ? 0 : G == 16 ? 1 : 2;  // kr::schedule_index(G): the schedule for G lanes
   extern __shared__ __align__(16) float smem[];
   __shared__ int s_group;
-  __shared__ float2 s_sin[512];
+  __shared__ float2 s_sin[kr::kSinEntries];
   kr::stage_sin(s_sin);  // the group loop's first barrier precedes its use
   const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31;
   const kr::Lanes<G> L(wl);
@@ -2359,7 +2359,7 @@ __global__ void fma_probe_kernel(float *out, int iters) {
 
 namespace {
 __global__ void sincos_probe_kernel(const float *x, int n, float *s, float *c) {
-  __shared__ float2 tab[512];
+  __shared__ float2 tab[kr::kSinEntries];
   kr::stage_sin(tab);
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

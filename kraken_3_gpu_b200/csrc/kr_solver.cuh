@@ -186,7 +186,8 @@ static __device__ __noinline__ float2 sincos_f64(float a) {
 // cycles); two 8-byte shared loads take a few bank conflicts each.
 __device__ __forceinline__ float sincos_near(const float2 *tab, float a, float *s, float *c) {
   const float t = fmaf(a, 0x1.45f306p6f, 12582912.f);  // 256/pi; the sum's low bits hold k
-  const float2 ts = tab[__float_as_int(t) & 511], tc = tab[(__float_as_int(t) + 128) & 511];
+  const float2 *e = tab + (__float_as_int(t) & 511);
+  const float2 ts = e[0], tc = e[128];
   const float4 T = make_float4(ts.x, ts.y, tc.x, tc.y);
   const float k = fsub(t, 12582912.f);
   const float r1 = fmaf(-k, 0x1.921fb6p-7f, a), rl = fmul(-k, -0x1.777a5cp-32f);
@@ -207,10 +208,12 @@ __device__ __forceinline__ float sincos_near(const float2 *tab, float a, float *
 }
 constexpr float kSinCosNearMax = 64.f;
 
-// The table into shared memory, by every thread of the block; __syncthreads
-// before its first use.
+// The table into shared memory, by every thread of the block, its first
+// quarter repeated at the end for the cosine; __syncthreads before its first
+// use.
+constexpr int kSinEntries = 640;
 __device__ __forceinline__ void stage_sin(float2 *tab) {
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = kSinNear[i];
+  for (int i = threadIdx.x; i < kSinEntries; i += blockDim.x) tab[i] = kSinNear[i & 511];
 }
 
 __device__ __forceinline__ void sincos_r(const float2 *tab, float a, float *s, float *c) {
@@ -704,8 +707,8 @@ template <int G>
 __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
   const float alpha_m = fmul(S.comp_m, K.invH2);
   const float4 *rec = S.recs + 3 * L.lane;
-  float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
   for (int p = 0; p < S.npass; p++) {
+    const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
     const unsigned ab = __float_as_uint(r0.x);
     const int A = ab & 0xff, B = (ab >> 8) & 0xff, m = (ab >> 16) & 0xff;
     const bool joint = (ab & kRecJoint) != 0;
@@ -714,16 +717,14 @@ __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, b
     const PinArgs U{r0.y, r0.z, r0.w, 0.f, r1.x, r1.y, r1.z, r1.w, 0.f, joint};
     const AngleArgs V{r2.x, r2.y, r2.z, mo.x, alpha_m, r1.y, r1.w, true};
     const float yw = r2.w;
-    // the next pass's records: the loads wait on nothing the sweep computes
     rec += 3 * G;
-    if (p + 1 < S.npass) { r0 = rec[0]; r1 = rec[1]; r2 = rec[2]; }
     const bool held = joint || ((ab & kRecIdle) == 0 && b.w == 0.f);  // b.w: an anchor's broken flag
     const float l0 = first || !joint ? 0.f : mo.y;
     const float lx0 = first || joint ? 0.f : mo.x, ly0 = first || joint ? 0.f : mo.y;
     float lx = lx0, ly = ly0, l = l0;
     const bool op = pin_near<false>(S.tab, U, held, a, b, lx, ly);
     const bool oa = angle_near<false>(V, yw, joint, a.z, b.z, l);
-    if (!(op && oa && alpha_m < 0x1p59f)) {
+    if (__builtin_expect(!(op && oa && alpha_m < 0x1p59f), 0)) {
       const UnitOut o = unit_any(U, V, held, joint, false, S.Q[A], S.Q[B], lx0, ly0, l0);
       a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;
     }
@@ -771,7 +772,7 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
       float lx = d.x, ly = d.y, l = d.z;
       const bool op = pin_near<true>(S.tab, U, pin, a, b, lx, ly) && (!pin || (ab & kPinTame) != 0);
       const bool oa = angle_near<true>(V, yw, angle, a.z, b.z, l);
-      if (!(op && oa && (ab & kBounded))) {
+      if (__builtin_expect(!(op && oa && (ab & kBounded)), 0)) {
         const UnitOut o = unit_any(U, V, pin, angle, A == B, S.Q[A], hasB ? S.Q[B] : anchor, d.x, d.y, d.z);
         a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;
       }
@@ -814,7 +815,8 @@ __device__ __forceinline__ float2 near_unpack(unsigned w) {
                      __uint_as_float(0x4b000000u | (w >> 16)) - 8421376.f);
 }
 __device__ __forceinline__ bool near_holds(const float2 ref, float x, float y, unsigned mask) {
-  return fmaxf(fabsf(x - ref.x), fabsf(y - ref.y)) <= ((mask & kNearBit) ? kNearMove : kFarMove) && x == x && y == y;
+  const float r = (mask & kNearBit) ? kNearMove : kFarMove;
+  return fabsf(x - ref.x) <= r && fabsf(y - ref.y) <= r;
 }
 // false only if the rect lies outside the box x0..x1 x y0..y1 (extents of
 // either sign; NaN counts as inside)
@@ -945,24 +947,13 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
   if (moved) S.Q[j] = q;
 }
 
-// One collision pass of the island.  Listed bodies with one or two points
-// take a lane each; the points of a body with more (the mantle's eight) are
-// evaluated side by side, and one lane repeats them in order from the first
-// that corrects -- until then none has moved the body.
+// The listed bodies of a collision pass.  Those with one or two points take a
+// lane each; the points of a body with more (the mantle's eight) are evaluated
+// side by side, and one lane repeats them in order from the first that
+// corrects -- until then none has moved the body.
 template <int G>
-__device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 *__restrict__ rects, int nR,
-                                               float near_d, const Lanes<G> &L) {
-  bool stale = !N.valid();
-  if (!stale) {
-    bool moved = false;
-#pragma unroll 2
-    for (int j = L.lane; j < S.nb; j += G) {
-      const float4 q = S.Q[j];
-      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, __float_as_uint(q.w));
-    }
-    stale = L.ballot(moved) != 0;
-  }
-  if (stale) N.w = near_rebuild<G>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
+__device__ __forceinline__ void collide_listed(Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
+                                               const Lanes<G> &L) {
   for (int t = L.lane; t < N.few(); t += G) {
     const int j = S.list[t];
     const float4 q = S.Q[j];
@@ -990,6 +981,35 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
       if (m) first = base + __ffs(m) - 1;
     }
     if (first >= 0 && L.lane == 0) collide_points(S, N, rects, nR, j, q, sa, ca, first);
+  }
+}
+template <int G>
+__device__ __noinline__ void collide_listed_call(Island S, Near N, const float4 *__restrict__ rects, int nR, Lanes<G> L) {
+  collide_listed<G>(S, N, rects, nR, L);
+}
+
+// One collision pass of the island.  OutOfLine: the listed bodies (most passes
+// have none) as a call -- for the kernel with the net, whose step is larger
+// than the instruction caches: 8,000 creatures under the net 35 -> 32 ms; the
+// others are 3 % faster with it in line.
+template <int G, bool OutOfLine>
+__device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 *__restrict__ rects, int nR,
+                                               float near_d, const Lanes<G> &L) {
+  bool stale = !N.valid();
+  if (!stale) {
+    bool moved = false;
+#pragma unroll 1
+    for (int j = L.lane; j < S.nb; j += G) {
+      const float4 q = S.Q[j];
+      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, __float_as_uint(q.w));
+    }
+    stale = L.ballot(moved) != 0;
+  }
+  if (stale) N.w = near_rebuild<G>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
+  if (OutOfLine) {
+    if (N.w & 0xffffu) collide_listed_call<G>(S, N, rects, nR, L);
+  } else {
+    collide_listed<G>(S, N, rects, nR, L);
   }
   L.sync();
 }
@@ -1031,22 +1051,25 @@ __device__ __forceinline__ bool grip_breaks(const SolverConsts &K, float lx, flo
 // iterations x (solve passes, collisions), finalize), then grip break.
 // U: unroll factor of the substep loop (1: a loop; 2: its body twice per
 // trip, remainder handled) -- the same operations in the same order, so the
-// results do not depend on it; the batched engine's autotuner picks it.
-template <bool World, int G, int U = 1>
+// results do not depend on it; the batched engine's autotuner picks it.  The
+// loops inside are not unrolled: an env step's code has to stay in the
+// instruction caches (the pass loop unrolled twice: 16,384 creatures 154 ->
+// 219 ms; the body loops not unrolled: 8,000 under the policy 31 -> 27 ms).
+template <bool World, int G, int U = 1, bool OutOfLine = false>
 __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
                                             const float4 *__restrict__ rects, int nR, float near_d,
                                             const Lanes<G> &L, Near &N) {
 #pragma unroll U
   for (int s = 0; s < K.substeps; s++) {
-#pragma unroll 2
+#pragma unroll 1
     for (int i = L.lane; i < S.nb; i += G) integrate_body<World>(K, S, i);
     L.sync();
     for (int it = 0; it < K.iterations; it++) {
       if constexpr (World) solve_world<G>(S, it == 0, L);
       else solve_engine<G>(K, S, it == 0, L);
-      collide_island<G>(S, N, rects, nR, near_d, L);
+      collide_island<G, OutOfLine>(S, N, rects, nR, near_d, L);
     }
-#pragma unroll 2
+#pragma unroll 1
     for (int i = L.lane; i < S.nb; i += G) finalize_body<World>(K, S, i);
     L.sync();
   }

@@ -93,7 +93,7 @@ __device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, i
 // plain kernel and its allocation-free variant).
 __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   extern __shared__ __align__(16) float smem[];
-  __shared__ float2 s_sin[512];
+  __shared__ float2 s_sin[kr::kSinEntries];
   kr::stage_sin(s_sin);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
