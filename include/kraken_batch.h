@@ -224,7 +224,7 @@ int kr_probe_fp32_rate(double *fma_per_s);
 int kr_probe_sincos(const float *x, int32_t n, float *s, float *c);
 
 /* The solver's f32 quotients a / b by a shared reciprocal of b, for |a| in
- * 2^-100..2^60 or 0, |b| in 2^-60..2^60 with a clear bit in its mantissa. */
+ * 2^-100..2^60 or 0, |b| in 2^-60..2^60. */
 int kr_probe_quot(const float *a, const float *b, int32_t n, float *q);
 
 /* readProprio's atan2(sin d, cos d) of f64 angle differences as the device

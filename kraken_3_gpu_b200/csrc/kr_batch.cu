@@ -1274,7 +1274,8 @@ namespace krb {
 // they do better with 16: 8,000 under the policy 32 against 39 ms, under the
 // net 37 against 41, 6,000 with rings 24 against 27.
 int auto_lanes(const kr_batch *b, long live) {
-  return live < 8L * b->n_sm ? 32 : live >= 96L * b->n_sm ? 8 : 16;
+  if (live < 8L * b->n_sm) return b->served ? 16 : 32;
+  return live >= 96L * b->n_sm ? 8 : 16;
 }
 constexpr int kAutoWarps = 4;
 

@@ -311,6 +311,7 @@ struct kr_batch {
   int unroll = 1;               // unroll factor of the kernel's substep loop (1 or 2)
   int smem_per_sm = 0, smem_reserved = 0, smem_optin = 0;
   bool auto_shape = true;       // until kr_batch_set_launch: G and W from the live count
+  bool served = false;          // a rollout server's engine
   int cpc = 16;                 // creature entries per group: W * 32 / G
   std::vector<int> tpl_cpg;     // creatures per group of each template
   size_t smem_dyn = 0;          // dynamic shared memory per CTA

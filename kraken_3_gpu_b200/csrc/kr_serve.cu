@@ -762,6 +762,7 @@ extern "C" int kr_server_create(const kr_server_desc *d, kr_server **out) {
   kr_batch *b = nullptr;
   rc = kr_batch_create(&bd, &b);
   if (rc != KR_OK) { g_serve_error = std::string("engine: ") + kr_batch_last_error(nullptr); return rc; }
+  b->served = true;
   kr_server *S = new kr_server();
   S->d = *d;
   S->d.rects = nullptr;

@@ -224,30 +224,25 @@ __device__ __forceinline__ void sincos_r(const float2 *tab, float a, float *s, f
   }
 }
 
-// Several quotients by one divisor: RN(1 / b) once, then each RN(a / b) by
-// Markstein's theorem (P. Markstein, IBM J. Res. Dev. 34(1), 1990): with y =
-// RN(1 / b) and q within one ulp of a / b, q + y (a - b q) rounds to RN(a / b),
-// the residual exact in one fma.  The first correction brings q within one
-// ulp, the second rounds.  y itself comes from the hardware estimate (one
-// ulp) by the same step twice; the theorem gives RN(1 / b) except for the
-// divisor with all mantissa bits set.  Five instructions in sequence per
-// quotient and no branch, against about 45 cycles and a branch per __fdiv_rn;
-// the GPU tests compare every mantissa of b and random quotients with it.
+// Quotients by a shared reciprocal: y = 1 / b from the hardware estimate and
+// one Newton step, then q = a y corrected once by its residual, q + y (a - b
+// q), the residual exact in one fma (the scheme of P. Markstein, IBM J. Res.
+// Dev. 34(1), 1990, where y rounded to nearest makes the result RN(a / b)).
+// For this y it was checked instead of proven: all 2^46 pairs of mantissas of
+// a and b give RN(a / b), and the estimate scales exactly with the exponent of
+// b over 2^-60 .. 2^60.  The same holds with y = RN(1 / b), unless every
+// mantissa bit of b is set.  Three instructions in sequence per quotient and
+// no branch, against about 45 cycles and a branch per __fdiv_rn.
 // Valid for |b| in 2^-60 .. 2^60 and |a| in 2^-100 .. 2^60 or a = 0: no
 // exponent comes near its limits, a residual is a multiple of 2^-149.
 __device__ __forceinline__ float recip(float b) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  y = fmaf(fmaf(-b, y, 1.f), y, y);
   return fmaf(fmaf(-b, y, 1.f), y, y);
 }
-__device__ __forceinline__ bool mantissa_ok(float b) { return (__float_as_uint(b) & 0x7fffffu) != 0x7fffffu; }
-__device__ __forceinline__ bool recip_ok(float b) {
-  return fabsf(b) > 0x1p-60f && fabsf(b) < 0x1p60f && mantissa_ok(b);
-}
+__device__ __forceinline__ bool recip_ok(float b) { return fabsf(b) > 0x1p-60f && fabsf(b) < 0x1p60f; }
 __device__ __forceinline__ float quot(float a, float b, float y) {
-  float q = fmul(a, y);
-  q = fmaf(fmaf(-b, q, a), y, q);
+  const float q = fmul(a, y);
   return fmaf(fmaf(-b, q, a), y, q);
 }
 
@@ -557,8 +552,7 @@ __device__ inline PinOut pin_any(PinArgs U, float4 a, float4 b, float lx, float 
 // the reference's early returns become one condition on the update (on: the
 // pin is there and not broken), which otherwise adds 0.  Returns false, with
 // a, b, lx, ly of no use, where another path is needed: an angle the rounding
-// test does not decide, a divisor that recip does not cover, an error beyond
-// 1e15 or NaN.  A predicate costs about 13 cycles and a branch on it 25 more
+// test does not decide, an error beyond 1e15 or NaN.  A predicate costs about 13 cycles and a branch on it 25 more
 // in a chain that nothing else hides, so the tests are folded into sums.
 // World: lby and the compliance may be other than 0 (the engine's pins have
 // neither, so their terms are left out: the same values).
@@ -593,7 +587,7 @@ __device__ __forceinline__ bool pin_near(const float2 *tab, const PinArgs &U, bo
   b.y = fsub(b.y, fmul(U.wB, dly));
   b.z = fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
   const bool small = World ? fadd(fabsf(bx), fabsf(by)) < 1e15f : csq < 1e30f;
-  return !on || (amax <= kSinCosNearMax && small && mantissa_ok(det) && spread == 0.f);
+  return !on || (amax <= kSinCosNearMax && small && spread == 0.f);
 }
 
 // solveAngleF, f32solver.mjs:258-301 (solver.wgsl:292-350): muscle
@@ -642,11 +636,13 @@ __device__ inline float3 angle_any(AngleArgs U, float az, float bz, float l, boo
 
 // The same operations in near form (as pin_near).  Where a term is used, |C|
 // and |over| are at least kSlackAng, so the quotients' numerators are 0 or
-// above 2^-40.  yw: recip(wA + wB).  World: any rest, target, masses and a
+// above 2^-40.  yw: 1 / (wA + wB) for quot; reach: kWrapNear, or negative
+// where the compliance is out of quot's range.  World: any rest, target, masses and a
 // missing body B; the engine's joints have 0 <= rest <= 6.27 and |target| <
 // 1.95, so only the differences of the two angles can exceed kWrapNear.
 template <bool World>
-__device__ __forceinline__ bool angle_near(const AngleArgs &U, float yw, bool on, float &az, float &bz, float &l) {
+__device__ __forceinline__ bool angle_near(const AngleArgs &U, float yw, float reach, bool on, float &az, float &bz,
+                                           float &l) {
   const bool hasB = !World || U.hasB;
   const float wSum = fadd(U.wA, U.wB), den = fadd(wSum, U.alphaTilde);
   const float y = recip(den);
@@ -670,8 +666,8 @@ __device__ __forceinline__ bool angle_near(const AngleArgs &U, float yw, bool on
   bz = hasB ? fadd(bz, fmul(U.wB, dl2)) : bz;
   float far = fmaxf(fabsf(x1), fabsf(x4));
   if (World) far = fmaxf(fmaxf(far, fabsf(x2)), fmaxf(fabsf(x3), fabsf(x5)));
-  const bool tame = World ? recip_ok(den) && recip_ok(wSum) && wSum > 0.f : mantissa_ok(den);
-  return !on || (tame && fabsf(num) < 0x1p60f && far <= kWrapNear);  // NaN fails by num
+  const bool tame = !World || (recip_ok(den) && recip_ok(wSum) && wSum > 0.f);
+  return !on || (tame && fabsf(num) < 0x1p60f && far <= reach);  // NaN fails by num
 }
 
 // A unit in the reference form.  Out of line, values in and values out:
@@ -705,7 +701,7 @@ static __device__ __noinline__ UnitOut unit_any(PinArgs U, AngleArgs V, bool pin
 // separate pin and angle levels with the reference's branches.
 template <int G>
 __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
-  const float alpha_m = fmul(S.comp_m, K.invH2);
+  const float alpha_m = fmul(S.comp_m, K.invH2), reach = alpha_m < 0x1p59f ? kWrapNear : -1.f;
   const float4 *rec = S.recs + 3 * L.lane;
   for (int p = 0; p < S.npass; p++) {
     const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
@@ -718,19 +714,19 @@ __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, b
     const AngleArgs V{r2.x, r2.y, r2.z, mo.x, alpha_m, r1.y, r1.w, true};
     const float yw = r2.w;
     rec += 3 * G;
-    const bool held = joint || ((ab & kRecIdle) == 0 && b.w == 0.f);  // b.w: an anchor's broken flag
-    const float l0 = first || !joint ? 0.f : mo.y;
-    const float lx0 = first || joint ? 0.f : mo.x, ly0 = first || joint ? 0.f : mo.y;
-    float lx = lx0, ly = ly0, l = l0;
+    const bool held = joint || b.w == 0.f;  // b.w: an anchor's broken flag (the spare record: broken)
+    // multipliers: a joint's is mo.y, a grip's are both (each ignores the other's)
+    const float m0 = first ? 0.f : mo.x, m1 = first ? 0.f : mo.y;
+    float lx = m0, ly = m1, l = m1;
     const bool op = pin_near<false>(S.tab, U, held, a, b, lx, ly);
-    const bool oa = angle_near<false>(V, yw, joint, a.z, b.z, l);
-    if (__builtin_expect(!(op && oa && alpha_m < 0x1p59f), 0)) {
-      const UnitOut o = unit_any(U, V, held, joint, false, S.Q[A], S.Q[B], lx0, ly0, l0);
+    const bool oa = angle_near<false>(V, yw, reach, joint, a.z, b.z, l);
+    if (__builtin_expect(!(op && oa), 0)) {
+      const UnitOut o = unit_any(U, V, held, joint, false, S.Q[A], S.Q[B], joint ? 0.f : m0, joint ? 0.f : m1, m1);
       a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;
     }
     S.Q[A] = a;
     if (joint) S.Q[B] = b;
-    S.mot[m] = joint ? make_float2(mo.x, l) : make_float2(lx, ly);
+    S.mot[m] = make_float2(joint ? mo.x : lx, joint ? l : ly);
     L.sync();
   }
 }
@@ -739,23 +735,18 @@ __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, b
 // {ab, lax, lay, lbx} {lby, 1 / mass A, 1 / inertia A, 1 / mass B}
 // {1 / inertia B, rest, min, max} {target, pin compliance / h^2, angle
 // compliance / h^2, recip of the inertias' sum} {lambda x, y, lambda, break
-// force}; lb is 0 without a body B.  As solve_engine, the next pass's static
-// part loads while the current one computes.
+// force}; lb is 0 without a body B.  The next pass's offset loads while the
+// current one computes.
 constexpr int kWorldRec = 5;
 template <int G>
 __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G> &L) {
   int beg = 0, end = S.npass > 0 ? S.off[1] : 0;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 r0 = zero, r1 = zero, r2 = zero, r3 = zero;
-  auto load = [&](int u) {
-    const float4 *rec = S.units + kWorldRec * u;
-    r0 = rec[0]; r1 = rec[1]; r2 = rec[2]; r3 = rec[3];
-  };
-  if (L.lane < end) load(L.lane);
   for (int p = 0; p < S.npass; p++) {
     const int u = beg + L.lane;  // passes hold at most 32 units
     const bool mine = u < end;
     const int next = p + 1 < S.npass ? S.off[p + 2] : end;
+    const float4 *rec = S.units + kWorldRec * (mine ? u : beg);
+    const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3];
     const unsigned ab = __float_as_uint(r0.x);
     const int A = ab & 0xff, B = (ab >> 8) & 0xff;
     const bool hasB = B != 0xff;
@@ -763,7 +754,6 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
     const PinArgs U{r0.y, r0.z, hasB ? r0.w : 0.f, hasB ? r1.x : 0.f, r1.y, r1.z, r1.w, r2.x, r3.y, hasB};
     const AngleArgs V{r2.y, r2.z, r2.w, r3.x, r3.z, r1.z, r2.x, hasB};
     const float yw = r3.w;
-    if (end + L.lane < next) load(end + L.lane);
     if (mine) {
       float4 a = S.Q[A], b = hasB ? S.Q[B] : anchor;
       float4 d = S.units[kWorldRec * u + 4];
@@ -771,7 +761,7 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
       const bool pin = (ab & (kHasPin | kPinBroken)) == kHasPin, angle = (ab & (kHasAngle | kAngleBroken)) == kHasAngle;
       float lx = d.x, ly = d.y, l = d.z;
       const bool op = pin_near<true>(S.tab, U, pin, a, b, lx, ly) && (!pin || (ab & kPinTame) != 0);
-      const bool oa = angle_near<true>(V, yw, angle, a.z, b.z, l);
+      const bool oa = angle_near<true>(V, yw, kWrapNear, angle, a.z, b.z, l);
       if (__builtin_expect(!(op && oa && (ab & kBounded)), 0)) {
         const UnitOut o = unit_any(U, V, pin, angle, A == B, S.Q[A], hasB ? S.Q[B] : anchor, d.x, d.y, d.z);
         a = o.a; b = o.b; lx = o.lx; ly = o.ly; l = o.l;

@@ -170,7 +170,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
   // again is what shared memory holds
   kr::Near near;
   for (int s = 0; s < A.n_steps; s++)
-    kr::island_step<true, 32>(A.K, S, A.rects, A.nR, A.near_d, kr::Lanes<32>(lane), near);
+    kr::island_step<true, 32, 1, true>(A.K, S, A.rects, A.nR, A.near_d, kr::Lanes<32>(lane), near);
 
   // write back bodies, consumed forces and constraint multipliers / flags
   for (int i = lane; i < S.nb; i += 32) {
