@@ -2108,27 +2108,15 @@ extern "C" int kr_batch_live(kr_batch *b, int32_t *live) {
   return KR_OK;
 }
 
-// Device buffers of bodies in the public layout, one per readback lane, for a
-// read of n slots (one lane if one buffer holds them); kept with the engine,
-// at most 4 x 4 MB.  Returns 0 where there is no memory for them.
-static int bodies_buffers(kr_batch *b, int n) {
-  constexpr size_t kSlot = 6 * kr::kMaxTplBodies * sizeof(float);
-  const size_t slots = std::min<size_t>(n, kr::Readback::kChunk / kSlot);
-  if (b->bodies_slots < slots) {
-    for (float *&p : b->d_bodies) {
-      if (p) cudaFree(p);
-      p = nullptr;
-    }
-    b->bodies_slots = slots;
+// The readback lanes' device buffer of bodies in the public layout, allocated
+// by the first read and kept with the engine; null without memory for it.
+static float *bodies_buffer(kr_batch *b, size_t bytes) {
+  std::lock_guard<std::mutex> lock(b->bodies_mu);
+  if (!b->d_bodies && cudaMalloc(&b->d_bodies, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    b->d_bodies = nullptr;
   }
-  const int lanes = (size_t)n > b->bodies_slots ? kr::Readback::kLanes : 1;
-  for (int i = 0; i < lanes; i++)
-    if (!b->d_bodies[i] && cudaMalloc(&b->d_bodies[i], b->bodies_slots * kSlot) != cudaSuccess) {
-      cudaGetLastError();
-      b->d_bodies[i] = nullptr;
-      return 0;
-    }
-  return lanes;
+  return b->d_bodies;
 }
 
 extern "C" int kr_batch_read_state(kr_batch *b, int32_t first, int32_t n, float *bodies, float *grips,
@@ -2137,22 +2125,27 @@ extern "C" int kr_batch_read_state(kr_batch *b, int32_t first, int32_t n, float 
   if (first < 0 || n < 0 || first + n > b->capacity) return b->fail(KR_ERR_INVALID, "read range outside the slots");
   if (n == 0) return KR_OK;
   // A kernel puts the bodies in the public layout (on the host that was 438
-  // strided element copies a slot), chunk by chunk into a lane's buffer; grips
+  // strided element copies a slot), chunk by chunk into a lane's part of
+  // the engine's buffer; grips
   // are laid out as they are read.
   constexpr size_t kPer = 6 * kr::kMaxTplBodies;
   cudaError_t e = cudaSuccess;
   if (bodies) {
-    const int lanes = bodies_buffers(b, n);
+    constexpr size_t kSlot = kPer * sizeof(float);
+    constexpr int kSlots = (int)(kr::Readback::kChunk / kSlot);  // a lane's
     const float *state = b->d_state + (size_t)first * kStateStride;
-    if (lanes > 0) {
-      e = b->rb.read(reinterpret_cast<char *>(bodies), (size_t)n * kPer * sizeof(float), b->stream,
-                     b->bodies_slots * kPer * sizeof(float), [&](int lane, size_t off, size_t bytes, cudaStream_t st) {
-                       const int i0 = (int)(off / (kPer * sizeof(float))), k = (int)(bytes / (kPer * sizeof(float)));
+    if (float *buf = bodies_buffer(b, kr::Readback::kLanes * kSlots * kSlot)) {
+      // a read without the lanes has the whole buffer
+      const size_t chunk = kSlots * kSlot * (n * kSlot < kr::Readback::kLeast ? kr::Readback::kLanes : 1);
+      e = b->rb.read(reinterpret_cast<char *>(bodies), n * kSlot, b->stream, chunk,
+                     [&](int lane, size_t off, size_t bytes, cudaStream_t st) {
+                       const int i0 = (int)(off / kSlot), k = (int)(bytes / kSlot);
+                       float *out = buf + (size_t)lane * kSlots * kPer;
                        bodies_kernel<<<(unsigned)((k * kPer + 255) / 256), 256, 0, st>>>(
-                           state + (size_t)i0 * kStateStride, b->d_bodies[lane], k);
-                       return reinterpret_cast<const char *>(b->d_bodies[lane]);
+                           state + (size_t)i0 * kStateStride, out, k);
+                       return reinterpret_cast<const char *>(out);
                      });
-    } else {  // no device memory for the buffers
+    } else {  // no device memory for the buffer
       std::vector<float> blk((size_t)std::min(n, 1024) * kStateStride);
       for (int i0 = 0; i0 < n && e == cudaSuccess; i0 += 1024) {
         const int k = std::min(1024, n - i0);
@@ -2257,8 +2250,7 @@ extern "C" int kr_batch_set_stream(kr_batch *b, void *stream) {
 extern "C" void kr_batch_destroy(kr_batch *b) {
   if (!b) return;
   cudaDeviceSynchronize();
-  for (float *p : b->d_bodies)
-    if (p) cudaFree(p);
+  if (b->d_bodies) cudaFree(b->d_bodies);
   void *ptrs[] = {b->d_tpl, const_cast<float4 *>(b->T.body), const_cast<float4 *>(b->T.pts),
                   const_cast<float4 *>(b->T.recs), const_cast<int *>(b->T.arm_tip), const_cast<int *>(b->T.arm_seg0),
                   const_cast<int *>(b->T.arm_segs), b->d_rects, b->d_map_off, b->d_map_cull, b->d_rects64,

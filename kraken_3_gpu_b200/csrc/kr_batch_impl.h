@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <map>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -331,11 +332,11 @@ struct kr_batch {
   int *d_steps = nullptr, *h_steps = nullptr;  // every slot's step counter after a slice
   cudaStream_t ctl = nullptr;          // the stop word's copy while a slice runs
   cudaEvent_t slice_start = nullptr, slice_end = nullptr;
-  // readbacks: pinned chunks, and per lane a device buffer of bodies in the
+  // readbacks: pinned chunks, and the lanes' device buffer of bodies in the
   // public layout
   kr::Readback rb;
-  float *d_bodies[kr::Readback::kLanes] = {nullptr};
-  size_t bodies_slots = 0;             // slots each of them holds
+  float *d_bodies = nullptr;
+  std::mutex bodies_mu;
   int last_slices = 0, last_kernels = 0;  // of the last kr_batch_run
   long long last_creature_launches = 0;    // ... live creatures per slice, summed
 

@@ -27,7 +27,6 @@
 #include <vector>
 
 #include "../../include/kraken_b200.h"
-#include "kr_readback.h"
 #include "kr_solver.cuh"
 #include "kr_units.h"
 
@@ -251,7 +250,6 @@ struct kr_world {
   bool uploaded = false;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  kr::Readback rb;
   std::string err;
 
   int fail(int code, const std::string &msg) {
@@ -665,13 +663,6 @@ extern "C" int kr_download(kr_world *w, float *bodies, uint32_t *cons) {
   if (!w->uploaded) return w->fail(KR_ERR_STATE, "download before upload");
   cudaError_t e;
   const size_t nb = sizeof(float) * 12 * (size_t)w->nB, nc = cons ? sizeof(uint32_t) * 20 * (size_t)w->nC : 0;
-  if (nc > kr::Readback::kChunk) {
-    // a large world: in chunks by several threads
-    if (bodies && (e = w->rb.read(bodies, w->d_bodies, nb, w->stream)) != cudaSuccess)
-      return w->cuda_fail(e, "download(bodies)");
-    if ((e = w->rb.read(cons, w->d_cons, nc, w->stream)) != cudaSuccess) return w->cuda_fail(e, "download(cons)");
-    return KR_OK;
-  }
   if (bodies && (e = cudaMemcpyAsync(bodies, w->d_bodies, nb, cudaMemcpyDeviceToHost, w->stream)) != cudaSuccess)
     return w->cuda_fail(e, "download(bodies)");
   if (nc && (e = cudaMemcpyAsync(cons, w->d_cons, nc, cudaMemcpyDeviceToHost, w->stream)) != cudaSuccess)

@@ -285,3 +285,27 @@ def test_noalloc_schedule_equals_the_handles_step(islands, nb, nc, steps):
         assert np.array_equal(dev[1].cpu().numpy(), cons.view(np.int32))
     finally:
         L.kr_destroy(h)
+
+
+@pytest.mark.parametrize("n", [2393, 2395, 3001])
+def test_large_readbacks_equal_small_ones(n):
+    """Reads on both sides of where the readback's lanes start (4 MB: 2,394
+    slots' bodies, 2,341 slots' rings of 8), with a last chunk that is not
+    full: the whole read equals reads of 250 slots, also from two threads at
+    once."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from kraken_3_gpu_b200 import batch, workloads
+    w = workloads.uneven(n=n, n_maps=2, seed=4, h_min=3, h_max=9)
+    eng = batch.BatchEngine(w.maps, w.n, obs_ring=8)
+    workloads.spawn_all(eng, w)
+    eng.run(9)
+    parts = [eng.read_state(i, min(250, n - i)) for i in range(0, n, 250)]
+    obs = np.concatenate([eng.read_obs(i, min(250, n - i)) for i in range(0, n, 250)])
+    with ThreadPoolExecutor(2) as pool:
+        whole = list(pool.map(lambda _: (eng.read_state(), eng.read_obs()), range(2)))
+    for st, ob in whole:
+        for f in ("px", "py", "vx", "vy", "ang", "av", "grips", "steps"):
+            assert np.array_equal(st[f], np.concatenate([p[f] for p in parts])), f
+        assert np.array_equal(ob, obs)
+    eng.close()
