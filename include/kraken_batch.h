@@ -237,11 +237,9 @@ int kr_probe_wrap(const double *d, int32_t n, double *out);
  * creatures), warps per CTA (1..16, at most 64 creatures per CTA) and CTAs
  * per SM (0 = 16 / warps).  A CTA gets an equal share of the SM's shared
  * memory; a group of one body template holds as many creatures as fit in it.
- * Until this is called the engine picks the shape per launch: 32 lanes x 4
- * warps below 16 live creatures per SM, 16 lanes x 8 warps below 96 (8
- * lanes when most creatures run the fused policy or the net, or an
- * observation ring is kept), else 8 lanes x 8 warps -- x 16 warps in one CTA
- * per SM when most creatures run the net or a ring is kept;
+ * Until this is called the engine picks the shape per launch, CTAs of 4
+ * warps: 32 lanes below 8 live creatures per SM (16 in a rollout server), 16
+ * lanes below 96, else 8.
  * lanes_per_creature = 0 returns to that (the other arguments are
  * ignored).  Results do not depend on the launch
  * shape. */

@@ -1,10 +1,12 @@
 // kr_world.cu -- the gpuworld.js drop-in: handle, schedule and the plain
-// step kernel (one launch per kr_step call, one warp per creature).
+// step kernel (one launch per kr_step call of up to 128 env steps, one warp per
+// creature).
 //
 // Device buffers hold the reference's own AoS blocks (48 B bodies, 80 B
 // constraints, 16 B forces / collision points), so upload and download are
 // single copies and mirrorInto/packControls keep their exact field offsets.
-// The kernel stages each creature into shared memory as SoA for the launch.
+// The kernel stages each creature into shared memory for the launch, bodies and
+// solve units as 16-byte records.
 //
 // Schedule.  The reference runs one dispatch per colour class
 // (gpuworld.js:353-366); a colour class is body-disjoint, so the classes in
