@@ -2287,8 +2287,8 @@ extern "C" int kr_batch_set_stream(kr_batch *b, void *stream) {
 extern "C" void kr_batch_destroy(kr_batch *b) {
   if (!b) return;
   cudaDeviceSynchronize();
-  if (b->d_bodies) cudaFree(b->d_bodies);
-  void *ptrs[] = {b->d_tpl, const_cast<float4 *>(b->T.body), const_cast<float4 *>(b->T.pts),
+  free_part(b->main);
+  void *ptrs[] = {b->d_bodies, b->d_tpl, const_cast<float4 *>(b->T.body), const_cast<float4 *>(b->T.pts),
                   const_cast<float4 *>(b->T.recs), const_cast<int *>(b->T.arm_tip), const_cast<int *>(b->T.arm_seg0),
                   const_cast<int *>(b->T.arm_segs), b->d_rects, b->d_map_off, b->d_map_cull, b->d_rects64,
                   b->d_state, b->d_grip, b->d_glam, b->d_cd, b->d_ctrl, b->d_meta, b->d_obs,
