@@ -214,8 +214,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4) plain_step_kernel(Step
   plain_step_body(A);
 }
 
+// The copy runs on the handle's stream: after the steps that still read the
+// old table, before those that read the new one (the handle's stream does not
+// wait for the legacy one, on which a plain copy would run).
 template <typename T>
-cudaError_t dev_upload(T **dptr, size_t *cap, const std::vector<T> &v) {
+cudaError_t dev_upload(T **dptr, size_t *cap, const std::vector<T> &v, cudaStream_t st) {
   size_t n = std::max<size_t>(v.size(), 1);
   if (*dptr == nullptr || *cap < n) {
     if (*dptr) cudaFree(*dptr);
@@ -225,7 +228,7 @@ cudaError_t dev_upload(T **dptr, size_t *cap, const std::vector<T> &v) {
     *cap = n;
   }
   if (v.empty()) return cudaSuccess;
-  return cudaMemcpy(*dptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  return cudaMemcpyAsync(*dptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
 }  // namespace
@@ -380,7 +383,7 @@ extern "C" int kr_create(const kr_solver_params *params, uint32_t n_bodies, uint
     return cleanup_fail(e, "cudaMalloc(control staging)");
   if ((e = cudaMalloc(&w->d_forces, sizeof(float) * 4 * n_bodies)) != cudaSuccess)
     return cleanup_fail(e, "cudaMalloc(forces)");
-  if ((e = cudaMemset(w->d_forces, 0, sizeof(float) * 4 * n_bodies)) != cudaSuccess)
+  if ((e = cudaMemsetAsync(w->d_forces, 0, sizeof(float) * 4 * n_bodies, w->stream)) != cudaSuccess)
     return cleanup_fail(e, "cudaMemset(forces)");
   std::vector<float4> r4(n_rects);
   double half_thick = 0.0, r_max = 0.0;
@@ -403,15 +406,16 @@ extern "C" int kr_create(const kr_solver_params *params, uint32_t n_bodies, uint
   w->near_d = std::isfinite(cull) && cull < 1e30 ? (float)cull : 1e30f;
   if ((e = cudaMalloc(&w->d_rects, sizeof(float4) * n_rects)) != cudaSuccess)
     return cleanup_fail(e, "cudaMalloc(rects)");
-  if ((e = cudaMemcpy(w->d_rects, r4.data(), sizeof(float4) * n_rects, cudaMemcpyHostToDevice)) !=
-      cudaSuccess)
+  if ((e = cudaMemcpyAsync(w->d_rects, r4.data(), sizeof(float4) * n_rects, cudaMemcpyHostToDevice,
+                           w->stream)) != cudaSuccess)
     return cleanup_fail(e, "cudaMemcpy(rects)");
   if ((e = cudaMalloc(&w->d_coll, sizeof(uint4) * std::max<uint32_t>(n_coll_pts, 1))) != cudaSuccess)
     return cleanup_fail(e, "cudaMalloc(collPts)");
   if (n_coll_pts &&
-      (e = cudaMemcpy(w->d_coll, coll_pts, sizeof(uint4) * n_coll_pts, cudaMemcpyHostToDevice)) !=
-          cudaSuccess)
+      (e = cudaMemcpyAsync(w->d_coll, coll_pts, sizeof(uint4) * n_coll_pts, cudaMemcpyHostToDevice,
+                           w->stream)) != cudaSuccess)
     return cleanup_fail(e, "cudaMemcpy(collPts)");
+  if ((e = cudaStreamSynchronize(w->stream)) != cudaSuccess) return cleanup_fail(e, "create(sync)");
   w->h_coll_range.assign(2 * (size_t)n_bodies, 0u);
   if (coll_range) std::memcpy(w->h_coll_range.data(), coll_range, sizeof(uint32_t) * 2 * n_bodies);
   *out = w;
@@ -544,13 +548,15 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
     maxP = std::max(maxP, np);
     maxLv = std::max(maxLv, nlv);
   }
-  cudaError_t e;
-  if ((e = dev_upload(&w->d_isl, &w->c_isl, isl)) != cudaSuccess) return w->cuda_fail(e, "upload(islands)");
-  if ((e = dev_upload(&w->d_ibodies, &w->c_ibodies, h_bodies)) != cudaSuccess) return w->cuda_fail(e, "upload(island bodies)");
-  if ((e = dev_upload(&w->d_units, &w->c_units, h_units)) != cudaSuccess) return w->cuda_fail(e, "upload(island units)");
-  if ((e = dev_upload(&w->d_ipts, &w->c_ipts, h_pts)) != cudaSuccess) return w->cuda_fail(e, "upload(island points)");
-  if ((e = dev_upload(&w->d_bpt, &w->c_bpt, h_bpt)) != cudaSuccess) return w->cuda_fail(e, "upload(body point ranges)");
-  if ((e = dev_upload(&w->d_pass, &w->c_pass, h_pass)) != cudaSuccess) return w->cuda_fail(e, "upload(passes)");
+  // steps in flight read the tables that are replaced or freed now
+  cudaError_t e = cudaStreamSynchronize(w->stream);
+  if (e != cudaSuccess) return w->cuda_fail(e, "upload(steps in flight)");
+  if ((e = dev_upload(&w->d_isl, &w->c_isl, isl, w->stream)) != cudaSuccess) return w->cuda_fail(e, "upload(islands)");
+  if ((e = dev_upload(&w->d_ibodies, &w->c_ibodies, h_bodies, w->stream)) != cudaSuccess) return w->cuda_fail(e, "upload(island bodies)");
+  if ((e = dev_upload(&w->d_units, &w->c_units, h_units, w->stream)) != cudaSuccess) return w->cuda_fail(e, "upload(island units)");
+  if ((e = dev_upload(&w->d_ipts, &w->c_ipts, h_pts, w->stream)) != cudaSuccess) return w->cuda_fail(e, "upload(island points)");
+  if ((e = dev_upload(&w->d_bpt, &w->c_bpt, h_bpt, w->stream)) != cudaSuccess) return w->cuda_fail(e, "upload(body point ranges)");
+  if ((e = dev_upload(&w->d_pass, &w->c_pass, h_pass, w->stream)) != cudaSuccess) return w->cuda_fail(e, "upload(passes)");
   w->nI = nI;
   // round up so every per-warp region keeps 16-byte alignment of its arrays
   w->maxB = (maxB + 3) & ~3;

@@ -1,11 +1,69 @@
-"""Handles over their lifetime: what closing one gives back."""
+"""Handles over their lifetime: what closing one gives back, and an upload
+that replaces a world while its steps are in flight."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from kraken_3_gpu_b200 import batch
+from kraken_3_gpu_b200 import _native, batch
 from oracle import binding as ob
 
 pytestmark = pytest.mark.gpu
+
+_F32P, _U32P = C.POINTER(C.c_float), C.POINTER(C.c_uint32)
+PARAMS = _native.SolverParams(1 / 120, 2, 4, 3.0, 3.0, 360.0, 18.0)
+RECTS = np.array([[0, 0, 400, 14], [0, 286, 400, 14], [0, 0, 14, 300], [386, 0, 14, 300]], np.float32)
+
+
+def _world(n, nc):
+    """A drop-in handle of n bodies without collision points and nc constraints."""
+    h = C.c_void_p()
+    _native.check(_native.lib().kr_create(C.byref(PARAMS), n, nc, RECTS.ctypes.data_as(_F32P), len(RECTS), None, 0,
+                                          None, C.byref(h)))
+    return h
+
+
+def _bodies(n, seed):
+    r = np.random.default_rng(seed)
+    b = np.zeros((n, 12), np.float32)
+    b[:, 0], b[:, 1], b[:, 6] = r.uniform(30, 350, n), r.uniform(30, 250, n), r.uniform(-3, 3, n)
+    b[:, 2:4], b[:, 7] = b[:, :2], b[:, 6]
+    b[:, 9], b[:, 10] = 1 / r.uniform(1, 20, n), 1 / r.uniform(20, 900, n)
+    return b
+
+
+def _chains(n, size):
+    """Pin and angle constraints along chains of `size` bodies out of n, as
+    many records as 2 n (the last ones pin single bodies to the world)."""
+    cons = np.zeros((2 * n, 20), np.float32)
+    cu = cons.view(np.uint32)
+    k = 0
+    for i in range(n):
+        if i % size != size - 1:
+            for t in (0, 1):
+                cu[k, 0], cu[k, 1], cu[k, 2] = i, i + 1, t
+                k += 1
+    for i in range(2 * n - k):
+        cu[k, 0], cu[k, 1], cu[k, 2] = i % n, 0xFFFFFFFF, 0
+        cons[k, 6:8] = 100 + i % 90
+        k += 1
+    cons[:, 4], cons[:, 8] = 6.0, 1e-5
+    cons[:, 11], cons[:, 12], cons[:, 16] = -1, 1, 400
+    return cons
+
+
+def _upload(h, bodies, cons):
+    _native.check(_native.lib().kr_upload(h, bodies.ctypes.data_as(_F32P), cons.ctypes.data_as(_U32P), None, None), h)
+
+
+def _step(h, steps):
+    _native.check(_native.lib().kr_step(h, steps), h)
+
+
+def _download(h, n, nc):
+    bodies, cons = np.zeros((n, 12), np.float32), np.zeros((nc, 20), np.float32)
+    _native.check(_native.lib().kr_download(h, bodies.ctypes.data_as(_F32P), cons.ctypes.data_as(_U32P)), h)
+    return bodies.view(np.uint32), cons.view(np.uint32)
 
 
 def _free_bytes():
@@ -37,3 +95,27 @@ def test_closed_engines_give_their_memory_back():
     for _ in range(300):
         one()
     assert before - _free_bytes() < 4 << 20
+
+
+@pytest.mark.parametrize("size", [(40, 3), (2, 48)])
+def test_upload_during_steps_equals_a_fresh_handle(size):
+    """kr_step returns while its launches (of up to 128 env steps each) run;
+    an upload of another constraint structure right behind it replaces the
+    tables that they read, and must wait for them."""
+    n = 1920
+    first, second = _chains(n, size[0]), _chains(n, size[1])
+    a, b = _world(n, 2 * n), _world(n, 2 * n)
+    try:
+        for turn in range(3):
+            _upload(a, _bodies(n, 1), first)
+            _step(a, 300)
+            _upload(a, _bodies(n, 2 + turn), second)
+            _step(a, 20)
+            got = _download(a, n, 2 * n)
+            _upload(b, _bodies(n, 2 + turn), second)
+            _step(b, 20)
+            want = _download(b, n, 2 * n)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    finally:
+        for h in (a, b):
+            _native.lib().kr_destroy(h)
