@@ -452,6 +452,15 @@ constexpr unsigned kHasPin = 1u << 16, kPinBroken = 1u << 17, kHasAngle = 1u << 
                    // two bodies whose inverse masses are finite (an update of 0 times them is 0)
                    kBounded = 1u << 22;
 
+// The flags by which a drop-in unit takes the short forms below: its pin is
+// tame or it has none (a disabled pin's levers enter sums with 0, so they must
+// be finite too), its masses are bounded
+__device__ inline unsigned unit_forms(bool has_pin, bool self, float lax, float lay, float lbx, float lby, float wA,
+                                      float wIA, float wB, float wIB) {
+  return (!has_pin || pin_tame(lax, lay, lbx, lby, wA, wIA, wB, wIB) ? kPinTame : 0u) |
+         (!self && fabsf(wA) + fabsf(wIA) + fabsf(wB) + fabsf(wIB) < 1e30f ? kBounded : 0u);
+}
+
 // The speed clamp of integrateF and finalizeF.  A squared speed of at most
 // 0.999 maxSpeed^2 has a length of at most maxSpeed however it rounds, so the
 // square root is taken only near the limit.
@@ -587,7 +596,8 @@ __device__ __forceinline__ bool pin_near(const float2 *tab, const PinArgs &U, bo
   b.y = fsub(b.y, fmul(U.wB, dly));
   b.z = fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
   const bool small = World ? fadd(fabsf(bx), fabsf(by)) < 1e15f : csq < 1e30f;
-  return !on || (amax <= kSinCosNearMax && small && spread == 0.f);
+  // (a lever of a disabled pin must come out finite: 0 times it is added)
+  return amax <= kSinCosNearMax && (!on || (small && spread == 0.f));
 }
 
 // solveAngleF, f32solver.mjs:258-301 (solver.wgsl:292-350): muscle
@@ -760,7 +770,7 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
       if (first) d.x = d.y = d.z = 0.f;
       const bool pin = (ab & (kHasPin | kPinBroken)) == kHasPin, angle = (ab & (kHasAngle | kAngleBroken)) == kHasAngle;
       float lx = d.x, ly = d.y, l = d.z;
-      const bool op = pin_near<true>(S.tab, U, pin, a, b, lx, ly) && (!pin || (ab & kPinTame) != 0);
+      const bool op = pin_near<true>(S.tab, U, pin, a, b, lx, ly) && (ab & kPinTame) != 0;
       const bool oa = angle_near<true>(V, yw, kWrapNear, angle, a.z, b.z, l);
       if (__builtin_expect(!(op && oa && (ab & kBounded)), 0)) {
         const UnitOut o = unit_any(U, V, pin, angle, A == B, S.Q[A], hasB ? S.Q[B] : anchor, d.x, d.y, d.z);

@@ -149,7 +149,6 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
       r0.w = __uint_as_float(w1.z); r1.x = __uint_as_float(w1.w);
       r3.y = kr::fmul(__uint_as_float(w2.x), A.K.invH2);
       brk = __uint_as_float(w4.x);
-      if (kr::pin_tame(r0.y, r0.z, has_b ? r0.w : 0.f, has_b ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y)) ab |= kr::kPinTame;
     }
     if (t.z >= 0) {
       const uint4 *c4 = reinterpret_cast<const uint4 *>(A.cons + 20 * (size_t)t.z);
@@ -160,7 +159,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
       r3.z = kr::fmul(__uint_as_float(w2.x), A.K.invH2);
       r3.w = kr::recip(kr::fadd(wa.y, wb.y));
     }
-    if (bA != bB && wa.x + wa.y + wb.x + wb.y < 1e30f) ab |= kr::kBounded;
+    ab |= kr::unit_forms(t.y >= 0, bA == bB, r0.y, r0.z, has_b ? r0.w : 0.f, has_b ? r1.x : 0.f, wa.x, wa.y, wb.x, wb.y);
     r0.x = __uint_as_float(ab);
     float4 *rec = S.units + kr::kWorldRec * u;
     rec[0] = r0; rec[1] = r1; rec[2] = r2; rec[3] = r3; rec[4] = make_float4(0.f, 0.f, 0.f, brk);

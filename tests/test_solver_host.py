@@ -1,0 +1,73 @@
+"""Device functions of csrc/kr_solver.cuh run on the CPU (tests/cuda_on_host.h),
+where a test can look at more than a step's results: which form a value takes,
+and how many rects a collision pass reads."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "kraken_3_gpu_b200", "csrc")
+
+COMMON = r'''
+#include <cstdio>
+#include <random>
+#include <vector>
+#include "cuda_on_host.h"
+using namespace kr;
+static float2 g_tab[kSinEntries];
+static float bits(unsigned u) { return __uint_as_float(u); }
+static bool same(float4 a, float4 b) { return std::memcmp(&a, &b, sizeof a) == 0; }
+'''
+
+
+def _run(tmp_path, body, *args):
+    src = tmp_path / "t.cpp"
+    src.write_text(COMMON + body)
+    exe = tmp_path / "t"
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-mfma", "-w", "-I", HERE, "-I", CSRC, "-o",
+                    str(exe), str(src)], check=True)
+    out = subprocess.run([str(exe), *args], capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0, out.stdout + out.stderr
+    return out.stdout
+
+
+DISABLED = r'''
+// one unit of two bodies whose pin and angle constraint are broken (or not
+// there): both bodies must stay as they are, whatever the records hold
+int main() {
+  stage_sin(g_tab);
+  const float inf = kInf, nan = bits(0x7fc00000u);
+  const float angles[] = {0.3f, 60.f, 70.f, 1e4f, 1e17f, 1e30f, -3e38f, inf, -inf};
+  const float levers[] = {7.f, 1e25f, inf, nan};
+  const float masses[] = {0.25f, 0.f, 1e31f, inf, -inf};
+  int n = 0;
+  for (float az : angles) for (float bz : angles) for (float lev : levers) for (float im : masses)
+  for (int ref = 0; ref < 3; ref++) for (int pin = 0; pin < 2; pin++) for (int world = 0; world < 2; world++) {
+    float4 Q[2] = {make_float4(10.f, 20.f, az, 0.f), make_float4(14.f, 22.f, bz, 0.f)}, in[2] = {Q[0], Q[1]};
+    float4 body[2] = {make_float4(im, ref == 1 ? im : 0.01f, 0.f, 0.f), make_float4(0.5f, ref == 2 ? im : 0.02f, 0.f, 0.f)};
+    const float lax = pin ? lev : 0.f, lay = pin ? 2.f : 0.f, lbx = pin ? 3.f : 0.f, lby = pin ? lev : 0.f;
+    const float wB = world ? 0.f : body[1].x, wIB = world ? 0.f : body[1].y;
+    const unsigned ab = 0u | (world ? 0xffu : 1u) << 8 | kHasAngle | kAngleBroken | (pin ? kHasPin | kPinBroken : 0u) |
+                        unit_forms(pin, false, lax, lay, world ? 0.f : lbx, world ? 0.f : lby, body[0].x, body[0].y, wB, wIB);
+    float4 rec[kWorldRec] = {{bits(ab), lax, lay, lbx}, {lby, body[0].x, body[0].y, wB}, {wIB, lev, -1.f, 1.f},
+                             {lev, lev, lev, recip(fadd(body[0].y, wIB))}, {0.f, 0.f, 0.f, 100.f}};
+    Island S{};
+    int off[2] = {0, 1};
+    S.Q = Q; S.tab = g_tab; S.units = rec; S.nu = 1; S.npass = 1; S.off = off; S.nb = 2;
+    solve_world<1>(S, true, Lanes<1>(0));
+    solve_world<1>(S, false, Lanes<1>(0));
+    if (!same(Q[0], in[0]) || !same(Q[1], in[1])) {
+      std::printf("FAIL angles %g %g lever %g mass %g: %g %g\n", az, bz, lev, im, Q[0].z, Q[1].z);
+      return 1;
+    }
+    n++;
+  }
+  std::printf("ok %d\n", n);
+  return 0;
+}
+'''
+
+
+def test_disabled_constraints_leave_their_bodies_alone(tmp_path):
+    assert _run(tmp_path, DISABLED).startswith("ok")
