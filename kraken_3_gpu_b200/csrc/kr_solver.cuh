@@ -463,10 +463,10 @@ __device__ inline unsigned unit_forms(bool has_pin, bool self, float lax, float 
 
 // The speed clamp of integrateF and finalizeF.  A squared speed of at most
 // 0.999 maxSpeed^2 has a length of at most maxSpeed however it rounds, so the
-// square root is taken only near the limit.
+// square root is taken only near the limit (and where a square overflows).
 __device__ __forceinline__ void clamp_speed(const SolverConsts &K, float &vx, float &vy) {
   const float s2 = fadd(fmul(vx, vx), fmul(vy, vy));
-  if (s2 > (K.maxSpeed > 0.f ? 0.999f * K.maxSpeed * K.maxSpeed : -1.f)) {
+  if (!(s2 < (K.maxSpeed > 0.f ? 0.999f * K.maxSpeed * K.maxSpeed : -1.f))) {
     const float sp = fsqrt(s2);
     if (sp > K.maxSpeed) {
       const float k = fdiv(K.maxSpeed, sp);

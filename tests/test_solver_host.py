@@ -71,3 +71,41 @@ int main() {
 
 def test_disabled_constraints_leave_their_bodies_alone(tmp_path):
     assert _run(tmp_path, DISABLED).startswith("ok")
+
+
+CLAMP = r'''
+// clamp_speed against the reference's plain form for limits of every size
+int main() {
+  std::mt19937 r(3);
+  std::vector<float> lim = {0.f, -1.f, kInf, -kInf, bits(0x7fc00000u), 1.f, 360.f, 3e38f, 1e20f, 1.9e19f, 1.8e19f, 1e-18f, 1e-22f, 1e-23f, 1e-40f};
+  for (int i = 0; i < 200; i++) lim.push_back(bits(r() & 0x7f7fffffu));
+  long n = 0;
+  for (float m : lim) {
+    SolverConsts K{};
+    K.maxSpeed = m;
+    for (int i = 0; i < 20000; i++) {
+      float x, y;
+      const float a = std::fabs(m) < 1e38f ? std::fabs(m) : 1e38f;
+      if (i < 10000) { x = bits(r() & 0xff7fffffu); y = i % 3 ? bits(r() & 0xff7fffffu) : 0.f; }
+      else { const float t = 6.2831853f * (r() >> 8) / 16777216.f, s = 0.9f + 0.2f * (r() >> 8) / 16777216.f;
+             x = a * s * std::cos(t); y = a * s * std::sin(t); }
+      if (i % 1000 == 0) x = i % 2000 ? kInf : bits(0x7fc00000u);
+      float vx = x, vy = y, wx = x, wy = y;
+      clamp_speed(K, vx, vy);
+      const float sp = length2(wx, wy);
+      if (sp > m) { const float k = fdiv(m, sp); wx = fmul(wx, k); wy = fmul(wy, k); }
+      if (std::memcmp(&vx, &wx, 4) || std::memcmp(&vy, &wy, 4)) {
+        std::printf("FAIL limit %g of (%g, %g): (%g, %g) for (%g, %g)\n", m, x, y, vx, vy, wx, wy);
+        return 1;
+      }
+      n++;
+    }
+  }
+  std::printf("ok %ld\n", n);
+  return 0;
+}
+'''
+
+
+def test_speed_clamp_equals_the_plain_form(tmp_path):
+    assert _run(tmp_path, CLAMP).startswith("ok")
