@@ -71,6 +71,9 @@ class Readback {
     int dev = 0;
     cudaError_t status[kLanes] = {};
     if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+    // cudaStreamPerThread names another stream in every lane's thread, so the
+    // lanes start when the work on the caller's has finished
+    if (const cudaError_t e = cudaStreamSynchronize(st); e != cudaSuccess) return e;
     const int lanes = (int)std::min<size_t>(kLanes, n);
     auto run = [&](int lane) {
       cudaError_t e = cudaSetDevice(dev);
