@@ -1640,6 +1640,7 @@ extern "C" int kr_batch_create(const kr_batch_desc *desc, kr_batch **out) {
   K.substeps = p.substeps;
   K.iterations = p.iterations;
   cudaGetDevice(&dev);
+  b->rb.device = dev;
   cudaDeviceGetAttribute(&b->n_sm, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&b->smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&b->smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
@@ -2149,6 +2150,7 @@ extern "C" int kr_batch_live(kr_batch *b, int32_t *live) {
 // MB take 0.4 ms longer than 350 KB); null without memory for it.
 static float *bodies_buffer(kr_batch *b, size_t bytes) {
   std::lock_guard<std::mutex> lock(b->bodies_mu);
+  const kr::OnDevice on(b->rb.device);
   if (!b->d_bodies && cudaMalloc(&b->d_bodies, bytes) != cudaSuccess) {
     cudaGetLastError();
     b->d_bodies = nullptr;

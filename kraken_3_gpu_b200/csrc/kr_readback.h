@@ -17,8 +17,28 @@
 
 namespace kr {
 
+// `device` is the calling thread's current device while this lives
+class OnDevice {
+ public:
+  explicit OnDevice(int device) {
+    if (cudaGetDevice(&before_) != cudaSuccess) before_ = device;
+    if (before_ != device) cudaSetDevice(device);
+    device_ = device;
+  }
+  ~OnDevice() {
+    if (before_ != device_) cudaSetDevice(before_);
+  }
+  OnDevice(const OnDevice &) = delete;
+  OnDevice &operator=(const OnDevice &) = delete;
+
+ private:
+  int before_ = 0, device_ = 0;
+};
+
 class Readback {
  public:
+  int device = 0;  // of the streams and memory it reads from
+
   static constexpr int kLanes = 8;
   static constexpr size_t kChunk = size_t(512) << 10;
   static constexpr size_t kLeast = size_t(4) << 20;  // smaller reads are plain copies
@@ -56,6 +76,7 @@ class Readback {
   template <class Produce>
   cudaError_t read(char *dst, size_t bytes, cudaStream_t st, size_t chunk, Produce produce) {
     std::lock_guard<std::mutex> lock(mu_);
+    const OnDevice on(device);  // events and launches need it; copies on a stream do not
     const size_t n = (bytes + chunk - 1) / chunk;
     if (n < 2 || bytes < kLeast || chunk > kChunk || !prepare()) {
       for (size_t c = 0; c < n; c++) {
@@ -68,15 +89,13 @@ class Readback {
       }
       return cudaSuccess;
     }
-    int dev = 0;
     cudaError_t status[kLanes] = {};
-    if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
     // cudaStreamPerThread names another stream in every lane's thread, so the
     // lanes start when the work on the caller's has finished
     if (const cudaError_t e = cudaStreamSynchronize(st); e != cudaSuccess) return e;
     const int lanes = (int)std::min<size_t>(kLanes, n);
     auto run = [&](int lane) {
-      cudaError_t e = cudaSetDevice(dev);
+      cudaError_t e = cudaSetDevice(device);
       for (size_t c = lane; c < n && e == cudaSuccess; c += lanes) {
         const size_t off = c * chunk, k = std::min(chunk, bytes - off);
         const char *src = produce(lane, off, k, st);

@@ -96,3 +96,38 @@ int main() {
   return 0;
 }
 ''')
+
+
+def test_reads_need_no_current_device(tmp_path):
+    """An engine on device 1, read by threads whose current device is 0: every
+    call that depends on the current device is made under the engine's, and
+    the caller's is as it was afterwards."""
+    _run(tmp_path, r'''
+int main() {
+  Queue q1;
+  q1.device = 1;
+  const cudaStream_t st = reinterpret_cast<cudaStream_t>(&q1);
+  std::vector<char> src(size_t(9) << 20), dst(src.size());
+  for (size_t i = 0; i < src.size(); i++) src[i] = (char)(i * 31);
+  kr::Readback rb;
+  rb.device = 1;
+  bool wrong = false;
+  auto reader = [&] {
+    if (rb.read(dst.data(), src.data(), src.size(), st) != cudaSuccess || dst != src) wrong = true;
+    for (size_t bytes : {size_t(1000), src.size()}) {
+      std::fill(dst.begin(), dst.end(), 0);
+      const cudaError_t e = rb.read(dst.data(), bytes, st, kr::Readback::kChunk,
+                                    [&](int, size_t off, size_t, cudaStream_t s) {
+                                      if (t_device != of(s).device) wrong = true;
+                                      return (const char *)src.data() + off;
+                                    });
+      if (e != cudaSuccess || std::memcmp(dst.data(), src.data(), bytes)) wrong = true;
+    }
+    if (t_device != 0) wrong = true;
+  };
+  reader();
+  std::thread(reader).join();
+  std::printf(wrong ? "FAIL\n" : "ok\n");
+  return wrong;
+}
+''')
