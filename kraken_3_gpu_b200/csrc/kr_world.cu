@@ -69,9 +69,14 @@ struct StepArgs {
   DeviceTables T;
 };
 
-__host__ __device__ inline int warp_smem_words(int mb, int mu, int mp) {
+__host__ __device__ constexpr int warp_smem_words(int mb, int mu, int mp) {
   return 20 * mb + 4 * kr::kWorldRec * mu + 4 * mp + 4 * ((kr::kMaxCulled + 7) / 8) + mb;
 }
+
+// a block's dynamic shared memory when every warp holds the largest island
+constexpr int kMaxWorldSmem =
+    (int)sizeof(float) * kWarpsPerBlock *
+    warp_smem_words(KR_MAX_ISLAND_BODIES, KR_MAX_ISLAND_CONSTRAINTS, KR_MAX_ISLAND_COLLPTS);
 
 // Writable views of the statics while they are staged; the solver reads them
 // through the const pointers of kr::Island.
@@ -564,8 +569,10 @@ int build_schedule(kr_world *w, const float *bodies, const uint32_t *cons) {
   w->maxLv = maxLv;
   w->smem_bytes =
       sizeof(float) * kWarpsPerBlock * (size_t)warp_smem_words(w->maxB, w->maxU, w->maxP);
-  if ((e = cudaFuncSetAttribute(plain_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)w->smem_bytes)) != cudaSuccess)
+  // the limit belongs to the kernel, not to the handle: always the largest
+  // island's, so that no upload lowers it below another handle's launches
+  if ((e = cudaFuncSetAttribute(plain_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWorldSmem)) !=
+      cudaSuccess)
     return w->cuda_fail(e, "cudaFuncSetAttribute(plain_step_kernel)");
   return KR_OK;
 }

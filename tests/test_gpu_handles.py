@@ -119,3 +119,37 @@ def test_upload_during_steps_equals_a_fresh_handle(size):
     finally:
         for h in (a, b):
             _native.lib().kr_destroy(h)
+
+
+@pytest.mark.parametrize("nb,nc", [(40, 150), (160, 384)])
+def test_handles_of_unlike_islands_step_side_by_side(nb, nc):
+    """A handle whose island needs more shared memory than a launch has by
+    default, then the upload of a small one: both step, in either order, to
+    what each gives by itself."""
+    cons = np.zeros((nc, 20), np.float32)
+    cu = cons.view(np.uint32)
+    for k in range(nc):
+        cu[k, 0], cu[k, 1] = (k, k + 1) if k < nb - 1 else (k % nb, 0xFFFFFFFF)
+    cons[nb - 1:, 6:8] = 150
+    cons[:, 4], cons[:, 8], cons[:, 16] = 6.0, 1e-5, 400
+    order = np.concatenate([np.arange(0, nb - 1, 2), np.arange(1, nb - 1, 2), np.arange(nb - 1, nc)])
+    cons = cons[order]
+    L = _native.lib()
+    alone = []
+    for n, c in ((nb, cons), (2, _chains(2, 2))):
+        h = _world(n, len(c))
+        _upload(h, _bodies(n, 5), c)
+        _step(h, 3)
+        alone.append(_download(h, n, len(c)))
+        L.kr_destroy(h)
+    a, b = _world(nb, nc), _world(2, 4)
+    try:
+        _upload(a, _bodies(nb, 5), cons)
+        _upload(b, _bodies(2, 5), _chains(2, 2))
+        _step(a, 3)
+        _step(b, 3)
+        for got, want in ((_download(a, nb, nc), alone[0]), (_download(b, 2, 4), alone[1])):
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    finally:
+        for h in (a, b):
+            L.kr_destroy(h)
