@@ -236,7 +236,10 @@ int kr_probe_wrap(const double *d, int32_t n, double *out);
 /* Launch shape: lanes per creature (32, 16 or 8: a warp carries 32 / lanes
  * creatures), warps per CTA (1..16, at most 64 creatures per CTA) and CTAs
  * per SM (0 = 16 / warps).  A CTA gets an equal share of the SM's shared
- * memory; a group of one body template holds as many creatures as fit in it.
+ * memory -- a larger one, with fewer CTAs per SM, where the creatures need
+ * it; a group of one body template holds as many creatures as fit in it.  A
+ * shape whose share is below a creature's and its template's fields at a word
+ * each is refused when it runs (KR_ERR_CAPACITY).
  * Until this is called the engine picks the shape per launch, CTAs of 4
  * warps: 32 lanes below 8 live creatures per SM (16 in a rollout server), 16
  * lanes below 96, else 8.

@@ -1101,30 +1101,64 @@ int upload_templates(kr_batch *b) {
   return KR_OK;
 }
 
+// The launch shapes that the interface takes: those in whose share of an SM's
+// shared memory one creature of every body shape fits at a word per field of
+// its bodies, constraints and collision points, beside its template.  The
+// records of the kernel are padded to the lanes of a creature, and the sine
+// table comes on top, so a shape within these limits can need more than its
+// share; plan_shape then takes fewer CTAs per SM.
+long limit_words(const TplDev &d) {
+  const int motors = d.arms * d.segs;
+  return 16 * r4(d.nb) + 13 * r4(d.nc) + 7 * r4(d.np) + r4(motors) + r4(motors + d.arms) + 4 * d.arms + 196;
+}
+
+// words of dynamic shared memory in a CTA's share when `ctas` run on an SM
+long share_words(const kr_batch *b, int ctas, long static_bytes) {
+  const long bytes = std::min<long>(b->smem_optin, (long)b->smem_per_sm / ctas - b->smem_reserved) - static_bytes;
+  return bytes / 16 * 4;
+}
+
 // Launch shape: creatures per group of every template and the dynamic shared
 // memory of a CTA.  A CTA gets an equal share of the SM's shared memory for
-// ctas_per_sm CTAs (default: 16 warps per SM); a template's group holds as
-// many creatures as fit in that share, at most W * 32 / G.
+// ctas_per_sm CTAs (default: 16 warps per SM), or for as many fewer as lets
+// an SM hold the most creatures of the template that fits worst (32 lanes, 1
+// warp, 6 x 7 bodies: 11 CTAs instead of 16, where none fits); a template's
+// group holds as many creatures as fit in that share, at most W * 32 / G.
 int plan_shape(kr_batch *b) {
   b->cpc = b->W * (32 / b->G);
-  const int ctas = b->ctas_per_sm > 0 ? b->ctas_per_sm : std::max(1, 16 / b->W);
-  long budget = std::min<long>(b->smem_optin, (long)b->smem_per_sm / ctas - b->smem_reserved) - kStaticSmem;
-  budget = (budget / 16) * 16;
-  const long words = budget / 4;
+  const int asked = b->ctas_per_sm > 0 ? b->ctas_per_sm : std::max(1, 16 / b->W);
+  const int v = kr::schedule_index(b->G);
+  for (const TplDev &d : b->h_tpl)
+    if (share_words(b, asked, 64) < limit_words(d))
+      return b->fail(KR_ERR_CAPACITY, "body " + std::to_string(d.arms) + "x" + std::to_string(d.segs) +
+                                          " does not fit the shared memory of " + std::to_string(asked) +
+                                          " CTAs per SM");
+  auto fits = [&](const TplDev &d, int ctas) {
+    const long room = share_words(b, ctas, kStaticSmem) - tpl_smem_words(d.npass[v], b->G, d.nb, d.np);
+    return (int)std::min<long>(b->cpc, std::max<long>(0, room) / creature_smem_words(d.nb, d.arms, d.segs));
+  };
+  b->ctas = asked;
+  int most = -1;
+  for (int ctas = asked; ctas >= 1; ctas--) {
+    int least = b->cpc;
+    for (const TplDev &d : b->h_tpl) least = std::min(least, fits(d, ctas));
+    if (ctas * least > most) {
+      most = ctas * least;
+      b->ctas = ctas;
+    }
+    if (least == b->cpc) break;
+  }
   b->tpl_cpg.assign(b->h_tpl.size(), 0);
   size_t need_max = 16;
   for (size_t t = 0; t < b->h_tpl.size(); t++) {
     const TplDev &d = b->h_tpl[t];
-    const long tw = tpl_smem_words(d.npass[kr::schedule_index(b->G)], b->G, d.nb, d.np);
-    const long cw = creature_smem_words(d.nb, d.arms, d.segs);
-    const long fit = (words - tw) / cw;
-    if (fit < 1)
+    const int cpg = fits(d, b->ctas);
+    if (cpg < 1)
       return b->fail(KR_ERR_CAPACITY, "body " + std::to_string(d.arms) + "x" + std::to_string(d.segs) +
-                                          " does not fit the shared memory of " + std::to_string(ctas) +
-                                          " CTAs per SM");
-    const int cpg = (int)std::min<long>(b->cpc, fit);
+                                          " does not fit the shared memory of a CTA");
     b->tpl_cpg[t] = cpg;
-    need_max = std::max(need_max, (size_t)(tw + (long)cpg * cw) * sizeof(float));
+    need_max = std::max(need_max, (size_t)(tpl_smem_words(d.npass[v], b->G, d.nb, d.np) +
+                                           (long)cpg * creature_smem_words(d.nb, d.arms, d.segs)) * sizeof(float));
   }
   b->smem_dyn = need_max;
   b->shape_dirty = false;
@@ -1198,8 +1232,7 @@ int build_groups(kr_batch *b, Part &p, int max_steps) {
   // wave of the resident CTAs, smaller groups (whole warps) spread them over
   // every SM instead of packing a few SMs.
   const int cpw = 32 / b->G;
-  const int ctas = b->ctas_per_sm > 0 ? b->ctas_per_sm : std::max(1, 16 / b->W);
-  const long slots = (long)b->n_sm * ctas;
+  const long slots = (long)b->n_sm * b->ctas;
   std::vector<int> n_t(b->h_tpl.size(), 0), size_t_(b->h_tpl.size(), 0);
   for (int i = 0; i < n_live; i++) n_t[p.g_tpl[i]]++;
   long full_groups = 0;

@@ -315,6 +315,7 @@ struct kr_batch {
   bool served = false;          // a rollout server's engine
   int cpc = 16;                 // creature entries per group: W * 32 / G
   std::vector<int> tpl_cpg;     // creatures per group of each template
+  int ctas = 1;                 // CTAs per SM that share an SM's shared memory (plan_shape)
   size_t smem_dyn = 0;          // dynamic shared memory per CTA
   bool shape_dirty = true;
   // policy: pw_stride floats per individual (device layout), individual of

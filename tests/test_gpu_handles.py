@@ -153,3 +153,37 @@ def test_handles_of_unlike_islands_step_side_by_side(nb, nc):
     finally:
         for h in (a, b):
             L.kr_destroy(h)
+
+
+# the launch shapes in whose share of an SM's shared memory a creature fits at a
+# word per field: by body, lanes, warps and CTAs per SM (0: 16 / warps), taken or not
+SHAPES = [(6, 7, 32, 1, 0, True), (6, 7, 32, 1, 16, True), (6, 7, 32, 1, 17, True), (6, 7, 32, 1, 19, False),
+          (6, 7, 16, 1, 16, True), (4, 5, 32, 1, 16, True), (8, 9, 32, 2, 0, True), (8, 9, 32, 1, 0, False),
+          (8, 9, 8, 16, 1, True), (1, 1, 32, 1, 32, True), (2, 2, 8, 2, 32, True)]
+
+
+@pytest.mark.parametrize("arms,segs,lanes,warps,ctas,taken", SHAPES)
+def test_launch_shapes_taken_and_refused(arms, segs, lanes, warps, ctas, taken):
+    """What kr_batch_set_launch takes runs, with the automatic shape's results,
+    also where the kernel's records need more than the shape's share of the
+    shared memory; what is too large for it is refused when it runs."""
+    n = 70
+    r = np.random.default_rng(3)
+    args = (np.full(n, arms), np.full(n, segs), np.zeros(n, int), r.uniform(300, 1000, n), r.uniform(300, 500, n),
+            r.uniform(0, 6, n), r.integers(5, 20, n))
+    out = []
+    for shape in (None, (warps, ctas, lanes)):
+        eng = batch.BatchEngine([ob.make_map_rects(seed=3)], n)
+        eng.spawn(0, *args)
+        if shape:
+            eng.set_launch(shape[0], shape[1], lanes_per_creature=shape[2])
+        if shape and not taken:
+            with pytest.raises(_native.KrError) as e:
+                eng.run(20)
+            assert e.value.code == _native.KR_ERR_CAPACITY
+        else:
+            eng.run(20)
+            out.append(eng.read_state())
+        eng.close()
+    if taken:
+        assert all(np.array_equal(out[0][f], out[1][f]) for f in out[0])
