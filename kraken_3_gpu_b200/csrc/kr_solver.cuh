@@ -162,9 +162,10 @@ static __device__ __noinline__ float2 sincos_f64(float a) {
 // h + (l - err) and h + (l + err) round to one f32, that is the rounding of
 // the exact value and of the f64 value above, whose own error err includes.
 // Returns the distance of the two roundings, 0 where the values stand; where
-// it is not (about one value in 3,000) and for |a| > kSinCosNearMax
-// sincos_f64 decides.  The f64 chain cost 241 cycles, mostly conversions
-// (18 cycles each) and the serial reduction and series.
+// it is not (one value in 2,400 to 4,700 of an octave from 2^-7 up, one in
+// 1,300 between 2^-8 and 2^-7, fewer and fewer below, none below 2^-13) and
+// for |a| > kSinCosNearMax sincos_f64 decides.  The f64 chain cost 241 cycles,
+// mostly conversions (18 cycles each) and the serial reduction and series.
 //
 // a = k pi/256 + r1 + rl: p1 = pi/256 to 24 bits, so r1 = a - k p1 is exact
 // (a multiple of 2^-31 below 2^-7.3, or a itself for k = 0), and rl = -k p2
@@ -176,10 +177,15 @@ static __device__ __noinline__ float2 sincos_f64(float a) {
 // because |S| is 0 or above |C r1|).  Error: r^2 (|m| <= r^2 / 2) times
 // below 12 units of 2^-24 for the roundings of r, r^2, m and the two sums
 // it enters, Sl m among them, times |S| (cos: |C|); |k| 2^-53 for the
-// roundings of rl, n, its sum and p2 (2^-55.4 |k| each); below 2^-43 for
-// r^5 / 120 (2^-43.7), the other roundings and the f64 value (2^-51).  All
-// 1.8e8 arguments of each sign from 2^-20 to 64: no value accepted that
-// differs from sincos_f64's.
+// roundings of rl, n, its sum and p2 (2^-55.4 |k| each); r^2 2^-28.9 for r^5 /
+// 120 (|r| <= pi / 512).  Every term vanishes with a, so an angle of 0, as
+// fixed bodies have it, and small ones are decided like any other (a bound of
+// 2^-43 in the place of the last term left all below 2^-18 to sincos_f64: 256
+// chains on fixed bodies at angle 0, 100 steps, 9.8 ms, now 4.0).  What is
+// left, below 2^-47 (the other roundings, the f64 value), has no term: that
+// the bound holds is checked, not proven, over all 2,231,369,730 arguments
+// from -64 to 64 -- no accepted value differs from sincos_f64's
+// (tests/test_solver_host.py repeats it).
 //
 // tab: kSinNear in shared memory.  As 16-byte __ldg gathers its look-ups were
 // the longest part of a pin (32 lanes, 32 lines: two of them 360 of 550
@@ -194,7 +200,7 @@ __device__ __forceinline__ float sincos_near(const float2 *tab, float a, float *
   const float r = fadd(r1, rl), rr = fmul(r, r);
   const float n = fmaf(fmul(r, rr), -1.f / 6, rl);
   const float m = fmul(rr, fmaf(rr, 1.f / 24, -0.5f));
-  const float w = fmul(rr, 0x1.8p-22f), e0 = fmaf(fabsf(k), 0x1p-53f, 0x1p-43f);
+  const float w = fmul(rr, 0x1.8p-22f), e0 = fmaf(fabsf(k), 0x1p-53f, fmul(rr, 0x1.1p-29f));
   const float es = fmaf(fabsf(T.x), w, e0), ec = fmaf(fabsf(T.z), w, e0);
   const float qs = fmul(T.z, r1), hs = fadd(T.x, qs);
   const float ls = fadd(fmaf(T.x, m, fmaf(T.z, n, fmaf(T.w, r1, T.y))),

@@ -11,6 +11,7 @@ CSRC = os.path.join(os.path.dirname(HERE), "kraken_3_gpu_b200", "csrc")
 
 COMMON = r'''
 #include <cstdio>
+#include <cstdlib>
 #include <random>
 #include <vector>
 #include "cuda_on_host.h"
@@ -25,7 +26,7 @@ def _run(tmp_path, body, *args):
     src = tmp_path / "t.cpp"
     src.write_text(COMMON + body)
     exe = tmp_path / "t"
-    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-mfma", "-w", "-I", HERE, "-I", CSRC, "-o",
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-mfma", "-w", "-pthread", "-I", HERE, "-I", CSRC, "-o",
                     str(exe), str(src)], check=True)
     out = subprocess.run([str(exe), *args], capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stdout + out.stderr
@@ -109,3 +110,58 @@ int main() {
 
 def test_speed_clamp_equals_the_plain_form(tmp_path):
     assert _run(tmp_path, CLAMP).startswith("ok")
+
+
+SINCOS = r'''
+#include <thread>
+// sincos_near against sincos_f64: no accepted value may differ, and how many
+// it leaves to sincos_f64 per octave of the argument.  argv[1]: every step-th
+// argument of an octave (1: all of them)
+struct Count { long n = 0, refused = 0, wrong = 0; };
+static Count octave(int e, unsigned step) {  // exponent field e of the argument, both signs
+  Count c;
+  const unsigned first = e < 0 ? 0 : (unsigned)e << 23, last = first + (1u << 23);
+  for (unsigned u = first; u < last; u += step)
+    for (int sign = 0; sign < 2; sign++) {
+      const float a = bits(u | (unsigned)sign << 31);
+      if (std::fabs(a) > kSinCosNearMax) continue;
+      float s, co;
+      c.n++;
+      if (sincos_near(g_tab, a, &s, &co) != 0.f) { c.refused++; continue; }
+      const float2 f = sincos_f64(a);
+      if (std::memcmp(&s, &f.x, 4) || std::memcmp(&co, &f.y, 4)) {
+        if (!c.wrong++) std::printf("FAIL sin/cos of %a: %a %a for %a %a\n", a, s, co, f.x, f.y);
+      }
+    }
+  return c;
+}
+int main(int argc, char **argv) {
+  stage_sin(g_tab);
+  const unsigned step = (unsigned)std::max(1, std::atoi(argv[1]));
+  std::vector<Count> per(134);  // exponent fields 0 (zero and subnormal) .. 133 (64)
+  std::vector<std::thread> th;
+  const int nt = (int)std::thread::hardware_concurrency();
+  for (int t = 0; t < nt; t++)
+    th.emplace_back([&, t] { for (int e = t; e < 134; e += nt) per[e] = octave(e, step); });
+  for (auto &t : th) t.join();
+  long n = 0, refused = 0, wrong = 0;
+  for (int e = 0; e < 134; e++) {
+    n += per[e].n; refused += per[e].refused; wrong += per[e].wrong;
+    if (argc > 2 && per[e].n) std::printf("2^%d: %ld of %ld\n", e - 127, per[e].refused, per[e].n);
+    // at most one in 500 of an octave
+    if (per[e].refused > per[e].n / 500 + 1) { std::printf("FAIL 2^%d: %ld of %ld refused\n", e - 127, per[e].refused, per[e].n); wrong++; }
+  }
+  float s, c;
+  for (float a : {0.f, -0.f})
+    if (sincos_near(g_tab, a, &s, &c) != 0.f || s != 0.f || c != 1.f) { std::printf("FAIL %g\n", a); wrong++; }
+  std::printf(wrong ? "FAIL\n" : "ok %ld arguments, %ld refused\n", n, refused);
+  return wrong != 0;
+}
+'''
+
+
+def test_sines_near_zero_take_the_short_form(tmp_path):
+    """0, the angle of most hand-made bodies, and small angles are decided by
+    the f32 sine as others are; every 1,009th argument of each octave up to
+    64 (KRAKEN_SINCOS_STEP=1: every argument, 20 s of 8 cores)."""
+    assert _run(tmp_path, SINCOS, os.environ.get("KRAKEN_SINCOS_STEP", "1009")).startswith("ok")
