@@ -989,9 +989,19 @@ __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const f
     if (first >= 0 && L.lane == 0) collide_points(S, N, rects, nR, j, q, sa, ca, first);
   }
 }
+// (the members it needs one by one: a struct of the size of Island would pass
+// through local memory)
 template <int G>
-__device__ __noinline__ void collide_listed_call(Island S, Near N, const float4 *__restrict__ rects, int nR, Lanes<G> L) {
-  collide_listed<G>(S, N, rects, nR, L);
+__device__ __noinline__ void collide_listed_call(const float4 *P, float4 *Q, const float4 *body, const float4 *pts,
+                                                 const float2 *tab, unsigned short *cull, unsigned char *list, int nb,
+                                                 unsigned near, const float4 *__restrict__ rects, int nR,
+                                                 int warp_lane) {
+  Island S{};
+  S.P = const_cast<float4 *>(P); S.Q = Q; S.body = body; S.pts = pts; S.tab = tab;
+  S.cull = cull; S.list = list; S.nb = nb;
+  Near N;
+  N.w = near;
+  collide_listed<G>(S, N, rects, nR, Lanes<G>(warp_lane));
 }
 
 // One collision pass of the island.  OutOfLine: the listed bodies (most passes
@@ -1013,7 +1023,8 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
   }
   if (stale) N.w = near_rebuild<G>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
   if (OutOfLine) {
-    if (N.w & 0xffffu) collide_listed_call<G>(S, N, rects, nR, L);
+    if (N.w & 0xffffu) collide_listed_call<G>(S.P, S.Q, S.body, S.pts, S.tab, S.cull, S.list, S.nb, N.w, rects, nR,
+                                                L.base + L.lane);
   } else {
     collide_listed<G>(S, N, rects, nR, L);
   }
