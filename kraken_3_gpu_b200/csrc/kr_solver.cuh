@@ -811,6 +811,9 @@ struct Near {
   __device__ __forceinline__ bool full() const { return (w >> 25) & 1; }
 };
 constexpr int kFewPoints = 2;
+// mask of a body that meets no rect (immovable or without points; no other
+// mask has rect bits without kNearBit): it needs no reference
+constexpr unsigned kExempt = 1u;
 
 // A reference position in one word: x and y rounded to integers + 2^15
 __device__ __forceinline__ unsigned near_pack(float x, float y) {
@@ -832,19 +835,20 @@ __device__ __forceinline__ bool in_box(const float4 r, float x0, float x1, float
 
 // New references, near list, masks and body lists from the bodies' predicted
 // positions.  near_d = D + kCullPad.  Out of line: it runs once per several
-// dozen passes.
-template <int G>
+// dozen passes.  World: bodies that meet no rect may be among them (the batched
+// engine's templates have none).
+template <int G, bool World>
 __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4 *body, unsigned short *cull,
                                           unsigned char *list, int nb, const float4 *__restrict__ rects, int nR,
                                           float near_d, Lanes<G> L) {
   int few_n = 0, many_n = 0, n = 0;
   float lx = kInf, ly = kInf, hx = -kInf, hy = -kInf;
   bool bad = nR > 65535;
+  auto exempt = [&](int j) { return World && (body[j].x == 0.f || (__float_as_int(body[j].w) >> 16) == 0); };
   for (int j = L.lane; j < nb; j += G) {
-    const float4 bd = body[j];
-    if (bd.x == 0.f || (__float_as_int(bd.w) >> 16) == 0) continue;
+    if (exempt(j)) continue;
     const float4 q = Q[j];
-    const float e = bd.z + near_d + kFarMove + kCullPad;
+    const float e = body[j].z + near_d + kFarMove + kCullPad;
     if (!(fabsf(q.x) < 32000.f && fabsf(q.y) < 32000.f && e < 1e6f)) { bad = true; continue; }
     lx = fminf(lx, q.x - e); hx = fmaxf(hx, q.x + e);
     ly = fminf(ly, q.y - e); hy = fmaxf(hy, q.y + e);
@@ -879,7 +883,9 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
       const float4 bd = body[j];
       const int cnt = __float_as_int(bd.w) >> 16;
       unsigned mask = 0u;
-      if (bd.x != 0.f && cnt != 0) {
+      if (exempt(j)) {
+        Q[j].w = __uint_as_float(kExempt);
+      } else {
         const float4 q = Q[j];
         if (full) {
           mask = 1u;
@@ -898,9 +904,6 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
           P[j].w = __uint_as_float(w);
         }
         Q[j].w = __uint_as_float(mask);
-      } else if (!full) {
-        // a body without points meets no rect: the reference only has to hold
-        P[j].w = __uint_as_float(near_pack(fminf(fmaxf(Q[j].x, -32000.f), 32000.f), fminf(fmaxf(Q[j].y, -32000.f), 32000.f)));
       }
       few = (mask & ~kNearBit) != 0u && cnt <= kFewPoints;
       many = (mask & ~kNearBit) != 0u && cnt > kFewPoints;
@@ -1008,7 +1011,7 @@ __device__ __noinline__ void collide_listed_call(const float4 *P, float4 *Q, con
 // have none) as a call -- for the kernel with the net, whose step is larger
 // than the instruction caches: 8,000 creatures under the net 35 -> 32 ms; the
 // others are 3 % faster with it in line.
-template <int G, bool OutOfLine>
+template <int G, bool World, bool OutOfLine>
 __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 *__restrict__ rects, int nR,
                                                float near_d, const Lanes<G> &L) {
   bool stale = !N.valid();
@@ -1017,11 +1020,12 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
 #pragma unroll 1
     for (int j = L.lane; j < S.nb; j += G) {
       const float4 q = S.Q[j];
+      if (World && __float_as_uint(q.w) == kExempt) continue;
       moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, __float_as_uint(q.w));
     }
     stale = L.ballot(moved) != 0;
   }
-  if (stale) N.w = near_rebuild<G>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
+  if (stale) N.w = near_rebuild<G, World>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
   if (OutOfLine) {
     if (N.w & 0xffffu) collide_listed_call<G>(S.P, S.Q, S.body, S.pts, S.tab, S.cull, S.list, S.nb, N.w, rects, nR,
                                                 L.base + L.lane);
@@ -1084,7 +1088,7 @@ __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
     for (int it = 0; it < K.iterations; it++) {
       if constexpr (World) solve_world<G>(S, it == 0, L);
       else solve_engine<G>(K, S, it == 0, L);
-      collide_island<G, OutOfLine>(S, N, rects, nR, near_d, L);
+      collide_island<G, World, OutOfLine>(S, N, rects, nR, near_d, L);
     }
 #pragma unroll 1
     for (int i = L.lane; i < S.nb; i += G) finalize_body<World>(K, S, i);

@@ -165,3 +165,106 @@ def test_sines_near_zero_take_the_short_form(tmp_path):
     the f32 sine as others are; every 1,009th argument of each octave up to
     64 (KRAKEN_SINCOS_STEP=1: every argument, 20 s of 8 cores)."""
     assert _run(tmp_path, SINCOS, os.environ.get("KRAKEN_SINCOS_STEP", "1009")).startswith("ok")
+
+
+NEAR = r'''
+// Collision passes of a group of bodies that drift, are thrown about and are
+// pulled back into walls, against the fold over every rect; and the rects that
+// the passes read.  argv: offset of the whole scene, rects, far anchors (an
+// immovable body and one without points, this far away; 0: at the scene),
+// pull (px a body is put back into the nearest wall in every pass), spread,
+// more rects, all far away
+struct Scene {
+  std::vector<float4> rects, P, Q, body, pts;
+  std::vector<unsigned short> cull = std::vector<unsigned short>(64);
+  std::vector<unsigned char> list;
+  Island S{};
+};
+int main(int, char **argv) {
+  stage_sin(g_tab);
+  const float off = std::atof(argv[1]), anchors = std::atof(argv[3]), pull = std::atof(argv[4]), spread = std::atof(argv[5]);
+  const int nr = std::atoi(argv[2]);
+  std::mt19937 r(11);
+  auto u = [&](float a, float b) { return a + (b - a) * (r() >> 8) / 16777216.f; };
+  Scene s;
+  auto rect = [&](float x, float y, float w, float h) { s.rects.push_back(make_float4(off + x, off + y, off + x + w, off + y + h)); };
+  rect(0, 0, 1400, 14); rect(0, 786, 1400, 14); rect(0, 0, 14, 800); rect(1386, 0, 14, 800);
+  for (int i = 4; i < nr; i++) rect(u(20, 1360), u(20, 760), u(3, 8), u(3, 8));
+  for (int i = 0; i < std::atoi(argv[6]); i++) rect(5000 + 10 * i, 5000, 5, 5);
+  const int nb = 24;
+  s.P.resize(nb); s.Q.resize(nb); s.body.resize(nb); s.list.resize(nb);
+  for (int j = 0; j < nb; j++) {
+    const bool fixed = j == 3, bare = j == 4;
+    const int n = bare ? 0 : j == 0 ? 8 : 1 + j % 2;
+    const float far = fixed || bare ? anchors : 0.f;
+    s.Q[j] = make_float4(off + far + 640 + spread * u(-1, 1), off + far + 400 + spread * u(-1, 1), u(-3, 3), 0.f);
+    const int at = (int)s.pts.size();
+    float reach = 0.f;
+    for (int k = 0; k < n; k++) {
+      s.pts.push_back(make_float4(u(-9, 9), u(-9, 9), u(2, 9), 0.f));
+      reach = std::max(reach, length2(s.pts.back().x, s.pts.back().y) + 1.f);
+    }
+    s.body[j] = make_float4(fixed ? 0.f : 0.2f, 0.01f, reach, __int_as_float(at | n << 16));
+  }
+  Island &S = s.S;
+  S.P = s.P.data(); S.Q = s.Q.data(); S.body = s.body.data(); S.pts = s.pts.data(); S.tab = g_tab;
+  S.cull = s.cull.data(); S.list = s.list.data(); S.nb = nb;
+  const int nR = (int)s.rects.size();
+  const float near_d = 9.f + 2.f + kCullPad;
+  const Lanes<1> L(0);
+  Near N;
+  long hits = 0, wrong = 0, loads = 0;
+  const int kSteps = 400, kPasses = 8;
+  for (int step = 0; step < kSteps; step++) {
+    for (int pass = 0; pass < kPasses; pass++) {
+      for (int j = 0; j < nb; j++) {
+        float4 &q = s.Q[j];
+        if (s.body[j].x == 0.f) continue;
+        q.x += u(-0.8f, 0.8f); q.y += u(-0.8f, 0.8f); q.z += u(-0.1f, 0.1f);
+        if (pull != 0.f && j % 5 == 0) { q.x = off + 700.f + 3.f * j; q.y = off + 14.f - pull; }
+      }
+      std::vector<float4> want = s.Q;
+      for (int j = 0; j < nb; j++) {
+        if (s.body[j].x == 0.f) continue;
+        float sa, ca;
+        sincos_r(g_tab, want[j].z, &sa, &ca);
+        const int pr = __float_as_int(s.body[j].w);
+        for (int k = 0; k < pr >> 16; k++) {
+          const float4 pt = s.pts[(pr & 0xffff) + k];
+          SdfFold f;
+          const float x = fadd(want[j].x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
+          const float y = fadd(want[j].y, fadd(fmul(pt.x, sa), fmul(pt.y, ca)));
+          for (const float4 &c : s.rects) f.add(c, x, y);
+          float dx, dy;
+          if (f.push(pt.z, &dx, &dy)) { want[j].x = fadd(want[j].x, dx); want[j].y = fadd(want[j].y, dy); hits++; }
+        }
+      }
+      const long before = g_rect_loads;
+      collide_island<1, true, false>(S, N, s.rects.data(), nR, near_d, L);
+      loads += g_rect_loads - before;
+      for (int j = 0; j < nb; j++)
+        if (std::memcmp(&s.Q[j], &want[j], 12)) {
+          if (!wrong++) std::printf("FAIL step %d pass %d body %d: %a %a for %a %a\n", step, pass, j, s.Q[j].x, s.Q[j].y, want[j].x, want[j].y);
+        }
+    }
+    if (step % 50 == 49)  // thrown across the scene
+      for (int j = 0; j < nb; j++)
+        if (s.body[j].x != 0.f) { s.Q[j].x = off + 640 + spread * u(-1, 1); s.Q[j].y = off + 400 + spread * u(-1, 1); }
+  }
+  std::printf(wrong ? "FAIL %ld wrong\n" : "ok %.1f rects a pass, %ld hits\n", wrong ? (double)wrong : (double)loads / (kSteps * kPasses), hits);
+  return wrong != 0;
+}
+'''
+
+
+def _loads(tmp_path, offset=0, rects=300, anchors=0, pull=0, spread=110, more=0):
+    out = _run(tmp_path, NEAR, *map(str, (offset, rects, anchors, pull, spread, more)))
+    assert out.startswith("ok"), out
+    words = out.split()
+    assert int(words[-2]) > 0
+    return float(words[1])
+
+
+def test_bodies_that_meet_no_rect_cost_no_rebuild(tmp_path):
+    """An immovable body and one without points, out of any reference's range."""
+    assert _loads(tmp_path, anchors=50000) <= 1.02 * _loads(tmp_path)
