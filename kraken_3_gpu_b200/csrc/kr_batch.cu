@@ -104,7 +104,7 @@ __host__ __device__ inline int tpl_smem_words(int npass, int G, int nb, int np) 
 __host__ __device__ inline int mot_words(int arms, int segs) { return r4(2 * (kr::grip_pair0(arms, segs) + arms + 1)); }
 __host__ __device__ inline int creature_smem_words(int nb, int arms, int segs) {
   return 4 * nb + 4 * (nb + arms + 1) + mot_words(arms, segs) + r4(arms) + r4(arms * segs + arms) +
-         r4((kr::kMaxCulled + 1) / 2) + r4((nb + 3) / 4);
+         kr::kCullWords + r4((nb + 3) / 4);
 }
 
 struct TplSmem {
@@ -138,7 +138,7 @@ __device__ inline void carve_creature(kr::Island &S, CreatureSmem &X, const TplS
   S.brk = p; p += r4(td.arms);
   S.grip0 = kr::grip_pair0(td.arms, td.segs);
   X.ctrl = p; p += r4(AS + td.arms);
-  S.cull = reinterpret_cast<unsigned short *>(p); p += r4((kr::kMaxCulled + 1) / 2);
+  S.cull = reinterpret_cast<unsigned short *>(p); p += kr::kCullWords;
   S.list = reinterpret_cast<unsigned char *>(p);
   // statics shared by the CTA
   S.recs = P.recs; S.body = P.body; S.pts = P.pts;

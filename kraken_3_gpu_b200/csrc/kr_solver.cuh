@@ -377,6 +377,8 @@ struct SdfFold {
 // touched a wall: 16,384 mixed creatures 308 -> 289 ms, 1,024 creatures x 400
 // steps 31.8 -> 29.0 ms.
 constexpr int kMaxCulled = 62;      // near list entries; bit b of a mask covers entries b << shift ...
+constexpr int kCullWords = 32;      // the near list, two entries a word, and the references' origin behind it
+static_assert(2 * kCullWords >= kMaxCulled + 2, "");
 constexpr unsigned kNearBit = 1u << 31;  // of a mask: the body holds within kNearMove only
 constexpr float kNearMove = 8.f, kFarMove = 32.f;
 constexpr float kCullPad = 1.f;     // rounding of the box tests
@@ -432,7 +434,7 @@ struct Island {
   const float2 *tab;   // kSinNear in shared memory
   const float4 *body;  // inverse mass, inverse inertia, reach, point offset | count << 16
   const float4 *pts;   // collision points: x, y, radius, body; grouped per body in groupCollPoints order
-  unsigned short *cull;       // near list (kMaxCulled rect indices)
+  unsigned short *cull;       // near list (kMaxCulled rect indices), origin
   unsigned char *list;        // bodies with near rects: one or two points from the front, more from the back
   int nb;
   // drop-in world: one dynamic record of 5 float4 per unit, pass offsets
@@ -800,7 +802,8 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
 // (a struct returned by the out-of-line rebuild would live in local memory):
 // listed bodies with at most kFewPoints points, listed bodies with more, near
 // list entries, entries per mask bit (log2), valid (every body has a
-// reference), full (no usable list: every body against every rect).
+// reference), full (no usable list: every body against every rect), shifted
+// (the references have an origin).
 struct Near {
   unsigned w = 0;
   __device__ __forceinline__ int few() const { return w & 0xff; }
@@ -809,19 +812,34 @@ struct Near {
   __device__ __forceinline__ int shift() const { return (w >> 23) & 1; }
   __device__ __forceinline__ bool valid() const { return (w >> 24) & 1; }
   __device__ __forceinline__ bool full() const { return (w >> 25) & 1; }
+  __device__ __forceinline__ bool shifted() const { return (w >> 27) & 1; }
 };
 constexpr int kFewPoints = 2;
+constexpr float kRefRange = 32000.f;   // of a reference's coordinates about the origin
+constexpr float kOriginStep = 16384.f;
 // mask of a body that meets no rect (immovable or without points; no other
 // mask has rect bits without kNearBit): it needs no reference
 constexpr unsigned kExempt = 1u;
 
-// A reference position in one word: x and y rounded to integers + 2^15
-__device__ __forceinline__ unsigned near_pack(float x, float y) {
-  return (unsigned)(__float2int_rn(x) + 32768) | ((unsigned)(__float2int_rn(y) + 32768) << 16);
+// A reference position in one word: x and y rounded to integers + 2^15, less
+// the origin, which is ox, oy times kOriginStep: 0 while every body is within
+// kRefRange, else kept behind the near list.
+__device__ __forceinline__ unsigned near_pack(float x, float y, int ox, int oy) {
+  return (unsigned)(__float2int_rn(x) + 32768 - ox * (int)kOriginStep) |
+         ((unsigned)(__float2int_rn(y) + 32768 - oy * (int)kOriginStep) << 16);
 }
-__device__ __forceinline__ float2 near_unpack(unsigned w) {
-  return make_float2(__uint_as_float(0x4b000000u | (w & 0xffffu)) - 8421376.f,
-                     __uint_as_float(0x4b000000u | (w >> 16)) - 8421376.f);
+// bias: near_bias of the origin (every sum is an integer below 2^24, so exact)
+__device__ __forceinline__ float2 near_unpack(unsigned w, const float2 bias) {
+  return make_float2(__uint_as_float(0x4b000000u | (w & 0xffffu)) - bias.x,
+                     __uint_as_float(0x4b000000u | (w >> 16)) - bias.y);
+}
+__device__ __forceinline__ float2 near_bias(int ox, int oy) {
+  return make_float2(8421376.f - kOriginStep * (float)ox, 8421376.f - kOriginStep * (float)oy);
+}
+__device__ __forceinline__ float2 near_bias(const unsigned short *cull, const Near &N) {
+  float2 bias = make_float2(8421376.f, 8421376.f);
+  if (N.shifted()) bias = near_bias((short)cull[kMaxCulled], (short)cull[kMaxCulled + 1]);
+  return bias;
 }
 __device__ __forceinline__ bool near_holds(const float2 ref, float x, float y, unsigned mask) {
   const float r = (mask & kNearBit) ? kNearMove : kFarMove;
@@ -843,19 +861,34 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
                                           float near_d, Lanes<G> L) {
   int few_n = 0, many_n = 0, n = 0;
   float lx = kInf, ly = kInf, hx = -kInf, hy = -kInf;
-  bool bad = nR > 65535;
+  bool bad = nR > 65535, out = false;
   auto exempt = [&](int j) { return World && (body[j].x == 0.f || (__float_as_int(body[j].w) >> 16) == 0); };
   for (int j = L.lane; j < nb; j += G) {
     if (exempt(j)) continue;
     const float4 q = Q[j];
     const float e = body[j].z + near_d + kFarMove + kCullPad;
-    if (!(fabsf(q.x) < 32000.f && fabsf(q.y) < 32000.f && e < 1e6f)) { bad = true; continue; }
+    if (!(fabsf(q.x) < 1e6f && fabsf(q.y) < 1e6f && e < 1e6f)) { bad = true; continue; }
+    out |= !(fabsf(q.x) < kRefRange && fabsf(q.y) < kRefRange);
     lx = fminf(lx, q.x - e); hx = fmaxf(hx, q.x + e);
     ly = fminf(ly, q.y - e); hy = fmaxf(hy, q.y + e);
   }
   lx = L.min(lx); ly = L.min(ly);
   hx = L.max(hx); hy = L.max(hy);
   bool full = L.ballot(bad) != 0;
+  const bool shifted = L.ballot(out) != 0 && !full;
+  int ox = 0, oy = 0;
+  if (shifted) {
+    ox = __float2int_rn((lx + hx) * (0.5f / kOriginStep));
+    oy = __float2int_rn((ly + hy) * (0.5f / kOriginStep));
+    for (int j = L.lane; j < nb; j += G)
+      bad |= !exempt(j) && !(fabsf(Q[j].x - kOriginStep * ox) < kRefRange && fabsf(Q[j].y - kOriginStep * oy) < kRefRange);
+    full = L.ballot(bad) != 0;  // farther apart than references reach
+    if (L.lane == 0) {
+      cull[kMaxCulled] = (unsigned short)ox;
+      cull[kMaxCulled + 1] = (unsigned short)oy;
+    }
+  }
+  const float2 bias = near_bias(ox, oy);
   // the near list, with the wide move if it fits
   float move = kFarMove;
   for (int base = 0; base < nR && !full; base += G) {
@@ -890,8 +923,8 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
         if (full) {
           mask = 1u;
         } else {
-          const unsigned w = near_pack(q.x, q.y);
-          const float2 ref = near_unpack(w);
+          const unsigned w = near_pack(q.x, q.y, ox, oy);
+          const float2 ref = near_unpack(w, bias);
           const float e = bd.z + near_d, en = e + kNearMove, ef = e + kFarMove;
           bool wide = move == kNearMove;
 #pragma unroll 4
@@ -916,7 +949,8 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
   }
   L.sync();
   return full ? (unsigned)few_n | ((unsigned)many_n << 8) | (1u << 25)
-              : (unsigned)few_n | ((unsigned)many_n << 8) | ((unsigned)n << 16) | ((unsigned)shift << 23) | (1u << 24);
+              : (unsigned)few_n | ((unsigned)many_n << 8) | ((unsigned)n << 16) | ((unsigned)shift << 23) | (1u << 24) |
+                    (shifted ? 1u << 27 : 0u);
 }
 
 // The fold at (x, y) over a body's near rects (or every rect)
@@ -950,7 +984,7 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
       q.y = fadd(q.y, dy);
       moved = true;
       // pushed away from its reference: its near set may miss a rect
-      all = N.full() || !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, mask);
+      all = N.full() || !near_holds(near_unpack(__float_as_uint(S.P[j].w), near_bias(S.cull, N)), q.x, q.y, mask);
     }
   }
   if (moved) S.Q[j] = q;
@@ -1017,11 +1051,12 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
   bool stale = !N.valid();
   if (!stale) {
     bool moved = false;
+    const float2 bias = near_bias(S.cull, N);
 #pragma unroll 1
     for (int j = L.lane; j < S.nb; j += G) {
       const float4 q = S.Q[j];
       if (World && __float_as_uint(q.w) == kExempt) continue;
-      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w)), q.x, q.y, __float_as_uint(q.w));
+      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w), bias), q.x, q.y, __float_as_uint(q.w));
     }
     stale = L.ballot(moved) != 0;
   }

@@ -70,7 +70,7 @@ struct StepArgs {
 };
 
 __host__ __device__ constexpr int warp_smem_words(int mb, int mu, int mp) {
-  return 20 * mb + 4 * kr::kWorldRec * mu + 4 * mp + 4 * ((kr::kMaxCulled + 7) / 8) + mb;
+  return 20 * mb + 4 * kr::kWorldRec * mu + 4 * mp + kr::kCullWords + mb;
 }
 
 // a block's dynamic shared memory when every warp holds the largest island
@@ -90,7 +90,7 @@ __device__ inline void carve(kr::Island &S, StageView &V, float *base, int mb, i
   V.body = q; q += mb;
   S.units = q; q += kr::kWorldRec * mu;
   V.pts = q; q += mp;
-  S.cull = reinterpret_cast<unsigned short *>(q); q += (kr::kMaxCulled + 7) / 8;
+  S.cull = reinterpret_cast<unsigned short *>(q); q += kr::kCullWords / 4;
   S.list = reinterpret_cast<unsigned char *>(q);
   S.body = V.body; S.pts = V.pts;
 }

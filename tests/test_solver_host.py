@@ -265,6 +265,14 @@ def _loads(tmp_path, offset=0, rects=300, anchors=0, pull=0, spread=110, more=0)
     return float(words[1])
 
 
+@pytest.mark.parametrize("offset", [31500, 100000, -200000, 990000])
+def test_near_sets_hold_anywhere(tmp_path, offset):
+    """A scene far from the origin gives the full fold's bits, and its passes
+    read as many rects as at the origin (within a tenth: its coordinates
+    round, so its bodies drift differently)."""
+    assert _loads(tmp_path, offset) < 1.1 * _loads(tmp_path)
+
+
 def test_bodies_that_meet_no_rect_cost_no_rebuild(tmp_path):
     """An immovable body and one without points, out of any reference's range."""
     assert _loads(tmp_path, anchors=50000) <= 1.02 * _loads(tmp_path)
