@@ -802,8 +802,9 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
 // (a struct returned by the out-of-line rebuild would live in local memory):
 // listed bodies with at most kFewPoints points, listed bodies with more, near
 // list entries, entries per mask bit (log2), valid (every body has a
-// reference), full (no usable list: every body against every rect), shifted
-// (the references have an origin).
+// reference), full (no usable list: every body against every rect), tight (the
+// near list holds while the bodies stay within kNearMove of their references,
+// else kFarMove), shifted (the references have an origin).
 struct Near {
   unsigned w = 0;
   __device__ __forceinline__ int few() const { return w & 0xff; }
@@ -812,7 +813,10 @@ struct Near {
   __device__ __forceinline__ int shift() const { return (w >> 23) & 1; }
   __device__ __forceinline__ bool valid() const { return (w >> 24) & 1; }
   __device__ __forceinline__ bool full() const { return (w >> 25) & 1; }
+  __device__ __forceinline__ bool tight() const { return (w >> 26) & 1; }
   __device__ __forceinline__ bool shifted() const { return (w >> 27) & 1; }
+  // the mask of every entry of the near list
+  __device__ __forceinline__ unsigned whole() const { return (1u << ((n() + shift()) >> shift())) - 1u; }
 };
 constexpr int kFewPoints = 2;
 constexpr float kRefRange = 32000.f;   // of a reference's coordinates about the origin
@@ -841,8 +845,7 @@ __device__ __forceinline__ float2 near_bias(const unsigned short *cull, const Ne
   if (N.shifted()) bias = near_bias((short)cull[kMaxCulled], (short)cull[kMaxCulled + 1]);
   return bias;
 }
-__device__ __forceinline__ bool near_holds(const float2 ref, float x, float y, unsigned mask) {
-  const float r = (mask & kNearBit) ? kNearMove : kFarMove;
+__device__ __forceinline__ bool near_holds(const float2 ref, float x, float y, float r) {
   return fabsf(x - ref.x) <= r && fabsf(y - ref.y) <= r;
 }
 // false only if the rect lies outside the box x0..x1 x y0..y1 (extents of
@@ -881,7 +884,7 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
     ox = __float2int_rn((lx + hx) * (0.5f / kOriginStep));
     oy = __float2int_rn((ly + hy) * (0.5f / kOriginStep));
     for (int j = L.lane; j < nb; j += G)
-      bad |= !exempt(j) && !(fabsf(Q[j].x - kOriginStep * ox) < kRefRange && fabsf(Q[j].y - kOriginStep * oy) < kRefRange);
+      bad |= !exempt(j) && !near_holds(make_float2(kOriginStep * ox, kOriginStep * oy), Q[j].x, Q[j].y, kRefRange);
     full = L.ballot(bad) != 0;  // farther apart than references reach
     if (L.lane == 0) {
       cull[kMaxCulled] = (unsigned short)ox;
@@ -950,7 +953,7 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
   L.sync();
   return full ? (unsigned)few_n | ((unsigned)many_n << 8) | (1u << 25)
               : (unsigned)few_n | ((unsigned)many_n << 8) | ((unsigned)n << 16) | ((unsigned)shift << 23) | (1u << 24) |
-                    (shifted ? 1u << 27 : 0u);
+                    (move == kNearMove ? 1u << 26 : 0u) | (shifted ? 1u << 27 : 0u);
 }
 
 // The fold at (x, y) over a body's near rects (or every rect)
@@ -972,7 +975,7 @@ __device__ __forceinline__ SdfFold near_fold(const Island &S, const Near &N, con
 __device__ __forceinline__ void collide_points(Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
                                                int j, float4 q, float sa, float ca, int from) {
   const int pr = __float_as_int(S.body[j].w), off = pr & 0xffff, cnt = pr >> 16;
-  const unsigned mask = __float_as_uint(q.w);
+  unsigned mask = __float_as_uint(q.w);
   bool all = N.full(), moved = false;
   for (int k = from; k < cnt; k++) {
     const float4 pt = S.pts[off + k];
@@ -983,8 +986,14 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
       q.x = fadd(q.x, dx);
       q.y = fadd(q.y, dy);
       moved = true;
-      // pushed away from its reference: its near set may miss a rect
-      all = N.full() || !near_holds(near_unpack(__float_as_uint(S.P[j].w), near_bias(S.cull, N)), q.x, q.y, mask);
+      // pushed away from its reference its near set may miss a rect, farther
+      // away the near list too (a body that its joints hold in a wall is pushed
+      // by more than kNearMove in every pass)
+      if (!N.full()) {
+        const float2 ref = near_unpack(__float_as_uint(S.P[j].w), near_bias(S.cull, N));
+        mask = near_holds(ref, q.x, q.y, kNearMove) ? __float_as_uint(q.w) : N.whole();
+        all = !near_holds(ref, q.x, q.y, N.tight() ? kNearMove : kFarMove);
+      }
     }
   }
   if (moved) S.Q[j] = q;
@@ -1055,8 +1064,10 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
 #pragma unroll 1
     for (int j = L.lane; j < S.nb; j += G) {
       const float4 q = S.Q[j];
-      if (World && __float_as_uint(q.w) == kExempt) continue;
-      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w), bias), q.x, q.y, __float_as_uint(q.w));
+      const unsigned mask = __float_as_uint(q.w);
+      if (World && mask == kExempt) continue;
+      moved |= !near_holds(near_unpack(__float_as_uint(S.P[j].w), bias), q.x, q.y,
+                           (mask & kNearBit) ? kNearMove : kFarMove);
     }
     stale = L.ballot(moved) != 0;
   }

@@ -276,3 +276,11 @@ def test_near_sets_hold_anywhere(tmp_path, offset):
 def test_bodies_that_meet_no_rect_cost_no_rebuild(tmp_path):
     """An immovable body and one without points, out of any reference's range."""
     assert _loads(tmp_path, anchors=50000) <= 1.02 * _loads(tmp_path)
+
+
+def test_bodies_held_in_a_wall_fold_over_the_near_list(tmp_path):
+    """Bodies pushed out of a wall by more than their near set's margin in every
+    pass: their remaining points fold over the group's list, not over the map.
+    3,000 more rects on it cost a look each at a rebuild, which a drift of 0.8
+    px a pass makes rarer than one pass in 20."""
+    assert _loads(tmp_path, pull=9, more=3000) - _loads(tmp_path, pull=9) < 3000 / 20
