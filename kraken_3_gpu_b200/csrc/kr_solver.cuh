@@ -801,10 +801,11 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
 // State of the near sets, the same in every lane of the group, in one word
 // (a struct returned by the out-of-line rebuild would live in local memory):
 // listed bodies with at most kFewPoints points, listed bodies with more, near
-// list entries, entries per mask bit (log2), valid (every body has a
-// reference), full (no usable list: every body against every rect), tight (the
-// near list holds while the bodies stay within kNearMove of their references,
-// else kFarMove), shifted (the references have an origin).
+// list entries (dense: log2 of the rects per bit of the list), entries per
+// mask bit (log2), valid (every body that can meet a rect has a reference),
+// full (no usable list: every body against every rect), dense (more near rects
+// than a list holds: its words are a bit map of the map's rects), shifted (the
+// references have an origin).
 struct Near {
   unsigned w = 0;
   __device__ __forceinline__ int few() const { return w & 0xff; }
@@ -813,11 +814,12 @@ struct Near {
   __device__ __forceinline__ int shift() const { return (w >> 23) & 1; }
   __device__ __forceinline__ bool valid() const { return (w >> 24) & 1; }
   __device__ __forceinline__ bool full() const { return (w >> 25) & 1; }
-  __device__ __forceinline__ bool tight() const { return (w >> 26) & 1; }
+  __device__ __forceinline__ bool dense() const { return (w >> 26) & 1; }
   __device__ __forceinline__ bool shifted() const { return (w >> 27) & 1; }
   // the mask of every entry of the near list
   __device__ __forceinline__ unsigned whole() const { return (1u << ((n() + shift()) >> shift())) - 1u; }
 };
+constexpr int kMapWords = kCullWords - 1;  // of the bit map; the origin stays behind it
 constexpr int kFewPoints = 2;
 constexpr float kRefRange = 32000.f;   // of a reference's coordinates about the origin
 constexpr float kOriginStep = 16384.f;
@@ -892,25 +894,28 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
     }
   }
   const float2 bias = near_bias(ox, oy);
-  // the near list, with the wide move if it fits
-  float move = kFarMove;
-  for (int base = 0; base < nR && !full; base += G) {
+  // the near list, or the bit map where it does not fit
+  for (int base = 0; base < nR && !full && n <= kMaxCulled; base += G) {
     const int i = base + L.lane;
-    const float d = kFarMove - move;
-    const bool keep = i < nR && in_box(__ldg(rects + i), lx + d, hx - d, ly + d, hy - d);
+    const bool keep = i < nR && in_box(__ldg(rects + i), lx, hx, ly, hy);
     const unsigned m = L.ballot(keep);
     const int at = n + __popc(m & ((1u << L.lane) - 1u));
     if (keep && at < kMaxCulled) cull[at] = (unsigned short)i;
     n += __popc(m);
-    if (n > kMaxCulled) {
-      full = move == kNearMove;
-      move = kNearMove;
-      n = 0;
-      base = -G;
-      L.sync();
+  }
+  const bool dense = n > kMaxCulled;
+  unsigned *map = reinterpret_cast<unsigned *>(cull);
+  if (dense) {
+    for (n = 0; (nR - 1) >> n >= 32 * kMapWords; n++) {}
+    L.sync();
+    for (int w = L.lane; w < kMapWords; w += G) {
+      unsigned bits = 0u;
+      for (int i = w << (5 + n); i < min((w + 1) << (5 + n), nR); i++)
+        if (in_box(__ldg(rects + i), lx, hx, ly, hy)) bits |= 1u << ((i >> n) & 31);
+      map[w] = bits;
     }
   }
-  const int shift = n > 31 ? 1 : 0;
+  const int shift = n > 31 && !dense ? 1 : 0;
   L.sync();
   for (int base = 0; base < nb; base += G) {
     const int j = base + L.lane;
@@ -929,12 +934,19 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
           const unsigned w = near_pack(q.x, q.y, ox, oy);
           const float2 ref = near_unpack(w, bias);
           const float e = bd.z + near_d, en = e + kNearMove, ef = e + kFarMove;
-          bool wide = move == kNearMove;
-#pragma unroll 4
-          for (int i = 0; i < n; i++) {
-            const float4 r = __ldg(rects + cull[i]);
+          bool wide = false;
+          auto look = [&](int i, unsigned bit) {
+            const float4 r = __ldg(rects + i);
             wide |= in_box(r, ref.x - ef, ref.x + ef, ref.y - ef, ref.y + ef);
-            if (in_box(r, ref.x - en, ref.x + en, ref.y - en, ref.y + en)) mask |= 1u << (i >> shift);
+            if (in_box(r, ref.x - en, ref.x + en, ref.y - en, ref.y + en)) mask |= bit;
+          };
+          if (dense) {
+            for (int w = 0; w < kMapWords; w++)
+              for (unsigned m = map[w]; m; m &= m - 1u)
+                for (int i = (32 * w + __ffs(m) - 1) << n, e = min(i + (1 << n), nR); i < e; i++) look(i, 1u);
+          } else {
+#pragma unroll 4
+            for (int i = 0; i < n; i++) look(cull[i], 1u << (i >> shift));
           }
           if (wide) mask |= kNearBit;
           P[j].w = __uint_as_float(w);
@@ -953,15 +965,30 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
   L.sync();
   return full ? (unsigned)few_n | ((unsigned)many_n << 8) | (1u << 25)
               : (unsigned)few_n | ((unsigned)many_n << 8) | ((unsigned)n << 16) | ((unsigned)shift << 23) | (1u << 24) |
-                    (move == kNearMove ? 1u << 26 : 0u) | (shifted ? 1u << 27 : 0u);
+                    (dense ? 1u << 26 : 0u) | (shifted ? 1u << 27 : 0u);
 }
 
-// The fold at (x, y) over a body's near rects (or every rect)
+// The fold at (x, y) over a body's near rects; over those of the dense list or
+// of all rects that can matter at this point (near_d = D + kCullPad, which
+// covers the box test's rounding below 1e6 px).
 __device__ __forceinline__ SdfFold near_fold(const Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
-                                             bool all, unsigned mask, float x, float y) {
+                                             float near_d, bool all, unsigned mask, float x, float y) {
   SdfFold f;
-  if (all) {
-    for (int i = 0; i < nR; i++) f.add(__ldg(rects + i), x, y);
+  if (all || N.dense()) {
+    const float d = fabsf(x) < 1e6f && fabsf(y) < 1e6f ? near_d : kInf;
+    const int g = N.dense() ? N.n() : 0;
+#pragma unroll 1
+    for (int base = 0; base < nR; base += 32 << g) {
+#pragma unroll 1
+      for (unsigned m = all ? ~0u : reinterpret_cast<const unsigned *>(S.cull)[base >> (5 + g)]; m; m &= m - 1u) {
+        const int i0 = base + ((__ffs(m) - 1) << g), e = min(i0 + (1 << g), nR);
+#pragma unroll 1
+        for (int i = i0; i < e; i++) {
+          const float4 r = __ldg(rects + i);
+          if (in_box(r, x - d, x + d, y - d, y + d)) f.add(r, x, y);
+        }
+      }
+    }
   } else {
     for (unsigned m = mask & ~kNearBit; m; m &= m - 1u) {
       const int b = (__ffs(m) - 1) << N.shift(), e = min(b + 1 + N.shift(), N.n());
@@ -973,7 +1000,7 @@ __device__ __forceinline__ SdfFold near_fold(const Island &S, const Near &N, con
 
 // The points [from, count) of body j in order, from its pose q
 __device__ __forceinline__ void collide_points(Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
-                                               int j, float4 q, float sa, float ca, int from) {
+                                               float near_d, int j, float4 q, float sa, float ca, int from) {
   const int pr = __float_as_int(S.body[j].w), off = pr & 0xffff, cnt = pr >> 16;
   unsigned mask = __float_as_uint(q.w);
   bool all = N.full(), moved = false;
@@ -982,7 +1009,7 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
     const float wx = fadd(q.x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
     const float wy = fadd(q.y, fadd(fmul(pt.x, sa), fmul(pt.y, ca)));
     float dx, dy;
-    if (near_fold(S, N, rects, nR, all, mask, wx, wy).push(pt.z, &dx, &dy)) {
+    if (near_fold(S, N, rects, nR, near_d, all, mask, wx, wy).push(pt.z, &dx, &dy)) {
       q.x = fadd(q.x, dx);
       q.y = fadd(q.y, dy);
       moved = true;
@@ -992,7 +1019,7 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
       if (!N.full()) {
         const float2 ref = near_unpack(__float_as_uint(S.P[j].w), near_bias(S.cull, N));
         mask = near_holds(ref, q.x, q.y, kNearMove) ? __float_as_uint(q.w) : N.whole();
-        all = !near_holds(ref, q.x, q.y, N.tight() ? kNearMove : kFarMove);
+        all = !near_holds(ref, q.x, q.y, kFarMove);
       }
     }
   }
@@ -1005,13 +1032,13 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
 // corrects -- until then none has moved the body.
 template <int G>
 __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
-                                               const Lanes<G> &L) {
+                                               float near_d, const Lanes<G> &L) {
   for (int t = L.lane; t < N.few(); t += G) {
     const int j = S.list[t];
     const float4 q = S.Q[j];
     float sa, ca;
     sincos_r(S.tab, q.z, &sa, &ca);
-    collide_points(S, N, rects, nR, j, q, sa, ca, 0);
+    collide_points(S, N, rects, nR, near_d, j, q, sa, ca, 0);
   }
   for (int t = 0; t < N.many(); t++) {
     const int j = S.list[S.nb - 1 - t];
@@ -1027,12 +1054,12 @@ __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const f
         const float wx = fadd(q.x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
         const float wy = fadd(q.y, fadd(fmul(pt.x, sa), fmul(pt.y, ca)));
         float dx, dy;
-        hit = near_fold(S, N, rects, nR, N.full(), __float_as_uint(q.w), wx, wy).push(pt.z, &dx, &dy);
+        hit = near_fold(S, N, rects, nR, near_d, N.full(), __float_as_uint(q.w), wx, wy).push(pt.z, &dx, &dy);
       }
       const unsigned m = L.ballot(hit);
       if (m) first = base + __ffs(m) - 1;
     }
-    if (first >= 0 && L.lane == 0) collide_points(S, N, rects, nR, j, q, sa, ca, first);
+    if (first >= 0 && L.lane == 0) collide_points(S, N, rects, nR, near_d, j, q, sa, ca, first);
   }
 }
 // (the members it needs one by one: a struct of the size of Island would pass
@@ -1040,14 +1067,14 @@ __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const f
 template <int G>
 __device__ __noinline__ void collide_listed_call(const float4 *P, float4 *Q, const float4 *body, const float4 *pts,
                                                  const float2 *tab, unsigned short *cull, unsigned char *list, int nb,
-                                                 unsigned near, const float4 *__restrict__ rects, int nR,
+                                                 unsigned near, const float4 *__restrict__ rects, int nR, float near_d,
                                                  int warp_lane) {
   Island S{};
   S.P = const_cast<float4 *>(P); S.Q = Q; S.body = body; S.pts = pts; S.tab = tab;
   S.cull = cull; S.list = list; S.nb = nb;
   Near N;
   N.w = near;
-  collide_listed<G>(S, N, rects, nR, Lanes<G>(warp_lane));
+  collide_listed<G>(S, N, rects, nR, near_d, Lanes<G>(warp_lane));
 }
 
 // One collision pass of the island.  OutOfLine: the listed bodies (most passes
@@ -1073,10 +1100,10 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
   }
   if (stale) N.w = near_rebuild<G, World>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
   if (OutOfLine) {
-    if (N.w & 0xffffu) collide_listed_call<G>(S.P, S.Q, S.body, S.pts, S.tab, S.cull, S.list, S.nb, N.w, rects, nR,
+    if (N.w & 0xffffu) collide_listed_call<G>(S.P, S.Q, S.body, S.pts, S.tab, S.cull, S.list, S.nb, N.w, rects, nR, near_d,
                                                 L.base + L.lane);
   } else {
-    collide_listed<G>(S, N, rects, nR, L);
+    collide_listed<G>(S, N, rects, nR, near_d, L);
   }
   L.sync();
 }

@@ -284,3 +284,14 @@ def test_bodies_held_in_a_wall_fold_over_the_near_list(tmp_path):
     3,000 more rects on it cost a look each at a rebuild, which a drift of 0.8
     px a pass makes rarer than one pass in 20."""
     assert _loads(tmp_path, pull=9, more=3000) - _loads(tmp_path, pull=9) < 3000 / 20
+
+
+@pytest.mark.parametrize("rects,spread", [(900, 110), (1500, 110), (1500, 320), (4000, 320)])
+def test_crowded_groups_fold_over_a_map_of_near_rects(tmp_path, rects, spread):
+    """More near rects than the list holds, at one, two and eight rects a bit:
+    the full fold's bits.  At one a bit a fold reads the rects near the group,
+    336 px of 1,340 x 740, and not the map: with the rebuilds less than three
+    tenths of it."""
+    points = 8 + 11 + 2 * 11  # of the 22 bodies that move and have points
+    loads = _loads(tmp_path, rects=rects, spread=spread)
+    assert rects > 992 or loads < 0.3 * rects * points
