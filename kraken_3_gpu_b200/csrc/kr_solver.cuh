@@ -13,6 +13,7 @@
 // and the WGSL `%` uses the exact truncated quotient (f32solver.mjs:36-51).
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "kr_sincos_tab.h"
 #include "kr_units.h"
@@ -370,12 +371,20 @@ struct SdfFold {
 // if no rect is that near): a bit mask over the creature's near list (the
 // rects near any of its bodies, ascending).
 // Bodies move a few px per env step, so the sets are rebuilt every few steps
-// instead of once per collision pass, and a body whose set is empty needs
-// nothing but the test that it still is near its reference.  A pass used to
-// reduce the bounding box of the bodies over the lanes and cull the map's
-// rects against it each time, the largest part of a pass in which no body
-// touched a wall: 16,384 mixed creatures 308 -> 289 ms, 1,024 creatures x 400
-// steps 31.8 -> 29.0 ms.
+// instead of once per collision pass (3 % of the passes on the default maps),
+// and a body whose set is empty needs nothing but the test that it still is
+// near its reference.
+//
+// The list takes the rects within the widest of three moves for which it fits,
+// kFarMove, half of it or kNearMove: a body that its joints hold in a wall is
+// pushed by more than kNearMove in every pass, and its remaining points fold
+// over the list as far as the list holds, else over the map.  A group with
+// more rects within kNearMove is dense: the list's words are a bit map of the
+// rects within kFarMove, 1 to 128 rects a bit.  A dense fold has more to
+// look at and diverges (256 chains among 405 small rects, 100 steps: 34 to 37
+// ms dense, 13.8 with a list within kNearMove), a fold over the map more yet
+// (1,024 creatures x 200 steps among 1,024 rects, where a few groups have no
+// list: 1,040 ms with every rect, 137 now).
 constexpr int kMaxCulled = 62;      // near list entries; bit b of a mask covers entries b << shift ...
 constexpr int kCullWords = 32;      // the near list, two entries a word, and the references' origin behind it
 static_assert(2 * kCullWords >= kMaxCulled + 2, "");
@@ -604,8 +613,11 @@ __device__ __forceinline__ bool pin_near(const float2 *tab, const PinArgs &U, bo
   b.y = fsub(b.y, fmul(U.wB, dly));
   b.z = fsub(b.z, fmul(U.wIB, fadd(fmul(pbx, dlx), fmul(pby, dly))));
   const bool small = World ? fadd(fabsf(bx), fabsf(by)) < 1e15f : csq < 1e30f;
-  // (a lever of a disabled pin must come out finite: 0 times it is added)
-  return amax <= kSinCosNearMax && (!on || (small && spread == 0.f));
+  // World: a disabled pin's levers must come out finite, since 0 times them is
+  // added (the engine's grips have the template's levers, and angles that are
+  // wrapped at 50 rad: 1 % of 12 creatures' step for a test that holds)
+  const bool near = amax <= kSinCosNearMax;
+  return World ? near && (!on || (small && spread == 0.f)) : !on || (near && small && spread == 0.f);
 }
 
 // solveAngleF, f32solver.mjs:258-301 (solver.wgsl:292-350): muscle
@@ -804,8 +816,9 @@ __device__ __forceinline__ void solve_world(Island &S, bool first, const Lanes<G
 // list entries (dense: log2 of the rects per bit of the list), entries per
 // mask bit (log2), valid (every body that can meet a rect has a reference),
 // full (no usable list: every body against every rect), dense (more near rects
-// than a list holds: its words are a bit map of the map's rects), shifted (the
-// references have an origin).
+// than a list holds: its words are a bit map of the map's rects, and bit b of a
+// mask covers word b), shifted (the references have an origin), tight (the list
+// holds while the bodies stay within near_reach(tight) of their references).
 struct Near {
   unsigned w = 0;
   __device__ __forceinline__ int few() const { return w & 0xff; }
@@ -816,10 +829,15 @@ struct Near {
   __device__ __forceinline__ bool full() const { return (w >> 25) & 1; }
   __device__ __forceinline__ bool dense() const { return (w >> 26) & 1; }
   __device__ __forceinline__ bool shifted() const { return (w >> 27) & 1; }
-  // the mask of every entry of the near list
+  __device__ __forceinline__ int tight() const { return (w >> 28) & 3; }
+  // the mask of the whole near list
   __device__ __forceinline__ unsigned whole() const { return (1u << ((n() + shift()) >> shift())) - 1u; }
 };
 constexpr int kMapWords = kCullWords - 1;  // of the bit map; the origin stays behind it
+// kFarMove, half of it, kNearMove
+__device__ __forceinline__ float near_reach(int tight) {
+  return __uint_as_float(__float_as_uint(kFarMove) - ((unsigned)tight << 23));
+}
 constexpr int kFewPoints = 2;
 constexpr float kRefRange = 32000.f;   // of a reference's coordinates about the origin
 constexpr float kOriginStep = 16384.f;
@@ -894,16 +912,25 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
     }
   }
   const float2 bias = near_bias(ox, oy);
-  // the near list, or the bit map where it does not fit
-  for (int base = 0; base < nR && !full && n <= kMaxCulled; base += G) {
+  // the near list, within the widest move for which it fits, or the bit map
+  int tight = 0;
+  bool dense = false;
+  for (int base = 0; base < nR && !full && !dense; base += G) {
     const int i = base + L.lane;
-    const bool keep = i < nR && in_box(__ldg(rects + i), lx, hx, ly, hy);
+    const float d = kFarMove - near_reach(tight);
+    const bool keep = i < nR && in_box(__ldg(rects + i), lx + d, hx - d, ly + d, hy - d);
     const unsigned m = L.ballot(keep);
     const int at = n + __popc(m & ((1u << L.lane) - 1u));
     if (keep && at < kMaxCulled) cull[at] = (unsigned short)i;
     n += __popc(m);
+    if (n > kMaxCulled) {
+      dense = near_reach(tight) == kNearMove;
+      tight = dense ? 0 : tight + 1;
+      n = 0;
+      base = -G;
+      L.sync();
+    }
   }
-  const bool dense = n > kMaxCulled;
   unsigned *map = reinterpret_cast<unsigned *>(cull);
   if (dense) {
     for (n = 0; (nR - 1) >> n >= 32 * kMapWords; n++) {}
@@ -934,7 +961,7 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
           const unsigned w = near_pack(q.x, q.y, ox, oy);
           const float2 ref = near_unpack(w, bias);
           const float e = bd.z + near_d, en = e + kNearMove, ef = e + kFarMove;
-          bool wide = false;
+          bool wide = tight != 0;
           auto look = [&](int i, unsigned bit) {
             const float4 r = __ldg(rects + i);
             wide |= in_box(r, ref.x - ef, ref.x + ef, ref.y - ef, ref.y + ef);
@@ -943,7 +970,7 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
           if (dense) {
             for (int w = 0; w < kMapWords; w++)
               for (unsigned m = map[w]; m; m &= m - 1u)
-                for (int i = (32 * w + __ffs(m) - 1) << n, e = min(i + (1 << n), nR); i < e; i++) look(i, 1u);
+                for (int i = (32 * w + __ffs(m) - 1) << n, e = min(i + (1 << n), nR); i < e; i++) look(i, 1u << w);
           } else {
 #pragma unroll 4
             for (int i = 0; i < n; i++) look(cull[i], 1u << (i >> shift));
@@ -965,30 +992,38 @@ __device__ __noinline__ unsigned near_rebuild(float4 *P, float4 *Q, const float4
   L.sync();
   return full ? (unsigned)few_n | ((unsigned)many_n << 8) | (1u << 25)
               : (unsigned)few_n | ((unsigned)many_n << 8) | ((unsigned)n << 16) | ((unsigned)shift << 23) | (1u << 24) |
-                    (dense ? 1u << 26 : 0u) | (shifted ? 1u << 27 : 0u);
+                    (dense ? 1u << 26 : 0u) | (shifted ? 1u << 27 : 0u) | ((unsigned)tight << 28);
 }
 
-// The fold at (x, y) over a body's near rects; over those of the dense list or
-// of all rects that can matter at this point (near_d = D + kCullPad, which
+// The fold at (x, y) over a body's near rects, or every rect.  Wide: for groups
+// whose state is dense or full; of a dense list's words and of all rects it
+// takes those that can matter at this point (near_d = D + kCullPad, which
 // covers the box test's rounding below 1e6 px).
+template <bool Wide>
 __device__ __forceinline__ SdfFold near_fold(const Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
                                              float near_d, bool all, unsigned mask, float x, float y) {
   SdfFold f;
-  if (all || N.dense()) {
+  if constexpr (Wide) {
     const float d = fabsf(x) < 1e6f && fabsf(y) < 1e6f ? near_d : kInf;
-    const int g = N.dense() ? N.n() : 0;
-#pragma unroll 1
-    for (int base = 0; base < nR; base += 32 << g) {
-#pragma unroll 1
-      for (unsigned m = all ? ~0u : reinterpret_cast<const unsigned *>(S.cull)[base >> (5 + g)]; m; m &= m - 1u) {
-        const int i0 = base + ((__ffs(m) - 1) << g), e = min(i0 + (1 << g), nR);
-#pragma unroll 1
-        for (int i = i0; i < e; i++) {
-          const float4 r = __ldg(rects + i);
-          if (in_box(r, x - d, x + d, y - d, y + d)) f.add(r, x, y);
+    auto take = [&](int i) {
+      const float4 r = __ldg(rects + i);
+      if (in_box(r, x - d, x + d, y - d, y + d)) f.add(r, x, y);
+    };
+    if (all) {
+#pragma unroll 4
+      for (int i = 0; i < nR; i++) take(i);
+    } else {
+      const int g = N.n();
+      for (unsigned words = mask & ~kNearBit; words; words &= words - 1u) {
+        const int w = __ffs(words) - 1;
+        for (unsigned m = reinterpret_cast<const unsigned *>(S.cull)[w]; m; m &= m - 1u) {
+          const int i0 = (32 * w + __ffs(m) - 1) << g, e = min(i0 + (1 << g), nR);
+          for (int i = i0; i < e; i++) take(i);
         }
       }
     }
+  } else if (all) {
+    for (int i = 0; i < nR; i++) f.add(__ldg(rects + i), x, y);
   } else {
     for (unsigned m = mask & ~kNearBit; m; m &= m - 1u) {
       const int b = (__ffs(m) - 1) << N.shift(), e = min(b + 1 + N.shift(), N.n());
@@ -999,27 +1034,29 @@ __device__ __forceinline__ SdfFold near_fold(const Island &S, const Near &N, con
 }
 
 // The points [from, count) of body j in order, from its pose q
+template <bool Wide>
 __device__ __forceinline__ void collide_points(Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
                                                float near_d, int j, float4 q, float sa, float ca, int from) {
   const int pr = __float_as_int(S.body[j].w), off = pr & 0xffff, cnt = pr >> 16;
   unsigned mask = __float_as_uint(q.w);
-  bool all = N.full(), moved = false;
+  const bool full = Wide && N.full();
+  bool all = full, moved = false;
   for (int k = from; k < cnt; k++) {
     const float4 pt = S.pts[off + k];
     const float wx = fadd(q.x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
     const float wy = fadd(q.y, fadd(fmul(pt.x, sa), fmul(pt.y, ca)));
     float dx, dy;
-    if (near_fold(S, N, rects, nR, near_d, all, mask, wx, wy).push(pt.z, &dx, &dy)) {
+    if (near_fold<Wide>(S, N, rects, nR, near_d, all, mask, wx, wy).push(pt.z, &dx, &dy)) {
       q.x = fadd(q.x, dx);
       q.y = fadd(q.y, dy);
       moved = true;
       // pushed away from its reference its near set may miss a rect, farther
       // away the near list too (a body that its joints hold in a wall is pushed
       // by more than kNearMove in every pass)
-      if (!N.full()) {
+      if (!full) {
         const float2 ref = near_unpack(__float_as_uint(S.P[j].w), near_bias(S.cull, N));
-        mask = near_holds(ref, q.x, q.y, kNearMove) ? __float_as_uint(q.w) : N.whole();
-        all = !near_holds(ref, q.x, q.y, kFarMove);
+        mask = near_holds(ref, q.x, q.y, kNearMove) ? __float_as_uint(q.w) : Wide ? ~kNearBit : N.whole();
+        all = !near_holds(ref, q.x, q.y, near_reach(N.tight()));
       }
     }
   }
@@ -1030,7 +1067,7 @@ __device__ __forceinline__ void collide_points(Island &S, const Near &N, const f
 // lane each; the points of a body with more (the mantle's eight) are evaluated
 // side by side, and one lane repeats them in order from the first that
 // corrects -- until then none has moved the body.
-template <int G>
+template <int G, bool Wide>
 __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const float4 *__restrict__ rects, int nR,
                                                float near_d, const Lanes<G> &L) {
   for (int t = L.lane; t < N.few(); t += G) {
@@ -1038,7 +1075,7 @@ __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const f
     const float4 q = S.Q[j];
     float sa, ca;
     sincos_r(S.tab, q.z, &sa, &ca);
-    collide_points(S, N, rects, nR, near_d, j, q, sa, ca, 0);
+    collide_points<Wide>(S, N, rects, nR, near_d, j, q, sa, ca, 0);
   }
   for (int t = 0; t < N.many(); t++) {
     const int j = S.list[S.nb - 1 - t];
@@ -1054,17 +1091,17 @@ __device__ __forceinline__ void collide_listed(Island &S, const Near &N, const f
         const float wx = fadd(q.x, fsub(fmul(pt.x, ca), fmul(pt.y, sa)));
         const float wy = fadd(q.y, fadd(fmul(pt.x, sa), fmul(pt.y, ca)));
         float dx, dy;
-        hit = near_fold(S, N, rects, nR, near_d, N.full(), __float_as_uint(q.w), wx, wy).push(pt.z, &dx, &dy);
+        hit = near_fold<Wide>(S, N, rects, nR, near_d, Wide && N.full(), __float_as_uint(q.w), wx, wy).push(pt.z, &dx, &dy);
       }
       const unsigned m = L.ballot(hit);
       if (m) first = base + __ffs(m) - 1;
     }
-    if (first >= 0 && L.lane == 0) collide_points(S, N, rects, nR, near_d, j, q, sa, ca, first);
+    if (first >= 0 && L.lane == 0) collide_points<Wide>(S, N, rects, nR, near_d, j, q, sa, ca, first);
   }
 }
 // (the members it needs one by one: a struct of the size of Island would pass
 // through local memory)
-template <int G>
+template <int G, bool Wide>
 __device__ __noinline__ void collide_listed_call(const float4 *P, float4 *Q, const float4 *body, const float4 *pts,
                                                  const float2 *tab, unsigned short *cull, unsigned char *list, int nb,
                                                  unsigned near, const float4 *__restrict__ rects, int nR, float near_d,
@@ -1074,7 +1111,7 @@ __device__ __noinline__ void collide_listed_call(const float4 *P, float4 *Q, con
   S.cull = cull; S.list = list; S.nb = nb;
   Near N;
   N.w = near;
-  collide_listed<G>(S, N, rects, nR, near_d, Lanes<G>(warp_lane));
+  collide_listed<G, Wide>(S, N, rects, nR, near_d, Lanes<G>(warp_lane));
 }
 
 // One collision pass of the island.  OutOfLine: the listed bodies (most passes
@@ -1099,12 +1136,13 @@ __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 
     stale = L.ballot(moved) != 0;
   }
   if (stale) N.w = near_rebuild<G, World>(S.P, S.Q, S.body, S.cull, S.list, S.nb, rects, nR, near_d, L);
-  if (OutOfLine) {
-    if (N.w & 0xffffu) collide_listed_call<G>(S.P, S.Q, S.body, S.pts, S.tab, S.cull, S.list, S.nb, N.w, rects, nR, near_d,
-                                                L.base + L.lane);
-  } else {
-    collide_listed<G>(S, N, rects, nR, near_d, L);
-  }
+  auto call = [&](auto wide) {
+    collide_listed_call<G, decltype(wide)::value>(S.P, S.Q, S.body, S.pts, S.tab, S.cull, S.list, S.nb, N.w, rects, nR,
+                                                  near_d, L.base + L.lane);
+  };
+  if (__builtin_expect(N.full() || N.dense(), 0)) call(std::true_type{});
+  else if (!OutOfLine) collide_listed<G, false>(S, N, rects, nR, near_d, L);
+  else if (N.w & 0xffffu) call(std::false_type{});
   L.sync();
 }
 

@@ -286,12 +286,12 @@ def test_bodies_held_in_a_wall_fold_over_the_near_list(tmp_path):
     assert _loads(tmp_path, pull=9, more=3000) - _loads(tmp_path, pull=9) < 3000 / 20
 
 
-@pytest.mark.parametrize("rects,spread", [(900, 110), (1500, 110), (1500, 320), (4000, 320)])
+@pytest.mark.parametrize("rects,spread", [(600, 110), (700, 110), (900, 110), (1500, 110), (1500, 320), (4000, 320)])
 def test_crowded_groups_fold_over_a_map_of_near_rects(tmp_path, rects, spread):
-    """More near rects than the list holds, at one, two and eight rects a bit:
-    the full fold's bits.  At one a bit a fold reads the rects near the group,
-    336 px of 1,340 x 740, and not the map: with the rebuilds less than three
-    tenths of it."""
+    """A list that fits within 16 or 8 px only, and more near rects than it
+    holds, at one, two and eight rects a bit: the full fold's bits.  Up to one
+    a bit a fold reads the rects near the group, 336 px of 1,340 x 740, and not
+    the map: with the rebuilds less than three tenths of it."""
     points = 8 + 11 + 2 * 11  # of the 22 bodies that move and have points
     loads = _loads(tmp_path, rects=rects, spread=spread)
     assert rects > 992 or loads < 0.3 * rects * points
