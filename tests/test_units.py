@@ -130,3 +130,9 @@ def program(tmp_path_factory):
 def test_units_keep_the_list_order(program):
     out = subprocess.run([program], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0 and out.stdout.startswith("ok"), out.stdout
+
+
+def test_every_shape_needs_the_fewest_passes(program):
+    """Bodies of two arms and segments or more: no schedule is longer than the
+    larger of the arms (each joins the mantle) and the units over the lanes."""
+    assert subprocess.run([program], capture_output=True, text=True, timeout=120).stdout == "ok 0\n"
