@@ -95,8 +95,9 @@ def test_steps_of_one_call_equal_single_steps_and_the_oracle(seed, steps):
     for c, f in ((0, "px"), (1, "py"), (4, "vx"), (5, "vy"), (6, "ang"), (8, "av")):
         assert np.array_equal(got[:, c], o.arr(f).astype(np.float32)), f
     assert [bool(v) for v in out[0][1].view(np.uint32)[:, 17]] == [bool(c.broken) for c in o.constraints]
-    # the run has what it is for: walls, bodies far from where they started, a grip that broke on the way
-    assert hits > 100 and np.abs(got[:, :2] - start).max() > 64
+    # the run has what it is for: walls, bodies beyond any collision reference's
+    # 32 px of where they started, a grip that broke on the way
+    assert hits > 100 and np.abs(got[:, :2] - start).max() > 32
     assert broke and broke[0] > 0 and len({c.broken for c in o.constraints}) == 2
 
 
