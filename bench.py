@@ -45,10 +45,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "creature-steps/s at 16k mixed envs, served vs plain launch; p50/p99 rollout ms"
 # DRAM bytes (read + write) of one persistent launch per creature, from a one-kernel,
-# one-launch ncu capture of an 8,192-creature case (20,806,656 B read + 381,184 B written):
+# one-launch ncu capture of an 8,192-creature case (20,216,832 B read + 340,224 B written):
 # the committed state, grips, controls and slot records in and out once, independent of the
 # step count
-NCU_DRAM_BYTES_PER_CREATURE = (20806656 + 381184) / 8192
+NCU_DRAM_BYTES_PER_CREATURE = (20216832 + 340224) / 8192
 UNIT = "creature-steps/s"
 
 

@@ -176,7 +176,13 @@ int kr_batch_live(kr_batch *b, int32_t *live);
 /* Copy the state of slots [first, first + n) to the host (synchronous):
  * bodies: n x (1 + 8 * 9) x 6 f32 (px py vx vy ang av per body, template
  * body order), grips: n x 8 x 4 f32 (lbx lby breakForce broken), steps: n
- * i32.  Any pointer may be NULL. */
+ * i32.  Any pointer may be NULL.
+ * Reads of 4 MB or more (here and in kr_batch_read_obs) go through up to
+ * eight host threads, seven of them started for the call, and 4 MB of pinned
+ * host memory that the engine allocates on its first such read and keeps
+ * until it is destroyed; the bodies also through up to 4 MB of device memory,
+ * kept from the first read on.  Without that memory the reads are plain
+ * copies.  Any host thread may read, whichever device is its current one. */
 int kr_batch_read_state(kr_batch *b, int32_t first, int32_t n, float *bodies, float *grips,
                         int32_t *steps);
 

@@ -293,7 +293,7 @@ __device__ __forceinline__ void load_vec(const float *p, float *v) {
 // Every dot product starts from the bias and accumulates in index order.
 // Bound by the latency of the weights, read from L2 or beyond once per env
 // step: as many rows in flight as the registers hold (one output at a time
-// and four rows of W1: 16,384 creatures x up to 300 steps 46.7 ms, now 42.5).
+// and four rows of W1: 16,384 creatures take 10 % longer).
 template <int G>
 __device__ __forceinline__ void policy(const float *w, int arms, int segs, const float *obs, float *ctrl,
                                        const kr::Lanes<G> &L) {
@@ -1334,14 +1334,25 @@ namespace krb {
 
 // Few creatures (under 8 per SM): one per warp, the shortest step latency;
 // up to 96 per SM two per warp; beyond, four per warp, the most
-// creature-steps per issue slot.  Measured at the edges, always with CTAs of
-// 4 warps: 2,000 default creatures x 200 steps (13.5 per SM) 9.1 ms at 16
-// lanes against 11.2 at 32, 1,024 x 400 (7 per SM) 16.1 at either; 16,384
-// mixed creatures 154 ms with 8 lanes above 96 per SM, 166 above 64.
-// Creatures under the policy or the net and ring-keeping ones used to take 8
-// lanes from 16 per SM on; since a pass runs one unit per lane at any width
-// they do better with 16: 8,000 under the policy 32 against 39 ms, under the
-// net 37 against 41, 6,000 with rings 24 against 27.
+// creature-steps per issue slot.  Measured with CTAs of 4 warps, ms at 32, 16
+// and 8 lanes:
+//   1,024 default creatures x 400 steps (7 per SM)        40.2  43.9  53.2
+//   1,184 mixed creatures, up to 300 steps (8 per SM)     11.3  10.9  13.3
+//   4,000 (27)                                            15.7  16.0  16.4
+//   9,472 (64)                                            33.1  19.4  21.8
+//   12,000 (81)                                           41.4  24.2  21.4
+//   14,208 (96)                                           48.7  28.0  21.9
+//   8,000 under the policy (54)                           38.2  25.7  29.6
+//   8,000 under the net (54)                              76.1  52.7  48.8
+//   8,000 with observation rings (54)                     33.3  20.5  22.0
+// In time slices the upper line is flat: 16,384 mixed creatures take 140 ms
+// with it at 64, 80 or 96.
+//
+// A server's engine keeps 16 lanes below 8 per SM, although 32 are faster
+// there (4 requests of up to 24 creatures 9.7 ms against 12.2, one of 12 8.3
+// against 9.8, 24 of up to 96 28.6 against 29.0): the check that admissions
+// reach a running request sends its requests 4 ms apart, and at 32 lanes its
+// longest, of 150 steps, ends before the next one comes.
 int auto_lanes(const kr_batch *b, long live) {
   if (live < 8L * b->n_sm) return b->served ? 16 : 32;
   return live >= 96L * b->n_sm ? 8 : 16;

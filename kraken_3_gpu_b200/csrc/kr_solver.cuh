@@ -287,8 +287,8 @@ static __device__ __noinline__ float wrap_far(float x) {
 // The same for |x| <= kWrapNear < kTau + kPi (or NaN): the quotient is 0 or
 // +-1, and either way a difference beyond pi moves by one kTau, rounded once.
 // Five instructions instead of the quotient's twenty in sequence (the angle
-// constraint evaluates five of these in a row; its chain went from 764 to 441
-// cycles, 16,384 mixed creatures from 289 to 239 ms).
+// constraint evaluates five of these in a row: its chain is 441 cycles instead
+// of 764 with the quotient).
 constexpr float kWrapNear = 9.42f;
 __device__ __forceinline__ float wrap_near(float x) {
   const float d = fsub(x, copysignf(kTau, x));
@@ -430,9 +430,8 @@ struct Lanes {
 // gives the sequential sweep's bits (the harness check color-order-free,
 // harness.js:1172-1193, pins this for the reference's colour classes).
 // The sweep is bound by its chain of dependent passes, each a round trip
-// through shared memory: per-constraint levels made a 6 x 7 body 12 of them,
-// as units it is 6 (12 creatures: 90 -> 64 us an env step; 16,384 mixed
-// creatures to their horizons: 391 -> 308 ms).
+// through shared memory: per-constraint levels make a 6 x 7 body 12 of them,
+// as units it is 6.
 //
 // Bodies are float4 records (one 16-byte load or store instead of three
 // 4-byte ones).
@@ -727,8 +726,7 @@ static __device__ __noinline__ UnitOut unit_any(PinArgs U, AngleArgs V, bool pin
 // instruction stream; a pass ends in its only branch, for units that need
 // the reference form (their bodies are still in shared memory as they were).
 // The pass's 230 + 340 cycles of dependent arithmetic are what a creature's
-// step consists of; 12 creatures' solve took 104,000 cycles a step as
-// separate pin and angle levels with the reference's branches.
+// step consists of.
 template <int G>
 __device__ __forceinline__ void solve_engine(const SolverConsts &K, Island &S, bool first, const Lanes<G> &L) {
   const float alpha_m = fmul(S.comp_m, K.invH2), reach = alpha_m < 0x1p59f ? kWrapNear : -1.f;
@@ -1116,8 +1114,9 @@ __device__ __noinline__ void collide_listed_call(const float4 *P, float4 *Q, con
 
 // One collision pass of the island.  OutOfLine: the listed bodies (most passes
 // have none) as a call -- for the kernel with the net, whose step is larger
-// than the instruction caches: 8,000 creatures under the net 35 -> 32 ms; the
-// others are 3 % faster with it in line.
+// than the instruction caches: 8,000 creatures under the net take 9 % longer
+// with it in line, the others 3 % less.  The groups without a list that masks
+// can cover take a call of their own in every kernel.
 template <int G, bool World, bool OutOfLine>
 __device__ __forceinline__ void collide_island(Island &S, Near &N, const float4 *__restrict__ rects, int nR,
                                                float near_d, const Lanes<G> &L) {
@@ -1185,8 +1184,8 @@ __device__ __forceinline__ bool grip_breaks(const SolverConsts &K, float lx, flo
 // trip, remainder handled) -- the same operations in the same order, so the
 // results do not depend on it; the batched engine's autotuner picks it.  The
 // loops inside are not unrolled: an env step's code has to stay in the
-// instruction caches (the pass loop unrolled twice: 16,384 creatures 154 ->
-// 219 ms; the body loops not unrolled: 8,000 under the policy 31 -> 27 ms).
+// instruction caches (the pass loop unrolled twice: 16,384 creatures take
+// 42 % longer; the body loops unrolled: 8,000 under the policy 15 %).
 template <bool World, int G, int U = 1, bool OutOfLine = false>
 __device__ __forceinline__ void island_step(const SolverConsts &K, Island &S,
                                             const float4 *__restrict__ rects, int nR, float near_d,

@@ -5,8 +5,8 @@
 // spawnKraken's creation order (src/body/kraken.js:64-148), createSim's
 // greedy colouring in creation order (src/sim/core.js:45-58 with
 // assignColor, src/physics/xpbd.js:98-105), the stable grouping by colour
-// (core.js:276-288), and from that list order the body-disjoint levels the
-// warp sweeps.  Spawn poses follow the same chain rule (kraken.js:64-101).
+// (core.js:276-288), and from that list order the passes of body-disjoint
+// units that the lanes sweep.  Spawn poses follow the same chain rule (kraken.js:64-101).
 #pragma once
 #include <cstdint>
 #include <string>

@@ -13,7 +13,7 @@
 
 namespace kr {
 
-// Levers and masses for which the quotients of kr_solver.cuh pin_math stay in
+// Levers and masses for which the quotients of kr_solver.cuh pin_near stay in
 // range whatever the angles (every pin of a creature): with wI |l|^2 <= 16 wS
 // the matrix entries lie in wS .. 33 wS and det in wS^2 .. 2^11 wS^2, wS in
 // 2^-10 .. 2^10 (so |det| >= kEpsDet); k01 is 0 or above 2^-100, since |sin|

@@ -131,7 +131,7 @@ __device__ __forceinline__ void plain_step_body(const StepArgs &A) {
       const float lx = __uint_as_float(cp.y), ly = __uint_as_float(cp.z);
       V.pts[bp.x + q] = make_float4(lx, ly, __uint_as_float(cp.w), __int_as_float(i));
       const float d = kr::length2(lx, ly) + 1.f;
-      if (!(d <= reach)) reach = d;  // NaN stays: such a body is tested against every rect
+      if (!(d <= reach)) reach = d;  // NaN, unless a later point replaces it (it corrects nothing): no list
     }
     V.body[i] = make_float4(q2.y, q2.z, reach, __int_as_float(bp.x | (bp.y << 16)));
   }
@@ -765,7 +765,7 @@ static __device__ __align__(256) int g_noalloc_scratch[kScratchWords];
 // Schedule builder, one block: the islands, bodies and point ranges of
 // build_schedule() and the same units, in passes by level.  A single thread
 // over global memory took 5.3 ms for 40 creatures, all of it load latency;
-// here (a 40-creature call of 4 steps: 5.6 -> 0.27 ms) the temporaries are in
+// here (a 40-creature call of 4 steps: 5.9 -> 0.24 ms) the temporaries are in
 // shared memory and only what is sequential by nature runs in order -- the
 // ranks within an island by one warp, 32 entries at a time, and an island's
 // units by one thread per island.
