@@ -1316,7 +1316,10 @@ template <int G>
 cudaError_t launch_g(const BatchArgs &A, kr_batch *b, cudaStream_t st, int n_groups, int *grid_out) {
   auto *fn = b->unroll == 2 ? (b->d_net ? batch_kernel<G, true, 2> : batch_kernel<G, false, 2>)
                             : (b->d_net ? batch_kernel<G, true, 1> : batch_kernel<G, false, 1>);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem_dyn);
+  // the limit belongs to the kernel, not to the engine: always what a CTA can
+  // have, so that no engine's launch lowers it under another's
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       b->smem_optin - (int)kStaticSmem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * b->W, b->smem_dyn);

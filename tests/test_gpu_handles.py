@@ -187,3 +187,38 @@ def test_launch_shapes_taken_and_refused(arms, segs, lanes, warps, ctas, taken):
         eng.close()
     if taken:
         assert all(np.array_equal(out[0][f], out[1][f]) for f in out[0])
+
+
+def test_engines_of_two_threads_launch_side_by_side():
+    """Two engines whose CTAs need unlike amounts of shared memory, each driven
+    by a thread of its own: every launch goes through, and to the state that
+    each engine reaches by itself."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    maps = [ob.make_map_rects(seed=3)]
+
+    def engine(arms, segs, n):
+        r = np.random.default_rng(arms)
+        eng = batch.BatchEngine(maps, n)
+        eng.spawn(0, np.full(n, arms), np.full(n, segs), np.zeros(n, int), r.uniform(300, 1000, n),
+                  r.uniform(300, 500, n), r.uniform(0, 6, n), np.full(n, 400))
+        return eng
+
+    def drive(eng):
+        for _ in range(400):
+            eng.run(1)
+        return eng.read_state()
+
+    shapes = ((8, 9, 6), (1, 1, 6))
+    alone = []
+    for s in shapes:
+        eng = engine(*s)
+        alone.append(drive(eng))
+        eng.close()
+    engines = [engine(*s) for s in shapes]
+    with ThreadPoolExecutor(2) as pool:
+        got = list(pool.map(drive, engines))
+    for a, g in zip(alone, got):
+        assert all(np.array_equal(a[f], g[f]) for f in a)
+    for eng in engines:
+        eng.close()
