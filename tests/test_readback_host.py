@@ -9,6 +9,7 @@ import subprocess
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "kraken_3_gpu_b200", "csrc")
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
 
 FAKE = r'''
 #include <cstdio>
@@ -72,7 +73,7 @@ def _run(tmp_path, body):
     src = tmp_path / "t.cpp"
     src.write_text(FAKE + body)
     exe = tmp_path / "t"
-    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-pthread", "-I", CSRC, "-I", "/usr/local/cuda/include", "-o",
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-pthread", "-I", CSRC, "-I", CUDA_INCLUDE, "-o",
                     str(exe), str(src)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0 and out.stdout.startswith("ok"), out.stdout + out.stderr
